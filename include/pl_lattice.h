@@ -227,6 +227,17 @@ int pl_debug_direct_index(int enable);
 int pl_direct_index_min_entries(int batch, int n_spatial_dims, const int* spatial_dims, float theta_gamma,
                                 int64_t* min_entries);
 
+/* A cheaper way to learn whether a call fits its max_entries than pl_lattice_stats: pl_watch_next_call makes the
+ * next filter or build call of this host thread report its counters as soon as its lattice is complete, and
+ * pl_await_watched_call waits for that report (not for the whole call: splat, blur and slice are still running)
+ * and returns what pl_stats would hold.  `stream` is the call's stream; it must not be being captured.  A watched
+ * call that returned an error is not awaited.  No counterpart in the reference (it prints or exits:
+ * src/PermutohedralLatticeGPU.cuh:49-55,442-445). */
+int pl_watch_next_call(void* stream);
+
+/* See pl_watch_next_call.  BLOCKS until the report is there.  No counterpart in the reference. */
+int pl_await_watched_call(int64_t* num_entries, int* device_status, void* stream);
+
 /* Copies the counters of the last call that used `workspace` to the host.  SYNCHRONISES `stream`.
  * workspace == NULL reads the counters of the last pl_lattice_filter_f32_noalloc call on the current
  * device (its scratch is inside the library, so that caller has no pointer to pass).

@@ -50,6 +50,22 @@ struct Header {   // first 256 bytes of the workspace
     u32 pad[56];
 };
 
+// Where a watched call reports (pl_watch_next_call): one word of mapped host memory.  The link kernel writes
+// sequence << 40 | status bits << 32 | entries there before it does anything else: everything that can make a
+// call fail has happened by then, and the host, which polls the word, goes on while the device still splats,
+// blurs and slices.
+constexpr u32 WATCH_SEQ_MASK = 0xFFFFFFu;
+struct Watch {
+    u64* word;   // null: nobody is watching
+    u32 seq;
+};
+__device__ __forceinline__ void report_to(const Watch& w, const Header* hdr) {
+    if (w.word && blockIdx.x == 0 && threadIdx.x == 0) {
+        const u64 v = ((u64)w.seq << 40) | ((u64)(hdr->status & 0xFFu) << 32) | (u64)hdr->num_entries;
+        asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(w.word), "l"(v) : "memory");
+    }
+}
+
 struct Layout {   // byte offsets into the workspace
     size_t tile_info, rec, rec_w, srec, list_keys, list_ref, vid, vkeys, table, nbr, v0, v1, v64, total;
     u64 max_entries;   // capacity of entry- and vertex-indexed arrays

@@ -89,8 +89,9 @@ template <int PD>
 __global__ void __launch_bounds__(256)
 link_neighbours_direct(const Header* hdr, Direct d, const u32* __restrict__ table, u32* __restrict__ list_ref,
                        const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys,
-                       int* __restrict__ nbr, u64 max_entries) {
+                       int* __restrict__ nbr, u64 max_entries, Watch watch) {
     after_previous_kernel();
+    report_to(watch, hdr);
     constexpr int KW = Cfg<PD>::KW;
     if (hdr->status != 0) return;
     resolve_entries(hdr, list_ref, vid);

@@ -458,8 +458,9 @@ __global__ void __launch_bounds__(256)
 link_neighbours(const Header* hdr, const u64* __restrict__ table,
                 const Key<Cfg<PD>::KW>* __restrict__ list_keys, u32* __restrict__ list_ref,
                 const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys, int* __restrict__ nbr,
-                u64 max_entries, void* zero_rows_ptr, u32 zero_row_bytes) {
+                u64 max_entries, void* zero_rows_ptr, u32 zero_row_bytes, Watch watch) {
     after_previous_kernel();
+    report_to(watch, hdr);
     constexpr int KW = Cfg<PD>::KW;
     if (hdr->status != 0) return;
     resolve_entries(hdr, list_ref, vid);

@@ -31,6 +31,7 @@
 #include <stdio.h>
 #include <string.h>
 #include <utility>
+#include <vector>
 
 #include "common.cuh"
 #include "lattice_build.cuh"
@@ -59,11 +60,64 @@ static int cuda_fail(cudaError_t e, const char* where) {
     snprintf(g_cuda_error, sizeof(g_cuda_error), "%s: %s", where, cudaGetErrorString(e));
     return PL_CUDA_ERROR;
 }
+
 #define PL_CUDA(call)                                   \
     do {                                                \
         cudaError_t e_ = (call);                        \
         if (e_ != cudaSuccess) return cuda_fail(e_, #call); \
     } while (0)
+
+// Pinned words in which watched calls (pl_watch_next_call) report their counters: a 64-byte line each, handed
+// to a thread when it first watches a call and taken back when the thread ends (the pool is as large as the
+// number of threads that ever watched at the same time, in pages of 64 lines).  The sequence number, which goes
+// with the line, tells its reports apart: a late one of a call that was given up on is not mistaken for the
+// next call's.
+struct alignas(64) WatchLine {
+    u64 word;
+    u32 seq;
+};
+static std::mutex g_watch_mutex;
+static std::vector<WatchLine*>& watch_pool() {
+    static std::vector<WatchLine*>* pool = new std::vector<WatchLine*>();   // outlives every thread
+    return *pool;
+}
+struct Watcher {
+    WatchLine* line = nullptr;
+    bool armed = false;     // the next call of this thread reports
+    bool launched = false;  // a call that reports has been queued
+    ~Watcher() {
+        if (!line) return;
+        std::lock_guard<std::mutex> lock(g_watch_mutex);
+        watch_pool().push_back(line);
+    }
+};
+static thread_local Watcher g_watcher;
+
+static int take_watch_line(WatchLine** out) {
+    std::lock_guard<std::mutex> lock(g_watch_mutex);
+    std::vector<WatchLine*>& pool = watch_pool();
+    if (pool.empty()) {
+        void* p = nullptr;
+        PL_CUDA(cudaHostAlloc(&p, 64 * sizeof(WatchLine), cudaHostAllocPortable | cudaHostAllocMapped));
+        memset(p, 0, 64 * sizeof(WatchLine));
+        for (int i = 0; i < 64; i++) pool.push_back(static_cast<WatchLine*>(p) + i);
+    }
+    *out = pool.back();
+    pool.pop_back();
+    return PL_OK;
+}
+
+// What a call passes to its link kernel: where to report, or nothing.
+static Watch take_watch() {
+    Watch w = {nullptr, 0u};
+    if (g_watcher.armed) {
+        w.word = &g_watcher.line->word;
+        w.seq = g_watcher.line->seq;
+        g_watcher.armed = false;
+        g_watcher.launched = true;
+    }
+    return w;
+}
 
 // Kernel launch with the error check of every other runtime call.  overlap: with programmatic stream
 // serialisation, i.e. the kernel may become resident while the kernel before it in the stream drains (it waits
@@ -417,7 +471,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
                 PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
                 PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
                 PL_LAUNCH_AFTER(OV_LINK, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                                 L.max_entries);
+                                                                 L.max_entries, take_watch());
             }
         }
         if (!use_direct) {
@@ -429,7 +483,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2);
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, nbr,
-                                                      L.max_entries, zrows, vinit.row_bytes);
+                                                      L.max_entries, zrows, vinit.row_bytes, take_watch());
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[2], st));
     } else {
@@ -522,14 +576,14 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
             PL_LAUNCH((clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
             PL_LAUNCH((insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH((link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                             L.max_entries);
+                                                             L.max_entries, take_watch());
         }
     }
     if (!use_direct) {
         PL_LAUNCH((clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2);
         PL_LAUNCH((insert_entries<KW>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, vinit);
         PL_LAUNCH((link_neighbours<PD>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, nbr, L.max_entries,
-                                                  nullptr, 0u);
+                                                  nullptr, 0u, take_watch());
     }
     PL_LAUNCH((splat_tiles_f64<PD>), tile_grid(g), TP, Splat64<PD>::BYTES, st, g, input, hdr, tile_info, rec, rec_w,
                                                                       list_ref, v0, vd);
@@ -1039,6 +1093,57 @@ int pl_debug_direct_index(int enable) {
 int pl_profile_next_call(void** stage_events) {
     g_stage_events = reinterpret_cast<cudaEvent_t*>(stage_events);
     return PL_OK;
+}
+
+int pl_watch_next_call(void* stream) {
+    Watcher& w = g_watcher;
+    w.armed = w.launched = false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PL_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        snprintf(g_cuda_error, sizeof(g_cuda_error), "pl_watch_next_call: the stream is being captured");
+        return PL_CUDA_ERROR;
+    }
+    if (!w.line) {
+        const int rc = take_watch_line(&w.line);
+        if (rc != PL_OK) return rc;
+    }
+    w.line->seq = (w.line->seq + 1) & WATCH_SEQ_MASK;
+    if (w.line->seq == 0) w.line->seq = 1;
+    w.armed = true;
+    return PL_OK;
+}
+
+int pl_await_watched_call(int64_t* num_entries, int* device_status, void* stream) {
+    Watcher& w = g_watcher;
+    w.armed = false;
+    if (!num_entries || !device_status || !w.launched) return PL_INVALID_ARGUMENT;
+    w.launched = false;
+    volatile u64* word = &w.line->word;
+    bool drained = false;
+    for (unsigned spin = 1;; spin++) {
+        const u64 v = *word;
+        if ((u32)(v >> 40) == w.line->seq) {
+            *num_entries = (int64_t)(u32)v;
+            *device_status = PL_OK;
+            for (int code = PL_INVALID_ARGUMENT; code <= PL_INTERNAL_ERROR; code++)
+                if ((v >> 32) & (1u << code)) *device_status = code;
+            return PL_OK;
+        }
+        if (drained) {
+            snprintf(g_cuda_error, sizeof(g_cuda_error), "pl_await_watched_call: the call ended without a report");
+            return PL_CUDA_ERROR;
+        }
+        // now and then: has the stream failed, or run empty (then the report is there, or never comes)?
+        if ((spin & 0xFFFu) == 0) {
+            const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+            if (e != cudaSuccess && e != cudaErrorNotReady) return cuda_fail(e, "pl_await_watched_call");
+            drained = e == cudaSuccess;
+        }
+#if defined(__x86_64__) && !defined(__CUDA_ARCH__)
+        __builtin_ia32_pause();
+#endif
+    }
 }
 
 int pl_lattice_stats(const void* workspace, pl_stats* stats, void* stream) {

@@ -37,9 +37,11 @@ def release_workspaces():
 #     - same memory, same version counter, same shape: a layer's backward call, the next iteration on the same
 #     image - builds the same lattice, so it runs with that call's bound and nothing needs checking;
 #   * any other call is VERIFIED: it runs with 1.5 x the largest entry count per item seen for its kind (a
-#     quarter of the worst case the first time), the stream is synchronised and the device status read, and
-#     the call is repeated with four times the bound as long as the lattice did not fit.  One
-#     synchronisation per new reference image.
+#     quarter of the worst case the first time), its counters are awaited, and the call is repeated with four
+#     times the bound as long as the lattice did not fit.  The counters arrive in a word of pinned memory when
+#     the lattice is complete (pl_await_watched_call), while the device still splats, blurs and slices: waiting
+#     for the whole stream instead left the GPU idle for 50 us after every new reference image (grey 1024 x 1024,
+#     forward + backward: 460 us with that wait).
 # Callers that own a synchronisation point of their own (HostPipeline) ask for verify="deferred" instead: the
 # call's counters are copied to pinned host memory behind it and looked at in check_pending(); a call that did
 # not fit has filled its output with NaN, and the caller repeats it.
@@ -155,29 +157,51 @@ def _run_sized(kind, identity, batch, worst, device, stream, launch, verify="aut
         return launch(known[1]), known[1]          # the same lattice as a call that fitted this bound
     max_entries = _guess_bound(kind, batch, worst, floor)
     repeated = False
+    L = capi.lib()
     while True:
-        ws = launch(max_entries)
-        if max_entries == 0:                       # the worst case cannot overflow: nothing to verify
-            if repeated:                           # (but what the lattice needed is worth knowing for the next call)
-                st = lattice_stats(ws, stream)
-                _entries_per_item[kind] = max(_entries_per_item.get(kind, 0.0), st.num_entries / max(batch, 1))
+        if max_entries == 0 and not repeated:      # the worst case cannot overflow: nothing to verify
+            ws = launch(max_entries)
             break
-        repeated = True
-        st = lattice_stats(ws, stream)
-        if st.device_status == capi.PL_CAPACITY_EXCEEDED:
+        capi.check(L.pl_watch_next_call(stream), "pl_watch_next_call")
+        ws = launch(max_entries)
+        entries, status = ctypes.c_int64(0), ctypes.c_int(0)
+        capi.check(L.pl_await_watched_call(ctypes.byref(entries), ctypes.byref(status), stream),
+                   "pl_await_watched_call")
+        if status.value == capi.PL_CAPACITY_EXCEEDED:
+            repeated = True
             grown = max_entries * FIRST_GUESS_DIVISOR
             max_entries = 0 if grown >= worst else grown
             continue
-        if st.device_status != capi.PL_OK:
-            raise capi.PlError(st.device_status, "lattice filter (device)")
-        _entries_per_item[kind] = max(_entries_per_item.get(kind, 0.0), st.num_entries / max(batch, 1))
+        if status.value != capi.PL_OK:
+            raise capi.PlError(status.value, "lattice filter (device)")
+        # (after a repeat at the worst case too: what the lattice needed is worth knowing for the next call)
+        _entries_per_item[kind] = max(_entries_per_item.get(kind, 0.0), entries.value / max(batch, 1))
         break
     _verified[kind] = (identity, max_entries)
     return ws, max_entries
 
 
 def _stream_handle(device):
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream's handle on `device` (a CUDA device with an index), without building a Stream object."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+class _OnDevice:
+    """torch.cuda.device(device) for the usual case too, in which that device is current already and there is
+    nothing to switch or to put back."""
+
+    def __init__(self, device):
+        self.index, self.before = device.index, -1
+
+    def __enter__(self):
+        current = torch.cuda.current_device()
+        if current != self.index:
+            self.before = current
+            torch.cuda.set_device(self.index)
+
+    def __exit__(self, *exc):
+        if self.before >= 0:
+            torch.cuda.set_device(self.before)
 
 
 def _check_tensor(t, name, dtype=None):
@@ -222,16 +246,57 @@ class FilterCall:
         self.vd = self.c + 1
         self.theta = (float(theta_alpha), float(theta_beta), float(theta_gamma))
         self.max_entries = 0   # the bound the last call on this geometry ran with (0: worst case)
+        self.c_sdims = capi.int_array(self.sdims)
 
     def workspace_bytes(self, max_entries=0, dtype=torch.float32, mode="atomic"):
         nbytes = ctypes.c_size_t(0)
-        head = (self.batch, self.n, self.pd, self.vd, len(self.sdims), capi.int_array(self.sdims), int(max_entries))
+        head = (self.batch, self.n, self.pd, self.vd, len(self.sdims), self.c_sdims, int(max_entries))
         if dtype == torch.float64:
             rc = capi.lib().pl_workspace_bytes_f64(*head, ctypes.byref(nbytes))
         else:
             rc = capi.lib().pl_workspace_bytes(*head, capi.MODES[mode], ctypes.byref(nbytes))
         capi.check(rc, "pl_workspace_bytes")
         return nbytes.value
+
+
+class _Plan:
+    """What calls of one geometry share: the FilterCall, its kind, worst case and floor of the sizing policy, and
+    the workspace sizes asked for so far."""
+
+    def __init__(self, device, call, dtype):
+        if not capi.lib().pl_supported(call.pd, call.vd):
+            raise capi.PlError(capi.PL_UNSUPPORTED_DIMS, "lattice_filter(pd=%d, vd=%d)" % (call.pd, call.vd))
+        self.call, self.dtype = call, dtype
+        self.kind = _kind(device, call)
+        self.worst = call.batch * call.n * (call.pd + 1)
+        self.floor = _direct_index_floor(call) if call.batch and call.n else 0
+        self._bytes = {}
+
+    def bytes(self, bound, mode):
+        key = (bound, mode)
+        nbytes = self._bytes.get(key)
+        if nbytes is None:
+            if len(self._bytes) >= 16:
+                self._bytes.clear()
+            nbytes = self._bytes[key] = self.call.workspace_bytes(bound, self.dtype, mode)
+        return nbytes
+
+
+_plans = {}        # arguments of a call that fix its geometry -> _Plan; emptied when it has grown to MOST_PLANS
+MOST_PLANS = 256
+
+
+def _plan_of(x, ref, bilateral, theta_alpha, theta_beta, theta_gamma):
+    key = (x.device.index, x.dtype, x.shape, None if ref is None else ref.shape, bool(bilateral), theta_alpha,
+           theta_beta, theta_gamma)
+    plan = _plans.get(key)
+    if plan is None:
+        plan = _Plan(x.device, FilterCall(tuple(x.shape), None if ref is None else tuple(ref.shape), bilateral,
+                                          theta_alpha, theta_beta, theta_gamma), x.dtype)
+        if len(_plans) >= MOST_PLANS:
+            _plans.clear()
+        _plans[key] = plan
+    return plan
 
 
 def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha=1.0,
@@ -254,38 +319,38 @@ def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha
     if bilateral:
         _check_tensor(reference_image, "reference_image", x.dtype)
         ref = reference_image.contiguous()
-    call = FilterCall(tuple(x.shape), None if ref is None else tuple(ref.shape), bilateral,
-                      theta_alpha, theta_beta, theta_gamma)
-    if not capi.lib().pl_supported(call.pd, call.vd):
-        raise capi.PlError(capi.PL_UNSUPPORTED_DIMS, "lattice_filter(pd=%d, vd=%d)" % (call.pd, call.vd))
+    plan = _plan_of(x, ref, bilateral, theta_alpha, theta_beta, theta_gamma)
+    call = FilterCall.__new__(FilterCall)      # the caller's own copy: it says what bound this call ran with
+    call.__dict__.update(plan.call.__dict__)
     if out is None:
         out = torch.empty_like(x)
     if call.batch == 0 or call.n == 0:
         return out, None, call
+    L = capi.lib()
     stream = _stream_handle(x.device)
     owner = stream if workspace_owner is None else workspace_owner
-    worst = call.batch * call.n * (call.pd + 1)
 
     def launch(bound):
-        nbytes = call.workspace_bytes(bound, x.dtype, mode)
-        ws = workspace if workspace is not None else _workspace(x.device, owner, nbytes)
+        ws = workspace
+        if ws is None:
+            ws = _workspace(x.device, owner, plan.bytes(bound, mode))
         head = (out.data_ptr(), x.data_ptr(), 0 if ref is None else ref.data_ptr(), call.batch,
-                len(call.sdims), capi.int_array(call.sdims), call.c, call.r, int(call.bilateral),
-                call.theta[0], call.theta[1], call.theta[2], int(bool(reverse)), ws.data_ptr(),
-                ws.numel(), int(bound))
+                len(call.sdims), call.c_sdims, call.c, call.r, call.bilateral,
+                call.theta[0], call.theta[1], call.theta[2], bool(reverse), ws.data_ptr(),
+                ws.numel(), bound)
         if f64:
-            capi.check(capi.lib().pl_lattice_filter_f64(*head, stream), "pl_lattice_filter_f64")
+            rc = L.pl_lattice_filter_f64(*head, stream)
         else:
-            capi.check(capi.lib().pl_lattice_filter_f32(*head, capi.MODES[mode], stream),
-                       "pl_lattice_filter_f32")
+            rc = L.pl_lattice_filter_f32(*head, capi.MODES[mode], stream)
+        if rc != capi.PL_OK:
+            capi.check(rc, "pl_lattice_filter_f64" if f64 else "pl_lattice_filter_f32")
         return ws
 
-    with torch.cuda.device(x.device):
+    with _OnDevice(x.device):
         if max_entries is None and workspace is None:
-            ws, max_entries = _run_sized(_kind(x.device, call), _identity(reference_image if bilateral else None,
-                                                                          call.batch),
-                                         call.batch, worst, x.device, stream, launch, verify=verify,
-                                         floor=_direct_index_floor(call))
+            ws, max_entries = _run_sized(plan.kind, _identity(reference_image if bilateral else None, call.batch),
+                                         call.batch, plan.worst, x.device, stream, launch, verify=verify,
+                                         floor=plan.floor)
         else:
             max_entries = int(max_entries or 0)
             ws = launch(max_entries)
@@ -309,7 +374,7 @@ def lattice_stats(workspace, stream=None, device=None):
         device = torch.device("cuda", torch.cuda.current_device())
     if stream is None:
         stream = _stream_handle(device)
-    with torch.cuda.device(device):
+    with _OnDevice(device):
         capi.check(capi.lib().pl_lattice_stats(0 if workspace is None else workspace.data_ptr(),
                                                ctypes.byref(st), stream), "pl_lattice_stats")
     return st
@@ -362,7 +427,7 @@ class Lattice:
                 ws.data_ptr(), ws.numel(), int(bound), stream), "pl_lattice_build_f32")
             return ws
 
-        with torch.cuda.device(device):
+        with _OnDevice(device):
             if max_entries is None:
                 worst = call.batch * call.n * (call.pd + 1)
                 # verified like a filter call: once per reference image, not again for a lattice rebuilt on it
@@ -391,7 +456,7 @@ class Lattice:
             out = torch.empty_like(x)
         if self.workspace is None:
             return out
-        with torch.cuda.device(self.device):
+        with _OnDevice(self.device):
             capi.check(capi.lib().pl_lattice_apply_f32(
                 out.data_ptr(), x.data_ptr(), x.shape[-1], int(bool(reverse)), capi.MODES[mode], call.batch,
                 call.n, call.pd, len(call.sdims), capi.int_array(call.sdims), self.workspace.data_ptr(),
@@ -418,7 +483,7 @@ class _LatticeFilterReuseFunction(torch.autograd.Function):
     def backward(ctx, grad):
         (reference_image,) = ctx.saved_tensors
         g = ctx.lattice.apply(grad, True, ctx.mode)
-        ref_grad = torch.zeros_like(reference_image) if reference_image is not None else None
+        ref_grad = torch.zeros_like(reference_image) if ctx.needs_input_grad[1] else None
         return g, ref_grad, None, None, None, None, None, None
 
 
@@ -440,7 +505,7 @@ class _LatticeFilterFunction(torch.autograd.Function):
         bilateral, theta_alpha, theta_beta, theta_gamma, mode = ctx.args
         g, _, _ = lattice_filter_raw(grad, reference_image, bilateral, theta_alpha, theta_beta,
                                      theta_gamma, True, mode)
-        ref_grad = torch.zeros_like(reference_image) if reference_image is not None else None
+        ref_grad = torch.zeros_like(reference_image) if ctx.needs_input_grad[1] else None
         return g, ref_grad, None, None, None, None, None, None
 
 
@@ -452,10 +517,20 @@ def lattice_filter(input_image, reference_image, bilateral=True, theta_alpha=1.0
     it there (same results; the reference always rebuilds).
     The thetas are float attributes of the op (src/LatticeFilterKernel.cpp:36-38): they are rounded to
     float32 here and widened again for float64 tensors, as the reference does (:131-142)."""
+    thetas = (_as_attr(theta_alpha), _as_attr(theta_beta), _as_attr(theta_gamma))
+    if not (torch.is_grad_enabled() and (input_image.requires_grad or (
+            reference_image is not None and reference_image.requires_grad))):
+        # nothing to differentiate: the autograd function would only add its own cost (a tenth of a small call)
+        if not reuse_lattice:
+            return lattice_filter_raw(input_image, reference_image, bool(bilateral), *thetas, bool(reverse), mode)[0]
+        return Lattice(reference_image, tuple(input_image.shape[:-1]), bool(bilateral), *thetas,
+                       max_channels=input_image.shape[-1], mode=mode).apply(input_image, bool(reverse), mode)
     fn = _LatticeFilterReuseFunction if reuse_lattice else _LatticeFilterFunction
-    as_attr = lambda v: ctypes.c_float(float(v)).value
-    return fn.apply(input_image, reference_image, bool(bilateral), as_attr(theta_alpha), as_attr(theta_beta),
-                    as_attr(theta_gamma), bool(reverse), mode)
+    return fn.apply(input_image, reference_image, bool(bilateral), *thetas, bool(reverse), mode)
+
+
+def _as_attr(v):
+    return ctypes.c_float(float(v)).value
 
 
 def compute_positions(reference_image, spatial_dims, spatial_std, feature_std, dtype=None):
@@ -477,7 +552,7 @@ def compute_positions(reference_image, spatial_dims, spatial_std, feature_std, d
         dtype = torch.float32 if dtype is None else dtype
     pos = torch.empty((n, len(sdims) + r), dtype=dtype, device=device)
     fn = capi.lib().pl_compute_positions_f64 if dtype == torch.float64 else capi.lib().pl_compute_positions_f32
-    with torch.cuda.device(device):
+    with _OnDevice(device):
         capi.check(fn(0 if ref is None else ref.data_ptr(), pos.data_ptr(), n, r, len(sdims),
                       capi.int_array(sdims), float(spatial_std), float(feature_std), _stream_handle(device)),
                    "pl_compute_positions")
@@ -528,7 +603,7 @@ def filter_positions(input_values, positions, reverse=False, mode="atomic", max_
                 capi.check(capi.lib().pl_filter_f32(*head, capi.MODES[mode], stream), "pl_filter_f32")
             return w
 
-        with torch.cuda.device(x.device):
+        with _OnDevice(x.device):
             if max_entries is None and workspace is None:
                 kind = (x.device.index, "positions", n, pd)
                 ws, max_entries = _run_sized(kind, _identity(positions, batch), batch, batch * n * (pd + 1), x.device,
@@ -565,7 +640,7 @@ def export_lattice(workspace, stats, batch, n, pd, vd, positions=None, reference
     vitem = torch.zeros((m,), dtype=torch.int32, device=device)
     pv = torch.zeros((batch, n, pd + 1), dtype=torch.int32, device=device)
     pw = torch.zeros((batch, n, pd + 1), dtype=dtype, device=device)
-    with torch.cuda.device(device):
+    with _OnDevice(device):
         if positions is not None:
             rc = fn(workspace.data_ptr(), positions.contiguous().data_ptr(), 0,
                     batch, n, pd, vd, 0, None, 0, 1.0, 1.0, int(max_entries),
