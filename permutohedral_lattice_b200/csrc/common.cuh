@@ -50,6 +50,20 @@ struct Header {   // first 256 bytes of the workspace
     u32 pad[56];
 };
 
+// Sketch of the lattice's size, behind the header (zeroed with it): a bitmap in which build_tiles sets one bit
+// for every key whose hash falls into a 2^-shift part of the hash range.  The bits set tell clear_table how many
+// DISTINCT keys there are (linear counting), so that the table is sized by vertices and not by entries, of which
+// there are up to 40 times as many.  The shift keeps the bitmap at most about half full in the worst case.
+constexpr int SKETCH_LOG2 = 16;
+constexpr int SKETCH_WORDS = (1 << SKETCH_LOG2) / 32;
+constexpr u64 SKETCH_MIN_ENTRIES = 1ull << 18;   // below, a table sized by entries is small anyway
+
+// Number of this thread in a grid of one or two dimensions, and how many there are.
+__device__ __forceinline__ u64 grid_thread() {
+    return (u64)(blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+}
+__device__ __forceinline__ u64 grid_threads() { return (u64)gridDim.x * gridDim.y * blockDim.x; }
+
 // Where a watched call reports (pl_watch_next_call): one word of mapped host memory.  The link kernel writes
 // sequence << 40 | status bits << 32 | entries there before it does anything else: everything that can make a
 // call fail has happened by then, and the host, which polls the word, goes on while the device still splats,
@@ -60,7 +74,7 @@ struct Watch {
     u32 seq;
 };
 __device__ __forceinline__ void report_to(const Watch& w, const Header* hdr) {
-    if (w.word && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (w.word && grid_thread() == 0) {
         const u64 v = ((u64)w.seq << 40) | ((u64)(hdr->status & 0xFFu) << 32) | (u64)hdr->num_entries;
         asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(w.word), "l"(v) : "memory");
     }
@@ -82,11 +96,13 @@ struct Cfg {
     static constexpr int KW = (PD + 1 + 3) / 4;          // 16-bit fields: PD coordinates + item
     static constexpr int TP = (PD <= 8) ? 256 : 128;     // points per tile = threads per CTA
     static constexpr int SPLATS = TP * (PD + 1);
-    static constexpr int LS = (5 * SPLATS <= 4 * 1024)   ? 1024
-                              : (5 * SPLATS <= 4 * 2048) ? 2048
-                              : (5 * SPLATS <= 4 * 4096) ? 4096
-                              : (5 * SPLATS <= 4 * 8192) ? 8192
-                                                         : 16384;   // shared hash slots (>= 1.25 * SPLATS)
+    // 16-bit slots of the tile's hash: at least 2.5 per splat
+    static constexpr int LSLOG = (5 * SPLATS <= 2 * 2048)    ? 11
+                                 : (5 * SPLATS <= 2 * 4096)  ? 12
+                                 : (5 * SPLATS <= 2 * 8192)  ? 13
+                                                             : 14;
+    static constexpr int LS = 1 << LSLOG;
+    static_assert(5 * SPLATS <= 2 * LS && SPLATS <= 65535, "slots hold 16-bit splat numbers");
     // The tile's splats sorted by entry, as build_tiles leaves them for the splat kernels: cut into windows
     // of WL splats, each followed by one spare 8-byte word (lanes that walk neighbouring windows in step then
     // read words an odd number of 8-byte words apart: no shared-memory bank collisions), SREC words per tile
@@ -94,24 +110,44 @@ struct Cfg {
     static constexpr int WL = 8 * (PD + 1);
     static constexpr int SREC = (SPLATS + SPLATS / WL + 1 + 1) & ~1;
     __host__ __device__ static constexpr int srec_slot(int pos) { return pos + pos / WL; }
-    // build_tiles assembles that list in the memory of its key list, which is therefore at least as large
-    static constexpr size_t BUILD_KEYS = sizeof(Key<KW>) * SPLATS > sizeof(uint2) * SREC ? sizeof(Key<KW>) * SPLATS
-                                                                                        : sizeof(uint2) * SREC;
-    static constexpr size_t BUILD_SMEM = BUILD_KEYS + sizeof(int) * LS + sizeof(u16) * SPLATS;
+    // What build_tiles keeps of the keys in shared memory (see TileKeys): every splat's key up to pd = 8, one
+    // record per point above (a key of 16 coordinates for each of 17 splats would leave room for two CTAs an SM).
+    static constexpr bool COMPACT = PD > 8;
+    static constexpr int CW = (PD + 1) / 2;                                  // 32-bit words of two coordinates
+    static constexpr int KEY_WORDS = COMPACT ? CW + 4 : CW <= 2 ? CW : 4;    // words of one key (point record)
+    // build_tiles assembles the sorted list in the memory of its keys, which is therefore at least as large
+    static constexpr size_t KEY_BYTES = sizeof(u32) * (size_t)KEY_WORDS * (COMPACT ? TP : SPLATS);
+    __host__ __device__ static constexpr size_t build_keys(bool sorted) {
+        return sorted && sizeof(uint2) * SREC > KEY_BYTES ? sizeof(uint2) * SREC : KEY_BYTES;
+    }
+    __host__ __device__ static constexpr size_t build_smem(bool sorted) {
+        return build_keys(sorted) + sizeof(u16) * LS + (COMPACT ? 2 : 1) * sizeof(u16) * SPLATS;
+    }
 };
 
+// Hash of a key: a sum of words times odd constants (linear, so that the hash of a neighbouring lattice point is
+// the sum plus a constant, see link_neighbours), then a mix.
+__host__ __device__ constexpr u64 hash_factor(int j) {
+    u64 z = 0x9E3779B97F4A7C15ull * (u64)(j + 1);   // splitmix64 sequence
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return (z ^ (z >> 31)) | 1ull;
+}
+template <int KW>
+__device__ __forceinline__ u64 linear_hash(const Key<KW>& k) {
+    u64 h = 0;
+#pragma unroll
+    for (int j = 0; j < KW; j++) h += k.w[j] * hash_factor(j);
+    return h;
+}
+__device__ __forceinline__ u64 mix_hash(u64 h) {
+    h ^= h >> 32;
+    h *= 0xC4CEB9FE1A85EC53ull;
+    return h ^ (h >> 29);
+}
 template <int KW>
 __device__ __forceinline__ u64 hash_key(const Key<KW>& k) {
-    u64 h = 0x9E3779B97F4A7C15ull;
-#pragma unroll
-    for (int j = 0; j < KW; j++) {
-        h ^= k.w[j];
-        h *= 0xFF51AFD7ED558CCDull;
-        h ^= h >> 32;
-    }
-    h *= 0xC4CEB9FE1A85EC53ull;
-    h ^= h >> 29;
-    return h;
+    return mix_hash(linear_hash<KW>(k));
 }
 
 template <int KW>
@@ -145,25 +181,11 @@ __device__ __forceinline__ u16 key_get(const Key<KW>& k, int f) {
 
 // 0x0001 in every coordinate field of key word j.
 template <int PD>
-__device__ __forceinline__ constexpr u64 coord_ones(int j) {
+__host__ __device__ constexpr u64 coord_ones(int j) {
     u64 m = 0;
     for (int f = 4 * j; f < 4 * j + 4; f++)
         if (f < PD) m |= 1ull << (16 * (f & 3));
     return m;
-}
-
-// Cheap 32-bit hash for the per-tile shared-memory table (placement only).
-template <int KW>
-__device__ __forceinline__ u32 tile_hash(const Key<KW>& k) {
-    u32 h = 0;
-#pragma unroll
-    for (int j = 0; j < KW; j++) {
-        h = (h ^ (u32)k.w[j]) * 0x9E3779B1u;
-        h = (h ^ (u32)(k.w[j] >> 32)) * 0x85EBCA77u;
-    }
-    h ^= h >> 15;
-    h *= 0x2C1B3C6Du;
-    return h ^ (h >> 13);
 }
 
 // Tile of this CTA.  Tile kernels run on a 3-D grid (tile column, tile row, item * outer + outer index)

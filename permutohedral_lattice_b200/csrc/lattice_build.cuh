@@ -16,30 +16,191 @@ struct is_double { static constexpr bool value = false; };
 template <>
 struct is_double<double> { static constexpr bool value = true; };
 
-// Up to pd = 5 six CTAs fit an SM's shared memory; capping the registers for that (40 per thread, a
-// few bytes of spills at pd = 5) measured 13 % faster than five CTAs with 48.
+// x << s with 0 for every shift beyond the word (negative ones included).
+__device__ __forceinline__ u32 shift_in(u32 x, u32 s) {
+    u32 y;
+    asm("shl.b32 %0, %1, %2;" : "=r"(y) : "r"(x), "r"(s));
+    return y;
+}
+
+// The keys of one point, remainder by remainder (src/PermutohedralLatticeCPU.h:297-304): coordinate i of the
+// remainder-r vertex is rem0_i + r - (PD+1) [rank_i > PD - r], so a step from r - 1 to r adds one to every
+// coordinate and takes PD+1 off the one of rank PD - r + 1.  Coordinates are packed two to a word, biased by
+// 0x8000 (no carries between them); `perm` holds the coordinate of every rank >= 1 in four bits.
+template <int PD>
+struct PointKeys {
+    static constexpr int CW = Cfg<PD>::CW;
+    static constexpr bool WIDE = PD > 8;
+    u32 w[CW];
+    u32 perm, perm_hi;   // coordinates of ranks 1..8 and 9..16
+    int last_rank;       // WIDE: rank of coordinate PD, which is not stored (else its nibble is 15: no coordinate)
+
+    template <typename S>
+    __device__ __forceinline__ void start(const S& s) {
+#pragma unroll
+        for (int j = 0; j < CW; j++) {
+            const u32 lo = rem0_low16<PD>(s, 2 * j);
+            w[j] = (2 * j + 1 < PD) ? __byte_perm(lo, rem0_low16<PD>(s, 2 * j + 1 < PD ? 2 * j + 1 : 0), 0x5410) ^ 0x80008000u
+                                    : (lo & 0xFFFFu) ^ 0x8000u;
+        }
+        perm = perm_hi = 0;
+#pragma unroll
+        for (int i = 1; i < PD; i++) {
+            perm += shift_in((u32)i, (u32)(4 * s.rank[i] - 4));
+            if constexpr (WIDE) perm_hi += shift_in((u32)i, (u32)(4 * s.rank[i] - 36));
+        }
+        if constexpr (!WIDE) perm += shift_in(15u, (u32)(4 * s.rank[PD] - 4));
+        last_rank = s.rank[PD];
+    }
+    // from remainder r - 1 to remainder r
+    __device__ __forceinline__ void step(int r) {
+        const int rank = PD - r + 1;
+        u32 c16;   // 16 x the coordinate of that rank
+        if constexpr (WIDE) {
+            c16 = ((rank > 8 ? perm_hi >> (4 * (rank - 9)) : perm >> (4 * (rank - 1))) & 15u) * 16u;
+            if (rank == last_rank) c16 = 512u;
+        } else {
+            c16 = ((rank > 1) ? perm >> (4 * (rank - 2)) : perm << 4) & 0xF0u;
+        }
+#pragma unroll
+        for (int j = 0; j < CW; j++) {
+            const u32 ones = (2 * j + 1 < PD) ? 0x00010001u : 1u;
+            w[j] += ones - shift_in((u32)(PD + 1), c16 - 32u * j);
+        }
+    }
+    // 32-bit hash of the key (of item `seed`): its high bits place the key in the tile's table
+    __device__ __forceinline__ u32 hash(u32 seed) const {
+        u32 h = seed;
+#pragma unroll
+        for (int j = 0; j < CW; j++) h += w[j] * (u32)(hash_factor(j + 8) >> 32 | 1u);
+        return h;
+    }
+};
+
+// What the tile keeps of its points' keys in shared memory.  Up to pd = 8: the coordinate words of every splat's
+// key.  Above (COMPACT): per point the remainder-0 key and the ranks of its coordinates, one byte each, from
+// which the key of any remainder follows.
+template <int PD>
+struct TileKeys {
+    static constexpr int TP = Cfg<PD>::TP, CW = Cfg<PD>::CW, KS = Cfg<PD>::KEY_WORDS;
+    static constexpr bool COMPACT = Cfg<PD>::COMPACT;
+    u32* s;
+    // coordinate words of splat `id` = r * TP + point
+    __device__ __forceinline__ void load(int id, int r, u32 (&k)[CW]) const {
+        if constexpr (COMPACT) {
+            const uint4* rec = reinterpret_cast<const uint4*>(s + (id - r * TP) * KS);
+            u32 rank[4];
+            const uint4 v = rec[CW / 4];
+            rank[0] = v.x; rank[1] = v.y; rank[2] = v.z; rank[3] = v.w;
+            const u32 above = (u32)(127 - (PD - r)) * 0x01010101u;   // rank + this has its top bit set iff rank > PD - r
+#pragma unroll
+            for (int j = 0; j < CW; j += 4) {
+                const uint4 q = rec[j / 4];
+                k[j] = q.x; k[j + 1] = q.y; k[j + 2] = q.z; k[j + 3] = q.w;
+            }
+#pragma unroll
+            for (int j = 0; j < CW; j++) {
+                const u32 taken = ((rank[j / 2] + above) >> 7) & 0x01010101u;
+                const u32 fields = __byte_perm(taken, 0u, (j & 1) ? 0x4342 : 0x4140);   // two 16-bit fields
+                k[j] += (u32)r * 0x00010001u - fields * (u32)(PD + 1);
+            }
+        } else if constexpr (KS == 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(s + id * 4);
+            const u32 t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < CW; j++) k[j] = t[j];
+        } else if constexpr (KS == 2) {
+            const uint2 v = *reinterpret_cast<const uint2*>(s + id * 2);
+            k[0] = v.x;
+            k[CW - 1] = v.y;
+        } else {
+            k[0] = s[id];
+        }
+    }
+    __device__ __forceinline__ void store(int id, const u32 (&k)[CW]) const {
+        if constexpr (KS == 4)
+            *reinterpret_cast<uint4*>(s + id * 4) = make_uint4(k[0], k[1 % CW], k[2 % CW], CW > 3 ? k[3 % CW] : 0u);
+        else if constexpr (KS == 2)
+            *reinterpret_cast<uint2*>(s + id * 2) = make_uint2(k[0], k[CW - 1]);
+        else
+            s[id] = k[0];
+    }
+    __device__ __forceinline__ bool same(int a, int b, int r) const {
+        u32 x[CW], y[CW];
+        load(a, r, x);
+        load(b, r, y);
+        u32 diff = 0;
+#pragma unroll
+        for (int j = 0; j < CW; j++) diff |= x[j] ^ y[j];
+        return diff == 0;
+    }
+    __device__ __forceinline__ u32 hash(int id, int r, u32 seed) const {
+        u32 k[CW];
+        load(id, r, k);
+        u32 h = seed;
+#pragma unroll
+        for (int j = 0; j < CW; j++) h += k[j] * (u32)(hash_factor(j + 8) >> 32 | 1u);
+        return h;
+    }
+    // the key as the global list holds it
+    __device__ __forceinline__ Key<Cfg<PD>::KW> global_key(int id, int r, int item) const {
+        constexpr int KW = Cfg<PD>::KW;
+        u32 k[CW];
+        load(id, r, k);
+        Key<KW> out;
+#pragma unroll
+        for (int j = 0; j < KW; j++) {
+            const u32 lo = (2 * j < CW) ? k[2 * j < CW ? 2 * j : 0] : 0u;
+            const u32 hi = (2 * j + 1 < CW) ? k[2 * j + 1 < CW ? 2 * j + 1 : 0] : 0u;
+            out.w[j] = (u64)lo | ((u64)hi << 32);
+        }
+        key_set<KW>(out, PD, (u16)item);
+        return out;
+    }
+};
+
+constexpr u32 TILE_SEED = 0x2C1B3C6Du;    // times the item: keys of different items sample independently
+constexpr int TILE_ROUNDS = 8;            // of the tile's de-duplication
+
+// One thread per point of the tile: features, enclosing simplex, weights, keys; then the tile's keys are
+// de-duplicated, its distinct keys appended to the global entry list, and every splat's entry number stored.
+//
+// De-duplication without atomics, in rounds: every splat writes its number into the slot of its key's hash (one
+// of the writers stays), and after a barrier reads the slot back.  If the number there is of the same key, that
+// splat represents the key, for all its splats alike, since all of them read that slot.  Keys that lost their slot
+// to another key go into the next round with another hash; with 2.5 slots a splat that leaves a few per cent of
+// them.  A splat still without representative after TILE_ROUNDS represents itself: the key then has two entries,
+// which the global table merges as it does those of different tiles.  (One compare-and-swap per splat on the slot,
+// as before, took a third of the kernel's shared-memory wavefronts, and its retries most of the divergence.)
+//
+// Bound by issue slots and the LSU pipe.  Up to pd = 5 six CTAs fit an SM: the registers are capped at 40 for it
+// (measured 13 % faster than five CTAs with 48).
 // SORTED (float calls that build a lattice for reuse): also leave every tile's splats sorted by entry in
 // `srec`, in the form the splat kernels walk, so that no later splat through this lattice sorts again.
 // It costs this kernel a quarter more time and saves every splat a fifth: worth it from the second
 // splat on, which is why the one-call filter does not ask for it.
+// sketch_shift < 0: no sketch of the lattice's size (see SKETCH_LOG2).
 template <int PD, typename R = float, bool SORTED = false>
-__global__ void __launch_bounds__(Cfg<PD>::TP, (PD <= 5 && !is_double<R>::value) ? 6 : 1)
+__global__ void __launch_bounds__(Cfg<PD>::TP, (PD <= 5 && !is_double<R>::value) ? 6 : (Cfg<PD>::COMPACT && !is_double<R>::value) ? 5 : 1)
 build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ reference,
             Header* hdr, int2* __restrict__ tile_info, u16* __restrict__ rec, R* __restrict__ rec_w,
-            uint2* __restrict__ srec, Key<Cfg<PD>::KW>* __restrict__ list_keys, u32 max_entries) {
+            uint2* __restrict__ srec, Key<Cfg<PD>::KW>* __restrict__ list_keys, u32 max_entries, int sketch_shift) {
     wait_for_previous_kernel();
-    constexpr int KW = Cfg<PD>::KW, TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, LS = Cfg<PD>::LS;
+    constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, LSLOG = Cfg<PD>::LSLOG;
+    constexpr bool COMPACT = Cfg<PD>::COMPACT;
+    constexpr int KEYS = (int)Cfg<PD>::build_keys(SORTED);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Key<KW>* keys_s = reinterpret_cast<Key<KW>*>(smem_raw);
-    int* hslots = reinterpret_cast<int*>(smem_raw + Cfg<PD>::BUILD_KEYS);
-    u16* lidx_s = reinterpret_cast<u16*>(smem_raw + Cfg<PD>::BUILD_KEYS + sizeof(int) * LS);
+    TileKeys<PD> keys;
+    keys.s = reinterpret_cast<u32*>(smem_raw);
+    u16* slots_s = reinterpret_cast<u16*>(smem_raw + KEYS);                       // [LS]
+    u16* lidx_s = slots_s + Cfg<PD>::LS;                                          // [SPLATS]
+    u16* rep_s = lidx_s + SPLATS;                                                 // [SPLATS], COMPACT only
     __shared__ int cnt_s[PD + 1], base_s;   // entries per remainder; first global entry of the tile
     __shared__ int wsum_s[TP / 32];
 
     PhaseClock pc(0);
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
-    for (int i = tid; i < LS; i += TP) hslots[i] = -1;
     if (tid <= PD) cnt_s[tid] = 0;
     if (tile == 0 && tid == 0) {
         hdr->capacity = max_entries;
@@ -48,9 +209,9 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 
     int item, pix, po, py, px;
     const bool valid = tile_point(g, tpos, tid, item, pix, po, py, px);
-    u32 slot[PD + 1];   // home slot of each key in the tile's hash, computed while the key is in registers
+    u32 slot2[PD / 2 + 1];   // slots of the splats' keys, two to a word
 #pragma unroll
-    for (int r = 0; r <= PD; r++) slot[r] = 0;
+    for (int r = 0; r <= PD / 2; r++) slot2[r] = 0;
     if (valid) {
         R f[PD];
         R w[PD + 1];
@@ -67,91 +228,121 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
         R* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
         for (int r = 0; r <= PD; r++) recw_tile[r * TP + tid] = w[r];
-        // Remainder-r vertex: coordinate i = rem0_i + r - (PD+1) [rank_i > PD - r]
-        // (src/PermutohedralLatticeCPU.h:297-304).  In packed form: start from the remainder-0 key,
-        // then per step add one to every coordinate field and take PD+1 off the one coordinate whose
-        // rank is PD - r + 1.
-        Key<KW> k;
+        PointKeys<PD> k;
+        k.start(s);
+        if constexpr (COMPACT) {
+            u32* mine = keys.s + tid * Cfg<PD>::KEY_WORDS;
 #pragma unroll
-        for (int j = 0; j < KW; j++) k.w[j] = 0;
+            for (int j = 0; j < Cfg<PD>::CW; j++) mine[j] = k.w[j];
 #pragma unroll
-        for (int i = 0; i < PD; i++) key_set<KW>(k, i, (u16)(s.rem0[i] + 0x8000));
-        key_set<KW>(k, PD, (u16)item);
-        keys_s[tid] = k;
-        slot[0] = tile_hash<KW>(k) & (LS - 1);
+            for (int j = 0; j < 4; j++)
+                mine[Cfg<PD>::CW + j] = (u32)s.rank[4 * j] | ((u32)s.rank[4 * j + 1] << 8) |
+                                        ((u32)s.rank[4 * j + 2] << 16) | ((u32)s.rank[4 * j + 3] << 24);
+        }
+        const u32 seed = (u32)item * TILE_SEED;
+        u32* sketch = reinterpret_cast<u32*>(hdr + 1);
 #pragma unroll
-        for (int r = 1; r <= PD; r++) {
-#pragma unroll
-            for (int i = 0; i < PD; i++)
-                k.w[i >> 2] -= (s.rank[i] == PD - r + 1) ? ((u64)(PD + 1) << (16 * (i & 3))) : 0ull;
-#pragma unroll
-            for (int j = 0; j < KW; j++) k.w[j] += coord_ones<PD>(j);
-            keys_s[r * TP + tid] = k;
-            slot[r] = tile_hash<KW>(k) & (LS - 1);
+        for (int r = 0; r <= PD; r++) {
+            if (r > 0) k.step(r);
+            if constexpr (!COMPACT) keys.store(r * TP + tid, k.w);
+            const u32 h = k.hash(seed);
+            const u32 slot = h >> (32 - LSLOG);
+            slots_s[slot] = (u16)(r * TP + tid);
+            slot2[r / 2] |= slot << (16 * (r & 1));
+            if (sketch_shift >= 0) {
+                const u32 x = (h ^ (h >> 15)) * 0x9E3779B1u;
+                if ((x >> 1) < (0x80000000u >> sketch_shift)) {
+                    const u32 bit = (h ^ (x << 7)) * 0x85EBCA77u >> (32 - SKETCH_LOG2);
+                    atomicOr(sketch + (bit >> 5), 1u << (bit & 31u));
+                }
+            }
         }
     }
     __syncthreads();
     pc.mark();
 
-    // de-duplicate: the first splat to claim a slot for a key represents it.  The first probes of all
-    // PD+1 keys are issued together (independent shared-memory accesses); most keys resolve there,
-    // the rest walk on one at a time.
-    int rep[PD + 1];
-    {
-        int cand[PD + 1];
-#pragma unroll
+    int rep[COMPACT ? 1 : PD + 1];   // the splat that represents each splat's key (COMPACT: in rep_s)
+    u32 open = 0;                    // splats without a representative
+    auto set_rep = [&](int r, int v) {
+        if constexpr (COMPACT) rep_s[r * TP + tid] = (u16)v;
+        else rep[r] = v;
+    };
+    auto get_rep = [&](int r) -> int {
+        if constexpr (COMPACT) return (int)rep_s[r * TP + tid];
+        else return rep[r];
+    };
+    if constexpr (COMPACT) {
+#pragma unroll 1
         for (int r = 0; r <= PD; r++) {
-            rep[r] = -1;
-            cand[r] = valid ? hslots[slot[r]] : -1;
-        }
-#pragma unroll
-        for (int r = 0; r <= PD; r++) {
-            if (valid && cand[r] < 0) {
-                cand[r] = atomicCAS(&hslots[slot[r]], -1, r * TP + tid);
-                if (cand[r] < 0) rep[r] = r * TP + tid;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r <= PD; r++) {
-            if (valid && rep[r] < 0 && key_equal<KW>(keys_s[cand[r]], keys_s[r * TP + tid])) rep[r] = cand[r];
-        }
-#pragma unroll
-        for (int r = 0; r <= PD; r++) {
-            if (valid && rep[r] < 0) {
-                const int me = r * TP + tid;
-                const Key<KW> k = keys_s[me];
-                u32 s = (slot[r] + 1) & (LS - 1);
-                int found = -1;
-                for (int it = 0; it < LS; it++) {
-                    int o = hslots[s];
-                    if (o < 0) {
-                        o = atomicCAS(&hslots[s], -1, me);
-                        if (o < 0) { found = me; break; }
-                    }
-                    if (key_equal<KW>(keys_s[o], k)) { found = o; break; }
-                    s = (s + 1) & (LS - 1);
+            const int me = r * TP + tid;
+            int c = me;
+            if (valid) {
+                c = slots_s[keys.hash(me, r, (u32)item * TILE_SEED) >> (32 - LSLOG)];
+                if (c != me && (c / TP != r || !keys.same(c, me, r))) {
+                    c = me;
+                    open |= 1u << r;
                 }
-                rep[r] = found;
+            }
+            set_rep(r, c);
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r <= PD; r++)
+            rep[r] = valid ? (int)slots_s[(slot2[r / 2] >> (16 * (r & 1))) & 0xFFFFu] : r * TP + tid;
+#pragma unroll
+        for (int r = 0; r <= PD; r++) {
+            const int me = r * TP + tid;
+            // a slot written by a splat of another remainder holds another key: the remainder is the key modulo PD+1
+            if (rep[r] != me && !keys.same(rep[r], me, r)) {
+                rep[r] = me;
+                open |= 1u << r;
             }
         }
     }
-    __syncthreads();
+    for (int round = 1; round <= TILE_ROUNDS; round++) {
+        if (!__syncthreads_or((int)open)) break;
+        auto next_slot = [&](int r) {
+            const u32 h = keys.hash(r * TP + tid, r, (u32)item * TILE_SEED) + (u32)round * 0x632BE5ABu;
+            return ((h ^ (h >> 13)) * 0x85EBCA77u) >> (32 - LSLOG);
+        };
+        if (open) {
+#pragma unroll (COMPACT ? 1 : PD + 1)
+            for (int r = 0; r <= PD; r++)
+                if ((open >> r) & 1u) slots_s[next_slot(r)] = (u16)(r * TP + tid);
+        }
+        __syncthreads();
+        if (open) {
+#pragma unroll (COMPACT ? 1 : PD + 1)
+            for (int r = 0; r <= PD; r++) {
+                if ((open >> r) & 1u) {
+                    const int me = r * TP + tid, c = slots_s[next_slot(r)];
+                    if (c == me || ((!COMPACT || c / TP == r) && keys.same(c, me, r))) {
+                        set_rep(r, c);
+                        open &= ~(1u << r);
+                    }
+                }
+            }
+        }
+    }
     pc.mark();
     // Number the tile's entries remainder by remainder (all entries of remainder 0 first, ...: the splat
     // stage, which walks the tile's splats in entry order, measured 4 % faster with this order than with
     // entries grouped by warp).  Per warp ONE shared-memory atomic instruction: lane r adds the warp's
     // number of new remainder-r entries to counter r.  The index stored now is relative to the
     // remainder's segment; the segment starts are known after the barrier.
-    int* run_s = hslots;   // the tile hash is dead from here on: its memory counts the splats of every entry
-    if constexpr (SORTED)
+    int* run_s = reinterpret_cast<int*>(slots_s);   // SORTED: the tile hash is dead, its memory counts the splats of every entry
+    if constexpr (SORTED) {
+        static_assert(sizeof(int) * SPLATS <= sizeof(u16) * Cfg<PD>::LS, "the counters fit the hash's memory");
+        __syncthreads();
         for (int i = tid; i < SPLATS; i += TP) run_s[i] = 0;
+    }
     {
         const int lane = tid & 31;
         unsigned owners[PD + 1];
         int mine = 0;
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
-            owners[r] = __ballot_sync(0xFFFFFFFFu, valid && rep[r] == r * TP + tid);
+            owners[r] = __ballot_sync(0xFFFFFFFFu, valid && get_rep(r) == r * TP + tid);
             mine = (lane == r) ? __popc(owners[r]) : mine;
         }
         int first = 0;
@@ -188,7 +379,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     u16* rec_tile = rec + (size_t)tile * SPLATS;
 #pragma unroll
     for (int r = 0; r <= PD; r++) {
-        lfin[r] = (valid && rep[r] >= 0) ? (u16)(seg[r] + lidx_s[rep[r]]) : (u16)0;   // the representative has the same remainder
+        lfin[r] = valid ? (u16)(seg[r] + lidx_s[get_rep(r)]) : (u16)0;   // the representative has the same remainder
         rec_tile[r * TP + tid] = lfin[r];
     }
     // The tile's splats sorted by entry (what the splat stage walks): a counting sort whose first half,
@@ -203,10 +394,10 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     if constexpr (!SORTED) let_next_kernel_start();   // what is left of this tile: its keys
     const int base = base_s;
     if (valid && base >= 0) {
-#pragma unroll
+#pragma unroll (COMPACT ? 1 : PD + 1)
         for (int r = 0; r <= PD; r++) {
             const int me = r * TP + tid;
-            if (rep[r] == me) list_keys[(size_t)base + lfin[r]] = keys_s[me];
+            if (get_rep(r) == me) list_keys[(size_t)base + (seg[r] + lidx_s[me])] = keys.global_key(me, r, item);
         }
     }
     if constexpr (SORTED && !is_double<R>::value) {
@@ -262,14 +453,44 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 }
 
 // ---------------------------------------------------------------------------------------------
-// clear_table: table capacity = power of two >= 2 * entries (at least 1024), chosen on the device.
+// clear_table: table capacity chosen on the device, a power of two: at least twice the entries (at least 1024),
+// or, where the call kept a sketch of the lattice's size, at least four times the vertices it tells of (twice
+// as many cost the probe chains of insert_entries more than the smaller table gained it).
 // ---------------------------------------------------------------------------------------------
-__global__ void clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2) {
+__global__ void __launch_bounds__(256)
+clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift) {
     after_previous_kernel();
     if (hdr->status != 0) return;
-    u32 need = 2u * hdr->num_entries;
+    __shared__ u32 bits_s[8];
+    u64 need = 2ull * hdr->num_entries;
+    if (sketch_shift >= 0 && need > (1ull << (sketch_shift + 10))) {
+        const uint4* sketch = reinterpret_cast<const uint4*>(hdr + 1);
+        u32 bits = 0;
+#pragma unroll
+        for (int i = 0; i < SKETCH_WORDS / 4 / 256; i++) {
+            const uint4 v = sketch[i * 256 + threadIdx.x];
+            bits += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+        }
+        bits = __reduce_add_sync(0xFFFFFFFFu, bits);
+        if ((threadIdx.x & 31) == 0) bits_s[threadIdx.x >> 5] = bits;
+        __syncthreads();
+        u32 set = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) set += bits_s[i];
+        // Distinct sampled keys: -B ln(share of bits still clear).  With 2^10 or more of them the error of the
+        // estimate stays below 4 % (one standard deviation), far from the factor by which the table is larger;
+        // with fewer there are at most about 2^(shift + 10) vertices, for which the smallest table has room.
+        const u32 clear = (1u << SKETCH_LOG2) - set;
+        if (clear > (1u << SKETCH_LOG2) / 64) {
+            const float sampled = -(float)(1 << SKETCH_LOG2) * logf((float)clear * (1.f / (1 << SKETCH_LOG2)));
+            u64 slots = (u64)(4.f * sampled * (float)(1u << sketch_shift));
+            const u64 least = 1ull << (sketch_shift + 11);
+            slots = slots < least ? least : slots;
+            need = slots < need ? slots : need;
+        }
+    }
     u32 lg = 10;
-    while (lg < max_log2 && (1ull << lg) < (u64)need) lg++;
+    while (lg < max_log2 && (1ull << lg) < need) lg++;
     if (blockIdx.x == 0 && threadIdx.x == 0) hdr->table_log2 = lg;
     const u64 cap = 1ull << lg;
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (u64)gridDim.x * blockDim.x)
@@ -333,9 +554,9 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
         const u32 t = rd.t[i], v = base + i;
         vid[t] = v;
         vkeys[v] = list_keys[t];
-        __threadfence();              // the key is visible before the slot says "vertex v"
-        relabel(rd.slot[i], v);
     }
+    if (tot) __threadfence();   // a key is visible before its slot says "vertex v"
+    for (u32 i = threadIdx.x; i < tot; i += 256) relabel(rd.slot[i], base + i);
     if (tot) {
         int2* nb = reinterpret_cast<int2*>(vi.nbr);
         for (int a = 0; a <= vi.pd; a++)
@@ -351,35 +572,9 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
     __syncthreads();
 }
 
-// Looks key `k` up in the table.  A slot holds (32-bit hash tag, index): the index of the vertex once its
-// creator's round has ended (VERTEX_FLAG set; full key in vkeys), before that the index of the entry that
-// created it (full key in list_keys, which the previous launch has completely written).  Returns the low
-// word of the matching slot, or 0xFFFFFFFF and the first empty slot met in `empty_slot` (~0 if the
-// table is full).
-template <int KW>
-__device__ __forceinline__ u32 table_probe(const u64* __restrict__ table, u64 mask,
-                                           const Key<KW>* __restrict__ list_keys,
-                                           const Key<KW>* __restrict__ vkeys, const Key<KW>& k, u64 h,
-                                           u64& empty_slot) {
-    const u32 tag = (u32)(h >> 32);
-    u64 s = h & mask;
-    for (u64 it = 0; it <= mask; it++) {
-        const u64 cur = table[s];
-        if (cur == EMPTY_SLOT) {
-            empty_slot = s;
-            return 0xFFFFFFFFu;
-        }
-        if ((u32)(cur >> 32) == tag) {
-            const u32 low = (u32)cur;
-            const Key<KW>& other = (low & VERTEX_FLAG) ? vkeys[low & ~VERTEX_FLAG] : list_keys[low];
-            if (key_equal<KW>(other, k)) return low;
-        }
-        s = (s + 1) & mask;
-    }
-    empty_slot = ~0ull;
-    return 0xFFFFFFFFu;
-}
-
+// A table slot holds (32-bit hash tag, index): the index of the vertex once its creator's round has ended
+// (VERTEX_FLAG set; full key in vkeys), before that the index of the entry that created it (full key in
+// list_keys, which the previous launch has completely written).
 template <int KW>
 __global__ void __launch_bounds__(256)
 insert_entries(Header* hdr, u64* __restrict__ table, const Key<KW>* __restrict__ list_keys,
@@ -428,7 +623,7 @@ insert_entries(Header* hdr, u64* __restrict__ table, const Key<KW>* __restrict__
             round_add_winner(rd, winner, t, (u32)my_slot);
         }
         finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 v) {
-            table[slot] = (__ldcg(&table[slot]) & 0xFFFFFFFF00000000ull) | (u64)(VERTEX_FLAG | v);
+            reinterpret_cast<u32*>(table)[2 * (u64)slot] = VERTEX_FLAG | v;   // the low word: the tag stays
         });
     }
 }
@@ -438,7 +633,7 @@ insert_entries(Header* hdr, u64* __restrict__ table, const Key<KW>* __restrict__
 __device__ __forceinline__ void resolve_entries(const Header* hdr, u32* __restrict__ list_ref,
                                                 const u32* __restrict__ vid) {
     const u32 T = hdr->num_entries;
-    for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < T; t += (u64)gridDim.x * blockDim.x) {
+    for (u64 t = grid_thread(); t < T; t += grid_threads()) {
         const u32 ref = list_ref[t];
         list_ref[t] = (ref & VERTEX_FLAG) ? (ref & ~VERTEX_FLAG) : vid[ref];
     }
@@ -451,17 +646,67 @@ __device__ __forceinline__ void resolve_entries(const Header* hdr, u32* __restri
 // One table lookup per (vertex v, axis a): the neighbour u whose key is v's key with every stored
 // coordinate +1, except coordinate a which moves by -PD (along axis PD no stored coordinate is
 // special; src/PermutohedralLatticeCPU.h:381-388).  Then u is v's "+" neighbour and v is u's "-"
-// neighbour, so the second lookup of the reference is not needed.  Keys are read in vertex order
-// (coalesced); every slot carries a vertex index by now, so a lookup is two dependent accesses.
+// neighbour, so the second lookup of the reference is not needed.
+// One thread per (vertex, axis), axis = blockIdx.y: neighbouring threads take neighbouring vertices of one axis,
+// so their key loads and their own slots of the neighbour table are contiguous.  The neighbour's key and the
+// linear part of its hash differ from the vertex's by constants of the axis.  Every slot carries a vertex index by
+// now, so a lookup is two dependent accesses, and one where there is no neighbour.  (One thread for all axes of a
+// vertex, its first probes in flight together, took up to twice as long: its key comparisons wait for one another.)
+template <int PD>
+__host__ __device__ constexpr u64 axis_word(int a, int j) {   // what moving along axis a adds to key word j
+    return coord_ones<PD>(j) - ((a < PD && (a >> 2) == j) ? (u64)(PD + 1) << (16 * (a & 3)) : 0ull);
+}
+template <int PD>
+__host__ __device__ constexpr u64 axis_hash(int a) {          // and to its linear hash
+    u64 h = 0;
+    for (int j = 0; j < Cfg<PD>::KW; j++) h += axis_word<PD>(a, j) * hash_factor(j);
+    return h;
+}
+template <int PD, int A>
+__device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mask,
+                                          const Key<Cfg<PD>::KW>* __restrict__ vkeys, u32 M, int* __restrict__ nbr,
+                                          u64 max_entries) {
+    constexpr int KW = Cfg<PD>::KW;
+    int* __restrict__ nbr_axis = nbr + 2 * (u64)A * max_entries;
+    for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < M; v += gridDim.x * blockDim.x) {
+        Key<KW> k = vkeys[v];
+        const u64 h = mix_hash(linear_hash<KW>(k) + axis_hash<PD>(A));
+#pragma unroll
+        for (int j = 0; j < KW; j++) k.w[j] += axis_word<PD>(A, j);
+        u64 s = h & mask;
+        for (u64 it = 0; it <= mask; it++) {
+            const u64 cur = table[s];
+            if (cur == EMPTY_SLOT) break;
+            if ((u32)(cur >> 32) == (u32)(h >> 32)) {
+                const u32 u = (u32)cur & ~VERTEX_FLAG;
+                if (key_equal<KW>(vkeys[u], k)) {
+                    nbr_axis[2 * (u64)v] = (int)u;
+                    nbr_axis[2 * (u64)u + 1] = (int)v;
+                    break;
+                }
+            }
+            s = (s + 1) & mask;
+        }
+    }
+}
+template <int PD, int A>
+struct LinkAxis {   // link_axis of the axis this block works on, chosen once per block
+    template <typename... Args>
+    __device__ static __forceinline__ void run(int axis, Args... args) {
+        if (axis == A)
+            link_axis<PD, A>(args...);
+        else if constexpr (A < PD)
+            LinkAxis<PD, A + 1>::run(axis, args...);
+    }
+};
+
 template <int PD>
 __global__ void __launch_bounds__(256)
-link_neighbours(const Header* hdr, const u64* __restrict__ table,
-                const Key<Cfg<PD>::KW>* __restrict__ list_keys, u32* __restrict__ list_ref,
+link_neighbours(const Header* hdr, const u64* __restrict__ table, u32* __restrict__ list_ref,
                 const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys, int* __restrict__ nbr,
                 u64 max_entries, void* zero_rows_ptr, u32 zero_row_bytes, Watch watch) {
     after_previous_kernel();
     report_to(watch, hdr);
-    constexpr int KW = Cfg<PD>::KW;
     if (hdr->status != 0) return;
     resolve_entries(hdr, list_ref, vid);
     const u32 M = hdr->num_vertices;
@@ -469,31 +714,9 @@ link_neighbours(const Header* hdr, const u64* __restrict__ table,
     if (zero_rows_ptr) {   // streaming stores that overlap the latency of the lookups below
         uint4* rows = reinterpret_cast<uint4*>(zero_rows_ptr);
         const u64 quads = (u64)M * (zero_row_bytes / 16);
-        for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (u64)gridDim.x * blockDim.x)
-            rows[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (u64 i = grid_thread(); i < quads; i += grid_threads()) rows[i] = make_uint4(0u, 0u, 0u, 0u);
     }
-    const u64 items = (u64)M * (PD + 1);
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < items; e += (u64)gridDim.x * blockDim.x) {
-        // axis-major: neighbouring threads take neighbouring vertices of one axis, so their key loads and
-        // their own slots of the neighbour table are contiguous (vertex-major, where the threads of a vertex
-        // share one key load, measured slower at pd = 5 and at pd = 16)
-        const int a = (int)(e / M);
-        const u32 v = (u32)(e - (u64)a * M);
-        const Key<KW> k = vkeys[v];
-        Key<KW> nk;
-#pragma unroll
-        for (int j = 0; j < KW; j++) nk.w[j] = 0;
-#pragma unroll
-        for (int i = 0; i < PD; i++) key_set<KW>(nk, i, (u16)(key_get<KW>(k, i) + ((i == a) ? -PD : 1)));
-        key_set<KW>(nk, PD, key_get<KW>(k, PD));
-        u64 unused;
-        const u32 low = table_probe<KW>(table, mask, list_keys, vkeys, nk, hash_key<KW>(nk), unused);
-        if (low != 0xFFFFFFFFu) {
-            const u32 u = low & ~VERTEX_FLAG;
-            nbr[((u64)a * max_entries + v) * 2] = (int)u;
-            nbr[((u64)a * max_entries + u) * 2 + 1] = (int)v;
-        }
-    }
+    LinkAxis<PD, 0>::run((int)blockIdx.y, table, mask, vkeys, M, nbr, max_entries);
 }
 
 }  // namespace pl

@@ -156,6 +156,17 @@ enum { OV_BLUR = 1, OV_INSERT = 2, OV_SPLAT = 4, OV_BLUR0 = 8, OV_SLICE = 16, OV
 #define PL_LAUNCH_AFTER(which, kernel, grid, block, smem, st, ...) \
     PL_CUDA(launch_kernel((PL_OVERLAP & (which)) != 0, kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
 
+// The header and the sketch behind it.
+constexpr size_t HEADER_BYTES = sizeof(Header) + sizeof(u32) * SKETCH_WORDS;
+
+// Sampling of the sketch (see SKETCH_LOG2): so that a lattice of max_entries vertices sets about half its bits.
+static int sketch_shift_of(u64 max_entries) {
+    if (max_entries < SKETCH_MIN_ENTRIES) return -1;
+    int shift = 0;
+    while (shift < 20 && (max_entries >> shift) > (1ull << (SKETCH_LOG2 - 1))) shift++;
+    return shift;
+}
+
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static int tp_of(int pd) { return pd <= 8 ? 256 : 128; }
@@ -243,7 +254,7 @@ static int make_layout(Layout& L, const Geom& g, int pd, int vd, int64_t max_ent
     while (slots < 2 * E) slots <<= 1;
     L.table_slots = slots;
     const size_t tile_splats = (size_t)tp_of(pd) * (pd + 1);
-    size_t off = align_up(sizeof(Header));
+    size_t off = align_up(HEADER_BYTES);
     L.tile_info = off; off += align_up(sizeof(int2) * (size_t)g.num_tiles);
     L.rec = off;       off += align_up(sizeof(u16) * tile_splats * (size_t)g.num_tiles);
     L.rec_w = off;     off += align_up((size_t)real_bytes * tile_splats * (size_t)g.num_tiles);
@@ -334,6 +345,16 @@ static bool bulk_rows_ok(const Geom& g, const void* ptr, int channels) {
     const long long row_bytes = 4ll * channels;
     return ((uintptr_t)ptr % 16 == 0) && (row_bytes * g.W) % 16 == 0 && (row_bytes * g.TX) % 16 == 0 &&
            (row_bytes * g.n) % 16 == 0 && (row_bytes * g.TX * g.TY) < (1ll << 31);
+}
+
+// link_neighbours: a row of blocks for each lattice axis, long enough that the rows run one after the other on a
+// large lattice: threads then work on one axis of a stretch of vertices at a time, whose neighbours along that axis
+// lie close together too.  (All axes at once, in rows that fill the GPU together, measured 96 instead of 72 us on
+// the 16-image dense-CRF batch.)  On a small one, no more blocks than there can be vertices for.
+template <int PD>
+static dim3 link_grid(int wide, u64 max_entries) {
+    const u64 blocks = (max_entries + 511) / 512;
+    return dim3((unsigned)(blocks < (u64)wide ? blocks : (u64)wide), PD + 1, 1);
 }
 
 // splat / slice for value dimension vd: the instantiation with vd fixed at compile time where there
@@ -427,13 +448,14 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     float* v1 = reinterpret_cast<float*>(ws + L.v1);
     long long* v64 = (mode == PL_MODE_DETERMINISTIC) ? reinterpret_cast<long long*>(ws + L.v64) : nullptr;
 
+    const int sketch_shift = sketch_shift_of(L.max_entries);
     cudaEvent_t* ev = g_stage_events;
     g_stage_events = nullptr;
     if (ev) PL_CUDA(cudaEventRecord(ev[0], st));
-    if (phases & PH_BUILD) PL_CUDA(cudaMemsetAsync(hdr, 0, sizeof(Header), st));
+    if (phases & PH_BUILD) PL_CUDA(cudaMemsetAsync(hdr, 0, sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header), st));
     if (g.num_tiles == 0) return PL_OK;
 
-    PL_TRY((ensure_dynamic_smem<build_tiles<PD, float>>(Cfg<PD>::BUILD_SMEM)));
+    PL_TRY((ensure_dynamic_smem<build_tiles<PD, float>>(Cfg<PD>::build_smem(false))));
     const int sms = num_sms();
     const int wide = sms * 8;
     int table_log2 = 0;
@@ -445,12 +467,12 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     if (phases & PH_BUILD) {
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
         if (phases & PH_APPLY) {
-            PL_LAUNCH((build_tiles<PD, float, false>), tile_grid(g), TP, Cfg<PD>::BUILD_SMEM, st, g, positions, reference, hdr,
-                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries);
+            PL_LAUNCH((build_tiles<PD, float, false>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr,
+                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         } else {
-            PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, true>>(Cfg<PD>::BUILD_SMEM)));
-            PL_LAUNCH((build_tiles<PD, float, true>), tile_grid(g), TP, Cfg<PD>::BUILD_SMEM, st, g, positions, reference, hdr,
-                                                                        tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries);
+            PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, true>>(Cfg<PD>::build_smem(true))));
+            PL_LAUNCH((build_tiles<PD, float, true>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
+                                                                        tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         }
         PL_COUNT_LAUNCHES(4);   // build_tiles and the three launches of the index stage below
         if (ev) PL_CUDA(cudaEventRecord(ev[1], st));
@@ -480,9 +502,9 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             vinit.rows = nullptr;
             // (behind the build that also sorts the splats the overlap measured slower: 1.66 against 1.61 ms for
             // a build and two applies)
-            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2);
+            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, vinit);
-            PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, nbr,
+            PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, list_ref, vid, vkeys, nbr,
                                                       L.max_entries, zrows, vinit.row_bytes, take_watch());
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[2], st));
@@ -549,16 +571,17 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* v0 = reinterpret_cast<double*>(ws + L.v0);
     double* v1 = reinterpret_cast<double*>(ws + L.v1);
 
-    PL_CUDA(cudaMemsetAsync(hdr, 0, sizeof(Header), st));
+    const int sketch_shift = sketch_shift_of(L.max_entries);
+    PL_CUDA(cudaMemsetAsync(hdr, 0, sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header), st));
     if (g.num_tiles == 0) return PL_OK;
-    PL_TRY((ensure_dynamic_smem<build_tiles<PD, double>>(Cfg<PD>::BUILD_SMEM)));
+    PL_TRY((ensure_dynamic_smem<build_tiles<PD, double>>(Cfg<PD>::build_smem(false))));
     PL_TRY((ensure_dynamic_smem<splat_tiles_f64<PD>>(Splat64<PD>::BYTES)));
     const int wide = num_sms() * 8;
     int table_log2 = 0;
     while ((1ull << table_log2) < L.table_slots) table_log2++;
     const int vp = padded_vd_f64(vd);
 
-    PL_LAUNCH((build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::BUILD_SMEM, st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries);
+    PL_LAUNCH((build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
     // spatial-only calls index their vertices directly, as the float calls do (the key bounds hold for
     // either arithmetic: the margin is far wider than any rounding)
     Direct direct;
@@ -580,9 +603,9 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         }
     }
     if (!use_direct) {
-        PL_LAUNCH((clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2);
+        PL_LAUNCH((clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         PL_LAUNCH((insert_entries<KW>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, vinit);
-        PL_LAUNCH((link_neighbours<PD>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, nbr, L.max_entries,
+        PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   nullptr, 0u, take_watch());
     }
     PL_LAUNCH((splat_tiles_f64<PD>), tile_grid(g), TP, Splat64<PD>::BYTES, st, g, input, hdr, tile_info, rec, rec_w,
@@ -1013,8 +1036,8 @@ int pl_export_lattice_f64(const void* workspace, const double* positions, const 
 #ifdef PL_PHASE_CLOCKS
 // Developer aid: resident CTAs per SM of the config-2 tile kernels, as the runtime computes them.
 int pl_debug_occupancy(int* out) {
-    PL_CUDA(cudaFuncSetAttribute(build_tiles<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<5>::BUILD_SMEM));
-    PL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out[0], build_tiles<5>, 256, Cfg<5>::BUILD_SMEM));
+    PL_CUDA(cudaFuncSetAttribute(build_tiles<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<5>::build_smem(false)));
+    PL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out[0], build_tiles<5>, 256, Cfg<5>::build_smem(false)));
     const size_t ss = SplatRows<5, 22, false>::BYTES;
     PL_CUDA(cudaFuncSetAttribute(splat_tiles_rows<5, 22, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ss));
     PL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out[1], splat_tiles_rows<5, 22, false>, 256, ss));
@@ -1022,7 +1045,7 @@ int pl_debug_occupancy(int* out) {
     const size_t sl = SliceFast<5, 22>::bytes(rows_cap);
     PL_CUDA(cudaFuncSetAttribute(slice_tiles_fast<5, 22>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl));
     PL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out[2], slice_tiles_fast<5, 22>, 256, sl));
-    out[3] = (int)Cfg<5>::BUILD_SMEM; out[4] = (int)ss; out[5] = (int)sl;
+    out[3] = (int)Cfg<5>::build_smem(false); out[4] = (int)ss; out[5] = (int)sl;
     cudaFuncAttributes fa;
     PL_CUDA(cudaFuncGetAttributes(&fa, splat_tiles_rows<5, 22, false>));
     out[6] = fa.numRegs; out[7] = (int)fa.sharedSizeBytes;

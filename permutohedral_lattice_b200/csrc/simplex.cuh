@@ -10,11 +10,14 @@
 // Compiles for the host too (PL_HD), so the arithmetic can be checked without a GPU.
 #pragma once
 #include <stdint.h>
+#include <utility>
 
 #ifdef __CUDACC__
 #define PL_HD __host__ __device__ __forceinline__
+#define PL_CX __host__ __device__ constexpr
 #else
 #define PL_HD inline
+#define PL_CX constexpr
 #endif
 
 #ifdef __CUDA_ARCH__
@@ -65,11 +68,71 @@ PL_HD float div_by_rcp(float a, float b, float rcp_b) {
 
 template <int PD>
 struct Simplex {
-    int rem0[PD + 1];  // nearest remainder-0 lattice point, per coordinate (multiple of PD+1)
     int rank[PD + 1];  // rank of each coordinate's residual, 0..PD
     float el[PD + 1];  // elevated position
-    float rem0f[PD + 1];  // rem0 as float
+    float rem0f[PD + 1];  // nearest remainder-0 lattice point, per coordinate (multiple of PD+1), as float
 };
+
+// Coordinate i of the remainder-0 point: as an integer, and as a word whose low 16 bits are that integer's (the
+// low mantissa bits of the float plus the rounding constant: no subtraction, no conversion).
+template <int PD>
+PL_HD int rem0_of(const Simplex<PD>& s, int i) { return exact_int(s.rem0f[i]); }
+template <int PD>
+PL_HD unsigned rem0_low16(const Simplex<PD>& s, int i) {
+    return (unsigned)PL_F2BITS(PL_FADD(s.rem0f[i], PL_ROUND_MAGIC));
+}
+
+// Smaller and larger of two floats; a NaN on either side gives NaN twice.
+PL_HD void sort_two(float& hi, float& lo) {
+#ifdef __CUDA_ARCH__
+    float a, b;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(a) : "f"(hi), "f"(lo));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(b) : "f"(hi), "f"(lo));
+    hi = a;
+    lo = b;
+#else
+    if (!(hi >= lo)) {
+        const float t = hi;
+        hi = lo;
+        lo = t;
+    }
+#endif
+}
+
+// Sorting network (Batcher's odd-even merge sort) for N values, cut down from the next power of two by leaving
+// out the comparators that reach beyond N.  Comparator number C as (smaller index, larger index).
+struct NetPair { int a, b; };
+PL_CX int net_size(int N, int C, NetPair* out) {   // number of comparators; *out <- the C-th
+    int P = 1, count = 0;
+    while (P < N) P *= 2;
+    for (int p = 1; p < P; p *= 2)
+        for (int k = p; k >= 1; k /= 2)
+            for (int j = k % p; j <= P - 1 - k; j += 2 * k)
+                for (int i = 0; i < k && i < P - j - k; i++)
+                    if ((i + j) / (2 * p) == (i + j + k) / (2 * p) && i + j + k < N) {
+                        if (out && count == C) { out->a = i + j; out->b = i + j + k; }
+                        count++;
+                    }
+    return count;
+}
+template <int N, int C>
+struct NetStep {
+    static PL_CX NetPair get() {
+        NetPair p = {0, 0};
+        net_size(N, C, &p);
+        return p;
+    }
+    static constexpr int a = get().a, b = get().b;
+};
+template <int N, int... C>
+PL_HD void run_network(float* v, std::integer_sequence<int, C...>) {
+    (sort_two(v[NetStep<N, C>::a], v[NetStep<N, C>::b]), ...);
+}
+template <int N>
+PL_HD void sort_descending(float* v) {
+    constexpr int COUNT = net_size(N, -1, nullptr);
+    run_network<N>(v, std::make_integer_sequence<int, COUNT>());
+}
 
 // src/PermutohedralLatticeCPU.h:220-273 (embed_position_vector, find_enclosing_simplex).
 // scale[i] must be the host-computed factors of compute_scale_factor (:194-217).
@@ -90,7 +153,7 @@ PL_HD void find_simplex(const float* pos, const float* scale, Simplex<PD>& s) {
     // up = down + PD + 1; when it is, both candidate pairs contain the same winner with a margin of
     // a whole cell, so the choice below is identical in every case.  floor() by the add-magic trick.
     const float inv_f = 1.0f / (float)(PD + 1);
-    int sum = 0;
+    float cells = 0.f;   // sum of the coordinates' cell numbers: small integers, exact
 #pragma unroll
     for (int i = 0; i <= PD; i++) {
         const float v = PL_FMUL(s.el[i], inv_f);
@@ -98,17 +161,19 @@ PL_HD void find_simplex(const float* pos, const float* scale, Simplex<PD>& s) {
         fl = (fl > v) ? PL_FSUB(fl, 1.0f) : fl;                          // -> floor
         const float down = PL_FMUL(fl, (float)(PD + 1));                 // exact: small integers
         const float up = PL_FADD(down, (float)(PD + 1));
-        s.rem0f[i] = (PL_FSUB(up, s.el[i]) < PL_FSUB(s.el[i], down)) ? up : down;
-        s.rem0[i] = exact_int(s.rem0f[i]);
-        sum += s.rem0[i];
+        const bool take_up = PL_FSUB(up, s.el[i]) < PL_FSUB(s.el[i], down);
+        s.rem0f[i] = take_up ? up : down;
+        cells = PL_FADD(cells, take_up ? PL_FADD(fl, 1.0f) : fl);
     }
-    sum /= (PD + 1);
+    const int sum = exact_int(cells);
 
+    // Rank of a residual: how many of the others are larger, equal ones in index order.  rank[j] starts as if
+    // all earlier ones were.
     float d[PD + 1];
 #pragma unroll
     for (int i = 0; i <= PD; i++) {
         d[i] = PL_FSUB(s.el[i], s.rem0f[i]);
-        s.rank[i] = 0;
+        s.rank[i] = i + sum;
     }
 #pragma unroll
     for (int i = 0; i < PD; i++) {
@@ -116,27 +181,26 @@ PL_HD void find_simplex(const float* pos, const float* scale, Simplex<PD>& s) {
         for (int j = i + 1; j <= PD; j++) {
             const int lt = d[i] < d[j] ? 1 : 0;   // arithmetic on the predicate: no branches
             s.rank[i] += lt;
-            s.rank[j] += 1 - lt;
+            s.rank[j] -= lt;
         }
     }
 #pragma unroll
     for (int i = 0; i <= PD; i++) {
-        s.rank[i] += sum;
         // wrap into 0..PD: +1 cell when below, -1 cell when above (selects, no branches)
-        const int wrap = (s.rank[i] < 0 ? 1 : 0) - (s.rank[i] > PD ? 1 : 0);
-        s.rank[i] += wrap * (PD + 1);
-        s.rem0[i] += wrap * (PD + 1);
-        s.rem0f[i] = (wrap > 0)   ? PL_FADD(s.rem0f[i], (float)(PD + 1))
-                     : (wrap < 0) ? PL_FSUB(s.rem0f[i], (float)(PD + 1))
-                                  : s.rem0f[i];
+        const bool below = s.rank[i] < 0, above = s.rank[i] > PD;
+        s.rank[i] += below ? PD + 1 : above ? -(PD + 1) : 0;
+        s.rem0f[i] = PL_FADD(s.rem0f[i], below ? (float)(PD + 1) : above ? -(float)(PD + 1) : 0.f);
     }
 }
 
 // Barycentric weights, one per remainder (src/PermutohedralLatticeCPU.h:275-286).  The reference
 // scatters +delta_i to slot pd-rank_i and -delta_i to slot pd-rank_i+1 of a zeroed array; each
 // slot k in 1..pd thus ends as fl(delta[rank = pd-k] - delta[rank = pd-k+1]) whatever the order,
-// slot pd+1 as -delta[rank = 0], and slot 0 gets the wrap-around in double.  Written here without
-// data-dependent array indexing.
+// slot pd+1 as -delta[rank = 0], and slot 0 gets the wrap-around in double.
+// The residuals by rank are the residuals in descending order: the rank counts the larger ones, and the wrap
+// moves the residuals it takes a whole cell down (up), below (above) all others, as it moves their ranks.  So
+// they are sorted by a network of two instructions a comparator (12 comparators at pd = 5) instead of being
+// picked by rank, which took 2 (pd + 1)^2.
 template <int PD>
 PL_HD void barycentric(const Simplex<PD>& s, float* bary /* PD+1 */) {
     // delta_i = (el_i - rem0_i) / (PD+1): the reference multiplies by the double 1/(PD+1) and rounds
@@ -147,15 +211,14 @@ PL_HD void barycentric(const Simplex<PD>& s, float* bary /* PD+1 */) {
     const float cl = (float)(c - (double)ch);
     float by_rank[PD + 1];
 #pragma unroll
-    for (int q = 0; q <= PD; q++) by_rank[q] = 0.f;
+    for (int i = 0; i <= PD; i++) by_rank[i] = PL_FSUB(s.el[i], s.rem0f[i]);
+    sort_descending<PD + 1>(by_rank);
 #pragma unroll
     for (int i = 0; i <= PD; i++) {
-        const float d = PL_FSUB(s.el[i], s.rem0f[i]);
+        const float d = by_rank[i];
         const float p = PL_FMUL(d, ch);
         const float e = PL_FMA(d, ch, -p);             // exact error of p
-        const float delta = PL_FADD(p, PL_FMA(d, cl, e));
-#pragma unroll
-        for (int q = 0; q <= PD; q++) by_rank[q] = (s.rank[i] == q) ? delta : by_rank[q];   // select, not branch
+        by_rank[i] = PL_FADD(p, PL_FMA(d, cl, e));
     }
 #pragma unroll
     for (int k = 1; k <= PD; k++) bary[k] = PL_FSUB(by_rank[PD - k], by_rank[PD - k + 1]);
@@ -165,7 +228,7 @@ PL_HD void barycentric(const Simplex<PD>& s, float* bary /* PD+1 */) {
 // Coordinate i (< PD) of the remainder-r vertex of the simplex (src/PermutohedralLatticeCPU.h:297-304).
 template <int PD>
 PL_HD int16_t vertex_coord(const Simplex<PD>& s, int i, int r) {
-    const int k = s.rem0[i] + r - ((s.rank[i] > PD - r) ? PD + 1 : 0);
+    const int k = rem0_of(s, i) + r - ((s.rank[i] > PD - r) ? PD + 1 : 0);
     return (int16_t)k;
 }
 
@@ -181,6 +244,9 @@ struct Simplex64 {
     int rank[PD + 1];
     double el[PD + 1];
 };
+
+template <int PD>
+PL_HD unsigned rem0_low16(const Simplex64<PD>& s, int i) { return (unsigned)s.rem0[i]; }
 
 template <int PD>
 PL_HD void find_simplex_f64(const double* pos, const double* scale, Simplex64<PD>& s) {
