@@ -8,6 +8,7 @@ device memory and streams only, every computation happens in libpl_lattice.so th
 import ctypes
 
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from . import capi
 
@@ -34,7 +35,7 @@ def release_workspaces():
 # `max_entries`; the bound that can never overflow, batch * points * (pd + 1), is 1.5 to 40 times what the
 # benchmark configurations use.  So by default (max_entries=None) a call is sized from what the lattice needs:
 #   * a call whose reference image (or positions) is the tensor a VERIFIED call of the same kind just used
-#     - same memory, same version counter, same shape: a layer's backward call, the next iteration on the same
+#     - same storage, same version counter, same view: a layer's backward call, the next iteration on the same
 #     image - builds the same lattice, so it runs with that call's bound and nothing needs checking;
 #   * any other call is VERIFIED: it runs with 1.5 x the largest entry count per item seen for its kind (a
 #     quarter of the worst case the first time), its counters are awaited, and the call is repeated with four
@@ -48,7 +49,7 @@ def release_workspaces():
 # max_entries=0 asks for the worst case (never overflows, never synchronises), max_entries > 0 for that bound.
 # ---------------------------------------------------------------------------------------------------
 _entries_per_item = {}   # kind of call -> largest num_entries / batch seen
-_verified = {}           # kind of call -> (identity of the reference it ran on, the bound that sufficed)
+_verified = {}           # kind of call -> (identity of the reference it ran on, the bound that sufficed, weak reference)
 _pending = {}            # kind of call -> list of (event, pinned int32[3] = entries, vertices, status bits, bound, batch)
 _pinned_words = []       # pinned int32[3] buffers waiting to be used again (allocating pinned memory is slow)
 FIRST_GUESS_DIVISOR = 4
@@ -60,11 +61,13 @@ def _kind(device, call, from_positions=False):
 
 
 def _identity(t, batch):
-    """What makes two calls build the same lattice, as far as the host can tell: the same tensor (memory,
-    shape) that no torch operation has written to in between (version counter)."""
+    """What makes two calls build the same lattice, as far as the host can tell: the same view of the same storage
+    object that no torch operation has written to in between (version counter).  The storage object and not its
+    memory: a new tensor often gets the memory of one that is gone.  Its address stands for the object as long as
+    somebody holds a reference to it, which _run_sized does, a weak one that keeps no memory alive."""
     if t is None:
         return ("grid", batch)
-    return (t.data_ptr(), t._version, tuple(t.shape), t.dtype)
+    return (t.untyped_storage()._cdata, t.data_ptr(), t._version, tuple(t.shape), t.stride(), t.dtype)
 
 
 def _status_code(bits):
@@ -144,14 +147,16 @@ def _note_call(kind, ws, bound, batch, device):
     _pending.setdefault(kind, []).append((ev, host, bound, batch))
 
 
-def _run_sized(kind, identity, batch, worst, device, stream, launch, verify="auto", floor=0):
-    """Runs launch(max_entries) -> workspace under the default sizing policy.  Returns (workspace, max_entries)."""
+def _run_sized(kind, tensor, batch, worst, device, stream, launch, verify="auto", floor=0):
+    """Runs launch(max_entries) -> workspace under the default sizing policy.  Returns (workspace, max_entries).
+    tensor: what the lattice is built from, a reference image or positions (None: from the grid alone)."""
     if verify == "deferred":
         max_entries = _guess_bound(kind, batch, worst, floor)
         ws = launch(max_entries)
         if max_entries:
             _note_call(kind, ws, max_entries, batch, device)
         return ws, max_entries
+    identity = _identity(tensor, batch)
     known = _verified.get(kind)
     if known is not None and known[0] == identity:
         return launch(known[1]), known[1]          # the same lattice as a call that fitted this bound
@@ -177,7 +182,7 @@ def _run_sized(kind, identity, batch, worst, device, stream, launch, verify="aut
         # (after a repeat at the worst case too: what the lattice needed is worth knowing for the next call)
         _entries_per_item[kind] = max(_entries_per_item.get(kind, 0.0), entries.value / max(batch, 1))
         break
-    _verified[kind] = (identity, max_entries)
+    _verified[kind] = (identity, max_entries, None if tensor is None else StorageWeakRef(tensor.untyped_storage()))
     return ws, max_entries
 
 
@@ -348,7 +353,7 @@ def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha
 
     with _OnDevice(x.device):
         if max_entries is None and workspace is None:
-            ws, max_entries = _run_sized(plan.kind, _identity(reference_image if bilateral else None, call.batch),
+            ws, max_entries = _run_sized(plan.kind, reference_image if bilateral else None,
                                          call.batch, plan.worst, x.device, stream, launch, verify=verify,
                                          floor=plan.floor)
         else:
@@ -432,7 +437,7 @@ class Lattice:
                 worst = call.batch * call.n * (call.pd + 1)
                 # verified like a filter call: once per reference image, not again for a lattice rebuilt on it
                 self.workspace, self.max_entries = _run_sized(
-                    ("Lattice",) + _kind(device, call), _identity(reference_image if bilateral else None, call.batch),
+                    ("Lattice",) + _kind(device, call), reference_image if bilateral else None,
                     call.batch, worst, device, stream, build, floor=_direct_index_floor(call))
             else:
                 self.workspace = build(self.max_entries)
@@ -606,7 +611,7 @@ def filter_positions(input_values, positions, reverse=False, mode="atomic", max_
         with _OnDevice(x.device):
             if max_entries is None and workspace is None:
                 kind = (x.device.index, "positions", n, pd)
-                ws, max_entries = _run_sized(kind, _identity(positions, batch), batch, batch * n * (pd + 1), x.device,
+                ws, max_entries = _run_sized(kind, positions, batch, batch * n * (pd + 1), x.device,
                                              stream, launch)
             else:
                 max_entries = int(max_entries or 0)

@@ -99,6 +99,28 @@ def test_new_reference_is_verified_even_when_earlier_data_needed_far_less(policy
     assert np.array_equal(bits(out3.cpu().numpy()), bits(want3.cpu().numpy()))
 
 
+def test_new_tensor_in_the_memory_of_an_old_one_is_verified(policy):
+    """A reference image that got the memory, shape and version counter of one that is gone is another image."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from conftest import bits
+    x, ref = _data(3, blocky=False)
+    want, _, _ = plb.lattice_filter_raw(x, ref, mode="deterministic", max_entries=0, **KW)
+    flat = ref.new_empty(ref.shape)
+    flat.data.fill_(0.5)
+    where, version = flat.data_ptr(), flat._version
+    plb.lattice_filter_raw(x, flat, mode="deterministic", **KW)
+    del flat
+    again = ref.new_empty(ref.shape)
+    assert again.data_ptr() == where and again._version == version, "the allocator gave other memory: nothing tested"
+    again.data.copy_(ref)      # without the version counter, as a fresh upload would be
+    policy._entries_per_item.clear()
+    kind_before = dict(policy._verified)
+    out, _, _ = plb.lattice_filter_raw(x, again, mode="deterministic", **KW)
+    assert policy._verified != kind_before
+    assert np.array_equal(bits(out.cpu().numpy()), bits(want.cpu().numpy()))
+
+
 def test_deferred_call_that_does_not_fit_is_reported_and_succeeds_when_repeated(policy):
     import torch
     import permutohedral_lattice_b200 as plb
