@@ -1,0 +1,99 @@
+"""Lattice construction where its paths part: a hash table sized by a sketch of the vertices or by the entries, tiles
+whose keys are all distinct (several rounds of de-duplication) or all equal, verified calls from several threads.
+The structure is compared exactly."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device")
+    import gpu_helpers
+    return gpu_helpers
+
+
+@pytest.mark.parametrize("guide,theta", [("flat", (30.0, 0.2)), ("cells", (8.0, 0.1)), ("noise", (0.3, 0.01))])
+@pytest.mark.parametrize("size", [(128, 160), (256, 192)])
+def test_table_has_room_for_the_lattice(guide, theta, size, gpu, oracle):
+    """2 x 128 x 160 points x 6 lie below the size at which a sketch is kept, 2 x 256 x 192 x 6 above."""
+    rng = np.random.default_rng(53)
+    shape = (2,) + size
+    if guide == "flat":
+        ref = np.full(shape + (3,), 0.5, np.float32)
+    elif guide == "cells":
+        ref = np.kron(rng.random((2, size[0] // 16, size[1] // 16, 3)), np.ones((1, 16, 16, 1))).astype(np.float32)
+    else:
+        ref = rng.random(shape + (3,), dtype=np.float32)
+    inp = rng.random(shape + (1,), dtype=np.float32)
+    want, items = oracle.lattice_filter(inp, ref, True, *theta, 1.0, False, structure=True)
+    out, ws, call, _, rt = gpu.run_op(inp, ref, True, *theta, 1.0, False, max_entries=0)
+    st, (vk, vi, pv, pw) = gpu.export_op(ws, call, rt)
+    gpu.assert_structure_equal(vk, vi, pv, pw, items, guide)
+    gpu.assert_outputs_close(out.cpu().numpy(), want, guide)
+    assert st.table_slots >= 2 * st.num_vertices
+    # by vertices: four slots each, rounded up to a power of two (the sketch is 4 % off at most), or the smallest
+    # table that the sketch chooses; by entries: at least two slots an entry
+    assert st.table_slots <= max(4 * st.num_entries, 1024)
+    if size == (256, 192):
+        assert st.table_slots <= max(16 * st.num_vertices, 1 << 16)
+
+
+@pytest.mark.parametrize("pd", [1, 2, 3, 4, 5, 6, 7, 8, 16])
+@pytest.mark.parametrize("spread", [0.0, 1.0, 40.0])
+def test_tiles_of_equal_and_of_distinct_keys(pd, spread, gpu, oracle):
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(59)
+    n = 611
+    pos = (rng.standard_normal((2, n, pd)) * spread).astype(np.float32)
+    val = rng.random((2, n, 2), dtype=np.float32)
+    pt = torch.from_numpy(pos).cuda()
+    out, ws = plb.filter_positions(torch.from_numpy(val).cuda(), pt, max_entries=0)
+    st = plb.lattice_stats(ws)
+    vk, vi, pv, pw = plb.export_lattice(ws, st, 2, n, pd, 3, positions=pt)
+    items = [oracle.filter(val[i], pos[i]) for i in range(2)]
+    gpu.assert_structure_equal(vk, vi, pv, pw, items, "pd %d spread %g" % (pd, spread))
+    gpu.assert_outputs_close(out.cpu().numpy(), np.stack([o.out for o in items]), "pd %d spread %g" % (pd, spread))
+    # the rounds find every repeated key of a tile: as many entries as the tiles have distinct keys
+    tile = 128 if pd > 8 else 256
+    distinct = sum(len(set(map(bytes, items[i].pixel_keys()[a:a + tile].reshape(-1, pd))))
+                   for i in range(2) for a in range(0, n, tile))
+    assert st.num_entries == distinct
+
+
+def test_verified_calls_from_several_threads(gpu):
+    """Every thread's calls on new reference images wait for their own counters, on the thread's own stream."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(61)
+    refs = [torch.from_numpy(rng.random((1, 40 + 8 * i, 48, 3), dtype=np.float32)).cuda() for i in range(6)]
+    xs = [torch.rand(r.shape[:-1] + (2,), device="cuda") for r in refs]
+    want = [plb.lattice_filter_raw(x, r, True, 2.0, 0.05, mode="deterministic", max_entries=0)[0].clone()
+            for x, r in zip(xs, refs)]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(24):
+                    j = (i + k) % len(refs)
+                    got = plb.lattice_filter(xs[j], refs[j].clone(), True, 2.0, 0.05, mode="deterministic")
+                    torch.cuda.current_stream().synchronize()
+                    if not torch.equal(got, want[j]):
+                        wrong.append((k, j))
+        except Exception as e:   # noqa: BLE001 - reported below
+            wrong.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
