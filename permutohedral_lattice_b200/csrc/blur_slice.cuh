@@ -50,38 +50,42 @@ blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const float* __re
 // ascending order, reciprocal of the homogeneous channel in double, one multiply per channel).
 // The tile's vertex rows are staged once in shared memory.
 //
-// Fast form (VD known at compile time): one thread per point interpolates the whole row in
-// registers (float4 reads of the cached rows, row stride padded against bank conflicts), the
+// Fast form (rows of VP floats, VP known at compile time; up to 32): one thread per point interpolates the whole
+// row in registers (float4 reads of the cached rows, row stride padded against bank conflicts), the
 // output block is assembled in shared memory and leaves by bulk asynchronous copies when its rows
 // are 16-byte aligned.
 // Generic form (any vd): a group of lanes per point, one float4 of channels per lane.
 // ---------------------------------------------------------------------------------------------
-template <int PD, int VD>
+template <int PD, int VP>
 struct SliceFast {
-    static constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3;
+    static constexpr int TP = Cfg<PD>::TP;
     static constexpr int RS = VP + 4;   // words between cached rows: 16-byte aligned, spreads banks
-    static constexpr size_t OUT_BYTES = ((sizeof(float) * TP * C + 15) / 16) * 16;
-    // the output block reuses the space of the cached rows once every thread has read them
+    // the output block ([TP][C], C < VP) reuses the space of the cached rows once every thread has read them
     __host__ __device__ static size_t region(int rows_cap) {
-        const size_t rows = ((sizeof(float) * (size_t)rows_cap * RS + 15) / 16) * 16;
-        return rows > OUT_BYTES ? rows : OUT_BYTES;
+        const size_t rows = sizeof(float) * (size_t)rows_cap * RS, out = sizeof(float) * TP * VP;
+        return rows > out ? rows : out;
     }
     static size_t bytes(int rows_cap) { return region(rows_cap) + sizeof(int) * TP; }
+    // CTAs per SM asked of the compiler: what the row, the weights and the entry numbers of a point leave room for
+    static constexpr int NEED = VP + 2 * (PD + 1);
+    static constexpr int CTAS = TP != 256 ? (VP > 24 ? 6 : 8) : NEED <= 36 ? 5 : NEED <= 52 ? 4 : 3;
 };
 
-template <int PD, int VD>
-__global__ void __launch_bounds__(Cfg<PD>::TP, (Cfg<PD>::TP == 256) ? 5 : 8)
+// CT: the channels where they are fixed at compile time, else 0 (VP - 4 <= C < VP, a few registers more).
+template <int PD, int VP, int CT>
+__global__ void __launch_bounds__(Cfg<PD>::TP, SliceFast<PD, VP>::CTAS)
 slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const int2* __restrict__ tile_info,
                  const u16* __restrict__ rec, const float* __restrict__ rec_w,
-                 const u32* __restrict__ list_ref, const float* __restrict__ vsrc, int rows_cap, int bulk_ok) {
+                 const u32* __restrict__ list_ref, const float* __restrict__ vsrc, int channels, int rows_cap, int bulk_ok) {
     // Launched to overlap the tail of the last blur pass: the status word, the tile's range and the per-point
     // records are older than any blur pass and are fetched before the wait; the vertex rows after it.
-    constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, C = VD - 1, VP = (VD + 3) & ~3, QPR = VP / 4;
-    constexpr int RS = SliceFast<PD, VD>::RS;
+    const int C = CT ? CT : channels;
+    constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, QPR = VP / 4;
+    constexpr int RS = SliceFast<PD, VP>::RS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* rows_s = reinterpret_cast<float*>(smem_raw);                                         // [rows_cap][RS]
     float* out_s = reinterpret_cast<float*>(smem_raw);                                          // [TP][C], later
-    int* prow_s = reinterpret_cast<int*>(smem_raw + SliceFast<PD, VD>::region(rows_cap));       // [TP]
+    int* prow_s = reinterpret_cast<int*>(smem_raw + SliceFast<PD, VP>::region(rows_cap));       // [TP]
     if (call_failed(hdr)) {
         poison_tile_output(g, output, C);
         wait_for_previous_kernel();
@@ -169,9 +173,22 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     __syncthreads();   // every cached row has been read: the output block may overwrite them
     pc.mark();
     if (valid) {
-        const float inv = (float)(1.0 / (double)acc[C]);
+        const int last = C - (VP - 4);   // channels in the row's last quad; the next one is the homogeneous channel
+        const float norm = last == 0 ? acc[VP - 4] : last == 1 ? acc[VP - 3] : last == 2 ? acc[VP - 2] : acc[VP - 1];
+        const float inv = (float)(1.0 / (double)norm);
+        float* o = out_s + tid * C;
+        if (last == 0) {   // whole quads: rows a multiple of 16 bytes long would collide on banks as single floats
 #pragma unroll
-        for (int j = 0; j < C; j++) out_s[tid * C + j] = PL_FMUL(acc[j], inv);
+            for (int j = 0; j < VP - 4; j += 4)
+                *reinterpret_cast<float4*>(o + j) = make_float4(PL_FMUL(acc[j], inv), PL_FMUL(acc[j + 1], inv),
+                                                                PL_FMUL(acc[j + 2], inv), PL_FMUL(acc[j + 3], inv));
+        } else {
+#pragma unroll
+            for (int j = 0; j < VP - 4; j++) o[j] = PL_FMUL(acc[j], inv);
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+                if (j < last) o[VP - 4 + j] = PL_FMUL(acc[VP - 4 + j], inv);
+        }
     }
     if (bulk_ok) {
         fence_async_proxy();
@@ -186,10 +203,18 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
         pc.mark();
     } else {
         __syncthreads();
+        // element k = tid, tid + TP, ... is channel j of point p; (p, j) advance without a division
+        const int DP = TP / C, DJ = TP - DP * C;
+        int p = tid / C, j = tid - p * C;
         for (int k = tid; k < TP * C; k += TP) {
-            const int p = k / C, j = k - p * C;
             const int row = prow_s[p];
             if (row >= 0) output[(size_t)row * C + j] = out_s[k];
+            p += DP;
+            j += DJ;
+            if (j >= C) {
+                j -= C;
+                p++;
+            }
         }
     }
 }

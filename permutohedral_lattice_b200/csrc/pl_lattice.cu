@@ -338,6 +338,12 @@ static int rows_cap_for(int pd, int vd) {
     return cap;
 }
 
+// Widest row the splat stage takes: its tile's rows and twice its sorted list within 200 KB.
+static int widest_vd(int pd) {
+    const int tp = tp_of(pd);
+    return ((200 * 1024 - 16 * tp * (pd + 1) - 4 * tp) / (4 * tp)) & ~3;
+}
+
 // True when every contiguous run of a tile's points starts on a 16-byte boundary and has a size that is
 // a multiple of 16 bytes in a [points][channels] float array at `ptr`: then the tile's block can move
 // by bulk asynchronous copies.
@@ -357,32 +363,26 @@ static dim3 link_grid(int wide, u64 max_entries) {
     return dim3((unsigned)(blocks < (u64)wide ? blocks : (u64)wide), PD + 1, 1);
 }
 
-// splat / slice for value dimension vd: the instantiation with vd fixed at compile time where there
-// is one, else the generic one.
+// splat for value dimension VD, fixed at compile time, or (VD = 0) any other.
+// Rows of one float4 (VD <= 4) are summed by a thread each, wider ones by a group of lanes (splat.cuh).
 template <int PD, int VD, bool PRE>
 static int launch_splat_as(const Geom& g, const float* input, Header* hdr, const int2* tile_info, const u16* rec,
                            const float* rec_w, const uint2* srec, const u32* list_ref, float* v0, int vd,
                            cudaStream_t st) {
-    if constexpr (VD > 8 && VD <= 32) {   // wide rows: a quarter warp per window, conflict-free row reads
-        using SR = SplatRows<PD, VD, PRE>;
-        const size_t smem = SR::BYTES;
-        // five CTAs per SM need nearly all of the SM's shared memory: ask for the largest carve-out
-        PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, VD, PRE>>(smem, true)));
-        // bulk staging also needs 16-byte aligned landing zones inside the padded tile rows
-        const bool bulk = bulk_rows_ok(g, input, VD - 1) && g.TX <= 16 && (g.TX * (SR::VP - (VD - 1))) % 4 == 0;
-        PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_rows<PD, VD, PRE>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
-                                                                              srec, list_ref, v0, bulk ? 1 : 0);
-    } else if constexpr (VD > 0) {
+    if constexpr (VD > 0 && VD <= 4) {
         const size_t smem = SplatFast<PD, VD, PRE>::BYTES;
         PL_TRY((ensure_dynamic_smem<splat_tiles_fast<PD, VD, PRE>>(smem)));
         PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_fast<PD, VD, PRE>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                               srec, list_ref, v0, bulk_rows_ok(g, input, VD - 1) ? 1 : 0);
     } else {
-        const size_t smem = SplatGeneric<PD>::bytes(vd);
-        if (smem > 200 * 1024) return PL_UNSUPPORTED_DIMS;
-        PL_TRY((ensure_dynamic_smem<splat_tiles_generic<PD>>(smem)));
-        PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_generic<PD>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
-                                                                        list_ref, v0, vd);
+        const size_t smem = SplatRows<PD, VD, PRE>::bytes(vd);
+        if (vd > widest_vd(PD)) return PL_UNSUPPORTED_DIMS;
+        // five CTAs per SM need nearly all of the SM's shared memory: ask for the largest carve-out
+        PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, VD, PRE>>(smem, true)));
+        // bulk staging also needs 16-byte aligned landing zones inside the padded tile rows
+        const bool bulk = bulk_rows_ok(g, input, vd - 1) && g.TX <= 16 && (g.TX * (padded_vd(vd) - (vd - 1))) % 4 == 0;
+        PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_rows<PD, VD, PRE>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+                                                                              srec, list_ref, v0, vd, bulk ? 1 : 0);
     }
     return PL_OK;
 }
@@ -396,15 +396,16 @@ static int launch_splat(const Geom& g, const float* input, Header* hdr, const in
                      : launch_splat_as<PD, VD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v0, vd, st);
 }
 
-template <int PD, int VD>
+// slice for rows of VP floats (CT > 0: of CT channels), or (VP = 0) of more than 32.
+template <int PD, int VP, int CT = 0>
 static int launch_slice(const Geom& g, float* output, const Header* hdr, const int2* tile_info, const u16* rec,
                         const float* rec_w, const u32* list_ref, const float* vsrc, int vd, cudaStream_t st) {
-    if constexpr (VD > 0) {
-        int rows_cap = (40 * 1024) / (SliceFast<PD, VD>::RS * 4);
+    if constexpr (VP > 0) {
+        int rows_cap = (40 * 1024) / (SliceFast<PD, VP>::RS * 4);
         if (rows_cap > Cfg<PD>::SPLATS) rows_cap = Cfg<PD>::SPLATS;
-        const size_t smem = SliceFast<PD, VD>::bytes(rows_cap);
-        PL_TRY((ensure_dynamic_smem<slice_tiles_fast<PD, VD>>(smem)));
-        PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_fast<PD, VD>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, rows_cap, bulk_rows_ok(g, output, VD - 1) ? 1 : 0);
+        const size_t smem = SliceFast<PD, VP>::bytes(rows_cap);
+        PL_TRY((ensure_dynamic_smem<slice_tiles_fast<PD, VP, CT>>(smem)));
+        PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_fast<PD, VP, CT>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, vd - 1, rows_cap, bulk_rows_ok(g, output, vd - 1) ? 1 : 0);
     } else {
         const int rows_cap = rows_cap_for(PD, vd);
         const size_t fixed = sizeof(float) * Cfg<PD>::TP * SliceCfg<PD>::PW + sizeof(int) * Cfg<PD>::TP;
@@ -417,12 +418,25 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
     return PL_OK;
 }
 
-#define PL_DISPATCH_VD(FN, PD_, vd, ...)                                   \
-    ((vd) == 22  ? FN<PD_, 22>(__VA_ARGS__)                                 \
-     : (vd) == 4 ? FN<PD_, 4>(__VA_ARGS__)                                  \
-     : (vd) == 3 ? FN<PD_, 3>(__VA_ARGS__)                                  \
-     : (vd) == 2 ? FN<PD_, 2>(__VA_ARGS__)                                  \
-                 : FN<PD_, 0>(__VA_ARGS__))
+// The instantiation of splat (slice) for value dimension vd.
+#define PL_SPLAT_FOR(PD_, vd, ...)                  \
+    ((vd) == 22  ? launch_splat<PD_, 22>(__VA_ARGS__) \
+     : (vd) == 4 ? launch_splat<PD_, 4>(__VA_ARGS__)  \
+     : (vd) == 3 ? launch_splat<PD_, 3>(__VA_ARGS__)  \
+     : (vd) == 2 ? launch_splat<PD_, 2>(__VA_ARGS__)  \
+                 : launch_splat<PD_, 0>(__VA_ARGS__))
+#define PL_SLICE_FOR(PD_, vd, ...)                              \
+    ((vd) == 22            ? launch_slice<PD_, 24, 21>(__VA_ARGS__) \
+     : (vd) == 4           ? launch_slice<PD_, 4, 3>(__VA_ARGS__)   \
+     : padded_vd(vd) == 4  ? launch_slice<PD_, 4>(__VA_ARGS__)  \
+     : padded_vd(vd) == 8  ? launch_slice<PD_, 8>(__VA_ARGS__)  \
+     : padded_vd(vd) == 12 ? launch_slice<PD_, 12>(__VA_ARGS__) \
+     : padded_vd(vd) == 16 ? launch_slice<PD_, 16>(__VA_ARGS__) \
+     : padded_vd(vd) == 20 ? launch_slice<PD_, 20>(__VA_ARGS__) \
+     : padded_vd(vd) == 24 ? launch_slice<PD_, 24>(__VA_ARGS__) \
+     : padded_vd(vd) == 28 ? launch_slice<PD_, 28>(__VA_ARGS__) \
+     : padded_vd(vd) == 32 ? launch_slice<PD_, 32>(__VA_ARGS__) \
+                           : launch_slice<PD_, 0>(__VA_ARGS__))
 
 enum { PH_BUILD = 1, PH_APPLY = 2 };   // halves of a call: lattice structure / values through it
 
@@ -528,7 +542,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         PL_LAUNCH((convert_fixed), wide, 256, 0, st, hdr, v64, v0, padded_vd(vd));
         PL_COUNT_LAUNCHES(2);   // absmax_kernel, convert_fixed (the splat itself is counted below)
     } else {
-        rc = PL_DISPATCH_VD(launch_splat, PD, vd, g, input, hdr, tile_info, rec, rec_w, srec, !(phases & PH_BUILD), list_ref, v0, vd, st);
+        rc = PL_SPLAT_FOR(PD, vd, g, input, hdr, tile_info, rec, rec_w, srec, !(phases & PH_BUILD), list_ref, v0, vd, st);
     }
     if (rc != PL_OK) return rc;
     PL_COUNT_LAUNCHES(1 + 1);   // splat, slice (the blur launches are counted where they are issued)
@@ -544,7 +558,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     }
     PL_COUNT_LAUNCHES(PD + 1);
     if (ev) PL_CUDA(cudaEventRecord(ev[4], st));
-    rc = PL_DISPATCH_VD(launch_slice, PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, st);
+    rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, st);
     if (rc != PL_OK) return rc;
     if (ev) PL_CUDA(cudaEventRecord(ev[5], st));
     PL_CUDA(cudaGetLastError());

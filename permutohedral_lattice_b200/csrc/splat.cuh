@@ -11,10 +11,9 @@ namespace pl {
 // summed in registers, reading the tile's input rows from shared memory, and leaves the CTA as one
 // vector reduction per 16 bytes.  No floating-point atomics in shared memory.
 //
-// Narrow rows (VD <= 8, splat_tiles_fast): one THREAD sums a window of PD+1 sorted splats with the whole
+// Rows of one float4 (splat_tiles_fast): one THREAD sums a window of PD+1 sorted splats with the whole
 // row in registers; the input block arrives by bulk asynchronous copies when its rows are 16-byte aligned.
-// Wide rows (8 < VD <= 32, splat_tiles_rows): a quarter warp per window, see there.
-// Generic form (any vd): a group of lanes per entry, one float4 of channels per lane.
+// Wider rows (splat_tiles_rows): a group of lanes per window, see there.
 // ---------------------------------------------------------------------------------------------
 template <int PD>
 struct SplatCommon {
@@ -245,23 +244,26 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     flush_row<VP>(v0 + (size_t)vid_s[cur] * VP, acc);
 }
 
-// Wide rows (8 < VD <= 32): a QUARTER WARP per window.  The input block is staged with rows padded to VP
-// floats (16-byte aligned), so the 8 lanes of a quarter warp read one point's row as consecutive
-// float4 words: a 128-bit shared-memory load is served one quarter warp at a time, so every quarter
+// Rows of more than one float4: a GROUP OF LANES per window, one float4 of the row per lane (LW lanes: the power of
+// two that holds the row, a quarter warp for the 22 channels of the dense-CRF workload).  The input block is staged
+// with rows padded to VP floats (16-byte aligned), so the lanes of a group read one point's row as consecutive
+// float4 words: a 128-bit shared-memory load is served one quarter warp at a time, so with LW = 8 every quarter
 // reads its own row without bank conflicts whatever rows the other quarters read.  Lane h keeps
 // channels 4h .. 4h+3 of the running sum; the row's channel C is staged as 1 (homogeneous), the padding
 // as 0, so the loop has no channel tests.  A flush is one 16-byte vector reduction per lane.
+// VD = 0: any width, known at run time only (rows beyond 32 quads are walked once for every 32).
 // PRE: the lattice was built for reuse and holds every tile's splats already sorted, in the windowed form
 // (build_tiles with SORTED = true); the list then arrives by one bulk copy, the kernel needs no sort, no
 // counters, and fits five CTAs on an SM.
 template <int PD, int VD, bool PRE>
 struct SplatRows {
-    static constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, VP = (VD + 3) & ~3;
-    static constexpr int LR = VP / 4;                  // lanes that hold a piece of the row
-    static constexpr int WL = Cfg<PD>::WL;             // splats per window: TP / 8 windows
+    static constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS;
+    static constexpr int WL = Cfg<PD>::WL;             // splats between two spare words of the sorted list
     static constexpr int SORTED = Cfg<PD>::SREC;
-    static constexpr size_t BYTES = sizeof(float) * TP * VP + sizeof(uint2) * SORTED + (PRE ? 0 : sizeof(int) * SPLATS) +
-                                    sizeof(int) * TP;
+    static size_t bytes(int vd) {
+        return sizeof(float) * TP * (size_t)padded_vd(vd) + sizeof(uint2) * SORTED + (PRE ? 0 : sizeof(int) * SPLATS) +
+               sizeof(int) * TP;
+    }
 };
 
 // Five CTAs per SM (47-48 registers, no spills; with the sort's counters the five CTAs take nearly all of an
@@ -270,14 +272,14 @@ template <int PD, int VD, bool PRE>
 __global__ void __launch_bounds__(Cfg<PD>::TP, 5)
 splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
                  const u16* __restrict__ rec, const float* __restrict__ rec_w, const uint2* __restrict__ srec,
-                 const u32* __restrict__ list_ref, float* __restrict__ v0, int bulk_ok) {
+                 const u32* __restrict__ list_ref, float* __restrict__ v0, int vd, int bulk_ok) {
     // Launched to overlap the tail of the kernel before it (link_neighbours, or zero_rows in an apply): all
     // that the staging and the sort read (the input, the records and tile ranges of build_tiles, whose
     // failures are final by now) is older than that kernel, so they run before the wait; the window loop,
     // which reads the entries' vertices and adds to the zeroed rows, runs after it.
     using SR = SplatRows<PD, VD, PRE>;
-    constexpr int TP = SR::TP, SPLATS = SR::SPLATS, C = VD - 1, VP = SR::VP, LR = SR::LR, WL = SR::WL;
-    static_assert(LR <= 8, "a row must fit the 8 lanes of a quarter warp");
+    constexpr int TP = SR::TP, SPLATS = SR::SPLATS, WL = SR::WL;
+    const int C = (VD ? VD : vd) - 1, VP = padded_vd(VD ? VD : vd), LR = VP >> 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* in_s = reinterpret_cast<float*>(smem_raw);                         // [TP][VP]
     uint2* sorted_s = reinterpret_cast<uint2*>(in_s + TP * VP);               // [SORTED]
@@ -338,11 +340,10 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
         }
     } else {
         in_s[tid * VP + C] = 1.f;   // homogeneous channel, then padding
-#pragma unroll
         for (int j = C + 1; j < VP; j++) in_s[tid * VP + j] = 0.f;
         // element k = tid, tid + TP, ... of the tile's [point][channel] block; (point, channel) advance
         // without a division: TP = DP * C + DJ
-        constexpr int DP = TP / C, DJ = TP % C;
+        const int DP = TP / C, DJ = TP - DP * C;
         int p = tid / C, j = tid - p * C;
 #pragma unroll 3
         for (int it = 0; it < C; it++) {
@@ -362,7 +363,10 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     // did this thread see the copies complete within the bounded wait
     const bool arrived = (PRE || bulk_ok) ? mbar_wait(&bar, 0) : true;
     if (bulk_ok) {
-        constexpr int MAXE = (16 * C + 31) / 32;   // elements per lane of a tile row (TX <= 16)
+        // elements a lane reads before the first of them is written: the whole tile row (TX <= 16) where its size is
+        // known, else four at a time (an element moves towards the region's start and the elements after it lie
+        // behind its old place, so a trip never overwrites what a later one reads)
+        constexpr int MAXE = VD ? (16 * (VD - 1) + 31) / 32 : 4;
         for (int ly = warp; ly < g.TY; ly += TP / 32) {
             // valid points of this tile row: its first point's validity and the row's width
             const int p0 = ly * g.TX;
@@ -374,28 +378,32 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
             }
             float* region = in_s + (size_t)p0 * VP;
             const int n = count * C;
-            float tmp[MAXE];
-            int dst[MAXE];
             int pp = lane / C, jj = lane - pp * C;   // element e = lane + 32 m is channel jj of point pp
+            const int dp = 32 / C, dj = 32 - dp * C;
+#pragma unroll 1
+            for (int e0 = lane; e0 - lane < n; e0 += 32 * MAXE) {
+                float tmp[MAXE];
+                int dst[MAXE];
 #pragma unroll
-            for (int m = 0; m < MAXE; m++) {
-                const int e = lane + 32 * m;
-                tmp[m] = (e < n) ? region[land + e] : 0.f;
-                dst[m] = (e < n) ? pp * VP + jj : -1;
-                pp += 32 / C;
-                jj += 32 % C;
-                if (jj >= C) {
-                    jj -= C;
-                    pp++;
+                for (int m = 0; m < MAXE; m++) {
+                    const int e = e0 + 32 * m;
+                    tmp[m] = (e < n) ? region[land + e] : 0.f;
+                    dst[m] = (e < n) ? pp * VP + jj : -1;
+                    pp += dp;
+                    jj += dj;
+                    if (jj >= C) {
+                        jj -= C;
+                        pp++;
+                    }
                 }
-            }
-            __syncwarp();
+                __syncwarp();
 #pragma unroll
-            for (int m = 0; m < MAXE; m++)
-                if (dst[m] >= 0) region[dst[m]] = tmp[m];
+                for (int m = 0; m < MAXE; m++)
+                    if (dst[m] >= 0) region[dst[m]] = tmp[m];
+                if constexpr (VD > 0) break;   // one trip
+            }
             if (lane < g.TX) {
                 region[lane * VP + C] = 1.f;   // homogeneous channel, then padding
-#pragma unroll
                 for (int j = C + 1; j < VP; j++) region[lane * VP + j] = 0.f;
             }
         }
@@ -415,113 +423,45 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     wait_for_previous_kernel();
     if (call_failed(hdr)) return;   // a failure of the index stage
 
-    const int h = tid & 7, wnd = tid >> 3, first = wnd * WL;
-    const bool active = (h < LR) && (first < total);
-    if (active) {
-        const int count = min(WL, total - first);
-        const uint2* sp = sorted_s + wnd * (WL + 1);   // this window's words (see SplatCommon::slot)
-        const float4* in4 = reinterpret_cast<const float4*>(in_s) + h;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        int cur = (int)(sp[0].x >> 16);
-        u32 vcur = list_ref[base + cur];   // vertex of the running entry, fetched when the run starts
+    const int lw_log2 = LR > 16 ? 5 : LR > 8 ? 4 : LR > 4 ? 3 : LR > 2 ? 2 : LR > 1 ? 1 : 0;
+    const int LW = 1 << lw_log2, wl = LW * (PD + 1);   // lanes of a window, its splats
+    const int first = (tid >> lw_log2) * wl, end = min(first + wl, total);
+    constexpr bool ONE = VD > 16 && VD <= 32;          // known: a lane has one quad, a window is one stretch
+    if (first < end) {
+        for (int h = tid & (LW - 1); h < LR; h += LW) {
+            const float4* in4 = reinterpret_cast<const float4*>(in_s) + h;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            int cur = (int)(sorted_s[Cfg<PD>::srec_slot(first)].x >> 16);
+            u32 vcur = list_ref[base + cur];   // vertex of the running entry, fetched when the run starts
+            // a window lies between two spare words of the list, or (LW > 8) is a row of such stretches
+            for (int pos = first; pos < end; pos += WL) {
+                const uint2* sp = sorted_s + Cfg<PD>::srec_slot(pos);
+                const int count = min(WL, end - pos);
 #pragma unroll 4
-        for (int i = 0; i < count; i++) {
-            const uint2 pw = sp[i];
-            const int e = (int)(pw.x >> 16);
-            if (e != cur) {
-                red_add_v4(v0 + (size_t)vcur * VP + 4 * h, acc);
-                acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                cur = e;
-                vcur = list_ref[base + cur];
+                for (int i = 0; i < count; i++) {
+                    const uint2 pw = sp[i];
+                    const int e = (int)(pw.x >> 16);
+                    if (e != cur) {
+                        red_add_v4(v0 + (size_t)vcur * VP + 4 * h, acc);
+                        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                        cur = e;
+                        vcur = list_ref[base + cur];
+                    }
+                    const float wt = __uint_as_float(pw.y);
+                    const float4 x = in4[(pw.x & 0xFFFFu) * LR];
+                    acc.x = PL_FMA(wt, x.x, acc.x);
+                    acc.y = PL_FMA(wt, x.y, acc.y);
+                    acc.z = PL_FMA(wt, x.z, acc.z);
+                    acc.w = PL_FMA(wt, x.w, acc.w);
+                }
+                if constexpr (ONE) break;
             }
-            const float wt = __uint_as_float(pw.y);
-            const float4 x = in4[(pw.x & 0xFFFFu) * LR];
-            acc.x = PL_FMA(wt, x.x, acc.x);
-            acc.y = PL_FMA(wt, x.y, acc.y);
-            acc.z = PL_FMA(wt, x.z, acc.z);
-            acc.w = PL_FMA(wt, x.w, acc.w);
+            let_next_kernel_start();   // what is left of this thread's work: its last row
+            red_add_v4(v0 + (size_t)vcur * VP + 4 * h, acc);
+            if constexpr (ONE) break;
         }
-        let_next_kernel_start();   // what is left of this thread's work: its last row
-        red_add_v4(v0 + (size_t)vcur * VP + 4 * h, acc);
     }
     pc.mark(true);
-}
-
-template <int PD>
-struct SplatGeneric {
-    static constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS;
-    static size_t bytes(int vd) {
-        return sizeof(float) * (size_t)TP * padded_vd(vd) + sizeof(uint2) * SPLATS + 2 * sizeof(int) * SPLATS +
-               sizeof(int) * TP;
-    }
-};
-
-template <int PD>
-__global__ void __launch_bounds__(Cfg<PD>::TP)
-splat_tiles_generic(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
-                    const u16* __restrict__ rec, const float* __restrict__ rec_w,
-                    const u32* __restrict__ list_ref, float* __restrict__ v0, int vd) {
-    wait_for_previous_kernel();
-    constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, NW = TP / 32;
-    const int C = vd - 1, VP = padded_vd(vd), QPR = VP >> 2;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float* in_s = reinterpret_cast<float*>(smem_raw);                       // [TP][VP]
-    uint2* sorted_s = reinterpret_cast<uint2*>(in_s + (size_t)TP * VP);     // [SPLATS]
-    int* cur_s = reinterpret_cast<int*>(sorted_s + SPLATS);                 // [SPLATS]
-    int* off_s = cur_s + SPLATS;                                            // [SPLATS]
-    int* prow_s = off_s + SPLATS;                                           // [TP]
-    __shared__ int wsum_s[32];
-    if (call_failed(hdr)) return;
-    const TilePos tpos = this_tile(g);
-    const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
-    const int2 info = tile_info[tile];
-    const int base = info.x, nloc = info.y;
-
-    int item, pix;
-    const bool valid = tile_point(g, tpos, tid, item, pix);
-    prow_s[tid] = valid ? item * g.n + pix : -1;
-    for (int i = tid; i < nloc; i += TP) cur_s[i] = 0;
-    in_s[tid * VP + C] = 1.f;   // homogeneous channel, then padding
-    for (int j = C + 1; j < VP; j++) in_s[tid * VP + j] = 0.f;
-    __syncthreads();
-    for (int k = tid; k < TP * C; k += TP) {
-        const int p = k / C, j = k - p * C;
-        const int row = prow_s[p];
-        if (row >= 0) cp_async4(in_s + p * VP + j, input + (size_t)row * C + j);
-    }
-    float w[PD + 1];
-    int l[PD + 1];
-    const u16* rec_tile = rec + (size_t)tile * SPLATS;
-    const float* recw_tile = rec_w + (size_t)tile * SPLATS;
-#pragma unroll
-    for (int r = 0; r <= PD; r++) {
-        l[r] = valid ? rec_tile[r * TP + tid] : 0;
-        w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
-    }
-    SplatCommon<PD>::template sort_splats<0>(valid, l, w, nloc, sorted_s, cur_s, off_s, wsum_s);
-    cp_async_wait_all();
-    __syncthreads();
-
-    const LaneMap lm(QPR, lane);
-    if (!lm.active) return;
-    const float4* in4 = reinterpret_cast<const float4*>(in_s);
-    for (int e = warp * lm.ppw + lm.g; e < nloc; e += NW * lm.ppw) {
-        const int beg = cur_s[e], end = off_s[e];
-        float* vrow = v0 + (size_t)list_ref[base + e] * VP;
-        for (int q = lm.q0; q < QPR; q += lm.gs) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int sidx = beg; sidx < end; sidx++) {
-                const uint2 pw = sorted_s[sidx];
-                const float wt = __uint_as_float(pw.y);
-                const float4 x = in4[(pw.x & 0xFFFFu) * QPR + q];
-                acc.x = PL_FADD(acc.x, PL_FMUL(wt, x.x));
-                acc.y = PL_FADD(acc.y, PL_FMUL(wt, x.y));
-                acc.z = PL_FADD(acc.z, PL_FMUL(wt, x.z));
-                acc.w = PL_FADD(acc.w, PL_FMUL(wt, x.w));
-            }
-            red_add_v4(vrow + 4 * q, acc);
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1,0 +1,71 @@
+"""Splat and slice over value rows of every width class, against the oracle.
+
+Lanes of a splat window (1, 2, 4, 8, 16, 32) and the slice's row width change at the vd below and beside each of
+them; a channel count that is a multiple of four leaves the homogeneous channel a quad of its own.  The bounds are
+those of every comparison with the oracle (gpu_helpers): float sums of a few hundred terms in another order."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device")
+    import gpu_helpers
+    return gpu_helpers
+
+
+CHANNELS = [1, 2, 3, 4, 5, 7, 8, 11, 12, 15, 16, 19, 20, 21, 23, 24, 27, 28, 31, 32, 33, 47, 63, 64, 127, 130]
+
+
+@pytest.mark.parametrize("shape,r", [((35, 32), 3), ((18, 33), 3), ((19, 21), 1), ((301,), 2), ((5, 9, 11), 3)])
+def test_every_width_class(shape, r, gpu, oracle):
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(41)
+    ref = rng.random((2,) + shape + (r,), dtype=np.float32)
+    wide = rng.standard_normal((2,) + shape + (CHANNELS[-1],)).astype(np.float32)
+    wants = [oracle.lattice_filter(wide, ref, True, 4.0, 0.2, 1.0, reverse) for reverse in (False, True)]
+    rt = torch.from_numpy(ref).cuda()
+    lattice = plb.Lattice(rt, None, True, 4.0, 0.2, max_channels=CHANNELS[-1])
+    for c in CHANNELS:
+        x = torch.from_numpy(np.ascontiguousarray(wide[..., :c])).cuda()
+        for reverse in (False, True):
+            got = plb.lattice_filter(x, rt, True, 4.0, 0.2, reverse=reverse).cpu().numpy()
+            gpu.assert_outputs_close(got, wants[reverse][..., :c], "%d channels" % c)
+            got = lattice.apply(x, reverse).cpu().numpy()
+            gpu.assert_outputs_close(got, wants[reverse][..., :c], "%d channels, lattice kept" % c)
+
+
+@pytest.mark.parametrize("pd,n", [(16, 301), (8, 515), (7, 300), (1, 700)])
+def test_widths_on_the_positions_path(pd, n, gpu, oracle):
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(43)
+    pos = (rng.standard_normal((2, n, pd)) * 1.2).astype(np.float32)
+    wide = rng.standard_normal((2, n, 70)).astype(np.float32)
+    want = np.stack([oracle.filter(wide[i], pos[i], structure=False).out for i in range(2)])
+    for c in (3, 4, 6, 8, 10, 13, 17, 22, 26, 30, 40, 70):
+        x = torch.from_numpy(np.ascontiguousarray(wide[..., :c])).cuda()
+        got = plb.filter_positions(x, torch.from_numpy(pos).cuda())[0].cpu().numpy()
+        gpu.assert_outputs_close(got, want[..., :c], "pd %d, %d channels" % (pd, c))
+
+
+def test_rows_that_do_not_start_on_sixteen_bytes(gpu, oracle):
+    """An input that begins four bytes into its allocation is staged by 4-byte copies at every width."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(47)
+    shape = (1, 20, 32)
+    ref = rng.random(shape + (3,), dtype=np.float32)
+    rt = torch.from_numpy(ref).cuda()
+    for c in (3, 4, 10, 21, 31):
+        inp = rng.standard_normal(shape + (c,)).astype(np.float32)
+        flat = torch.empty(inp.size + 1, device="cuda")
+        x = flat[1:].view(inp.shape)
+        x.copy_(torch.from_numpy(inp))
+        out, _, _ = plb.lattice_filter_raw(x, rt, True, 4.0, 0.2, out=torch.empty(inp.size + 1, device="cuda")[1:].view(inp.shape))
+        gpu.assert_outputs_close(out.cpu().numpy(), oracle.lattice_filter(inp, ref, True, 4.0, 0.2), "%d channels" % c)
