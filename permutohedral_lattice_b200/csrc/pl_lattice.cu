@@ -589,7 +589,8 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     PL_CUDA(cudaMemsetAsync(hdr, 0, sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header), st));
     if (g.num_tiles == 0) return PL_OK;
     PL_TRY((ensure_dynamic_smem<build_tiles<PD, double>>(Cfg<PD>::build_smem(false))));
-    PL_TRY((ensure_dynamic_smem<splat_tiles_f64<PD>>(Splat64<PD>::BYTES)));
+    const size_t splat_smem = Splat64<PD>::bytes(vd);
+    PL_TRY((ensure_dynamic_smem<splat_tiles_f64<PD>>(splat_smem)));
     const int wide = num_sms() * 8;
     int table_log2 = 0;
     while ((1ull << table_log2) < L.table_slots) table_log2++;
@@ -622,7 +623,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   nullptr, 0u, take_watch());
     }
-    PL_LAUNCH((splat_tiles_f64<PD>), tile_grid(g), TP, Splat64<PD>::BYTES, st, g, input, hdr, tile_info, rec, rec_w,
+    PL_LAUNCH((splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                       list_ref, v0, vd);
     double* src = v0;
     double* dst = v1;

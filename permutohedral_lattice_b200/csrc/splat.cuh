@@ -15,6 +15,12 @@ namespace pl {
 // row in registers; the input block arrives by bulk asynchronous copies when its rows are 16-byte aligned.
 // Wider rows (splat_tiles_rows): a group of lanes per window, see there.
 // ---------------------------------------------------------------------------------------------
+// A sorted splat: point | entry << 16, and its weight.
+__device__ __forceinline__ uint2 splat_record(unsigned key, float w) { return make_uint2(key, __float_as_uint(w)); }
+__device__ __forceinline__ uint4 splat_record(unsigned key, double w) {
+    return make_uint4(key, 0u, (unsigned)__double2loint(w), (unsigned)__double2hiint(w));
+}
+
 template <int PD>
 struct SplatCommon {
     static constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, NW = TP / 32;
@@ -34,28 +40,27 @@ struct SplatCommon {
     }
 
     // Counting sort of the tile's splats by entry.  On return (after the trailing barrier) entry e's
-    // splats are sorted positions cur_s[e] .. cur_s[e] + count(e), each stored as
-    // (point | entry << 16, weight bits); off_s[e], when given, receives the end of the run.
+    // splats are the sorted positions from cur_s[e] on, each stored as
+    // (point | entry << 16, weight) (splat_record).
     // cur_s must be zero for e < nloc on entry.  One shared-memory atomic per splat: the value it
     // returns is the splat's offset inside its entry's run, so no second atomic pass is needed once the
     // run starts are known.  (Grouping equal entries of a warp with a match instruction first measured
     // slower than letting the atomics collide.)
-    template <int WL>
-    __device__ static __forceinline__ void sort_splats(bool valid, const int* l, const float* w, int nloc,
-                                                       uint2* sorted_s, int* cur_s, int* off_s, int* wsum_s) {
+    template <int WL, typename Rec, typename W>
+    __device__ static __forceinline__ void sort_splats(bool valid, const int* l, const W* w, int nloc,
+                                                       Rec* sorted_s, int* cur_s, int* wsum_s) {
         const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
         int off[PD + 1];
 #pragma unroll
         for (int r = 0; r <= PD; r++) off[r] = valid ? atomicAdd(&cur_s[l[r]], 1) : 0;
         __syncthreads();
-        int local[PD + 1], count[PD + 1];
+        int local[PD + 1];
         int sum = 0;
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
             const int i = tid * (PD + 1) + r;
             local[r] = sum;
-            count[r] = (i < nloc) ? cur_s[i] : 0;
-            sum += count[r];
+            sum += (i < nloc) ? cur_s[i] : 0;
         }
         int incl = sum;
 #pragma unroll
@@ -72,17 +77,14 @@ struct SplatCommon {
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
             const int i = tid * (PD + 1) + r;
-            if (i < nloc) {
-                cur_s[i] = excl + local[r];
-                if (off_s) off_s[i] = excl + local[r] + count[r];
-            }
+            if (i < nloc) cur_s[i] = excl + local[r];
         }
         __syncthreads();
         if (valid) {
 #pragma unroll
             for (int r = 0; r <= PD; r++) {
                 const int pos = cur_s[l[r]] + off[r];
-                sorted_s[slot<WL>(pos)] = make_uint2((unsigned)tid | ((unsigned)l[r] << 16), __float_as_uint(w[r]));
+                sorted_s[slot<WL>(pos)] = splat_record((unsigned)tid | ((unsigned)l[r] << 16), w[r]);
             }
         }
         __syncthreads();
@@ -198,7 +200,7 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
             l[r] = valid ? rec_tile[r * TP + tid] : 0;
             w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
         }
-        SplatCommon<PD>::template sort_splats<PD + 1>(valid, l, w, nloc, sorted_s, cur_s, nullptr, wsum_s);
+        SplatCommon<PD>::template sort_splats<PD + 1>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
     }
 
     if (bulk_ok) {
@@ -358,7 +360,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
         }
     }
 
-    if constexpr (!PRE) SplatCommon<PD>::template sort_splats<WL>(valid, l, w, nloc, sorted_s, cur_s, nullptr, wsum_s);
+    if constexpr (!PRE) SplatCommon<PD>::template sort_splats<WL>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
     pc.mark();
     // did this thread see the copies complete within the bounded wait
     const bool arrived = (PRE || bulk_ok) ? mbar_wait(&bar, 0) : true;
@@ -536,7 +538,7 @@ splat_tiles_det(Geom g, const float* __restrict__ input, Header* hdr, const int2
         l[r] = valid ? rec_tile[r * TP + tid] : 0;
         w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
     }
-    SplatCommon<PD>::template sort_splats<0>(valid, l, w, nloc, sorted_s, cur_s, nullptr, wsum_s);
+    SplatCommon<PD>::template sort_splats<0>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
     cp_async_wait_all();
     __syncthreads();
 

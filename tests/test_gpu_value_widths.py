@@ -69,3 +69,22 @@ def test_rows_that_do_not_start_on_sixteen_bytes(gpu, oracle):
         x.copy_(torch.from_numpy(inp))
         out, _, _ = plb.lattice_filter_raw(x, rt, True, 4.0, 0.2, out=torch.empty(inp.size + 1, device="cuda")[1:].view(inp.shape))
         gpu.assert_outputs_close(out.cpu().numpy(), oracle.lattice_filter(inp, ref, True, 4.0, 0.2), "%d channels" % c)
+
+
+@pytest.mark.parametrize("shape,r", [((35, 32), 3), ((18, 33), 3), ((301,), 2)])
+def test_every_width_class_in_double(shape, r, gpu, oracle):
+    """Rows of 1 to 32 pairs and beyond; blocks of 32 doubles, the last of them with the homogeneous channel alone."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from conftest import rel_l2
+    rng = np.random.default_rng(67)
+    ref = rng.random((2,) + shape + (r,))
+    wide = rng.standard_normal((2,) + shape + (130,))
+    rt = torch.from_numpy(ref).cuda()
+    for reverse in (False, True):
+        want = oracle.lattice_filter(wide, ref, True, 4.0, float(np.float32(0.2)), 1.0, reverse, dtype=np.float64)
+        for c in (1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 21, 31, 32, 33, 40, 62, 63, 64, 65, 96, 130):
+            x = torch.from_numpy(np.ascontiguousarray(wide[..., :c])).cuda()
+            got = plb.lattice_filter(x, rt, True, 4.0, 0.2, reverse=reverse).cpu().numpy()
+            # double sums in another order: the bound of every comparison in double with the oracle
+            assert rel_l2(got, want[..., :c]) <= 1e-12, "%d channels" % c
