@@ -127,29 +127,6 @@ splat_tiles_f64(Geom g, const double* __restrict__ input, Header* hdr, const int
     }
 }
 
-// One [1 2 1]/4 pass along a lattice axis (src/PermutohedralLatticeCPU.h:403-405).  One double2 per thread.
-__global__ void __launch_bounds__(256)
-blur_axis_f64(const Header* hdr, const int* __restrict__ nbr_axis, const double* __restrict__ src,
-              double* __restrict__ dst, int ppr /* double2 per row */) {
-    if (hdr->status != 0) return;
-    const u32 M = hdr->num_vertices;
-    const u64 items = (u64)M * ppr;
-    const double2* __restrict__ s = reinterpret_cast<const double2*>(src);
-    double2* __restrict__ d = reinterpret_cast<double2*>(dst);
-    const int2* __restrict__ nb = reinterpret_cast<const int2*>(nbr_axis);
-    const double2 zero = make_double2(0.0, 0.0);
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < items; e += (u64)gridDim.x * blockDim.x) {
-        const u32 v = (u32)(e / ppr);
-        const int j = (int)(e - (u64)v * ppr);
-        const int2 n = __ldg(nb + v);
-        const double2 b = s[e];
-        const double2 a = (n.x >= 0) ? s[(u64)n.x * ppr + j] : zero;
-        const double2 c = (n.y >= 0) ? s[(u64)n.y * ppr + j] : zero;
-        d[e] = make_double2(PL_DADD(PL_DADD(PL_DMUL(0.25, a.x), PL_DMUL(0.5, b.x)), PL_DMUL(0.25, c.x)),
-                            PL_DADD(PL_DADD(PL_DMUL(0.25, a.y), PL_DMUL(0.5, b.y)), PL_DMUL(0.25, c.y)));
-    }
-}
-
 // Slice (src/PermutohedralLatticeCPU.h:333-352): per point and channel the weighted sum over the
 // remainders in ascending order, then one multiply by the reciprocal of the homogeneous channel.
 // A group of lanes per point, a double2 of the row each (rows beyond a warp's 32 are walked 32 at a time); the

@@ -549,11 +549,11 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     if (ev) PL_CUDA(cudaEventRecord(ev[3], st));
     float* src = v0;
     float* dst = v1;
-    const int qpr = padded_vd(vd) / 4;
+    const u32 qpr = (u32)padded_vd(vd) / 4;
     for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * L.max_entries * 2;
-        PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis), wide, 256, 0, st, hdr, nb, src, dst, qpr);
+        PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<float4>), wide, 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
         float* tmp = src; src = dst; dst = tmp;
     }
     PL_COUNT_LAUNCHES(PD + 1);
@@ -629,7 +629,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* dst = v1;
     for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        PL_LAUNCH((blur_axis_f64), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, src, dst, vp / 2);
+        PL_LAUNCH((blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
     PL_LAUNCH((slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd);
