@@ -344,6 +344,12 @@ static int widest_vd(int pd) {
     return ((200 * 1024 - 16 * tp * (pd + 1) - 4 * tp) / (4 * tp)) & ~3;
 }
 
+// The same of the deterministic splat: its input block and one and a half sorted lists within 200 KB.
+static int widest_vd_fixed(int pd) {
+    const int tp = tp_of(pd);
+    return (200 * 1024 - 12 * tp * (pd + 1) - 4 * tp) / (4 * tp) + 1;
+}
+
 // True when every contiguous run of a tile's points starts on a 16-byte boundary and has a size that is
 // a multiple of 16 bytes in a [points][channels] float array at `ptr`: then the tile's block can move
 // by bulk asynchronous copies.
@@ -363,6 +369,11 @@ static dim3 link_grid(int wide, u64 max_entries) {
     return dim3((unsigned)(blocks < (u64)wide ? blocks : (u64)wide), PD + 1, 1);
 }
 
+// Bulk copies into padded rows (splat_tiles_rows) also need 16-byte aligned landing zones inside the tile rows.
+static bool bulk_staging_ok(const Geom& g, const float* input, int vd) {
+    return bulk_rows_ok(g, input, vd - 1) && g.TX <= 16 && (g.TX * (padded_vd(vd) - (vd - 1))) % 4 == 0;
+}
+
 // splat for value dimension VD, fixed at compile time, or (VD = 0) any other.
 // Rows of one float4 (VD <= 4) are summed by a thread each, wider ones by a group of lanes (splat.cuh).
 template <int PD, int VD, bool PRE>
@@ -378,12 +389,24 @@ static int launch_splat_as(const Geom& g, const float* input, Header* hdr, const
         const size_t smem = SplatRows<PD, VD, PRE>::bytes(vd);
         if (vd > widest_vd(PD)) return PL_UNSUPPORTED_DIMS;
         // five CTAs per SM need nearly all of the SM's shared memory: ask for the largest carve-out
-        PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, VD, PRE>>(smem, true)));
-        // bulk staging also needs 16-byte aligned landing zones inside the padded tile rows
-        const bool bulk = bulk_rows_ok(g, input, vd - 1) && g.TX <= 16 && (g.TX * (padded_vd(vd) - (vd - 1))) % 4 == 0;
-        PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_rows<PD, VD, PRE>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+        PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, VD, PRE, FloatSum, float>>(smem, true)));
+        const bool bulk = bulk_staging_ok(g, input, vd);
+        PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_rows<PD, VD, PRE, FloatSum, float>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                               srec, list_ref, v0, vd, bulk ? 1 : 0);
     }
+    return PL_OK;
+}
+
+// The deterministic splat: fixed-point sums, rows of any width.
+template <int PD, bool PRE>
+static int launch_splat_fixed(const Geom& g, const float* input, Header* hdr, const int2* tile_info, const u16* rec,
+                              const float* rec_w, const uint2* srec, const u32* list_ref, long long* v64, int vd,
+                              cudaStream_t st) {
+    const size_t smem = SplatRows<PD, 0, PRE>::bytes(vd);
+    PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, 0, PRE, FixedSum, long long>>(smem, true)));
+    const bool bulk = bulk_staging_ok(g, input, vd);
+    PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_rows<PD, 0, PRE, FixedSum, long long>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+                                                                          srec, list_ref, v64, vd, bulk ? 1 : 0);
     return PL_OK;
 }
 
@@ -534,11 +557,11 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     }
     int rc = PL_OK;
     if (v64) {
-        const size_t smem = SplatDet<PD>::bytes(vd);
-        if (smem > 200 * 1024) return PL_UNSUPPORTED_DIMS;
-        PL_TRY((ensure_dynamic_smem<splat_tiles_det<PD>>(smem)));
+        if (vd > widest_vd_fixed(PD)) return PL_UNSUPPORTED_DIMS;
         PL_LAUNCH((absmax_kernel), wide, 256, 0, st, input, (u64)g.batch * g.n * (vd - 1), hdr);
-        PL_LAUNCH((splat_tiles_det<PD>), tile_grid(g), TP, smem, st, g, input, hdr, tile_info, rec, rec_w, list_ref, v64, vd);
+        rc = (phases & PH_BUILD) ? launch_splat_fixed<PD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st)
+                                 : launch_splat_fixed<PD, true>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st);
+        if (rc != PL_OK) return rc;
         PL_LAUNCH((convert_fixed), wide, 256, 0, st, hdr, v64, v0, padded_vd(vd));
         PL_COUNT_LAUNCHES(2);   // absmax_kernel, convert_fixed (the splat itself is counted below)
     } else {

@@ -1,6 +1,7 @@
 // Splat stage: per-tile sort of the splats by entry and segmented reduction into the vertex rows
-// (register-resident, generic and deterministic fixed-point forms).
+// (a thread per window of narrow rows, a group of lanes per window of wider ones; float and fixed-point sums).
 #pragma once
+#include <type_traits>
 #include "common.cuh"
 
 namespace pl {
@@ -246,6 +247,66 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     flush_row<VP>(v0 + (size_t)vid_s[cur] * VP, acc);
 }
 
+// The deterministic mode's grid (PL_MODE_DETERMINISTIC): every product weight * value is rounded once to a multiple
+// of 2^-36 of the next power of two above max(|input|, 1), found by absmax_kernel, and summed as a 64-bit integer, in
+// registers and in global memory.  Integer addition is associative, so the sums do not depend on the order in which
+// splats, windows or tiles arrive: results are bitwise reproducible.  Finite inputs only.
+__device__ __forceinline__ int fixed_exponent(const Header* hdr) {   // 36 - e with 2^e > max(|input|, 1)
+    const u32 bits = max(hdr->absmax_bits, __float_as_uint(1.0f));
+    return 36 - ((int)((bits >> 23) & 0xFF) - 127 + 1);
+}
+
+// What a lane keeps of the running entry: four channels of its sum.
+struct FloatSum {
+    float4 a;
+    __device__ __forceinline__ explicit FloatSum(const Header*) {}
+    __device__ __forceinline__ void clear() { a = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void add(float wt, float4 x) {
+        a.x = PL_FMA(wt, x.x, a.x);
+        a.y = PL_FMA(wt, x.y, a.y);
+        a.z = PL_FMA(wt, x.z, a.z);
+        a.w = PL_FMA(wt, x.w, a.w);
+    }
+    __device__ __forceinline__ void flush(float* row) const { red_add_v4(row, a); }
+};
+// The same on the fixed-point grid.  A product scaled to the grid, t with |t| <= 2^36 and a little, is an integer
+// number of 2^15 (added to 1.5 * 2^38, whose last place that is) plus a rest of at most 2^14, exact in float, whose
+// nearest integer the same trick with 1.5 * 2^23 gives: together t rounded to the nearest integer, ties to even.  The
+// two halves of a window's sum, of at most 32 (pd + 1) terms, fit 32 bits each.  (Converting every product to double
+// and that to a 64-bit integer took two instructions of a sixteenth of the float rate each.)
+struct FixedSum {
+    static constexpr float M_HI = 412316860416.f, M_LO = 12582912.f;
+    int hi[4], lo[4];
+    float scale;
+    __device__ __forceinline__ explicit FixedSum(const Header* hdr) {
+        scale = __int_as_float((127 + fixed_exponent(hdr)) << 23);
+    }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int k = 0; k < 4; k++) hi[k] = lo[k] = 0;
+    }
+    __device__ __forceinline__ void add1(int k, float prod) {
+        const float t = PL_FMUL(prod, scale);
+        const float h = PL_FADD(t, M_HI);
+        const float l = PL_FADD(PL_FADD(t, -PL_FADD(h, -M_HI)), M_LO);
+        hi[k] += __float_as_int(h) - __float_as_int(M_HI);
+        lo[k] += __float_as_int(l) - __float_as_int(M_LO);
+    }
+    __device__ __forceinline__ void add(float wt, float4 x) {
+        add1(0, PL_FMUL(wt, x.x));
+        add1(1, PL_FMUL(wt, x.y));
+        add1(2, PL_FMUL(wt, x.z));
+        add1(3, PL_FMUL(wt, x.w));
+    }
+    __device__ __forceinline__ void flush(long long* row) const {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const long long sum = (long long)hi[k] * 32768 + (long long)lo[k];
+            if (sum) atomicAdd(reinterpret_cast<u64*>(row + k), (u64)sum);
+        }
+    }
+};
+
 // Rows of more than one float4: a GROUP OF LANES per window, one float4 of the row per lane (LW lanes: the power of
 // two that holds the row, a quarter warp for the 22 channels of the dense-CRF workload).  The input block is staged
 // with rows padded to VP floats (16-byte aligned), so the lanes of a group read one point's row as consecutive
@@ -254,6 +315,7 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
 // channels 4h .. 4h+3 of the running sum; the row's channel C is staged as 1 (homogeneous), the padding
 // as 0, so the loop has no channel tests.  A flush is one 16-byte vector reduction per lane.
 // VD = 0: any width, known at run time only (rows beyond 32 quads are walked once for every 32).
+// Sum: float sums into rows of floats, or fixed-point sums into rows of 64-bit integers (V: type of a row's cell).
 // PRE: the lattice was built for reuse and holds every tile's splats already sorted, in the windowed form
 // (build_tiles with SORTED = true); the list then arrives by one bulk copy, the kernel needs no sort, no
 // counters, and fits five CTAs on an SM.
@@ -270,11 +332,11 @@ struct SplatRows {
 
 // Five CTAs per SM (47-48 registers, no spills; with the sort's counters the five CTAs take nearly all of an
 // SM's shared memory): 4 % faster than four at 16 items, and 2048 tiles (two items) take three waves, not four.
-template <int PD, int VD, bool PRE>
-__global__ void __launch_bounds__(Cfg<PD>::TP, 5)
+template <int PD, int VD, bool PRE, typename Sum, typename V>
+__global__ void __launch_bounds__(Cfg<PD>::TP, std::is_same<Sum, FloatSum>::value ? 5 : 4)
 splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
                  const u16* __restrict__ rec, const float* __restrict__ rec_w, const uint2* __restrict__ srec,
-                 const u32* __restrict__ list_ref, float* __restrict__ v0, int vd, int bulk_ok) {
+                 const u32* __restrict__ list_ref, V* __restrict__ v0, int vd, int bulk_ok) {
     // Launched to overlap the tail of the kernel before it (link_neighbours, or zero_rows in an apply): all
     // that the staging and the sort read (the input, the records and tile ranges of build_tiles, whose
     // failures are final by now) is older than that kernel, so they run before the wait; the window loop,
@@ -432,7 +494,8 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     if (first < end) {
         for (int h = tid & (LW - 1); h < LR; h += LW) {
             const float4* in4 = reinterpret_cast<const float4*>(in_s) + h;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            Sum acc(hdr);
+            acc.clear();
             int cur = (int)(sorted_s[Cfg<PD>::srec_slot(first)].x >> 16);
             u32 vcur = list_ref[base + cur];   // vertex of the running entry, fetched when the run starts
             // a window lies between two spare words of the list, or (LW > 8) is a row of such stretches
@@ -444,22 +507,17 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
                     const uint2 pw = sp[i];
                     const int e = (int)(pw.x >> 16);
                     if (e != cur) {
-                        red_add_v4(v0 + (size_t)vcur * VP + 4 * h, acc);
-                        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                        acc.flush(v0 + (size_t)vcur * VP + 4 * h);
+                        acc.clear();
                         cur = e;
                         vcur = list_ref[base + cur];
                     }
-                    const float wt = __uint_as_float(pw.y);
-                    const float4 x = in4[(pw.x & 0xFFFFu) * LR];
-                    acc.x = PL_FMA(wt, x.x, acc.x);
-                    acc.y = PL_FMA(wt, x.y, acc.y);
-                    acc.z = PL_FMA(wt, x.z, acc.z);
-                    acc.w = PL_FMA(wt, x.w, acc.w);
+                    acc.add(__uint_as_float(pw.y), in4[(pw.x & 0xFFFFu) * LR]);
                 }
                 if constexpr (ONE) break;
             }
             let_next_kernel_start();   // what is left of this thread's work: its last row
-            red_add_v4(v0 + (size_t)vcur * VP + 4 * h, acc);
+            acc.flush(v0 + (size_t)vcur * VP + 4 * h);
             if constexpr (ONE) break;
         }
     }
@@ -467,11 +525,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
 }
 
 // ---------------------------------------------------------------------------------------------
-// Deterministic splat (PL_MODE_DETERMINISTIC): the same sort-by-entry and segmented reduction, but
-// every product weight * value is rounded once onto a fixed-point grid and summed as a 64-bit
-// integer, in registers and in global memory.  Integer addition is associative, so the sums do not
-// depend on the order in which splats, windows or tiles arrive: results are bitwise reproducible.
-// Grid spacing: 2^-36 of the next power of two above max(|input|, 1), found by a first pass.
+// Deterministic mode: the input's largest magnitude before the splat, the sums as floats after it.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
@@ -484,100 +538,12 @@ absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
     if ((threadIdx.x & 31) == 0 && m) atomicMax(&hdr->absmax_bits, m);
 }
 
-// 2^(36 - e) with 2^e > max(|input|, 1); finite inputs only.
-__device__ __forceinline__ double fixed_scale(const Header* hdr) {
-    const u32 bits = max(hdr->absmax_bits, __float_as_uint(1.0f));
-    const int e = (int)((bits >> 23) & 0xFF) - 127 + 1;
-    return __longlong_as_double((long long)(1023 + 36 - e) << 52);
-}
-
-template <int PD>
-struct SplatDet {
-    static constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS;
-    static size_t bytes(int vd) {
-        return ((sizeof(float) * (size_t)TP * (vd - 1) + 15) / 16) * 16 + sizeof(uint2) * SPLATS +
-               sizeof(int) * SPLATS + sizeof(int) * TP;
-    }
-};
-
-template <int PD>
-__global__ void __launch_bounds__(Cfg<PD>::TP)
-splat_tiles_det(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
-                const u16* __restrict__ rec, const float* __restrict__ rec_w,
-                const u32* __restrict__ list_ref, long long* __restrict__ v64, int vd) {
-    after_previous_kernel();
-    constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, NW = TP / 32;
-    const int C = vd - 1, VP = padded_vd(vd);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float* in_s = reinterpret_cast<float*>(smem_raw);                                                // [TP][C]
-    uint2* sorted_s = reinterpret_cast<uint2*>(smem_raw + ((sizeof(float) * (size_t)TP * C + 15) / 16) * 16);
-    int* cur_s = reinterpret_cast<int*>(sorted_s + SPLATS);
-    int* prow_s = cur_s + SPLATS;
-    __shared__ int wsum_s[32];
-    if (call_failed(hdr)) return;
-    const TilePos tpos = this_tile(g);
-    const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
-    const int2 info = tile_info[tile];
-    const int base = info.x, nloc = info.y;
-    int item, pix;
-    const bool valid = tile_point(g, tpos, tid, item, pix);
-    prow_s[tid] = valid ? item * g.n + pix : -1;
-    for (int i = tid; i < nloc; i += TP) cur_s[i] = 0;
-    const int nvalid = __syncthreads_count(valid);
-    for (int k = tid; k < TP * C; k += TP) {
-        const int p = k / C, j = k - p * C;
-        const int row = prow_s[p];
-        if (row >= 0) cp_async4(in_s + k, input + (size_t)row * C + j);
-    }
-    float w[PD + 1];
-    int l[PD + 1];
-    const u16* rec_tile = rec + (size_t)tile * SPLATS;
-    const float* recw_tile = rec_w + (size_t)tile * SPLATS;
-#pragma unroll
-    for (int r = 0; r <= PD; r++) {
-        l[r] = valid ? rec_tile[r * TP + tid] : 0;
-        w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
-    }
-    SplatCommon<PD>::template sort_splats<0>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
-    cp_async_wait_all();
-    __syncthreads();
-
-    // warp-uniform walk over a contiguous chunk of the sorted splats, lanes over channels
-    const double scale = fixed_scale(hdr);
-    const int total = nvalid * (PD + 1);
-    const int chunk = (total + NW - 1) / NW;
-    const int beg = warp * chunk, end = min(total, beg + chunk);
-    if (beg >= end) return;
-    for (int j0 = 0; j0 < vd; j0 += 32) {
-        const int j = j0 + lane;
-        long long acc = 0;
-        int cur = (int)(sorted_s[beg].x >> 16);
-        for (int sidx = beg; sidx < end; sidx++) {
-            const uint2 pw = sorted_s[sidx];
-            const int e = (int)(pw.x >> 16);
-            if (e != cur) {
-                if (j < vd && acc)
-                    atomicAdd(reinterpret_cast<u64*>(v64 + (size_t)list_ref[base + cur] * VP + j), (u64)acc);
-                acc = 0;
-                cur = e;
-            }
-            if (j < vd) {
-                const float wt = __uint_as_float(pw.y);
-                const float prod = (j < C) ? PL_FMUL(wt, in_s[(pw.x & 0xFFFFu) * C + j]) : wt;
-                acc += __double2ll_rn(PL_DMUL((double)prod, scale));
-            }
-        }
-        if (j < vd && acc)
-            atomicAdd(reinterpret_cast<u64*>(v64 + (size_t)list_ref[base + cur] * VP + j), (u64)acc);
-    }
-}
-
 // fixed-point sums -> float rows
 __global__ void __launch_bounds__(256)
 convert_fixed(const Header* hdr, const long long* __restrict__ v64, float* __restrict__ v0, int vp) {
     after_previous_kernel();
     if (hdr->status != 0) return;
-    const double inv = 1.0 / fixed_scale(hdr);
+    const double inv = __longlong_as_double((long long)(1023 - fixed_exponent(hdr)) << 52);
     const u64 cells = (u64)hdr->num_vertices * vp;
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += (u64)gridDim.x * blockDim.x)
         v0[i] = (float)PL_DMUL(__ll2double_rn(v64[i]), inv);

@@ -88,3 +88,27 @@ def test_every_width_class_in_double(shape, r, gpu, oracle):
             got = plb.lattice_filter(x, rt, True, 4.0, 0.2, reverse=reverse).cpu().numpy()
             # double sums in another order: the bound of every comparison in double with the oracle
             assert rel_l2(got, want[..., :c]) <= 1e-12, "%d channels" % c
+
+
+@pytest.mark.parametrize("scale", [1e-3, 1.0, 1e3, 1e30])
+@pytest.mark.parametrize("shape,r", [((35, 32), 3), ((18, 33), 3), ((5, 9, 11), 1)])
+def test_fixed_point_sums_at_every_width(shape, r, scale, gpu, oracle):
+    """The deterministic mode at every lane count: identical bits from run to run and through a kept lattice."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from conftest import bits
+    rng = np.random.default_rng(71)
+    ref = rng.random((2,) + shape + (r,), dtype=np.float32)
+    wide = (scale * rng.standard_normal((2,) + shape + (70,))).astype(np.float32)
+    rt = torch.from_numpy(ref).cuda()
+    for c in (1, 3, 4, 6, 8, 13, 21, 30, 40, 70):
+        inp = np.ascontiguousarray(wide[..., :c])
+        x = torch.from_numpy(inp).cuda()
+        got = plb.lattice_filter(x, rt, True, 4.0, 0.2, mode="deterministic").cpu().numpy()
+        again = plb.lattice_filter(x, rt, True, 4.0, 0.2, mode="deterministic").cpu().numpy()
+        kept = plb.Lattice(rt, None, True, 4.0, 0.2, max_channels=c, mode="deterministic").apply(
+            x, mode="deterministic").cpu().numpy()
+        assert np.array_equal(bits(got), bits(again)) and np.array_equal(bits(got), bits(kept))
+        if scale <= 1e3:
+            # the grid, 2^-36 of at most 8e3, is 1e-7 of the weights and finer than that of the values
+            gpu.assert_outputs_close(got / scale, oracle.lattice_filter(inp, ref, True, 4.0, 0.2) / scale, "%d channels" % c)
