@@ -104,12 +104,12 @@ struct Cfg {
     static constexpr int LS = 1 << LSLOG;
     static_assert(5 * SPLATS <= 2 * LS && SPLATS <= 65535, "slots hold 16-bit splat numbers");
     // The tile's splats sorted by entry, as build_tiles leaves them for the splat kernels: cut into windows
-    // of WL splats, each followed by one spare 8-byte word (lanes that walk neighbouring windows in step then
-    // read words an odd number of 8-byte words apart: no shared-memory bank collisions), SREC words per tile
-    // (even: the list moves by bulk copies, whose sizes are multiples of 16 bytes).
+    // of WL splats, each followed by two spare 8-byte words: lanes that walk neighbouring windows in step read two
+    // splats at once, and windows an odd number of 16-byte words apart do not collide on shared-memory banks.  SREC
+    // words per tile (even: the list moves by bulk copies, whose sizes are multiples of 16 bytes).
     static constexpr int WL = 8 * (PD + 1);
-    static constexpr int SREC = (SPLATS + SPLATS / WL + 1 + 1) & ~1;
-    __host__ __device__ static constexpr int srec_slot(int pos) { return pos + pos / WL; }
+    static constexpr int SREC = SPLATS + 2 * (SPLATS / WL);
+    __host__ __device__ static constexpr int srec_slot(int pos) { return pos + 2 * (pos / WL); }
     // What build_tiles keeps of the keys in shared memory (see TileKeys): every splat's key up to pd = 8, one
     // record per point above (a key of 16 coordinates for each of 17 splats would leave room for two CTAs an SM).
     static constexpr bool COMPACT = PD > 8;

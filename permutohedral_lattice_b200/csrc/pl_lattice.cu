@@ -174,7 +174,7 @@ static int kw_of(int pd) { return (pd + 1 + 3) / 4; }
 // 8-byte words of a tile's sorted splat list (Cfg<PD>::SREC)
 static int srec_words_of(int pd) {
     const int splats = tp_of(pd) * (pd + 1), wl = 8 * (pd + 1);
-    return (splats + splats / wl + 1 + 1) & ~1;
+    return splats + 2 * (splats / wl);
 }
 
 static bool pd_supported(int pd) {

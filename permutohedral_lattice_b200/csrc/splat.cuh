@@ -28,14 +28,14 @@ struct SplatCommon {
     // Words of the sorted list when it is cut into windows (one spare word per window, WL >= PD + 1).
     static constexpr int SORTED = SPLATS + TP;
 
-    // WL > 0 stores sorted position pos at slot(pos): the list is cut into windows of WL splats, each
-    // followed by one spare word.  Splats of one entry (written together by neighbouring lanes) land in
+    // Sorted position pos is stored at slot(pos): the list is cut into windows of WL splats, each followed by two
+    // spare words (Cfg<PD>::WL, see there) or by one.  Splats of one entry (written together by neighbouring lanes) land in
     // neighbouring words, and lanes that walk neighbouring windows in step read words WL + 1 apart: an
     // odd number of 8-byte words, so neither side collides on shared-memory banks.
     template <int WL>
     __device__ static __forceinline__ int slot(int pos) {
-        if constexpr (WL == 0)
-            return pos;
+        if constexpr (WL == Cfg<PD>::WL)
+            return Cfg<PD>::srec_slot(pos);
         else
             return pos + pos / WL;
     }
@@ -487,7 +487,8 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     wait_for_previous_kernel();
     if (call_failed(hdr)) return;   // a failure of the index stage
 
-    const int lw_log2 = LR > 16 ? 5 : LR > 8 ? 4 : LR > 4 ? 3 : LR > 2 ? 2 : LR > 1 ? 1 : 0;
+    // (two lanes at least, so that a window starts on an even splat)
+    const int lw_log2 = LR > 16 ? 5 : LR > 8 ? 4 : LR > 4 ? 3 : LR > 2 ? 2 : 1;
     const int LW = 1 << lw_log2, wl = LW * (PD + 1);   // lanes of a window, its splats
     const int first = (tid >> lw_log2) * wl, end = min(first + wl, total);
     constexpr bool ONE = VD > 16 && VD <= 32;          // known: a lane has one quad, a window is one stretch
@@ -502,18 +503,24 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
             for (int pos = first; pos < end; pos += WL) {
                 const uint2* sp = sorted_s + Cfg<PD>::srec_slot(pos);
                 const int count = min(WL, end - pos);
-#pragma unroll 4
-                for (int i = 0; i < count; i++) {
-                    const uint2 pw = sp[i];
-                    const int e = (int)(pw.x >> 16);
+auto one = [&](unsigned key, unsigned weight) {
+                    const int e = (int)(key >> 16);
                     if (e != cur) {
                         acc.flush(v0 + (size_t)vcur * VP + 4 * h);
                         acc.clear();
                         cur = e;
                         vcur = list_ref[base + cur];
                     }
-                    acc.add(__uint_as_float(pw.y), in4[(pw.x & 0xFFFFu) * LR]);
+                    acc.add(__uint_as_float(weight), in4[(key & 0xFFFFu) * LR]);
+                };
+                int i = 0;
+#pragma unroll 2
+                for (; i + 1 < count; i += 2) {   // two splats a load
+                    const uint4 pw = *reinterpret_cast<const uint4*>(sp + i);
+                    one(pw.x, pw.y);
+                    one(pw.z, pw.w);
                 }
+                if (i < count) one(sp[i].x, sp[i].y);
                 if constexpr (ONE) break;
             }
             let_next_kernel_start();   // what is left of this thread's work: its last row
