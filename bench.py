@@ -53,8 +53,8 @@ def parse_args():
                     help="the timed blocks of --steps steps are repeated until they fill this much device time")
     ap.add_argument("--no-weak", action="store_true", help="skip the extra weak-scaling measurement at N > 1")
     ap.add_argument("--channels", type=int, default=0,
-                    help="override the channel count of configuration 2 / 5 (value widths without a register-resident "
-                         "instantiation run the generic splat / slice kernels)")
+                    help="override the channel count of configuration 2 / 5 (widths other than 1, 2, 3 and 21 run the splat "
+                         "whose width is known at run time only)")
     ap.add_argument("--headline-only", action="store_true",
                     help="only the device-resident measurement (no end-to-end, gather, reuse, graph or weak-scaling "
                          "legs): short runs for profiler captures")
