@@ -75,7 +75,7 @@ struct Watch {
 };
 __device__ __forceinline__ void report_to(const Watch& w, const Header* hdr) {
     if (w.word && grid_thread() == 0) {
-        const u64 v = ((u64)w.seq << 40) | ((u64)(hdr->status & 0xFFu) << 32) | (u64)hdr->num_entries;
+        const u64 v = ((u64)w.seq << 40) | ((u64)(__ldcg(&hdr->status) & 0xFFu) << 32) | (u64)hdr->num_entries;
         asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(w.word), "l"(v) : "memory");
     }
 }

@@ -38,6 +38,7 @@
 #include "direct_index.cuh"
 #include "splat.cuh"
 #include "blur_slice.cuh"
+#include "small.cuh"
 #include "export.cuh"
 #include "fp64.cuh"
 #include "crf.cuh"
@@ -461,6 +462,14 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
      : padded_vd(vd) == 32 ? launch_slice<PD_, 32>(__VA_ARGS__) \
                            : launch_slice<PD_, 0>(__VA_ARGS__))
 
+// Which calls take the one-cluster kernels of small.cuh, by the bounds the host knows.
+// RGB calls one after another, wide -> one cluster, us a call: 33x45, 573 entries 43 -> 34; 48x56, 806 entries 43 -> 36;
+// 8910 entries, all vertices, 59 -> 67; 16128 of them 73 -> 108: the two lines cross at about 6700 entries.  A blur of
+// SMALL_ITEMS pieces is two trips a thread and pass, as many as the index has where the lines cross.
+constexpr u64 SMALL_ENTRIES = 6144, SMALL_ITEMS = 16384;
+static bool small_index(const Layout& L) { return L.max_entries <= SMALL_ENTRIES; }
+static bool small_blur(const Layout& L, u32 vpr) { return L.max_entries * vpr <= SMALL_ITEMS; }
+
 enum { PH_BUILD = 1, PH_APPLY = 2 };   // halves of a call: lattice structure / values through it
 
 template <int PD>
@@ -511,7 +520,6 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             PL_LAUNCH((build_tiles<PD, float, true>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         }
-        PL_COUNT_LAUNCHES(4);   // build_tiles and the three launches of the index stage below
         if (ev) PL_CUDA(cudaEventRecord(ev[1], st));
         Direct direct;
         bool use_direct = false;
@@ -533,7 +541,11 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
                                                                  L.max_entries, take_watch());
             }
         }
-        if (!use_direct) {
+        const bool small = !use_direct && small_index(L);
+        PL_COUNT_LAUNCHES(small ? 2 : 4);   // build_tiles and the launches of the index stage
+        if (small) {
+            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch());
+        } else if (!use_direct) {
             // the value rows are zeroed by the link launch, whose lookups leave the memory system idle
             void* zrows = vinit.rows;
             vinit.rows = nullptr;
@@ -573,13 +585,17 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     float* src = v0;
     float* dst = v1;
     const u32 qpr = (u32)padded_vd(vd) / 4;
-    for (int step = 0; step <= PD; step++) {
+    if (small_blur(L, qpr)) {
+        PL_LAUNCH_AFTER(OV_BLUR, (blur_small<float4>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, nbr, L.max_entries, reinterpret_cast<float4*>(v0), reinterpret_cast<float4*>(v1), qpr, PD + 1, reverse);
+        PL_COUNT_LAUNCHES(1);
+        if (PD % 2 == 0) src = v1;   // an odd number of passes
+    } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * L.max_entries * 2;
         PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<float4>), wide, 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
         float* tmp = src; src = dst; dst = tmp;
+        PL_COUNT_LAUNCHES(1);
     }
-    PL_COUNT_LAUNCHES(PD + 1);
     if (ev) PL_CUDA(cudaEventRecord(ev[4], st));
     rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, st);
     if (rc != PL_OK) return rc;
@@ -640,7 +656,10 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
                                                              L.max_entries, take_watch());
         }
     }
-    if (!use_direct) {
+    const bool small = !use_direct && small_index(L);
+    if (small) {
+        PL_LAUNCH((index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch());
+    } else if (!use_direct) {
         PL_LAUNCH((clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         PL_LAUNCH((insert_entries<KW>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, vinit);
         PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, list_ref, vid, vkeys, nbr, L.max_entries,
@@ -650,13 +669,17 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
                                                                       list_ref, v0, vd);
     double* src = v0;
     double* dst = v1;
-    for (int step = 0; step <= PD; step++) {
+    const bool one_blur = small_blur(L, (u32)vp / 2);
+    if (one_blur) {
+        PL_LAUNCH((blur_small<double2>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, nbr, L.max_entries, reinterpret_cast<double2*>(v0), reinterpret_cast<double2*>(v1), (u32)vp / 2, PD + 1, reverse);
+        if (PD % 2 == 0) src = v1;   // an odd number of passes
+    } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         PL_LAUNCH((blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
     PL_LAUNCH((slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd);
-    PL_COUNT_LAUNCHES(4 + 1 + (PD + 1) + 1);   // build and index (3); splat; blur passes; slice
+    PL_COUNT_LAUNCHES((small ? 2 : 4) + 1 + (one_blur ? 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;
 }

@@ -97,3 +97,29 @@ def test_verified_calls_from_several_threads(gpu):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("pd,n", [(1, 8200), (2, 5470), (3, 4100), (5, 2735), (8, 1825), (16, 970)])
+def test_small_lattices_give_the_bits_of_wide_ones(pd, n, gpu, oracle):
+    """A bound of 6144 entries is the largest that takes the one-cluster index, and with it rows of up to two quads
+    take the one-cluster blur (16384 quads).  Deterministic sums make small and wide comparable."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(79)
+    pos = np.repeat(rng.standard_normal((1, (n + 4) // 5, pd)), 5, 1)[:, :n].astype(np.float32)
+    pt = torch.from_numpy(pos).cuda()
+    assert n * (pd + 1) > 16384   # the worst case: wide launches
+    for c in (1, 3, 4, 7, 8):
+        val = rng.standard_normal((1, n, c)).astype(np.float32)
+        x = torch.from_numpy(val).cuda()
+        for reverse in (False, True):
+            small = plb.filter_positions(x, pt, reverse=reverse, mode="deterministic", max_entries=6144)[0].clone()
+            wide = plb.filter_positions(x, pt, reverse=reverse, mode="deterministic", max_entries=0)[0].clone()
+            assert torch.equal(small, wide), "pd %d, %d channels" % (pd, c)
+        x64, p64 = x.double(), pt.double()
+        small = plb.filter_positions(x64, p64, max_entries=6144)[0].clone()
+        wide = plb.filter_positions(x64, p64, max_entries=0)[0].clone()
+        # double sums in varying order
+        assert float((small - wide).norm() / wide.norm()) <= 1e-12, "pd %d, %d channels in double" % (pd, c)
+    got = plb.filter_positions(x, pt, max_entries=6144)[0].cpu().numpy()[0]
+    gpu.assert_outputs_close(got, oracle.filter(val[0], pos[0], structure=False).out, "pd %d" % pd)
