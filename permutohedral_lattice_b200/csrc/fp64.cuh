@@ -48,7 +48,11 @@ splat_tiles_f64(Geom g, const double* __restrict__ input, Header* hdr, const int
     int* cur_s = reinterpret_cast<int*>(sorted_s + Splat64<PD>::SORTED);       // [SPLATS]
     int* prow_s = cur_s + SPLATS;                                              // [TP]
     __shared__ int wsum_s[32];
-    if (call_failed(hdr)) return;
+    // Launched to overlap the tail of link_neighbours, as splat_tiles_rows is: the input and the records are older.
+    if (call_failed(hdr)) {
+        wait_for_previous_kernel();
+        return;
+    }
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
     const int2 info = tile_info[tile];
@@ -89,6 +93,10 @@ splat_tiles_f64(Geom g, const double* __restrict__ input, Header* hdr, const int
         for (int j = max(chans, 0); j < width; j++) in_s[tid * width + j] = (j0 + j == C) ? 1.0 : 0.0;
         if (j0 == 0) SplatCommon<PD>::template sort_splats<WL>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
         cp_async_wait_all();
+        if (j0 == 0) {
+            wait_for_previous_kernel();     // from here on the entries' vertices and the zeroed rows
+            if (call_failed(hdr)) return;   // a failure of the index stage
+        }
         __syncthreads();
 
         const int pairs = width >> 1, lw_log2 = lanes_log2_f64(pairs);
@@ -146,6 +154,7 @@ slice_tiles_f64(Geom g, double* __restrict__ output, const Header* hdr, const in
     __shared__ int prow_s[TP];
     if (call_failed(hdr)) {
         poison_tile_output(g, output, C);
+        wait_for_previous_kernel();
         return;
     }
     const TilePos tpos = this_tile(g);
@@ -161,6 +170,7 @@ slice_tiles_f64(Geom g, double* __restrict__ output, const Header* hdr, const in
         w_s[r * TP + tid] = valid ? recw_tile[r * TP + tid] : 0.0;
         v_s[r * TP + tid] = valid ? list_ref[base + rec_tile[r * TP + tid]] : 0u;
     }
+    wait_for_previous_kernel();   // the last blur pass: all that was read up to here is older
     __syncwarp();   // a warp reads the points its own lanes have written
     const int lw_log2 = lanes_log2_f64(pairs), lw = 1 << lw_log2;
     const int h = lane & (lw - 1), group = lane >> lw_log2;

@@ -634,6 +634,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     int table_log2 = 0;
     while ((1ull << table_log2) < L.table_slots) table_log2++;
     const int vp = padded_vd_f64(vd);
+    const bool small_table = L.table_slots <= (1ull << 23);   // (as for float)
 
     PL_LAUNCH((build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
     // spatial-only calls index their vertices directly, as the float calls do (the key bounds hold for
@@ -650,35 +651,35 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     vinit.row_bytes = (u32)vp * 8u;
     if constexpr (PD <= MAX_SDIMS) {
         if (use_direct) {
-            PL_LAUNCH((clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
-            PL_LAUNCH((insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
+            PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
+            PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH((link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
                                                              L.max_entries, take_watch());
         }
     }
     const bool small = !use_direct && small_index(L);
     if (small) {
-        PL_LAUNCH((index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch());
+        PL_LAUNCH_AFTER(OV_CLEAR, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch());
     } else if (!use_direct) {
-        PL_LAUNCH((clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
-        PL_LAUNCH((insert_entries<KW>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, vinit);
+        PL_LAUNCH_AFTER(OV_CLEAR, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+        PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, list_keys, list_ref, vid, vkeys, vinit);
         PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   nullptr, 0u, take_watch());
     }
-    PL_LAUNCH((splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
+    PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                       list_ref, v0, vd);
     double* src = v0;
     double* dst = v1;
     const bool one_blur = small_blur(L, (u32)vp / 2);
     if (one_blur) {
-        PL_LAUNCH((blur_small<double2>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, nbr, L.max_entries, reinterpret_cast<double2*>(v0), reinterpret_cast<double2*>(v1), (u32)vp / 2, PD + 1, reverse);
+        PL_LAUNCH_AFTER(OV_BLUR, (blur_small<double2>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, nbr, L.max_entries, reinterpret_cast<double2*>(v0), reinterpret_cast<double2*>(v1), (u32)vp / 2, PD + 1, reverse);
         if (PD % 2 == 0) src = v1;   // an odd number of passes
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        PL_LAUNCH((blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+        PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
-    PL_LAUNCH((slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd);
+    PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd);
     PL_COUNT_LAUNCHES((small ? 2 : 4) + 1 + (one_blur ? 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;
