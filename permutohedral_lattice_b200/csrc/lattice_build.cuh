@@ -491,7 +491,17 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
     }
     u32 lg = 10;
     while (lg < max_log2 && (1ull << lg) < need) lg++;
-    if (blockIdx.x == 0 && threadIdx.x == 0) hdr->table_log2 = lg;
+    const u32 filter_log2 =
+        (lg >= FILTER_MIN_LOG2 && lg < max_log2) ? min(lg + FILTER_BITS_LOG2, FILTER_MAX_LOG2) : 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        hdr->table_log2 = lg;
+        hdr->filter_log2 = filter_log2;
+    }
+    if (filter_log2) {
+        uint4* filter = reinterpret_cast<uint4*>(filter_words(table, max_log2, filter_log2));
+        for (u64 i = grid_thread(); i < (1ull << (filter_log2 - 7)); i += grid_threads())
+            filter[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
     const u64 cap = 1ull << lg;
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (u64)gridDim.x * blockDim.x)
         table[i] = EMPTY_SLOT;
@@ -577,7 +587,7 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
 // list_keys, which the previous launch has completely written).
 template <int KW>
 __global__ void __launch_bounds__(256)
-insert_entries(Header* hdr, u64* __restrict__ table, const Key<KW>* __restrict__ list_keys,
+insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>* __restrict__ list_keys,
                u32* __restrict__ list_ref, u32* __restrict__ vid, Key<KW>* __restrict__ vkeys, VertexInit vi) {
     after_previous_kernel();
     __shared__ InsertRound rd;
@@ -585,6 +595,8 @@ insert_entries(Header* hdr, u64* __restrict__ table, const Key<KW>* __restrict__
     if (call_failed(hdr)) return;   // (its barrier also publishes rd.count)
     const u32 T = hdr->num_entries;
     const u64 mask = (1ull << hdr->table_log2) - 1;
+    const u32 filter_log2 = hdr->filter_log2;
+    u32* filter = filter_log2 ? filter_words(table, max_log2, filter_log2) : nullptr;
     const u32 stride = gridDim.x * 256u;
     for (u32 start = blockIdx.x * 256u; start < T;) {
         for (int c = 0; c < INSERT_CHUNKS && start < T; c++, start += stride) {
@@ -604,7 +616,16 @@ insert_entries(Header* hdr, u64* __restrict__ table, const Key<KW>* __restrict__
                     u64 cur = __ldcg(&table[s]);
                     if (cur == EMPTY_SLOT) {
                         cur = atomicCAS(&table[s], EMPTY_SLOT, mine);
-                        if (cur == EMPTY_SLOT) { ref = t; winner = true; my_slot = s; break; }
+                        if (cur == EMPTY_SLOT) {
+                            ref = t;
+                            winner = true;
+                            my_slot = s;
+                            if (filter) {
+                                const u32 bit = (u32)h & ((1u << filter_log2) - 1u);
+                                atomicOr(filter + (bit >> 5), 1u << (bit & 31u));
+                            }
+                            break;
+                        }
                     }
                     if ((u32)(cur >> 32) == (u32)(h >> 32)) {
                         const u32 low = (u32)cur;
@@ -663,7 +684,8 @@ __host__ __device__ constexpr u64 axis_hash(int a) {          // and to its line
     return h;
 }
 template <int PD, int A>
-__device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mask,
+__device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mask, const u32* __restrict__ filter,
+                                          u32 filter_mask,
                                           const Key<Cfg<PD>::KW>* __restrict__ vkeys, u32 M, int* __restrict__ nbr,
                                           u64 max_entries) {
     constexpr int KW = Cfg<PD>::KW;
@@ -671,6 +693,10 @@ __device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mas
     for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < M; v += gridDim.x * blockDim.x) {
         Key<KW> k = vkeys[v];
         const u64 h = mix_hash(linear_hash<KW>(k) + axis_hash<PD>(A));
+        if (filter) {
+            const u32 bit = (u32)h & filter_mask;
+            if (!((__ldg(filter + (bit >> 5)) >> (bit & 31u)) & 1u)) continue;
+        }
 #pragma unroll
         for (int j = 0; j < KW; j++) k.w[j] += axis_word<PD>(A, j);
         u64 s = h & mask;
@@ -702,7 +728,7 @@ struct LinkAxis {   // link_axis of the axis this block works on, chosen once pe
 
 template <int PD>
 __global__ void __launch_bounds__(256)
-link_neighbours(const Header* hdr, const u64* __restrict__ table, u32* __restrict__ list_ref,
+link_neighbours(const Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restrict__ list_ref,
                 const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys, int* __restrict__ nbr,
                 u64 max_entries, void* zero_rows_ptr, u32 zero_row_bytes, Watch watch) {
     after_previous_kernel();
@@ -716,7 +742,9 @@ link_neighbours(const Header* hdr, const u64* __restrict__ table, u32* __restric
         const u64 quads = (u64)M * (zero_row_bytes / 16);
         for (u64 i = grid_thread(); i < quads; i += grid_threads()) rows[i] = make_uint4(0u, 0u, 0u, 0u);
     }
-    LinkAxis<PD, 0>::run((int)blockIdx.y, table, mask, vkeys, M, nbr, max_entries);
+    const u32 filter_log2 = hdr->filter_log2;
+    const u32* filter = filter_log2 ? filter_words(table, max_log2, filter_log2) : nullptr;
+    LinkAxis<PD, 0>::run((int)blockIdx.y, table, mask, filter, (1u << filter_log2) - 1u, vkeys, M, nbr, max_entries);
 }
 
 }  // namespace pl

@@ -123,3 +123,16 @@ def test_small_lattices_give_the_bits_of_wide_ones(pd, n, gpu, oracle):
         assert float((small - wide).norm() / wide.norm()) <= 1e-12, "pd %d, %d channels in double" % (pd, c)
     got = plb.filter_positions(x, pt, max_entries=6144)[0].cpu().numpy()[0]
     gpu.assert_outputs_close(got, oracle.filter(val[0], pos[0], structure=False).out, "pd %d" % pd)
+
+
+def test_filter_in_front_of_a_large_table(gpu, oracle):
+    """2.9 M vertices in a table of 2^23 slots, half of what the workspace has room for: the lookups pass the filter."""
+    rng = np.random.default_rng(73)
+    ref = np.repeat(rng.random((1, 1024, 360, 3), dtype=np.float32), 2, 2)
+    inp = rng.random((1, 1024, 720, 1), dtype=np.float32)
+    want, items = oracle.lattice_filter(inp, ref, True, 3.0, 0.05, 1.0, False, structure=True)
+    out, ws, call, _, rt = gpu.run_op(inp, ref, True, 3.0, 0.05, 1.0, False, max_entries=0)
+    st, (vk, vi, pv, pw) = gpu.export_op(ws, call, rt)
+    assert st.table_slots == 1 << 23
+    gpu.assert_structure_equal(vk, vi, pv, pw, items, "large table")
+    gpu.assert_outputs_close(out.cpu().numpy(), want, "large table")
