@@ -534,15 +534,49 @@ auto one = [&](unsigned key, unsigned weight) {
 // ---------------------------------------------------------------------------------------------
 // Deterministic mode: the input's largest magnitude before the splat, the sums as floats after it.
 // ---------------------------------------------------------------------------------------------
+// One pass over the input, 16 bytes a load and four loads in flight (4-byte loads one by one reached 1.9 TB/s); the up
+// to three floats before the first 16-byte boundary and after the last go one by one.  2 x 512x512 x 21, forward +
+// backward: 491 -> 466 us.
 __global__ void __launch_bounds__(256)
 absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
     after_previous_kernel();
     u32 m = 0;
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (u64)gridDim.x * blockDim.x)
-        m = max(m, __float_as_uint(fabsf(input[i])));
+    auto take = [&](float x) { m = max(m, __float_as_uint(fabsf(x))); };
+    const u64 lead = min(count, (u64)(((16u - ((u32)(uintptr_t)input & 15u)) & 15u) >> 2));
+    const u64 quads = (count - lead) >> 2, tail = lead + 4 * quads, stride = (u64)gridDim.x * blockDim.x;
+    const u64 first = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+    const float4* __restrict__ in4 = reinterpret_cast<const float4*>(input + lead);
+    u64 i = first;
+    for (; i + 3 * stride < quads; i += 4 * stride) {
+        float4 x[4];
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, d));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(&hdr->absmax_bits, m);
+        for (int k = 0; k < 4; k++) x[k] = __ldg(in4 + i + k * stride);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            take(x[k].x);
+            take(x[k].y);
+            take(x[k].z);
+            take(x[k].w);
+        }
+    }
+    for (; i < quads; i += stride) {
+        const float4 x = __ldg(in4 + i);
+        take(x.x);
+        take(x.y);
+        take(x.z);
+        take(x.w);
+    }
+    if (first < lead) take(input[first]);
+    if (first < count - tail) take(input[tail + first]);
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    __shared__ u32 m_s[8];
+    if ((threadIdx.x & 31) == 0) m_s[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 1; k < 8; k++) m = max(m, m_s[k]);
+        if (m) atomicMax(&hdr->absmax_bits, m);
+    }
 }
 
 // fixed-point sums -> float rows

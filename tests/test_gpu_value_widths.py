@@ -112,3 +112,19 @@ def test_fixed_point_sums_at_every_width(shape, r, scale, gpu, oracle):
         if scale <= 1e3:
             # the grid, 2^-36 of at most 8e3, is 1e-7 of the weights and finer than that of the values
             gpu.assert_outputs_close(got / scale, oracle.lattice_filter(inp, ref, True, 4.0, 0.2) / scale, "%d channels" % c)
+
+
+def test_grid_follows_the_largest_value_wherever_it_lies(gpu):
+    """The largest magnitude among the floats before the first 16-byte boundary, in the vector loads or after the last
+    one: a grid too fine for it would overflow the sums, one too coarse lose the constant 1 around it."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    ref = torch.zeros((1, 16, 19, 1), device="cuda")
+    for offset in (0, 1, 2, 3):
+        for where in (0, 1, 3, 4, 150, 299, 300, 301, 302, 303):
+            flat = torch.ones(16 * 19 + offset, device="cuda")
+            x = flat[offset:].view(1, 16, 19, 1)
+            x.view(-1)[where] = -1e30
+            out, ws, _ = plb.lattice_filter_raw(x, ref, True, 4.0, 0.2, mode="deterministic")
+            bits = int(ws[16:20].view(torch.int32).item())      # the header's word for the largest magnitude
+            assert bits == int(np.float32(1e30).view(np.int32)), (offset, where)
