@@ -559,7 +559,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         if (ev) PL_CUDA(cudaEventRecord(ev[2], st));
     } else {
         if (ev) { PL_CUDA(cudaEventRecord(ev[1], st)); }
-        PL_LAUNCH((zero_rows), wide, 256, 0, st, hdr, v0, v64, padded_vd(vd));
+        PL_LAUNCH_AFTER(OV_CLEAR, (zero_rows), wide, 256, 0, st, hdr, v0, v64, padded_vd(vd));
         PL_COUNT_LAUNCHES(1);
         if (ev) { PL_CUDA(cudaEventRecord(ev[2], st)); }
     }
