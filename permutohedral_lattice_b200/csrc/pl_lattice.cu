@@ -464,9 +464,9 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
 
 // Which calls take the one-cluster kernels of small.cuh, by the bounds the host knows.
 // RGB calls one after another, wide -> one cluster, us a call: 33x45, 573 entries 43 -> 34; 48x56, 806 entries 43 -> 36;
-// 8910 entries, all vertices, 59 -> 67; 16128 of them 73 -> 108: the two lines cross at about 6700 entries.  A blur of
-// SMALL_ITEMS pieces is two trips a thread and pass, as many as the index has where the lines cross.
-constexpr u64 SMALL_ENTRIES = 6144, SMALL_ITEMS = 16384;
+// 8910 entries, all vertices, 59 -> 67; 16128 of them 73 -> 108: the two lines cross at about 6700 entries.  The blur
+// alone, all vertices: 8910 rows of one piece 58 -> 62, 16128 of them 73 -> 78, so one piece a thread at most.
+constexpr u64 SMALL_ENTRIES = 6144, SMALL_ITEMS = SMALL_CTAS * SMALL_THREADS;
 static bool small_index(const Layout& L) { return L.max_entries <= SMALL_ENTRIES; }
 static bool small_blur(const Layout& L, u32 vpr) { return L.max_entries * vpr <= SMALL_ITEMS; }
 
