@@ -8,6 +8,7 @@ device memory and streams only, every computation happens in libpl_lattice.so th
 import ctypes
 
 import torch
+from torch.autograd import forward_ad
 from torch.multiprocessing.reductions import StorageWeakRef
 
 from . import capi
@@ -523,7 +524,7 @@ def lattice_filter(input_image, reference_image, bilateral=True, theta_alpha=1.0
     The thetas are float attributes of the op (src/LatticeFilterKernel.cpp:36-38): they are rounded to
     float32 here and widened again for float64 tensors, as the reference does (:131-142)."""
     thetas = (_as_attr(theta_alpha), _as_attr(theta_beta), _as_attr(theta_gamma))
-    if not (torch.is_grad_enabled() and (input_image.requires_grad or (
+    if not _watched_by_torch() and not (torch.is_grad_enabled() and (input_image.requires_grad or (
             reference_image is not None and reference_image.requires_grad))):
         # nothing to differentiate: the autograd function would only add its own cost (a tenth of a small call)
         if not reuse_lattice:
@@ -532,6 +533,14 @@ def lattice_filter(input_image, reference_image, bilateral=True, theta_alpha=1.0
                        max_channels=input_image.shape[-1], mode=mode).apply(input_image, bool(reverse), mode)
     fn = _LatticeFilterReuseFunction if reuse_lattice else _LatticeFilterFunction
     return fn.apply(input_image, reference_image, bool(bilateral), *thetas, bool(reverse), mode)
+
+
+def _watched_by_torch():
+    """True while something other than reverse mode follows the tensors: a tracer, forward-mode differentiation, a
+    functorch transform.  None of them sees the kernels, which go through ctypes; the autograd function is what tells
+    a tracer that there was a call, and what makes the others refuse it."""
+    return (torch._C._get_tracing_state() is not None or forward_ad._current_level >= 0 or
+            torch._C._functorch.maybe_current_level() is not None or torch.compiler.is_compiling())
 
 
 def _as_attr(v):
