@@ -228,6 +228,9 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
         R* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
         for (int r = 0; r <= PD; r++) recw_tile[r * TP + tid] = w[r];
+        // COMPACT: a slot is written by the key that the steps below give and read by the one that the stored ranks
+        // give.  Where the ranks were no permutation the two differed, and the slot read was one that no splat had written.
+        if constexpr (COMPACT) settle_ranks<PD>(s);
         PointKeys<PD> k;
         k.start(s);
         if constexpr (COMPACT) {

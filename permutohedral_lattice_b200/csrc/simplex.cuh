@@ -225,6 +225,20 @@ PL_HD void barycentric(const Simplex<PD>& s, float* bary /* PD+1 */) {
     bary[0] = (float)PL_DADD((double)by_rank[PD], PL_DADD(1.0, (double)(-by_rank[0])));
 }
 
+// Makes the ranks 0..PD, each once, which is what they are unless the features are NaN, infinite or beyond the
+// integers of a float (double: of 16 bits).  Such a point has no simplex, but two ways of deriving its keys from its
+// ranks must still agree (build_tiles, pd > 8).
+template <int PD, typename S>
+PL_HD void settle_ranks(S& s) {
+    unsigned seen = 0;
+#pragma unroll
+    for (int i = 0; i <= PD; i++) seen |= (unsigned)s.rank[i] <= (unsigned)PD ? 1u << s.rank[i] : 0u;
+    if (seen != (2u << PD) - 1u) {
+#pragma unroll
+        for (int i = 0; i <= PD; i++) s.rank[i] = i;
+    }
+}
+
 // Coordinate i (< PD) of the remainder-r vertex of the simplex (src/PermutohedralLatticeCPU.h:297-304).
 template <int PD>
 PL_HD int16_t vertex_coord(const Simplex<PD>& s, int i, int r) {

@@ -56,6 +56,38 @@ extern "C" int simplex_host_f64(const double* pos, const double* scale, int n, i
     return 1;
 }
 
+// What build_tiles derives a point's keys from: the low 16 bits of its remainder-0 coordinates and its ranks, as the
+// simplex search leaves them and settled.
+template <int PD, typename S, typename R, void FIND(const R*, const R*, S&)>
+static void point_records(const R* pos, const R* scale, int n, uint16_t* low16, int* found, int* settled) {
+    for (int p = 0; p < n; p++) {
+        S s;
+        FIND(pos + (size_t)p * PD, scale, s);
+        for (int i = 0; i < PD; i++) low16[(size_t)p * PD + i] = (uint16_t)pl::rem0_low16<PD>(s, i);
+        for (int i = 0; i <= PD; i++) found[(size_t)p * (PD + 1) + i] = s.rank[i];
+        pl::settle_ranks<PD>(s);
+        for (int i = 0; i <= PD; i++) settled[(size_t)p * (PD + 1) + i] = s.rank[i];
+    }
+}
+template <int PD>
+static void records(const void* pos, const void* scale, int n, int f64, uint16_t* low16, int* found, int* settled) {
+    if (f64)
+        point_records<PD, pl::Simplex64<PD>, double, pl::find_simplex_f64<PD>>(
+            static_cast<const double*>(pos), static_cast<const double*>(scale), n, low16, found, settled);
+    else
+        point_records<PD, pl::Simplex<PD>, float, pl::find_simplex<PD>>(
+            static_cast<const float*>(pos), static_cast<const float*>(scale), n, low16, found, settled);
+}
+extern "C" int point_records_host(const void* pos, const void* scale, int n, int pd, int f64, uint16_t* low16,
+                                  int* found, int* settled) {
+    switch (pd) {
+        case 2: records<2>(pos, scale, n, f64, low16, found, settled); return 0;
+        case 5: records<5>(pos, scale, n, f64, low16, found, settled); return 0;
+        case 16: records<16>(pos, scale, n, f64, low16, found, settled); return 0;
+    }
+    return 1;
+}
+
 // a / b through the reciprocal-based division used for the features; rcp = RN(1 / b).
 extern "C" void div_by_rcp_host(const float* a, float b, int n, float* out) {
     const float rcp = 1.0f / b;

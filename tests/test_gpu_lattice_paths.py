@@ -136,3 +136,27 @@ def test_filter_in_front_of_a_large_table(gpu, oracle):
     assert st.table_slots == 1 << 23
     gpu.assert_structure_equal(vk, vi, pv, pw, items, "large table")
     gpu.assert_outputs_close(out.cpu().numpy(), want, "large table")
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_features_without_a_simplex_stay_in_their_own_points(dtype, gpu, oracle):
+    """pd = 16: item 0 has NaN, infinite and huge features, in full tiles and in a last tile of one point; item 1 has
+    none and is filtered as ever."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from conftest import rel_l2
+    from test_host_simplex import features_without_a_simplex
+    n = 4 * 128 + 1
+    pos = np.stack([np.resize(features_without_a_simplex(dtype)[::-1], (n, 16)),
+                    np.random.default_rng(83).standard_normal((n, 16)).astype(dtype)])
+    val = np.random.default_rng(89).random((2, n, 3)).astype(dtype)
+    pt = torch.from_numpy(pos).cuda()
+    for _ in range(3):   # the shared memory of a call holds what the one before left
+        out, ws = plb.filter_positions(torch.from_numpy(val).cuda(), pt, max_entries=0)
+        st = plb.lattice_stats(ws)
+        assert st.device_status == 0 and st.num_entries <= 2 * n * 17
+        _, vitem, pv, _ = plb.export_lattice(ws, st, 2, n, 16, 4, positions=pt)
+        assert int(pv.min()) >= 0 and int(pv.max()) < st.num_vertices
+        assert bool((vitem[pv[0].long()] == 0).all()) and bool((vitem[pv[1].long()] == 1).all())
+        want = oracle.filter(val[1], pos[1], structure=False, dtype=dtype).out
+        assert rel_l2(out[1].cpu().numpy(), want) <= (1e-12 if dtype == np.float64 else 1e-5)

@@ -105,3 +105,71 @@ def test_reciprocal_division_is_the_ieee_quotient(shim):
         out = np.empty_like(a)
         shim.div_by_rcp_host(a.ctypes.data_as(fp), ctypes.c_float(b), len(a), out.ctypes.data_as(fp))
         assert np.array_equal(bits(out), bits(a / np.float32(b))), b
+
+
+def point_records(shim, pos, scale):
+    n, pd = pos.shape
+    low16 = np.zeros((n, pd), np.uint16)
+    found, settled = np.zeros((n, pd + 1), np.int32), np.zeros((n, pd + 1), np.int32)
+    rc = shim.point_records_host(*(ctypes.c_void_p(a.ctypes.data) for a in (pos, scale)), n, pd,
+                                 int(pos.dtype == np.float64),
+                                 *(ctypes.c_void_p(a.ctypes.data) for a in (low16, found, settled)))
+    assert rc == 0
+    return low16, found, settled
+
+
+def keys_by_steps(low16, rank):
+    """Keys of every remainder as build_tiles steps from one to the next: a coordinate for every rank, packed in four
+    bits (ranks outside 1..16 fall out of the words)."""
+    n, pd = low16.shape
+    keys = np.zeros((n, pd + 1, pd), np.int64)
+    for p in range(n):
+        coord = [0] * 17
+        for i in range(1, pd):
+            if 1 <= rank[p, i] <= 16:
+                coord[rank[p, i]] = (coord[rank[p, i]] + i) & 15
+        k = low16[p].astype(np.int64)
+        keys[p, 0] = k
+        for r in range(1, pd + 1):
+            k = k + 1
+            taken = pd - r + 1
+            if taken != rank[p, pd]:
+                k[coord[taken]] -= pd + 1
+            keys[p, r] = k
+    return keys & 0xFFFF
+
+
+def keys_by_ranks(low16, rank):
+    """The same from the ranks, one byte each in four words."""
+    n, pd = low16.shape
+    keys = np.zeros((n, pd + 1, pd), np.int64)
+    for p in range(n):
+        words = [sum(int(rank[p, 4 * j + b]) << (8 * b) for b in range(4)) & 0xFFFFFFFF for j in range(pd // 4)]
+        for r in range(pd + 1):
+            for i in range(pd):
+                above = (words[i // 4] + (127 - (pd - r)) * 0x01010101) & 0xFFFFFFFF
+                keys[p, r, i] = int(low16[p, i]) + r - (pd + 1) * ((above >> (8 * (i & 3) + 7)) & 1)
+    return keys & 0xFFFF
+
+
+def features_without_a_simplex(dtype):
+    """pd = 16: tame points first, then NaN, infinite, huge and (double) merely large features."""
+    rng = np.random.default_rng(5)
+    pos = rng.standard_normal((60, 16)) * 3.0
+    pos[20:30, rng.integers(0, 16, 10)] = np.nan
+    pos[30:40, 3] = np.inf
+    pos[40:50] *= 1e9
+    pos[50:60] *= 1e5 if dtype == np.float64 else 1e30
+    return pos.astype(dtype)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_both_ways_to_a_key_agree_whatever_the_features(dtype, shim, oracle):
+    pos = features_without_a_simplex(dtype)
+    low16, found, settled = point_records(shim, pos, oracle.scale_factors(16, dtype))
+    assert np.array_equal(found[:20], settled[:20])                     # real simplices stay as they are
+    assert np.array_equal(np.sort(settled, 1), np.tile(np.arange(17), (60, 1)))
+    steps, ranks = keys_by_steps(low16, settled), keys_by_ranks(low16, settled)
+    assert np.array_equal(steps, ranks)
+    # without settling they part: a slot of the tile's hash is then read that nobody wrote
+    assert (keys_by_steps(low16, found) != keys_by_ranks(low16, found))[20:].any()
