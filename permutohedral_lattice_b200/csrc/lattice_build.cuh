@@ -125,11 +125,13 @@ struct TileKeys {
         else
             s[id] = k[0];
     }
+    // is splat a, of any remainder, one of splat b's remainder r with b's key
     __device__ __forceinline__ bool same(int a, int b, int r) const {
+        u32 diff = (u32)(a ^ b) & ~(u32)(TP - 1);
+        if (COMPACT && diff) return false;   // a record is read by point and remainder
         u32 x[CW], y[CW];
         load(a, r, x);
         load(b, r, y);
-        u32 diff = 0;
 #pragma unroll
         for (int j = 0; j < CW; j++) diff |= x[j] ^ y[j];
         return diff == 0;
@@ -170,8 +172,11 @@ constexpr int TILE_ROUNDS = 8;            // of the tile's de-duplication
 // splat represents the key, for all its splats alike, since all of them read that slot.  Keys that lost their slot
 // to another key go into the next round with another hash; with 2.5 slots a splat that leaves a few per cent of
 // them.  A splat still without representative after TILE_ROUNDS represents itself: the key then has two entries,
-// which the global table merges as it does those of different tiles.  (One compare-and-swap per splat on the slot,
-// as before, took a third of the kernel's shared-memory wavefronts, and its retries most of the divergence.)
+// which the global table merges as it does those of different tiles.  A splat stands only for splats of its own
+// remainder, because entries are numbered remainder by remainder.  Keys of two remainders differ (a key modulo PD+1 is
+// its remainder), but only until 16 bits, or the integers of a float, no longer hold their coordinates.
+// (One compare-and-swap per splat on the slot, as before, took a third of the kernel's shared-memory wavefronts, and
+// its retries most of the divergence.)
 //
 // Bound by issue slots and the LSU pipe.  Up to pd = 5 six CTAs fit an SM: the registers are capped at 40 for it
 // (measured 13 % faster than five CTAs with 48).
@@ -281,7 +286,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             int c = me;
             if (valid) {
                 c = slots_s[keys.hash(me, r, (u32)item * TILE_SEED) >> (32 - LSLOG)];
-                if (c != me && (c / TP != r || !keys.same(c, me, r))) {
+                if (c != me && !keys.same(c, me, r)) {
                     c = me;
                     open |= 1u << r;
                 }
@@ -295,7 +300,6 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
             const int me = r * TP + tid;
-            // a slot written by a splat of another remainder holds another key: the remainder is the key modulo PD+1
             if (rep[r] != me && !keys.same(rep[r], me, r)) {
                 rep[r] = me;
                 open |= 1u << r;
@@ -319,7 +323,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             for (int r = 0; r <= PD; r++) {
                 if ((open >> r) & 1u) {
                     const int me = r * TP + tid, c = slots_s[next_slot(r)];
-                    if (c == me || ((!COMPACT || c / TP == r) && keys.same(c, me, r))) {
+                    if (c == me || keys.same(c, me, r)) {
                         set_rep(r, c);
                         open &= ~(1u << r);
                     }

@@ -160,3 +160,25 @@ def test_features_without_a_simplex_stay_in_their_own_points(dtype, gpu, oracle)
         assert bool((vitem[pv[0].long()] == 0).all()) and bool((vitem[pv[1].long()] == 1).all())
         want = oracle.filter(val[1], pos[1], structure=False, dtype=dtype).out
         assert rel_l2(out[1].cpu().numpy(), want) <= (1e-12 if dtype == np.float64 else 1e-5)
+
+
+@pytest.mark.parametrize("pd", [1, 2, 3, 5, 8])
+def test_keys_beyond_their_range_stay_in_their_own_tiles(pd, gpu, oracle):
+    """Item 0 has features so large that splats of different remainders get one key; item 1 is filtered as ever, and
+    every splat of either item still points to a vertex of its own item."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from test_host_simplex import far_features
+    n = 3 * 256 + 1
+    pos = np.stack([far_features(pd, n), np.random.default_rng(97).standard_normal((n, pd)).astype(np.float32)])
+    val = np.random.default_rng(101).random((2, n, 3), dtype=np.float32)
+    pt = torch.from_numpy(pos).cuda()
+    for _ in range(3):
+        out, ws = plb.filter_positions(torch.from_numpy(val).cuda(), pt, max_entries=0)
+        st = plb.lattice_stats(ws)
+        assert st.device_status == 0 and st.num_entries <= 2 * n * (pd + 1)
+        _, vitem, pv, _ = plb.export_lattice(ws, st, 2, n, pd, 4, positions=pt)
+        assert int(pv.min()) >= 0 and int(pv.max()) < st.num_vertices
+        assert bool((vitem[pv[0].long()] == 0).all()) and bool((vitem[pv[1].long()] == 1).all())
+        want = oracle.filter(val[1], pos[1], structure=False).out
+        gpu.assert_outputs_close(out[1].cpu().numpy(), want, "pd %d" % pd)

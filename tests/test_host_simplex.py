@@ -173,3 +173,18 @@ def test_both_ways_to_a_key_agree_whatever_the_features(dtype, shim, oracle):
     assert np.array_equal(steps, ranks)
     # without settling they part: a slot of the tile's hash is then read that nobody wrote
     assert (keys_by_steps(low16, found) != keys_by_ranks(low16, found))[20:].any()
+
+
+def far_features(pd, n=256):
+    """Features beyond the integers of a float: neighbouring floats, whose low 16 bits differ by one."""
+    return (1e8 + np.random.default_rng(0).integers(0, 40, (n, pd)) * 8.0).astype(np.float32)
+
+
+def test_splats_of_two_remainders_can_have_one_key(shim, oracle):
+    """Why a tile's splat may only stand for splats of its own remainder."""
+    low16, found, _ = point_records(shim, far_features(2), oracle.scale_factors(2))
+    remainders = {}
+    for point in keys_by_steps(low16, found):
+        for r, key in enumerate(point):
+            remainders.setdefault(key.tobytes(), set()).add(r)
+    assert max(len(rs) for rs in remainders.values()) > 1
