@@ -235,6 +235,10 @@ int pl_direct_index_min_entries(int batch, int n_spatial_dims, const int* spatia
  * src/PermutohedralLatticeGPU.cuh:49-55,442-445). */
 int pl_watch_next_call(void* stream);
 
+/* Takes pl_watch_next_call back, for a caller that does not get as far as its call.  A filter or build call that fails
+ * ends the watch by itself.  No counterpart in the reference. */
+int pl_cancel_watch(void);
+
 /* See pl_watch_next_call.  BLOCKS until the report is there.  No counterpart in the reference. */
 int pl_await_watched_call(int64_t* num_entries, int* device_status, void* stream);
 

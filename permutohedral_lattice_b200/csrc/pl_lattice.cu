@@ -108,17 +108,24 @@ static int take_watch_line(WatchLine** out) {
     return PL_OK;
 }
 
-// What a call passes to its link kernel: where to report, or nothing.
-static Watch take_watch() {
+// What a call passes to its link kernel: where to report, or nothing.  A call that is being captured never reports: the
+// graph would write into the line at every replay.
+static Watch take_watch(cudaStream_t st) {
     Watch w = {nullptr, 0u};
-    if (g_watcher.armed) {
+    if (!g_watcher.armed) return w;
+    g_watcher.armed = false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
         w.word = &g_watcher.line->word;
         w.seq = g_watcher.line->seq;
-        g_watcher.armed = false;
         g_watcher.launched = true;
     }
     return w;
 }
+// In every filter and build entry point: the watch is for this call, however far it gets, and never for a later one.
+struct WatchScope {
+    ~WatchScope() { g_watcher.armed = false; }
+};
 
 // Kernel launch with the error check of every other runtime call.  overlap: with programmatic stream
 // serialisation, i.e. the kernel may become resident while the kernel before it in the stream drains (it waits
@@ -538,13 +545,13 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
                 PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
                 PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
                 PL_LAUNCH_AFTER(OV_LINK, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                                 L.max_entries, take_watch());
+                                                                 L.max_entries, take_watch(st));
             }
         }
         const bool small = !use_direct && small_index(L);
         PL_COUNT_LAUNCHES(small ? 2 : 4);   // build_tiles and the launches of the index stage
         if (small) {
-            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch());
+            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch(st));
         } else if (!use_direct) {
             // the value rows are zeroed by the link launch, whose lookups leave the memory system idle
             void* zrows = vinit.rows;
@@ -554,7 +561,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
-                                                      L.max_entries, zrows, vinit.row_bytes, take_watch());
+                                                      L.max_entries, zrows, vinit.row_bytes, take_watch(st));
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[2], st));
     } else {
@@ -654,17 +661,17 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
             PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH((link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                             L.max_entries, take_watch());
+                                                             L.max_entries, take_watch(st));
         }
     }
     const bool small = !use_direct && small_index(L);
     if (small) {
-        PL_LAUNCH_AFTER(OV_CLEAR, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch());
+        PL_LAUNCH_AFTER(OV_CLEAR, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch(st));
     } else if (!use_direct) {
         PL_LAUNCH_AFTER(OV_CLEAR, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
         PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
-                                                  nullptr, 0u, take_watch());
+                                                  nullptr, 0u, take_watch(st));
     }
     PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                       list_ref, v0, vd);
@@ -825,6 +832,7 @@ int pl_compute_positions_f32(const float* reference, float* positions, int n,
 int pl_filter_f32(float* output, const float* input, const float* positions, int batch, int n,
                   int pd, int vd, int reverse, void* workspace, size_t workspace_bytes,
                   int64_t max_entries, int mode, void* stream) {
+    WatchScope this_call;
     if (batch < 0 || n < 0 || batch > 65535) return PL_INVALID_ARGUMENT;
     if (!pl_supported(pd, vd)) return PL_UNSUPPORTED_DIMS;
     if (batch == 0 || n == 0) return PL_OK;
@@ -865,6 +873,7 @@ int pl_lattice_filter_f32(float* output, const float* input, const float* refere
                           int n_reference_channels, int bilateral, float theta_alpha,
                           float theta_beta, float theta_gamma, int reverse, void* workspace,
                           size_t workspace_bytes, int64_t max_entries, int mode, void* stream) {
+    WatchScope this_call;
     if (n_input_channels < 1) return PL_INVALID_ARGUMENT;
     Geom g;
     int pd = 0, n = 0;
@@ -884,6 +893,7 @@ int pl_lattice_filter_f32_noalloc(float* output, const float* input, const float
                                   int n_reference_channels, int bilateral, float theta_alpha,
                                   float theta_beta, float theta_gamma, int reverse, int64_t max_entries,
                                   void* stream) {
+    WatchScope this_call;
     if (n_input_channels < 1) return PL_INVALID_ARGUMENT;
     Geom g;
     int pd = 0, n = 0;
@@ -917,6 +927,7 @@ int pl_lattice_build_f32(const float* reference, int batch, int n_spatial_dims, 
                          int n_reference_channels, int bilateral, float theta_alpha, float theta_beta,
                          float theta_gamma, int max_value_dim, void* workspace, size_t workspace_bytes,
                          int64_t max_entries, void* stream) {
+    WatchScope this_call;
     Geom g;
     int pd = 0, n = 0;
     int rc = op_geom(g, batch, n_spatial_dims, spatial_dims, n_reference_channels, bilateral, theta_alpha,
@@ -931,6 +942,7 @@ int pl_lattice_build_f32(const float* reference, int batch, int n_spatial_dims, 
 
 int pl_lattice_build_positions_f32(const float* positions, int batch, int n, int pd, int max_value_dim,
                                    void* workspace, size_t workspace_bytes, int64_t max_entries, void* stream) {
+    WatchScope this_call;
     if (batch < 0 || n < 0 || batch > 65535) return PL_INVALID_ARGUMENT;
     if (!pl_supported(pd, max_value_dim)) return PL_UNSUPPORTED_DIMS;
     if (batch == 0 || n == 0) return PL_OK;
@@ -1031,6 +1043,7 @@ static int filter_common_f64(const Geom& g, double* output, const double* input,
 int pl_filter_f64(double* output, const double* input, const double* positions, int batch, int n, int pd,
                   int vd, int reverse, void* workspace, size_t workspace_bytes, int64_t max_entries,
                   void* stream) {
+    WatchScope this_call;
     if (batch < 0 || n < 0 || batch > 65535) return PL_INVALID_ARGUMENT;
     if (!pl_supported(pd, vd)) return PL_UNSUPPORTED_DIMS;
     if (batch == 0 || n == 0) return PL_OK;
@@ -1049,6 +1062,7 @@ int pl_lattice_filter_f64(double* output, const double* input, const double* ref
                           int n_reference_channels, int bilateral, double theta_alpha, double theta_beta,
                           double theta_gamma, int reverse, void* workspace, size_t workspace_bytes,
                           int64_t max_entries, void* stream) {
+    WatchScope this_call;
     if (n_input_channels < 1) return PL_INVALID_ARGUMENT;
     Geom g;
     int pd = 0, n = 0;
@@ -1196,6 +1210,11 @@ int pl_watch_next_call(void* stream) {
     w.line->seq = (w.line->seq + 1) & WATCH_SEQ_MASK;
     if (w.line->seq == 0) w.line->seq = 1;
     w.armed = true;
+    return PL_OK;
+}
+
+int pl_cancel_watch(void) {
+    g_watcher.armed = g_watcher.launched = false;
     return PL_OK;
 }
 

@@ -169,7 +169,11 @@ def _run_sized(kind, tensor, batch, worst, device, stream, launch, verify="auto"
             ws = launch(max_entries)
             break
         capi.check(L.pl_watch_next_call(stream), "pl_watch_next_call")
-        ws = launch(max_entries)
+        try:
+            ws = launch(max_entries)
+        except BaseException:
+            L.pl_cancel_watch()                    # no memory for the workspace, say: the watch was for this call alone
+            raise
         entries, status = ctypes.c_int64(0), ctypes.c_int(0)
         capi.check(L.pl_await_watched_call(ctypes.byref(entries), ctypes.byref(status), stream),
                    "pl_await_watched_call")

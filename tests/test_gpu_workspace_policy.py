@@ -174,3 +174,63 @@ def test_host_pipeline_gives_back_its_workspaces_when_closed(policy):
     assert mine                                   # one workspace per stream slot that was used
     pipe.close()
     assert not [k for k in policy._workspaces if isinstance(k[1], tuple) and k[1][:2] == ("HostPipeline", id(pipe))]
+
+
+def _watched(lib):
+    """What awaiting the watched call of this thread returns: (return code, entries)."""
+    import ctypes
+    import torch
+    entries, status = ctypes.c_int64(-1), ctypes.c_int(-1)
+    torch.cuda.synchronize()
+    rc = lib.pl_await_watched_call(ctypes.byref(entries), ctypes.byref(status), torch.cuda.current_stream().cuda_stream)
+    return rc, entries.value
+
+
+@pytest.mark.parametrize("failure", ["workspace", "argument", "memory", "empty"])
+def test_watch_of_a_call_that_failed_is_not_taken_by_the_next_one(policy, failure, monkeypatch):
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from permutohedral_lattice_b200 import capi
+    x, ref = _data(8)
+    _, ws, call = plb.lattice_filter_raw(x, ref, max_entries=0, **KW)
+    lib, stream = capi.lib(), torch.cuda.current_stream().cuda_stream
+    if failure == "memory":
+        policy._verified.clear()
+
+        def no_memory(*args):
+            raise torch.cuda.OutOfMemoryError("no memory for the workspace")
+
+        with monkeypatch.context() as m:
+            m.setattr(policy, "_workspace", no_memory)
+            with pytest.raises(torch.cuda.OutOfMemoryError):
+                plb.lattice_filter_raw(x, ref, **KW)
+    else:
+        assert lib.pl_watch_next_call(stream) == capi.PL_OK
+        batch, nbytes, out, want = call.batch, ws.numel(), x.data_ptr(), capi.PL_OK
+        if failure == "workspace":
+            nbytes, want = 16, capi.PL_WORKSPACE_TOO_SMALL
+        elif failure == "argument":
+            out, want = 0, capi.PL_INVALID_ARGUMENT
+        else:
+            batch = 0
+        assert lib.pl_lattice_filter_f32(out, x.data_ptr(), ref.data_ptr(), batch, len(call.sdims), call.c_sdims,
+                                         call.c, call.r, 1, *call.theta, 0, ws.data_ptr(), nbytes, 0, 0, stream) == want
+    plb.lattice_filter_raw(x, ref, max_entries=0, **KW)      # nobody watches this one
+    assert _watched(lib)[0] == capi.PL_INVALID_ARGUMENT
+
+
+def test_call_that_is_being_captured_is_not_watched(policy):
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from permutohedral_lattice_b200 import capi
+    x, ref = _data(9)
+    out, ws, _ = plb.lattice_filter_raw(x, ref, max_entries=0, **KW)
+    want, lib = out.clone(), capi.lib()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    assert lib.pl_watch_next_call(torch.cuda.current_stream().cuda_stream) == capi.PL_OK
+    with torch.cuda.graph(graph):
+        plb.lattice_filter_raw(x, ref, out=out, workspace=ws, **KW)
+    graph.replay()
+    assert _watched(lib)[0] == capi.PL_INVALID_ARGUMENT
+    assert torch.allclose(out, want, atol=1e-5)
