@@ -230,10 +230,18 @@ int pl_direct_index_min_entries(int batch, int n_spatial_dims, const int* spatia
 /* A cheaper way to learn whether a call fits its max_entries than pl_lattice_stats: pl_watch_next_call makes the
  * next filter or build call of this host thread report its counters as soon as its lattice is complete, and
  * pl_await_watched_call waits for that report (not for the whole call: splat, blur and slice are still running)
- * and returns what pl_stats would hold.  `stream` is the call's stream; it must not be being captured.  A watched
- * call that returned an error is not awaited.  No counterpart in the reference (it prints or exits:
+ * and returns the entries and the status up to there.  `stream` is the call's stream; it must not be being captured.
+ * A watched call that returned an error is not awaited.
+ * A filter call that fails after its report (PL_INTERNAL_ERROR: the splat gave up a bounded wait) fills its output
+ * with NaN, says so in pl_lattice_stats, and the next pl_watch_next_call of the thread returns that status, once, and
+ * watches nothing.  No counterpart in the reference (it prints or exits:
  * src/PermutohedralLatticeGPU.cuh:49-55,442-445). */
 int pl_watch_next_call(void* stream);
+
+/* device_status <- the status of a watched call, of any host thread, that failed after its report and that nobody has
+ * been told of yet; PL_OK if there is none.  Does not wait: calls that are still running are not looked at.
+ * No counterpart in the reference. */
+int pl_watched_calls_status(int* device_status);
 
 /* Takes pl_watch_next_call back, for a caller that does not get as far as its call.  A filter or build call that fails
  * ends the watch by itself.  No counterpart in the reference. */

@@ -28,6 +28,7 @@ EXPORTED_SYMBOLS = [
     "pl_workspace_bytes_f64", "pl_compute_positions_f64", "pl_filter_f64", "pl_lattice_filter_f64",
     "pl_export_lattice_f64", "pl_debug_direct_index", "pl_crf_update_f32", "pl_launch_count",
     "pl_direct_index_min_entries", "pl_watch_next_call", "pl_cancel_watch", "pl_await_watched_call",
+    "pl_watched_calls_status",
 ]
 STATIC_SCRATCH_BYTES = 64 << 20
 NUM_STAGE_EVENTS = 6
@@ -91,6 +92,7 @@ def lib():
         L.pl_crf_update_f32.argtypes = [vp, vp, vp, vp, vp, f, f, i64, i, vp]
         L.pl_profile_next_call.argtypes = [ctypes.POINTER(ctypes.c_void_p)]
         L.pl_watch_next_call.argtypes = [vp]
+        L.pl_watched_calls_status.argtypes = [ctypes.POINTER(i)]
         L.pl_cancel_watch.argtypes = []
         L.pl_await_watched_call.argtypes = [ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(i), vp]
         L.pl_launch_count.argtypes = []

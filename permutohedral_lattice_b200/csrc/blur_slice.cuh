@@ -90,7 +90,8 @@ template <int PD, int VP, int CT>
 __global__ void __launch_bounds__(Cfg<PD>::TP, SliceFast<PD, VP>::CTAS)
 slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const int2* __restrict__ tile_info,
                  const u16* __restrict__ rec, const float* __restrict__ rec_w,
-                 const u32* __restrict__ list_ref, const float* __restrict__ vsrc, int channels, int rows_cap, int bulk_ok) {
+                 const u32* __restrict__ list_ref, const float* __restrict__ vsrc, int channels, int rows_cap, int bulk_ok,
+                 Watch watch) {
     // Launched to overlap the tail of the last blur pass: the status word, the tile's range and the per-point
     // records are older than any blur pass and are fetched before the wait; the vertex rows after it.
     const int C = CT ? CT : channels;
@@ -102,6 +103,7 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     int* prow_s = reinterpret_cast<int*>(smem_raw + SliceFast<PD, VP>::region(rows_cap));       // [TP]
     if (call_failed(hdr)) {
         poison_tile_output(g, output, C);
+        report_late(watch, hdr);
         wait_for_previous_kernel();
         return;
     }
@@ -242,7 +244,7 @@ template <int PD>
 __global__ void __launch_bounds__(Cfg<PD>::TP)
 slice_tiles_generic(Geom g, float* __restrict__ output, const Header* hdr, const int2* __restrict__ tile_info,
                     const u16* __restrict__ rec, const float* __restrict__ rec_w,
-                    const u32* __restrict__ list_ref, const float* __restrict__ vsrc, int vd, int rows_cap) {
+                    const u32* __restrict__ list_ref, const float* __restrict__ vsrc, int vd, int rows_cap, Watch watch) {
     wait_for_previous_kernel();
     constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, PW = SliceCfg<PD>::PW;
     const int C = vd - 1, VP = padded_vd(vd), QPR = VP >> 2;
@@ -252,6 +254,7 @@ slice_tiles_generic(Geom g, float* __restrict__ output, const Header* hdr, const
     int* prow_s = reinterpret_cast<int*>(prec_s + (size_t)TP * PW);                 // [TP]
     if (call_failed(hdr)) {
         poison_tile_output(g, output, C);
+        report_late(watch, hdr);
         return;
     }
     const TilePos tpos = this_tile(g);

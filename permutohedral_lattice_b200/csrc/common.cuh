@@ -48,7 +48,8 @@ struct Header {   // first 256 bytes of the workspace
     u32 capacity;      // the max_entries the workspace was laid out for (written by build_tiles)
     u32 sorted;        // 1: the lattice was built for reuse and holds every tile's splats sorted by entry
     u32 filter_log2;   // bits of the vertex filter behind the table, as a logarithm; 0: none (see FILTER_BITS_LOG2)
-    u32 pad[55];
+    u32 reported;      // status bits that the call's watch has told the host of (see Watch)
+    u32 pad[54];
 };
 
 // Sketch of the lattice's size, behind the header (zeroed with it): a bitmap in which build_tiles sets one bit
@@ -77,19 +78,31 @@ __device__ __forceinline__ u64 grid_thread() {
 }
 __device__ __forceinline__ u64 grid_threads() { return (u64)gridDim.x * gridDim.y * blockDim.x; }
 
-// Where a watched call reports (pl_watch_next_call): one word of mapped host memory.  The link kernel writes
-// sequence << 40 | status bits << 32 | entries there before it does anything else: everything that can make a
-// call fail has happened by then, and the host, which polls the word, goes on while the device still splats,
-// blurs and slices.
+// Where a watched call reports (pl_watch_next_call): two words of mapped host memory.  The link kernel writes
+// sequence << 40 | status bits << 32 | entries into the first before it does anything else: whether the lattice fits,
+// and whether it could be built, is known by then, and the host, which polls the word, goes on while the device still
+// splats, blurs and slices.  What fails after that (the splat's bounded wait for its copies) the slice kernel, which
+// then fills the output with NaN, writes into the second word; the host looks there when it watches again.
 constexpr u32 WATCH_SEQ_MASK = 0xFFFFFFu;
 struct Watch {
-    u64* word;   // null: nobody is watching
+    u64* words;   // null: nobody is watching
     u32 seq;
 };
-__device__ __forceinline__ void report_to(const Watch& w, const Header* hdr) {
-    if (w.word && grid_thread() == 0) {
-        const u64 v = ((u64)w.seq << 40) | ((u64)(__ldcg(&hdr->status) & 0xFFu) << 32) | (u64)hdr->num_entries;
-        asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(w.word), "l"(v) : "memory");
+__device__ __forceinline__ void store_to_host(u64* word, u64 v) {
+    asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(word), "l"(v) : "memory");
+}
+__device__ __forceinline__ void report_to(const Watch& w, Header* hdr) {
+    if (w.words && grid_thread() == 0) {
+        const u32 status = __ldcg(&hdr->status);
+        hdr->reported = status;
+        store_to_host(w.words, ((u64)w.seq << 40) | ((u64)(status & 0xFFu) << 32) | (u64)hdr->num_entries);
+    }
+}
+// By the first thread of the grid of a slice kernel that has found the call failed.
+__device__ __forceinline__ void report_late(const Watch& w, const Header* hdr) {
+    if (w.words && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+        const u32 late = hdr->status & ~hdr->reported;
+        if (late) store_to_host(w.words + 1, late);
     }
 }
 

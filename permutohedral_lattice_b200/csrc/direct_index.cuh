@@ -87,7 +87,7 @@ insert_direct(Header* hdr, Direct d, u32* __restrict__ table, const Key<Cfg<PD>:
 // its slot (every slot carries a vertex index by now); the same result fills that neighbour's "-" slot.
 template <int PD>
 __global__ void __launch_bounds__(256)
-link_neighbours_direct(const Header* hdr, Direct d, const u32* __restrict__ table, u32* __restrict__ list_ref,
+link_neighbours_direct(Header* hdr, Direct d, const u32* __restrict__ table, u32* __restrict__ list_ref,
                        const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys,
                        int* __restrict__ nbr, u64 max_entries, Watch watch) {
     after_previous_kernel();

@@ -146,7 +146,7 @@ template <int PD>
 __global__ void __launch_bounds__(Cfg<PD>::TP)
 slice_tiles_f64(Geom g, double* __restrict__ output, const Header* hdr, const int2* __restrict__ tile_info,
                 const u16* __restrict__ rec, const double* __restrict__ rec_w,
-                const u32* __restrict__ list_ref, const double* __restrict__ vsrc, int vd) {
+                const u32* __restrict__ list_ref, const double* __restrict__ vsrc, int vd, Watch watch) {
     constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS;
     const int C = vd - 1, VP = padded_vd_f64(vd), pairs = VP >> 1;
     __shared__ double w_s[SPLATS];
@@ -154,6 +154,7 @@ slice_tiles_f64(Geom g, double* __restrict__ output, const Header* hdr, const in
     __shared__ int prow_s[TP];
     if (call_failed(hdr)) {
         poison_tile_output(g, output, C);
+        report_late(watch, hdr);
         wait_for_previous_kernel();
         return;
     }

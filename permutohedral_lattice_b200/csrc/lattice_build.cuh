@@ -735,7 +735,7 @@ struct LinkAxis {   // link_axis of the axis this block works on, chosen once pe
 
 template <int PD>
 __global__ void __launch_bounds__(256)
-link_neighbours(const Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restrict__ list_ref,
+link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restrict__ list_ref,
                 const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys, int* __restrict__ nbr,
                 u64 max_entries, void* zero_rows_ptr, u32 zero_row_bytes, Watch watch) {
     after_previous_kernel();

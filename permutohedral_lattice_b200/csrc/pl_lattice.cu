@@ -74,10 +74,14 @@ static int cuda_fail(cudaError_t e, const char* where) {
 // with the line, tells its reports apart: a late one of a call that was given up on is not mistaken for the
 // next call's.
 struct alignas(64) WatchLine {
-    u64 word;
+    u64 words[2];   // what the device writes (see Watch): the report, and the status bits of a failure after it
     u32 seq;
 };
 static std::mutex g_watch_mutex;
+static std::vector<WatchLine*>& watch_pages() {   // every page of 64 lines there is
+    static std::vector<WatchLine*>* pages = new std::vector<WatchLine*>();
+    return *pages;
+}
 static std::vector<WatchLine*>& watch_pool() {
     static std::vector<WatchLine*>* pool = new std::vector<WatchLine*>();   // outlives every thread
     return *pool;
@@ -101,6 +105,7 @@ static int take_watch_line(WatchLine** out) {
         void* p = nullptr;
         PL_CUDA(cudaHostAlloc(&p, 64 * sizeof(WatchLine), cudaHostAllocPortable | cudaHostAllocMapped));
         memset(p, 0, 64 * sizeof(WatchLine));
+        watch_pages().push_back(static_cast<WatchLine*>(p));
         for (int i = 0; i < 64; i++) pool.push_back(static_cast<WatchLine*>(p) + i);
     }
     *out = pool.back();
@@ -116,11 +121,21 @@ static Watch take_watch(cudaStream_t st) {
     g_watcher.armed = false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
-        w.word = &g_watcher.line->word;
+        w.words = g_watcher.line->words;
         w.seq = g_watcher.line->seq;
         g_watcher.launched = true;
     }
     return w;
+}
+static int code_of(u64 status_bits) {
+    int code = PL_OK;
+    for (int c = PL_INVALID_ARGUMENT; c <= PL_INTERNAL_ERROR; c++)
+        if (status_bits & (1u << c)) code = c;
+    return code;
+}
+// The failure after its report, if any, of a call that reported to this line; told once.
+static int take_late_failure(WatchLine* line) {
+    return code_of(__atomic_exchange_n(&line->words[1], 0ull, __ATOMIC_ACQ_REL));
 }
 // In every filter and build entry point: the watch is for this call, however far it gets, and never for a later one.
 struct WatchScope {
@@ -430,13 +445,13 @@ static int launch_splat(const Geom& g, const float* input, Header* hdr, const in
 // slice for rows of VP floats (CT > 0: of CT channels), or (VP = 0) of more than 32.
 template <int PD, int VP, int CT = 0>
 static int launch_slice(const Geom& g, float* output, const Header* hdr, const int2* tile_info, const u16* rec,
-                        const float* rec_w, const u32* list_ref, const float* vsrc, int vd, cudaStream_t st) {
+                        const float* rec_w, const u32* list_ref, const float* vsrc, int vd, Watch watch, cudaStream_t st) {
     if constexpr (VP > 0) {
         int rows_cap = (40 * 1024) / (SliceFast<PD, VP>::RS * 4);
         if (rows_cap > Cfg<PD>::SPLATS) rows_cap = Cfg<PD>::SPLATS;
         const size_t smem = SliceFast<PD, VP>::bytes(rows_cap);
         PL_TRY((ensure_dynamic_smem<slice_tiles_fast<PD, VP, CT>>(smem)));
-        PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_fast<PD, VP, CT>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, vd - 1, rows_cap, bulk_rows_ok(g, output, vd - 1) ? 1 : 0);
+        PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_fast<PD, VP, CT>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, vd - 1, rows_cap, bulk_rows_ok(g, output, vd - 1) ? 1 : 0, watch);
     } else {
         const int rows_cap = rows_cap_for(PD, vd);
         const size_t fixed = sizeof(float) * Cfg<PD>::TP * SliceCfg<PD>::PW + sizeof(int) * Cfg<PD>::TP;
@@ -444,7 +459,7 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
         if (smem > 200 * 1024) return PL_UNSUPPORTED_DIMS;
         PL_TRY((ensure_dynamic_smem<slice_tiles_generic<PD>>(smem)));
         PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_generic<PD>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w,
-                                                                        list_ref, vsrc, vd, rows_cap);
+                                                                        list_ref, vsrc, vd, rows_cap, watch);
     }
     return PL_OK;
 }
@@ -507,6 +522,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     if (ev) PL_CUDA(cudaEventRecord(ev[0], st));
     if (phases & PH_BUILD) PL_CUDA(cudaMemsetAsync(hdr, 0, sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header), st));
     if (g.num_tiles == 0) return PL_OK;
+    const Watch watch = (phases & PH_BUILD) ? take_watch(st) : Watch{nullptr, 0u};
 
     PL_TRY((ensure_dynamic_smem<build_tiles<PD, float>>(Cfg<PD>::build_smem(false))));
     const int sms = num_sms();
@@ -545,13 +561,13 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
                 PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
                 PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
                 PL_LAUNCH_AFTER(OV_LINK, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                                 L.max_entries, take_watch(st));
+                                                                 L.max_entries, watch);
             }
         }
         const bool small = !use_direct && small_index(L);
         PL_COUNT_LAUNCHES(small ? 2 : 4);   // build_tiles and the launches of the index stage
         if (small) {
-            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch(st));
+            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, watch);
         } else if (!use_direct) {
             // the value rows are zeroed by the link launch, whose lookups leave the memory system idle
             void* zrows = vinit.rows;
@@ -561,7 +577,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
-                                                      L.max_entries, zrows, vinit.row_bytes, take_watch(st));
+                                                      L.max_entries, zrows, vinit.row_bytes, watch);
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[2], st));
     } else {
@@ -604,7 +620,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         PL_COUNT_LAUNCHES(1);
     }
     if (ev) PL_CUDA(cudaEventRecord(ev[4], st));
-    rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, st);
+    rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch, st);
     if (rc != PL_OK) return rc;
     if (ev) PL_CUDA(cudaEventRecord(ev[5], st));
     PL_CUDA(cudaGetLastError());
@@ -634,6 +650,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     const int sketch_shift = sketch_shift_of(L.max_entries);
     PL_CUDA(cudaMemsetAsync(hdr, 0, sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header), st));
     if (g.num_tiles == 0) return PL_OK;
+    const Watch watch = take_watch(st);
     PL_TRY((ensure_dynamic_smem<build_tiles<PD, double>>(Cfg<PD>::build_smem(false))));
     const size_t splat_smem = Splat64<PD>::bytes(vd);
     PL_TRY((ensure_dynamic_smem<splat_tiles_f64<PD>>(splat_smem)));
@@ -661,17 +678,17 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
             PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH((link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                             L.max_entries, take_watch(st));
+                                                             L.max_entries, watch);
         }
     }
     const bool small = !use_direct && small_index(L);
     if (small) {
-        PL_LAUNCH_AFTER(OV_CLEAR, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, take_watch(st));
+        PL_LAUNCH_AFTER(OV_CLEAR, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, watch);
     } else if (!use_direct) {
         PL_LAUNCH_AFTER(OV_CLEAR, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
         PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
-                                                  nullptr, 0u, take_watch(st));
+                                                  nullptr, 0u, watch);
     }
     PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                       list_ref, v0, vd);
@@ -686,7 +703,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
-    PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd);
+    PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
     PL_COUNT_LAUNCHES((small ? 2 : 4) + 1 + (one_blur ? 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;
@@ -1207,9 +1224,27 @@ int pl_watch_next_call(void* stream) {
         const int rc = take_watch_line(&w.line);
         if (rc != PL_OK) return rc;
     }
+    const int late = take_late_failure(w.line);
+    if (late != PL_OK) {
+        snprintf(g_cuda_error, sizeof(g_cuda_error),
+                 "pl_watch_next_call: an earlier watched call failed after its report, its output holds NaN");
+        return late;
+    }
     w.line->seq = (w.line->seq + 1) & WATCH_SEQ_MASK;
     if (w.line->seq == 0) w.line->seq = 1;
     w.armed = true;
+    return PL_OK;
+}
+
+int pl_watched_calls_status(int* device_status) {
+    if (!device_status) return PL_INVALID_ARGUMENT;
+    *device_status = PL_OK;
+    std::lock_guard<std::mutex> lock(g_watch_mutex);
+    for (WatchLine* page : watch_pages())
+        for (int i = 0; i < 64; i++) {
+            const int late = take_late_failure(page + i);
+            if (late != PL_OK) *device_status = late;
+        }
     return PL_OK;
 }
 
@@ -1223,15 +1258,13 @@ int pl_await_watched_call(int64_t* num_entries, int* device_status, void* stream
     w.armed = false;
     if (!num_entries || !device_status || !w.launched) return PL_INVALID_ARGUMENT;
     w.launched = false;
-    volatile u64* word = &w.line->word;
+    volatile u64* word = &w.line->words[0];
     bool drained = false;
     for (unsigned spin = 1;; spin++) {
         const u64 v = *word;
         if ((u32)(v >> 40) == w.line->seq) {
             *num_entries = (int64_t)(u32)v;
-            *device_status = PL_OK;
-            for (int code = PL_INVALID_ARGUMENT; code <= PL_INTERNAL_ERROR; code++)
-                if ((v >> 32) & (1u << code)) *device_status = code;
+            *device_status = code_of((v >> 32) & 0xFFu);
             return PL_OK;
         }
         if (drained) {

@@ -43,7 +43,8 @@ def release_workspaces():
 #     times the bound as long as the lattice did not fit.  The counters arrive in a word of pinned memory when
 #     the lattice is complete (pl_await_watched_call), while the device still splats, blurs and slices: waiting
 #     for the whole stream instead left the GPU idle for 50 us after every new reference image (grey 1024 x 1024,
-#     forward + backward: 460 us with that wait).
+#     forward + backward: 460 us with that wait).  What can fail after that (the splat gives up a wait for its
+#     copies: never seen) leaves NaN and is raised by the next verified call of the thread or by check_pending().
 # Callers that own a synchronisation point of their own (HostPipeline) ask for verify="deferred" instead: the
 # call's counters are copied to pinned host memory behind it and looked at in check_pending(); a call that did
 # not fit has filled its output with NaN, and the caller repeats it.
@@ -54,6 +55,7 @@ _verified = {}           # kind of call -> (identity of the reference it ran on,
 _pending = {}            # kind of call -> list of (event, pinned int32[3] = entries, vertices, status bits, bound, batch)
 _pinned_words = []       # pinned int32[3] buffers waiting to be used again (allocating pinned memory is slow)
 FIRST_GUESS_DIVISOR = 4
+LATE_FAILURE = "an earlier lattice filter call failed on the device after its lattice was complete; its output holds NaN"
 HEADROOM = 1.5
 
 
@@ -97,7 +99,8 @@ def _look_at(kind, entry):
 
 def check_pending(wait=True):
     """Looks at the counters of every call made with verify="deferred" that has not been looked at yet;
-    wait=True synchronises with those calls first.  Raises PlError if one of them outgrew its workspace."""
+    wait=True synchronises with those calls first.  Raises PlError if one of them outgrew its workspace, or if a
+    verified call that has finished failed after its lattice was complete."""
     first_error = None
     for kind in list(_pending):
         keep = []
@@ -114,6 +117,10 @@ def check_pending(wait=True):
         _pending[kind] = keep
     if first_error is not None:
         raise first_error
+    status = ctypes.c_int(0)
+    capi.check(capi.lib().pl_watched_calls_status(ctypes.byref(status)), "pl_watched_calls_status")
+    if status.value != capi.PL_OK:
+        raise capi.PlError(status.value, LATE_FAILURE)
 
 
 def _guess_bound(kind, batch, worst, floor=0):
@@ -168,7 +175,9 @@ def _run_sized(kind, tensor, batch, worst, device, stream, launch, verify="auto"
         if max_entries == 0 and not repeated:      # the worst case cannot overflow: nothing to verify
             ws = launch(max_entries)
             break
-        capi.check(L.pl_watch_next_call(stream), "pl_watch_next_call")
+        rc = L.pl_watch_next_call(stream)
+        if rc != capi.PL_OK:
+            raise capi.PlError(rc, LATE_FAILURE if rc == capi.PL_INTERNAL_ERROR else "pl_watch_next_call")
         try:
             ws = launch(max_entries)
         except BaseException:

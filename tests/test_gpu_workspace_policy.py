@@ -234,3 +234,46 @@ def test_call_that_is_being_captured_is_not_watched(policy):
     graph.replay()
     assert _watched(lib)[0] == capi.PL_INVALID_ARGUMENT
     assert torch.allclose(out, want, atol=1e-5)
+
+
+@pytest.mark.parametrize("dtype,c", [("float32", 21), ("float32", 40), ("float64", 8)])
+@pytest.mark.parametrize("told_by", ["next call", "check_pending"])
+def test_failure_after_the_report_is_raised_later(policy, dtype, c, told_by):
+    """A verified call returns when its lattice is complete.  Here a copy on another stream then sets the status bit
+    that a splat which gives up its bounded wait would set (the rest of the call takes hundreds of microseconds more;
+    every kernel looks at the status when it starts, whatever it is)."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from permutohedral_lattice_b200 import capi
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    ref = torch.rand((8, 64, 64, 3), device="cuda", generator=gen).repeat_interleave(8, 1).repeat_interleave(8, 2)
+    ref = ref.to(getattr(torch, dtype)).contiguous()
+    x = torch.rand((8, 512, 512, c), device="cuda", generator=gen).to(ref.dtype)
+    kw = dict(bilateral=True, theta_alpha=8.0, theta_beta=0.1)
+    plb.lattice_filter_raw(x, ref, **kw)                      # the workspace has its size from here on
+    bit = torch.tensor([1 << capi.PL_INTERNAL_ERROR], dtype=torch.int32).pin_memory()
+    ws = policy._workspaces[(x.device.index, torch.cuda.current_stream().cuda_stream)]
+    status, side = ws[8:12].view(torch.int32), torch.cuda.Stream()
+    for _ in range(20):
+        torch.cuda.synchronize()
+        policy._verified.clear()
+        out, used, _ = plb.lattice_filter_raw(x, ref, **kw)
+        with torch.cuda.stream(side):
+            status.copy_(bit, non_blocking=True)
+        assert used.data_ptr() == ws.data_ptr()
+        torch.cuda.synchronize()
+        if torch.isnan(out).all():
+            break
+        try:                                                  # too late for some of the slice: again
+            plb.check_pending()
+        except plb.PlError:
+            pass
+    else:
+        pytest.fail("the copy never came before the slice")
+    policy._verified.clear()
+    with pytest.raises(plb.PlError) as err:
+        plb.check_pending() if told_by == "check_pending" else plb.lattice_filter_raw(x, ref, **kw)
+    assert err.value.status == capi.PL_INTERNAL_ERROR
+    plb.check_pending()                                       # told once
+    out, _, _ = plb.lattice_filter_raw(x, ref, **kw)
+    assert torch.isfinite(out).all()
