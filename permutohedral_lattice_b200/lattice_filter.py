@@ -385,12 +385,14 @@ def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha
 
 def lattice_stats(workspace, stream=None, device=None):
     """Counters of the last call that used `workspace` (synchronises the stream).  workspace=None reads
-    those of the last pl_lattice_filter_f32_noalloc call on `device` (default: the current one)."""
+    those of the last pl_lattice_filter_f32_noalloc call on `device` (whatever torch.cuda.device takes; default:
+    the current one)."""
     st = capi.PlStats()
     if workspace is not None:
         device = workspace.device
-    elif device is None:
-        device = torch.device("cuda", torch.cuda.current_device())
+    else:
+        index = torch.cuda.device(device).idx
+        device = torch.device("cuda", index if index is not None and index >= 0 else torch.cuda.current_device())
     if stream is None:
         stream = _stream_handle(device)
     with _OnDevice(device):

@@ -90,3 +90,16 @@ def test_noalloc_reports_a_max_entries_that_was_too_small():
     assert rc == capi.PL_OK
     assert plb.lattice_stats(None).device_status == capi.PL_OK
     assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("device", [None, "cuda", "cuda:0", 0])
+def test_stats_of_the_built_in_scratch_take_any_form_of_device(device):
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from permutohedral_lattice_b200 import capi
+    x = torch.rand((1, 20, 24, 3), device="cuda")
+    rc, _ = _call_noalloc(x, x, [20, 24], True, 4.0, 0.2, 1.0, False)
+    assert rc == capi.PL_OK
+    for d in (device, torch.device(device) if device is not None else None):
+        st = plb.lattice_stats(None, device=d)
+        assert st.device_status == capi.PL_OK and st.num_entries > 0
