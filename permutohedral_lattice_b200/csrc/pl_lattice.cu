@@ -25,11 +25,13 @@
 // side: geometry and workspace layout, launches, and the extern "C" entry points.
 #include <cuda_runtime.h>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <mutex>
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -1253,13 +1255,20 @@ int pl_cancel_watch(void) {
     return PL_OK;
 }
 
+// The report of a call whose stream is idle comes within some tens of microseconds: polled without a pause.  Where
+// it takes longer (earlier work in the stream), or the process has asked for waits that block, the thread sleeps
+// between polls and leaves its core to others; the sleep, 50 to 100 us with the system's timer slack, is then small
+// beside the wait and beside what the device still has to do after the report.
+constexpr auto WATCH_SPIN = std::chrono::microseconds(1000), WATCH_NAP = std::chrono::microseconds(20);
+
 int pl_await_watched_call(int64_t* num_entries, int* device_status, void* stream) {
     Watcher& w = g_watcher;
     w.armed = false;
     if (!num_entries || !device_status || !w.launched) return PL_INVALID_ARGUMENT;
     w.launched = false;
     volatile u64* word = &w.line->words[0];
-    bool drained = false;
+    const auto start = std::chrono::steady_clock::now();
+    bool drained = false, nap = false;
     for (unsigned spin = 1;; spin++) {
         const u64 v = *word;
         if ((u32)(v >> 40) == w.line->seq) {
@@ -1272,13 +1281,18 @@ int pl_await_watched_call(int64_t* num_entries, int* device_status, void* stream
             return PL_CUDA_ERROR;
         }
         // now and then: has the stream failed, or run empty (then the report is there, or never comes)?
-        if ((spin & 0xFFFu) == 0) {
+        if (nap || (spin & 0xFFFu) == 0) {
             const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
             if (e != cudaSuccess && e != cudaErrorNotReady) return cuda_fail(e, "pl_await_watched_call");
             drained = e == cudaSuccess;
+            unsigned flags = 0;
+            if (!nap && cudaGetDeviceFlags(&flags) == cudaSuccess)
+                nap = (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync ||
+                      std::chrono::steady_clock::now() - start > WATCH_SPIN;
+            if (nap && !drained) std::this_thread::sleep_for(WATCH_NAP);
         }
 #if defined(__x86_64__) && !defined(__CUDA_ARCH__)
-        __builtin_ia32_pause();
+        if (!nap) __builtin_ia32_pause();
 #endif
     }
 }

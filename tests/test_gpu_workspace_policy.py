@@ -277,3 +277,22 @@ def test_failure_after_the_report_is_raised_later(policy, dtype, c, told_by):
     plb.check_pending()                                       # told once
     out, _, _ = plb.lattice_filter_raw(x, ref, **kw)
     assert torch.isfinite(out).all()
+
+
+def test_waiting_for_a_report_leaves_the_core_to_others(policy):
+    """A verified call behind a long queue: the thread sleeps most of the wait."""
+    import time
+    import torch
+    import permutohedral_lattice_b200 as plb
+    x, ref = _data(10)
+    plb.lattice_filter_raw(x, ref, **KW)
+    big = torch.zeros(1 << 28, device="cuda")
+    torch.cuda.synchronize()
+    policy._verified.clear()
+    for _ in range(600):                     # some 0.3 ms each
+        big.add_(1.0)
+    wall, busy = time.perf_counter(), time.thread_time()
+    plb.lattice_filter_raw(x, ref, **KW)
+    wall, busy = time.perf_counter() - wall, time.thread_time() - busy
+    assert wall > 0.05, "the queue was empty before the call: nothing tested"
+    assert busy < 0.5 * wall
