@@ -107,7 +107,6 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
         wait_for_previous_kernel();
         return;
     }
-    PhaseClock pc(2);
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
     const int2 info = tile_info[tile];
@@ -152,7 +151,6 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     }
     cp_async_wait_all();
     __syncthreads();
-    pc.mark();
     float acc[VP];
 #pragma unroll
     for (int j = 0; j < VP; j++) acc[j] = 0.f;
@@ -187,7 +185,6 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
         }
     }
     __syncthreads();   // every cached row has been read: the output block may overwrite them
-    pc.mark();
     if (valid) {
         const int last = C - (VP - 4);   // channels in the row's last quad; the next one is the homogeneous channel
         const float norm = last == 0 ? acc[VP - 4] : last == 1 ? acc[VP - 3] : last == 2 ? acc[VP - 2] : acc[VP - 1];
@@ -209,14 +206,12 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     if (bulk_ok) {
         fence_async_proxy();
         __syncthreads();
-        pc.mark();
         if (tid < g.TY) {
             int first, count;
             if (tile_row(g, this_tile(g), tid, first, count))   // recomputed: keeps registers free above
                 bulk_store(output + (size_t)first * C, out_s + (size_t)tid * g.TX * C, (unsigned)count * C * 4u);
             bulk_store_finish();
         }
-        pc.mark();
     } else {
         __syncthreads();
         // element k = tid, tid + TP, ... is channel j of point p; (p, j) advance without a division

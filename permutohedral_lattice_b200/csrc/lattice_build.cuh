@@ -203,7 +203,6 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     __shared__ int cnt_s[PD + 1], base_s;   // entries per remainder; first global entry of the tile
     __shared__ int wsum_s[TP / 32];
 
-    PhaseClock pc(0);
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
     if (tid <= PD) cnt_s[tid] = 0;
@@ -267,7 +266,6 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
         }
     }
     __syncthreads();
-    pc.mark();
 
     int rep[COMPACT ? 1 : PD + 1];   // the splat that represents each splat's key (COMPACT: in rep_s)
     u32 open = 0;                    // splats without a representative
@@ -331,7 +329,6 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             }
         }
     }
-    pc.mark();
     // Number the tile's entries remainder by remainder (all entries of remainder 0 first, ...: the splat
     // stage, which walks the tile's splats in entry order, measured 4 % faster with this order than with
     // entries grouped by warp).  Per warp ONE shared-memory atomic instruction: lane r adds the warp's
@@ -397,7 +394,6 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
         for (int r = 0; r <= PD; r++) place[r] = valid ? atomicAdd(&run_s[lfin[r]], 1) : 0;
     }
     __syncthreads();
-    pc.mark();
     if constexpr (!SORTED) let_next_kernel_start();   // what is left of this tile: its keys
     const int base = base_s;
     if (valid && base >= 0) {
@@ -456,7 +452,6 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             bulk_store_finish();
         }
     }
-    pc.mark(true);
 }
 
 // ---------------------------------------------------------------------------------------------

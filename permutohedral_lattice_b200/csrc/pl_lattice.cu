@@ -1128,35 +1128,6 @@ int pl_export_lattice_f64(const void* workspace, const double* positions, const 
 #undef CALL
 }
 
-#ifdef PL_PHASE_CLOCKS
-// Developer aid: resident CTAs per SM of the config-2 tile kernels, as the runtime computes them.
-int pl_debug_occupancy(int* out) {
-    PL_CUDA(cudaFuncSetAttribute(build_tiles<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<5>::build_smem(false)));
-    PL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out[0], build_tiles<5>, 256, Cfg<5>::build_smem(false)));
-    const size_t ss = SplatRows<5, 22, false>::BYTES;
-    PL_CUDA(cudaFuncSetAttribute(splat_tiles_rows<5, 22, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ss));
-    PL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out[1], splat_tiles_rows<5, 22, false>, 256, ss));
-    int rows_cap = (40 * 1024) / (SliceFast<5, 22>::RS * 4);
-    const size_t sl = SliceFast<5, 22>::bytes(rows_cap);
-    PL_CUDA(cudaFuncSetAttribute(slice_tiles_fast<5, 22>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl));
-    PL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out[2], slice_tiles_fast<5, 22>, 256, sl));
-    out[3] = (int)Cfg<5>::build_smem(false); out[4] = (int)ss; out[5] = (int)sl;
-    cudaFuncAttributes fa;
-    PL_CUDA(cudaFuncGetAttributes(&fa, splat_tiles_rows<5, 22, false>));
-    out[6] = fa.numRegs; out[7] = (int)fa.sharedSizeBytes;
-    return PL_OK;
-}
-
-// Developer aid: copies (and clears) the per-kernel phase cycle counters, 8 x 16 values.  SYNCHRONISES.
-int pl_debug_phase_cycles(unsigned long long* out) {
-    PL_CUDA(cudaDeviceSynchronize());
-    PL_CUDA(cudaMemcpyFromSymbol(out, g_phase_cycles, sizeof(unsigned long long) * 8 * 16));
-    static unsigned long long zeros[8 * 16] = {0};
-    PL_CUDA(cudaMemcpyToSymbol(g_phase_cycles, zeros, sizeof(zeros)));
-    return PL_OK;
-}
-#endif
-
 int pl_crf_update_f32(float* q_out, const float* unaries, const float* q_bilateral, const float* q_spatial,
                       const float* compatibility, float bilateral_weight, float spatial_weight,
                       int64_t n_points, int n_labels, void* stream) {

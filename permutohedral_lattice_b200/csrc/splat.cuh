@@ -355,7 +355,6 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
         wait_for_previous_kernel();
         return;
     }
-    PhaseClock pc(1);
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
@@ -381,7 +380,6 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     if ((PRE || bulk_ok) && tid == 0) mbar_init(&bar, 1);
     const int nvalid = __syncthreads_count(valid);
     const int total = nvalid * (PD + 1);
-    pc.mark();
     // PRE: the tile's sorted splats arrive by one bulk copy, already in the windowed form the loop below reads
     constexpr unsigned REC_BYTES = PRE ? (unsigned)(sizeof(uint2) * SR::SORTED) : 0u;
     if ((PRE || bulk_ok) && tid == 0) {
@@ -423,7 +421,6 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     }
 
     if constexpr (!PRE) SplatCommon<PD>::template sort_splats<WL>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
-    pc.mark();
     // did this thread see the copies complete within the bounded wait
     const bool arrived = (PRE || bulk_ok) ? mbar_wait(&bar, 0) : true;
     if (bulk_ok) {
@@ -483,7 +480,6 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
         wait_for_previous_kernel();
         return;
     }
-    pc.mark();
     wait_for_previous_kernel();
     if (call_failed(hdr)) return;   // a failure of the index stage
 
@@ -528,7 +524,6 @@ auto one = [&](unsigned key, unsigned weight) {
             if constexpr (ONE) break;
         }
     }
-    pc.mark(true);
 }
 
 // ---------------------------------------------------------------------------------------------
