@@ -15,7 +15,8 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libpl_lattice.so")
 SOURCES = [os.path.join(CSRC, "pl_lattice.cu")]
 HEADERS = [os.path.join(CSRC, h) for h in ("simplex.cuh", "common.cuh", "lattice_build.cuh", "splat.cuh",
-                                             "blur_slice.cuh", "small.cuh", "export.cuh", "fp64.cuh", "direct_index.cuh", "direct_bounds.h", "crf.cuh")] + [
+                                             "blur_slice.cuh", "small.cuh", "export.cuh", "fp64.cuh", "direct_index.cuh", "direct_bounds.h", "crf.cuh",
+                                             "smem_limit.h")] + [
     os.path.join(ROOT, "include", "pl_lattice.h")]
 
 

@@ -44,6 +44,7 @@
 #include "export.cuh"
 #include "fp64.cuh"
 #include "crf.cuh"
+#include "smem_limit.h"
 
 namespace pl {
 
@@ -330,23 +331,20 @@ static int num_sms() {
     return g_num_sms;
 }
 
-// cudaFuncSetAttribute is a driver call and its effect lasts as long as the context: the dynamic
-// shared-memory limit (and carve-out preference) of a kernel is raised once per device, and again only
-// when a later call needs more than any call before it.
-constexpr int MAX_DEVICES = 64;
+// Raises a kernel's dynamic shared-memory limit (and sets its carve-out preference) when this call needs more than any
+// call before it on the current device.
 template <auto Kernel>
 static int ensure_dynamic_smem(size_t bytes, bool max_carveout = false) {
-    static std::atomic<size_t> granted[MAX_DEVICES];   // zero-initialised: nothing granted yet
+    static SmemLimit limit;
     int dev = -1;
     PL_CUDA(cudaGetDevice(&dev));
-    const bool cached = dev >= 0 && dev < MAX_DEVICES;
-    if (cached && granted[dev].load(std::memory_order_acquire) >= bytes + 1) return PL_OK;
-    PL_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    if (max_carveout)
-        PL_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     cudaSharedmemCarveoutMaxShared));
-    if (cached) granted[dev].store(bytes + 1, std::memory_order_release);
-    return PL_OK;
+    return limit.raise(dev, bytes, [&](size_t n) -> int {
+        PL_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n));
+        if (max_carveout)
+            PL_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared));
+        return PL_OK;
+    });
 }
 #define PL_TRY(call)                     \
     do {                                 \

@@ -99,6 +99,38 @@ def test_verified_calls_from_several_threads(gpu):
     assert not wrong
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_calls_of_several_widths_from_several_threads(dtype, gpu):
+    """Threads whose calls need more shared memory of the same kernels than one another's, all at once."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(67)
+    pos = torch.from_numpy(rng.standard_normal((1, 700, 7))).to(getattr(torch, dtype)).cuda()
+    xs = [torch.from_numpy(rng.random((1, 700, c))).to(pos.dtype).cuda() for c in (30, 5, 60, 9, 100, 16)]
+    got, wrong, together = [None] * len(xs), [], threading.Barrier(len(xs))
+    torch.cuda.synchronize()
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                together.wait(30)
+                got[k] = plb.filter_positions(xs[k], pos, max_entries=0)[0]
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:   # noqa: BLE001 - reported below
+            wrong.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(xs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    for x, g in zip(xs, got):
+        want = plb.filter_positions(x, pos, max_entries=0)[0]
+        # sums in varying order
+        assert float((g - want).norm() / want.norm()) <= (1e-12 if dtype == "float64" else 1e-5)
+
+
 @pytest.mark.parametrize("pd,n", [(1, 8200), (2, 5470), (3, 4100), (5, 2735), (8, 1825), (16, 970)])
 def test_small_lattices_give_the_bits_of_wide_ones(pd, n, gpu, oracle):
     """A bound of 6144 entries is the largest that takes the one-cluster index, and with it rows of one quad take
