@@ -138,8 +138,9 @@ int pl_lattice_apply_f32(float* output, const float* input, int n_input_channels
  * PL_STATIC_SCRATCH_BYTES on every GPU that loads the library, held until the process exits.
  * This entry point has no counterpart in the reference.
  *  - It calls no cudaMalloc / cudaFree and no allocating library routine.
- *  - A call whose pl_workspace_bytes exceeds PL_STATIC_SCRATCH_BYTES returns
- *    PL_WORKSPACE_TOO_SMALL before launching anything (pl_last_cuda_error then holds the two sizes);
+ *  - A call that needs more than PL_STATIC_SCRATCH_BYTES (what pl_workspace_bytes says, less 8 bytes and a
+ *    little for each of the batch * n * (pd + 1) splats, whose sorted order only a kept lattice stores)
+ *    returns PL_WORKSPACE_TOO_SMALL before launching anything (pl_last_cuda_error then holds the two sizes);
  *    a smaller max_entries shrinks the need.  Whether the lattice stayed within that max_entries is
  *    known only on the device: read it with pl_lattice_stats(NULL, &stats, stream) and check
  *    stats.device_status (on PL_CAPACITY_EXCEEDED the output holds NaN).

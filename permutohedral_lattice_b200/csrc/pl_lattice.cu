@@ -269,8 +269,9 @@ static int make_geom(Geom& g, int batch, int n, int pd, int n_sdims, const int* 
 
 // real_bytes: 4 for float calls, 8 for double calls (wider weights and value rows, no fixed-point sums).
 // with_fixed_point: the workspace also holds the 64-bit sums of the deterministic mode (float calls only).
+// with_sorted: it also holds every tile's splats sorted (float calls only; used by lattices built to be applied later).
 static int make_layout(Layout& L, const Geom& g, int pd, int vd, int64_t max_entries_arg, int real_bytes = 4,
-                       bool with_fixed_point = false) {
+                       bool with_fixed_point = false, bool with_sorted = true) {
     const u64 S = (u64)g.batch * (u64)g.n * (u64)(pd + 1);
     if (S >= 0x7FFFFFF0ull) return PL_INVALID_ARGUMENT;
     u64 E = (max_entries_arg <= 0 || (u64)max_entries_arg > S) ? S : (u64)max_entries_arg;
@@ -285,7 +286,7 @@ static int make_layout(Layout& L, const Geom& g, int pd, int vd, int64_t max_ent
     L.rec = off;       off += align_up(sizeof(u16) * tile_splats * (size_t)g.num_tiles);
     L.rec_w = off;     off += align_up((size_t)real_bytes * tile_splats * (size_t)g.num_tiles);
     L.srec = off;      // the splats of every tile sorted by entry (float calls: what their splat kernels walk)
-    if (real_bytes == 4) off += align_up(sizeof(uint2) * (size_t)srec_words_of(pd) * (size_t)g.num_tiles);
+    if (real_bytes == 4 && with_sorted) off += align_up(sizeof(uint2) * (size_t)srec_words_of(pd) * (size_t)g.num_tiles);
     L.list_keys = off; off += align_up(sizeof(u64) * kw_of(pd) * E);
     L.list_ref = off;  off += align_up(sizeof(u32) * E);
     L.vid = off;       off += align_up(sizeof(u32) * E);
@@ -747,10 +748,10 @@ static int run_export(const Geom& g, const R* positions, const R* reference, con
 static int filter_common(const Geom& g, float* output, const float* input, const float* positions,
                          const float* reference, int pd, int vd, int reverse, void* workspace,
                          size_t workspace_bytes, int64_t max_entries, int mode, cudaStream_t st,
-                         int phases = PH_BUILD | PH_APPLY) {
+                         int phases = PH_BUILD | PH_APPLY, bool with_sorted = true) {
     if (mode != PL_MODE_ATOMIC && mode != PL_MODE_DETERMINISTIC) return PL_INVALID_ARGUMENT;
     Layout L;
-    int rc = make_layout(L, g, pd, vd, max_entries, 4, mode == PL_MODE_DETERMINISTIC);
+    int rc = make_layout(L, g, pd, vd, max_entries, 4, mode == PL_MODE_DETERMINISTIC, with_sorted);
     if (rc != PL_OK) return rc;
     if (workspace_bytes < L.total) return PL_WORKSPACE_TOO_SMALL;
 #define CALL(P) run_filter<P>(g, output, input, positions, reference, vd, reverse, mode, workspace, L, st, phases)
@@ -921,9 +922,10 @@ int pl_lattice_filter_f32_noalloc(float* output, const float* input, const float
     if (!pl_supported(pd, vd)) return PL_UNSUPPORTED_DIMS;
     if (batch == 0 || n == 0) return PL_OK;
     if (!output || !input || (g.R > 0 && !reference)) return PL_INVALID_ARGUMENT;
-    // sizes beyond the built-in scratch are refused before anything is launched
+    // Sizes beyond the built-in scratch are refused before anything is launched.  The scratch has no room for sorted
+    // splats, which a lattice used once does not keep.
     Layout L;
-    rc = make_layout(L, g, pd, vd, max_entries);
+    rc = make_layout(L, g, pd, vd, max_entries, 4, false, false);
     if (rc != PL_OK) return rc;
     if (L.total > (size_t)PL_STATIC_SCRATCH_BYTES) {
         snprintf(g_cuda_error, sizeof(g_cuda_error),
@@ -934,10 +936,11 @@ int pl_lattice_filter_f32_noalloc(float* output, const float* input, const float
     void* scratch = nullptr;
     rc = static_scratch_of_current_device(&scratch);   // first call on a device: looks the address up
     if (rc != PL_OK) return rc;
-    // the call itself zeroes the counters it needs (the 256-byte header) and the value rows it sums
-    // into; everything else in the scratch is written before it is read
+    // the call itself zeroes the counters it needs (the header and, in calls that keep one, the sketch behind it) and
+    // the value rows it sums into; everything else in the scratch is written before it is read
     return filter_common(g, output, input, nullptr, reference, pd, vd, reverse, scratch,
-                         (size_t)PL_STATIC_SCRATCH_BYTES, max_entries, PL_MODE_ATOMIC, (cudaStream_t)stream);
+                         (size_t)PL_STATIC_SCRATCH_BYTES, max_entries, PL_MODE_ATOMIC, (cudaStream_t)stream,
+                         PH_BUILD | PH_APPLY, false);
 }
 
 int pl_lattice_build_f32(const float* reference, int batch, int n_spatial_dims, const int* spatial_dims,

@@ -72,6 +72,35 @@ def test_noalloc_refuses_sizes_beyond_its_scratch():
     assert np.abs(g - w).max() <= MAX_ABS_TOL
 
 
+def test_noalloc_needs_no_room_for_sorted_splats():
+    """The largest bound that the scratch took while the header had no sketch behind it and a tile's sorted splats took
+    240 bytes less is still taken."""
+    import ctypes
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from permutohedral_lattice_b200 import capi
+
+    def need(entries):
+        b = ctypes.c_size_t(0)
+        assert capi.lib().pl_workspace_bytes(1, 320 * 320, 5, 4, 2, capi.int_array([320, 320]), entries, 0,
+                                             ctypes.byref(b)) == capi.PL_OK
+        return b.value
+
+    scratch, grown = 64 << 20, 8192 + 240 * 400   # 400 tiles
+    lo, hi = 1000, 320 * 320 * 6
+    assert need(lo) - grown <= scratch < need(hi) - grown
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if need(mid) - grown <= scratch else (lo, mid)
+    x = torch.rand((1, 320, 320, 3), device="cuda")
+    ref = torch.full((1, 320, 320, 3), 0.5, device="cuda")
+    rc, out = _call_noalloc(x, ref, [320, 320], True, 8.0, 0.125, 1.0, False, max_entries=lo)
+    assert need(lo) > scratch and rc == capi.PL_OK
+    assert plb.lattice_stats(None).device_status == capi.PL_OK
+    want = plb.lattice_filter(x, ref, True, 8.0, 0.125)
+    assert float((out - want).norm() / want.norm()) <= REL_L2_TOL
+
+
 def test_noalloc_reports_a_max_entries_that_was_too_small():
     """The call itself returns PL_OK (nothing is known on the host); the device sets a status bit, every
     later kernel of the call stands down, and the output is filled with NaN.  Nothing faults."""
