@@ -306,6 +306,8 @@ MOST_PLANS = 256
 
 
 def _plan_of(x, ref, bilateral, theta_alpha, theta_beta, theta_gamma):
+    # the thetas as numbers: an array has no hash, and a tensor is a key by its identity, whatever it comes to hold
+    theta_alpha, theta_beta, theta_gamma = float(theta_alpha), float(theta_beta), float(theta_gamma)
     key = (x.device.index, x.dtype, x.shape, None if ref is None else ref.shape, bool(bilateral), theta_alpha,
            theta_beta, theta_gamma)
     plan = _plans.get(key)
