@@ -6,20 +6,25 @@
 //                   per point; the tile's keys are de-duplicated in a shared-memory hash; the
 //                   distinct keys become a contiguous run of "entries" in a global list and every
 //                   splat records the 16-bit index of its entry inside the tile.
-//   clear_table     sizes the global hash table from the entry count (on the device) and clears it.
+//   clear_table     sizes the global hash table (on the device) from the entry count or, in larger calls, from
+//                   build_tiles' sketch of the vertices, and clears it and the filter in front of it.
 //   insert_entries  one CAS per entry into the table; the first entry of a key owns a new vertex, whose
-//                   neighbour slots and value row the same launch initialises.
-//   link_neighbours entry -> vertex index; then the +-1 neighbours of every vertex along each of the
-//                   pd+1 axes: one table lookup per vertex and axis fills both directions.
+//                   neighbour slots the same launch initialises.
+//   link_neighbours entry -> vertex index; value rows zeroed; then the +-1 neighbours of every vertex along each
+//                   of the pd+1 axes: one table lookup per vertex and axis fills both directions.
 //   splat_tiles     one CTA per tile: input block staged in shared memory (bulk async copies), splats
 //                   sorted by entry, runs summed in registers, vector reductions into the vertex rows.
 //   blur_axis       pd+1 launches: V'[v] = (V[n1] + 2 V[v] + V[n2]) / 4, Jacobi, ping-pong buffers.
 //   slice_tiles     one CTA per tile: the tile's vertex rows staged in shared memory, each point
 //                   interpolates, divides by the homogeneous channel and writes its output row.
 //
-// A table slot is one 64-bit word (32-bit hash tag | index of the owning entry); full keys are
-// compared through the entry list, which a previous launch has completely written, so there are no
-// locks, no waiting and no duplicate vertices.  All device loops are bounded.
+// Small lattices take one launch for the three index kernels and one for all blur passes (small.cuh); spatial-only calls
+// index their vertices without hashing (direct_index.cuh).
+//
+// A table slot is one 64-bit word: 32-bit hash tag | index of the entry that created the vertex, which becomes the
+// vertex's own index when the creator's round ends.  Full keys are compared through the entry list, which a previous
+// launch has completely written, or through the vertex's key, so there are no locks, no waiting and no duplicate
+// vertices.  All device loops are bounded.
 //
 // Device code lives in the headers included below (one translation unit); this file holds the host
 // side: geometry and workspace layout, launches, and the extern "C" entry points.
@@ -362,13 +367,15 @@ static int rows_cap_for(int pd, int vd) {
     return cap;
 }
 
-// Widest row the splat stage takes: its tile's rows and twice its sorted list within 200 KB.
+// Widest row the splat stage takes: its tile's rows and twice its sorted list within 200 KB.  (The kernel's own need,
+// SplatRows::bytes, is a little less.)
 static int widest_vd(int pd) {
     const int tp = tp_of(pd);
     return ((200 * 1024 - 16 * tp * (pd + 1) - 4 * tp) / (4 * tp)) & ~3;
 }
 
-// The same of the deterministic splat: its input block and one and a half sorted lists within 200 KB.
+// The same of the deterministic splat: unpadded input rows and one and a half sorted lists within 200 KB.  (With its rows
+// padded the kernel asks for up to 209,408 bytes, at pd 4 and 8, of the 227 KB that a block may have.)
 static int widest_vd_fixed(int pd) {
     const int tp = tp_of(pd);
     return (200 * 1024 - 12 * tp * (pd + 1) - 4 * tp) / (4 * tp) + 1;

@@ -57,8 +57,8 @@ PL_HD int exact_int(float x) { return PL_F2BITS(PL_FADD(x, PL_ROUND_MAGIC)) - 0x
 // (float)c for 0 <= c < 2^23 (no conversion unit).
 PL_HD float small_int_to_float(int c) { return PL_FSUB(PL_BITS2F(0x4B000000 | c), 8388608.0f); }
 
-// Correctly rounded a / b from the correctly rounded reciprocal rcp_b = RN(1 / b): q = RN(a rcp_b),
-// exact remainder r = a - b q by fused multiply-add, result RN(q + r rcp_b).  For finite operands
+// Correctly rounded a / b from the correctly rounded reciprocal rcp_b = RN(1 / b) (Markstein, IBM J. Res. Dev. 34,
+// 1990): q = RN(a rcp_b), exact remainder r = a - b q by fused multiply-add, result RN(q + r rcp_b).  For finite operands
 // whose quotient and remainder stay in the normal range this equals the IEEE quotient.
 PL_HD float div_by_rcp(float a, float b, float rcp_b) {
     const float q = PL_FMUL(a, rcp_b);

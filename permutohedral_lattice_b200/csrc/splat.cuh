@@ -25,13 +25,15 @@ __device__ __forceinline__ uint4 splat_record(unsigned key, double w) {
 template <int PD>
 struct SplatCommon {
     static constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, NW = TP / 32;
-    // Words of the sorted list when it is cut into windows (one spare word per window, WL >= PD + 1).
+    // Words of the sorted list with one spare word a window of PD + 1 splats.
     static constexpr int SORTED = SPLATS + TP;
 
-    // Sorted position pos is stored at slot(pos): the list is cut into windows of WL splats, each followed by two
-    // spare words (Cfg<PD>::WL, see there) or by one.  Splats of one entry (written together by neighbouring lanes) land in
-    // neighbouring words, and lanes that walk neighbouring windows in step read words WL + 1 apart: an
-    // odd number of 8-byte words, so neither side collides on shared-memory banks.
+    // Sorted position pos is stored at slot(pos).  Splats of one entry, written together by neighbouring lanes, land in
+    // neighbouring words either way.
+    // WL = Cfg<PD>::WL (a group of lanes per window, 16 bytes a load): stretches of WL splats, two spare words after each,
+    // see there.
+    // WL = PD + 1 (a thread per window, 8 bytes a load): one spare word a window, so that lanes in step read words PD + 2
+    // apart: an odd distance, and no two on one bank, where PD is odd (5 above all).
     template <int WL>
     __device__ static __forceinline__ int slot(int pos) {
         if constexpr (WL == Cfg<PD>::WL)
@@ -499,7 +501,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
             for (int pos = first; pos < end; pos += WL) {
                 const uint2* sp = sorted_s + Cfg<PD>::srec_slot(pos);
                 const int count = min(WL, end - pos);
-auto one = [&](unsigned key, unsigned weight) {
+                auto one = [&](unsigned key, unsigned weight) {
                     const int e = (int)(key >> 16);
                     if (e != cur) {
                         acc.flush(v0 + (size_t)vcur * VP + 4 * h);

@@ -1,6 +1,6 @@
 """Splat and slice over value rows of every width class, against the oracle.
 
-Lanes of a splat window (1, 2, 4, 8, 16, 32) and the slice's row width change at the vd below and beside each of
+Lanes of a splat window (2, 4, 8, 16, 32; in double 1 too) and the slice's row width change at the vd below and beside each of
 them; a channel count that is a multiple of four leaves the homogeneous channel a quad of its own.  The bounds are
 those of every comparison with the oracle (gpu_helpers): float sums of a few hundred terms in another order."""
 import numpy as np
@@ -128,3 +128,21 @@ def test_grid_follows_the_largest_value_wherever_it_lies(gpu):
             out, ws, _ = plb.lattice_filter_raw(x, ref, True, 4.0, 0.2, mode="deterministic")
             bits = int(ws[16:20].view(torch.int32).item())      # the header's word for the largest magnitude
             assert bits == int(np.float32(1e30).view(np.int32)), (offset, where)
+
+
+@pytest.mark.parametrize("pd,atomic,deterministic", [(4, 176, 185), (5, 172, 182), (8, 160, 173), (16, 328, 349)])
+def test_widest_rows_taken_and_first_refused(pd, atomic, deterministic, gpu, oracle):
+    """The splat stage's limits on the value dimension, which have not moved since its first kernels."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from permutohedral_lattice_b200 import capi
+    rng = np.random.default_rng(103)
+    pos = rng.standard_normal((1, 300, pd)).astype(np.float32)
+    pt = torch.from_numpy(pos).cuda()
+    for mode, widest in (("atomic", atomic), ("deterministic", deterministic)):
+        val = rng.random((1, 300, widest - 1), dtype=np.float32)
+        got = plb.filter_positions(torch.from_numpy(val).cuda(), pt, mode=mode)[0].cpu().numpy()
+        gpu.assert_outputs_close(got[0], oracle.filter(val[0], pos[0], structure=False).out, "%s, vd %d" % (mode, widest))
+        with pytest.raises(plb.PlError) as err:
+            plb.filter_positions(torch.rand((1, 300, widest), device="cuda"), pt, mode=mode)
+        assert err.value.status == capi.PL_UNSUPPORTED_DIMS
