@@ -483,7 +483,9 @@ def main():
     if staged:
         dominant = max(kernel_names, key=lambda k: stage_ms[k])
         achieved = kernel_bytes[dominant] / max(kernel_ms[dominant] * 1e-3, 1e-12) / 1e9
-        traffic, traffic_source = measured_traffic(full.name, kernel_names[dominant], arm.b * n)
+        # (the capture is of the workload's own channels, in atomic mode, with a lattice a call)
+        captured = args.mode == "atomic" and not args.channels and not args.reuse_lattice
+        traffic, traffic_source = measured_traffic(full.name, kernel_names[dominant], arm.b * n) if captured else (None, None)
         roofline = {"bound": "hbm", "kernel": kernel_names[dominant], "achieved": achieved,
                     "peak": hbm_gbs, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / hbm_gbs,
                     "traffic": traffic, "traffic_source": traffic_source,
