@@ -552,12 +552,15 @@ def lattice_filter(input_image, reference_image, bilateral=True, theta_alpha=1.0
     return fn.apply(input_image, reference_image, bool(bilateral), *thetas, bool(reverse), mode)
 
 
+_is_tracing, _functorch_level, _is_compiling = (
+    torch._C._is_tracing, torch._C._functorch.maybe_current_level, torch.compiler.is_compiling)
+
+
 def _watched_by_torch():
     """True while something other than reverse mode follows the tensors: a tracer, forward-mode differentiation, a
     functorch transform.  None of them sees the kernels, which go through ctypes; the autograd function is what tells
     a tracer that there was a call, and what makes the others refuse it."""
-    return (torch._C._get_tracing_state() is not None or forward_ad._current_level >= 0 or
-            torch._C._functorch.maybe_current_level() is not None or torch.compiler.is_compiling())
+    return _is_tracing() or forward_ad._current_level >= 0 or _functorch_level() is not None or _is_compiling()
 
 
 def _as_attr(v):
