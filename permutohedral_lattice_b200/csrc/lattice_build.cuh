@@ -52,21 +52,28 @@ struct PointKeys {
         if constexpr (!WIDE) perm += shift_in(15u, (u32)(4 * s.rank[PD] - 4));
         last_rank = s.rank[PD];
     }
-    // from remainder r - 1 to remainder r
-    __device__ __forceinline__ void step(int r) {
+    __device__ __forceinline__ u32 moved16(int r) const {   // 16 x the coordinate that a step to r takes a cell off
         const int rank = PD - r + 1;
-        u32 c16;   // 16 x the coordinate of that rank
         if constexpr (WIDE) {
-            c16 = ((rank > 8 ? perm_hi >> (4 * (rank - 9)) : perm >> (4 * (rank - 1))) & 15u) * 16u;
-            if (rank == last_rank) c16 = 512u;
+            const u32 c16 = ((rank > 8 ? perm_hi >> (4 * (rank - 9)) : perm >> (4 * (rank - 1))) & 15u) * 16u;
+            return rank == last_rank ? 512u : c16;
         } else {
-            c16 = ((rank > 1) ? perm >> (4 * (rank - 2)) : perm << 4) & 0xF0u;
+            return ((rank > 1) ? perm >> (4 * (rank - 2)) : perm << 4) & 0xF0u;
         }
+    }
+    __device__ __forceinline__ u32 moves(u32 c16, int j) const {   // what that step adds to word j
+        return ((2 * j + 1 < PD) ? 0x00010001u : 1u) - shift_in((u32)(PD + 1), c16 - 32u * j);
+    }
+    // from remainder r - 1 to remainder r, and back
+    __device__ __forceinline__ void step(int r) {
+        const u32 c16 = moved16(r);
 #pragma unroll
-        for (int j = 0; j < CW; j++) {
-            const u32 ones = (2 * j + 1 < PD) ? 0x00010001u : 1u;
-            w[j] += ones - shift_in((u32)(PD + 1), c16 - 32u * j);
-        }
+        for (int j = 0; j < CW; j++) w[j] += moves(c16, j);
+    }
+    __device__ __forceinline__ void step_back(int r) {
+        const u32 c16 = moved16(r);
+#pragma unroll
+        for (int j = 0; j < CW; j++) w[j] -= moves(c16, j);
     }
     // 32-bit hash of the key (of item `seed`): its high bits place the key in the tile's table
     __device__ __forceinline__ u32 hash(u32 seed) const {
@@ -136,6 +143,15 @@ struct TileKeys {
         for (int j = 0; j < CW; j++) diff |= x[j] ^ y[j];
         return diff == 0;
     }
+    // the same for a splat b whose key the caller holds (COMPACT)
+    __device__ __forceinline__ bool same_as(int a, int b, int r, const u32 (&y)[CW]) const {
+        if ((u32)(a ^ b) & ~(u32)(TP - 1)) return false;
+        u32 x[CW], diff = 0;
+        load(a, r, x);
+#pragma unroll
+        for (int j = 0; j < CW; j++) diff |= x[j] ^ y[j];
+        return diff == 0;
+    }
     __device__ __forceinline__ u32 hash(int id, int r, u32 seed) const {
         u32 k[CW];
         load(id, r, k);
@@ -146,9 +162,12 @@ struct TileKeys {
     }
     // the key as the global list holds it
     __device__ __forceinline__ Key<Cfg<PD>::KW> global_key(int id, int r, int item) const {
-        constexpr int KW = Cfg<PD>::KW;
         u32 k[CW];
         load(id, r, k);
+        return global_key(k, item);
+    }
+    __device__ static __forceinline__ Key<Cfg<PD>::KW> global_key(const u32 (&k)[CW], int item) {
+        constexpr int KW = Cfg<PD>::KW;
         Key<KW> out;
 #pragma unroll
         for (int j = 0; j < KW; j++) {
@@ -202,10 +221,12 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     u16* rep_s = lidx_s + SPLATS;                                                 // [SPLATS], COMPACT only
     __shared__ int cnt_s[PD + 1], base_s;   // entries per remainder; first global entry of the tile
     __shared__ int wsum_s[TP / 32];
+    __shared__ int open_s;   // COMPACT: splats without representative
 
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
     if (tid <= PD) cnt_s[tid] = 0;
+    if (COMPACT && tid == 0) open_s = 0;
     if (tile == 0 && tid == 0) {
         hdr->capacity = max_entries;
         hdr->sorted = SORTED ? 1u : 0u;
@@ -216,6 +237,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     u32 slot2[PD / 2 + 1];   // slots of the splats' keys, two to a word
 #pragma unroll
     for (int r = 0; r <= PD / 2; r++) slot2[r] = 0;
+    PointKeys<PD> k;
     if (valid) {
         R f[PD];
         R w[PD + 1];
@@ -232,10 +254,9 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
         R* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
         for (int r = 0; r <= PD; r++) recw_tile[r * TP + tid] = w[r];
-        // COMPACT: a slot is written by the key that the steps below give and read by the one that the stored ranks
-        // give.  Where the ranks were no permutation the two differed, and the slot read was one that no splat had written.
+        // COMPACT: a point's own key is formed by steps, that of a splat it is compared with from the stored ranks.
+        // Where the ranks are no permutation the two differ.
         if constexpr (COMPACT) settle_ranks<PD>(s);
-        PointKeys<PD> k;
         k.start(s);
         if constexpr (COMPACT) {
             u32* mine = keys.s + tid * Cfg<PD>::KEY_WORDS;
@@ -255,7 +276,8 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             const u32 h = k.hash(seed);
             const u32 slot = h >> (32 - LSLOG);
             slots_s[slot] = (u16)(r * TP + tid);
-            slot2[r / 2] |= slot << (16 * (r & 1));
+            if constexpr (COMPACT) lidx_s[r * TP + tid] = (u16)slot;   // (there are no entry numbers yet)
+            else slot2[r / 2] |= slot << (16 * (r & 1));
             if (sketch_shift >= 0) {
                 const u32 x = (h ^ (h >> 15)) * 0x9E3779B1u;
                 if ((x >> 1) < (0x80000000u >> sketch_shift)) {
@@ -279,15 +301,16 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     };
     if constexpr (COMPACT) {
 #pragma unroll 1
-        for (int r = 0; r <= PD; r++) {
+        for (int r = PD; r >= 0; r--) {   // the key is that of remainder PD by now and goes back step by step
             const int me = r * TP + tid;
             int c = me;
             if (valid) {
-                c = slots_s[keys.hash(me, r, (u32)item * TILE_SEED) >> (32 - LSLOG)];
-                if (c != me && !keys.same(c, me, r)) {
+                c = slots_s[lidx_s[me]];
+                if (c != me && !keys.same_as(c, me, r, k.w)) {
                     c = me;
                     open |= 1u << r;
                 }
+                if (r > 0) k.step_back(r);
             }
             set_rep(r, c);
         }
@@ -304,26 +327,58 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             }
         }
     }
-    for (int round = 1; round <= TILE_ROUNDS; round++) {
-        if (!__syncthreads_or((int)open)) break;
-        auto next_slot = [&](int r) {
-            const u32 h = keys.hash(r * TP + tid, r, (u32)item * TILE_SEED) + (u32)round * 0x632BE5ABu;
-            return ((h ^ (h >> 13)) * 0x85EBCA77u) >> (32 - LSLOG);
-        };
+    auto next_slot = [&](int id, int r, int round) {
+        const u32 h = keys.hash(id, r, (u32)item * TILE_SEED) + (u32)round * 0x632BE5ABu;
+        return ((h ^ (h >> 13)) * 0x85EBCA77u) >> (32 - LSLOG);
+    };
+    if constexpr (COMPACT) {
+        // The open splats, a few in a hundred, are put in a list and the rounds run over that.  Looked for among all 17
+        // splats of a point, most warps had one or another of every remainder and went through hash and comparison
+        // for each: with it and the keys by steps 350 -> 286 us on 1 M points.  (With six splats a point, whose keys lie in shared memory as they are, the list and its barriers
+        // cost more than they saved: 160 -> 170 us on 16 x 512x512, pd 5.)
+        u16* const list = lidx_s;
+        __syncthreads();   // the slots kept there have been read
         if (open) {
-#pragma unroll (COMPACT ? 1 : PD + 1)
-            for (int r = 0; r <= PD; r++)
-                if ((open >> r) & 1u) slots_s[next_slot(r)] = (u16)(r * TP + tid);
+            int pos = atomicAdd(&open_s, __popc(open));
+            for (u32 rest = open; rest; rest &= rest - 1) list[pos++] = (u16)((__ffs(rest) - 1) * TP + tid);
         }
         __syncthreads();
-        if (open) {
-#pragma unroll (COMPACT ? 1 : PD + 1)
-            for (int r = 0; r <= PD; r++) {
-                if ((open >> r) & 1u) {
-                    const int me = r * TP + tid, c = slots_s[next_slot(r)];
-                    if (c == me || keys.same(c, me, r)) {
-                        set_rep(r, c);
-                        open &= ~(1u << r);
+        const int listed = open_s;
+        u32 todo = 0;   // of the list's splats number tid + m TP, those still open
+        for (int m = 0; tid + m * TP < listed; m++) todo |= 1u << m;
+        for (int round = 1; listed && round <= TILE_ROUNDS; round++) {
+            for (u32 rest = todo; rest; rest &= rest - 1) {
+                const int id = list[tid + (__ffs(rest) - 1) * TP];
+                slots_s[next_slot(id, id / TP, round)] = (u16)id;
+            }
+            __syncthreads();
+            for (u32 rest = todo; rest; rest &= rest - 1) {
+                const int m = __ffs(rest) - 1, id = list[tid + m * TP], c = slots_s[next_slot(id, id / TP, round)];
+                if (c == id || keys.same(c, id, id / TP)) {
+                    rep_s[id] = (u16)c;
+                    todo &= ~(1u << m);
+                }
+            }
+            if (!__syncthreads_or((int)todo)) break;
+        }
+    } else {
+        for (int round = 1; round <= TILE_ROUNDS; round++) {
+            if (!__syncthreads_or((int)open)) break;
+            if (open) {
+#pragma unroll
+                for (int r = 0; r <= PD; r++)
+                    if ((open >> r) & 1u) slots_s[next_slot(r * TP + tid, r, round)] = (u16)(r * TP + tid);
+            }
+            __syncthreads();
+            if (open) {
+#pragma unroll
+                for (int r = 0; r <= PD; r++) {
+                    if ((open >> r) & 1u) {
+                        const int me = r * TP + tid, c = slots_s[next_slot(me, r, round)];
+                        if (c == me || keys.same(c, me, r)) {
+                            rep[r] = c;
+                            open &= ~(1u << r);
+                        }
                     }
                 }
             }
@@ -400,7 +455,10 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 #pragma unroll (COMPACT ? 1 : PD + 1)
         for (int r = 0; r <= PD; r++) {
             const int me = r * TP + tid;
-            if (get_rep(r) == me) list_keys[(size_t)base + (seg[r] + lidx_s[me])] = keys.global_key(me, r, item);
+            if (get_rep(r) == me)
+                list_keys[(size_t)base + (seg[r] + lidx_s[me])] =
+                    COMPACT ? TileKeys<PD>::global_key(k.w, item) : keys.global_key(me, r, item);
+            if (COMPACT && r < PD) k.step(r + 1);
         }
     }
     if constexpr (SORTED && !is_double<R>::value) {
