@@ -366,6 +366,25 @@ __device__ __forceinline__ void poison_tile_output(const Geom& g, T* __restrict_
 // aligned: every row access below is a float4, and a row of 22 channels covers exactly three
 // 32-byte sectors.  Pad channels stay zero through splat and blur and are never sliced.
 // ---------------------------------------------------------------------------------------------
+// Two floats an instruction, each rounded as by the scalar one.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<u64*>(&a)), "l"(*reinterpret_cast<u64*>(&b)), "l"(*reinterpret_cast<u64*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    u64 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<u64*>(&a)), "l"(*reinterpret_cast<u64*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    u64 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<u64*>(&a)), "l"(*reinterpret_cast<u64*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+
 // Vector reduction into global memory (sm_90+): one L2 operation per 16 bytes.
 __device__ __forceinline__ void red_add_v4(float* addr, float4 v) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v.x), "f"(v.y), "f"(v.z),
