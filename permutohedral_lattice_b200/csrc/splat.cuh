@@ -140,8 +140,74 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
     for (int j = 0; j < VP; j++) acc[j] = 0.f;
 }
 
+// A tile with few entries for its splats (a volume, a smooth guide): points next to one another mostly share their
+// vertices, so that walking down a column of COLUMN points meets about as few runs as the sorted list cut into windows
+// does, and needs no sort.  One thread a column and remainder; nothing goes through shared memory: a point's row is read
+// PD + 1 times, from L1 after the first, neighbouring threads on neighbouring points.
+// Bound by its reductions and the latency of its loads.  Two volumes of 111x128x120 points, 20 splats an entry: 106 -> 83 us
+// (the sort kept the LSU pipe at 82 %).
+// In columns or sorted, us a call: pd 2, 21 channels, 2.4 splats an entry 354 / 352, 4.8 210 / 218, 14.7 128 / 139; pd 2, 2
+// channels, 2.4 splats 279 / 285, 14.7 114 / 126; pd 4, 9.6 splats 177 / 184, 42 splats 159 / 171; pd 5, 8 splats 201 / 197,
+// 13 splats 164 / 167, 36 splats (few vertices, which all tiles add to) 158 / 138.  Hence: up to pd 4, from 2 pd splats an
+// entry on.  Tiles of points in one dimension have no columns.
+constexpr int COLUMN = 8, COLUMNS_PD = 4;
+template <int PD>
+__device__ __forceinline__ bool in_columns(const Geom& g, int entries) {
+    return PD <= COLUMNS_PD && g.TX <= 16 && 2 * PD * entries <= Cfg<PD>::SPLATS;
+}
+template <int PD, int VD>
+__device__ __forceinline__ void splat_columns(const Geom& g, const TilePos& tpos, int base,
+                                              const float* __restrict__ input, const u16* __restrict__ rec_tile,
+                                              const float* __restrict__ recw_tile,
+                                              const u32* __restrict__ list_ref, float* __restrict__ v0) {
+    constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3, COLUMNS = TP / COLUMN, AHEAD = 4;
+    for (int i = threadIdx.x; i < (PD + 1) * COLUMNS; i += TP) {
+        const int r = i / COLUMNS, c = i % COLUMNS;
+        const int lx = c & (g.TX - 1), ly = (c >> g.tx_log2) * COLUMN;
+        const int x = tpos.tx * g.TX + lx, y = tpos.ty * g.TY + ly;
+        const int rows = x < g.W ? min(COLUMN, g.H - y) : 0;
+        if (rows <= 0) continue;
+        const u16* rp = rec_tile + r * TP + ly * g.TX + lx;
+        const float* wp = recw_tile + r * TP + ly * g.TX + lx;
+        const float* in = input + ((size_t)tpos.item * g.n + ((size_t)tpos.o * g.H + y) * g.W + x) * C;
+        const size_t step = (size_t)g.W * C;
+        float acc[VP];
+#pragma unroll
+        for (int j = 0; j < VP; j++) acc[j] = 0.f;
+        u32 cur = list_ref[base + rp[0]];
+#pragma unroll 1
+        for (int k0 = 0; k0 < rows; k0 += AHEAD) {   // AHEAD points' loads in flight
+            u32 v[AHEAD];
+            float w[AHEAD], xv[AHEAD][C];
+#pragma unroll
+            for (int k = 0; k < AHEAD; k++) {
+                const bool there = k0 + k < rows;
+                v[k] = there ? rp[(k0 + k) * g.TX] : 0u;
+                w[k] = there ? wp[(k0 + k) * g.TX] : 0.f;
+#pragma unroll
+                for (int j = 0; j < C; j++) xv[k][j] = there ? __ldg(in + (size_t)(k0 + k) * step + j) : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < AHEAD; k++) v[k] = (k0 + k < rows) ? list_ref[base + v[k]] : cur;
+#pragma unroll
+            for (int k = 0; k < AHEAD; k++) {
+                if (k0 + k < rows) {
+                    if (v[k] != cur) {
+                        flush_row<VP>(v0 + (size_t)cur * VP, acc);
+                        cur = v[k];
+                    }
+#pragma unroll
+                    for (int j = 0; j < C; j++) acc[j] = PL_FMA(w[k], xv[k][j], acc[j]);
+                    acc[C] = PL_FADD(acc[C], w[k]);
+                }
+            }
+        }
+        flush_row<VP>(v0 + (size_t)cur * VP, acc);
+    }
+}
+
 template <int PD, int VD, bool PRE>
-__global__ void __launch_bounds__(Cfg<PD>::TP)
+__global__ void __launch_bounds__(Cfg<PD>::TP, PD <= COLUMNS_PD ? 6 : 0)
 splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
                  const u16* __restrict__ rec, const float* __restrict__ rec_w, const uint2* __restrict__ srec,
                  const u32* __restrict__ list_ref, float* __restrict__ v0, int bulk_ok) {
@@ -162,6 +228,14 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     const int tid = threadIdx.x, tile = tpos.tile;
     const int2 info = tile_info[tile];
     const int base = info.x, nloc = info.y;
+    if constexpr (PD <= COLUMNS_PD) {
+        if (in_columns<PD>(g, nloc)) {
+            splat_columns<PD, VD>(g, tpos, base, input, rec + (size_t)tile * SPLATS, rec_w + (size_t)tile * SPLATS,
+                                  list_ref, v0);
+            let_next_kernel_start();
+            return;
+        }
+    }
 
     int item, pix;
     const bool valid = tile_point(g, tpos, tid, item, pix);
@@ -261,7 +335,7 @@ __device__ __forceinline__ int fixed_exponent(const Header* hdr) {   // 36 - e w
 // What a lane keeps of the running entry: four channels of its sum.
 struct FloatSum {
     float4 a;
-    __device__ __forceinline__ explicit FloatSum(const Header*) {}
+    __device__ __forceinline__ void start(const Header*) {}
     __device__ __forceinline__ void clear() { a = make_float4(0.f, 0.f, 0.f, 0.f); }
     __device__ __forceinline__ void add(float wt, float4 x) {
         const float2 w2 = make_float2(wt, wt);
@@ -282,7 +356,7 @@ struct FixedSum {
     static constexpr float M_HI = 412316860416.f, M_LO = 12582912.f;
     int hi[4], lo[4];
     float scale;
-    __device__ __forceinline__ explicit FixedSum(const Header* hdr) {
+    __device__ __forceinline__ void start(const Header* hdr) {
         scale = __int_as_float((127 + fixed_exponent(hdr)) << 23);
     }
     __device__ __forceinline__ void clear() {
@@ -337,6 +411,61 @@ struct SplatRows {
     }
 };
 
+// Walking columns of points (see splat_columns) for rows of more than one float4, up to pd = WIDE_COLUMNS_PD: a group of
+// lanes per column, as below, with the running sums of all PD + 1 remainders, so that a point's row is read once instead
+// of PD + 1 times and neither sorted nor spread to padded rows: lanes read single floats, and four neighbouring columns
+// with an odd number of channels never meet on a shared-memory bank.  Channel 0 of point (lx, ly) lies at
+// ly row_step + lx point_step; `splat_s` holds the vertex and weight of every splat.  8 x 512x512 x 21, pd 2: 99 -> 75 us.
+// (Running sums of four remainders are what the registers of five CTAs an SM hold.)
+constexpr int WIDE_COLUMNS_PD = 3;
+template <int PD, typename Sum, typename V>
+__device__ __forceinline__ void splat_wide_columns(const Geom& g, const TilePos& tpos, const Header* hdr,
+                                                   const float* in_s, int point_step, int row_step, const uint2* splat_s,
+                                                   V* __restrict__ v0, int C, int VP) {
+    constexpr int TP = Cfg<PD>::TP;
+    const int LR = VP >> 2;
+    const int lw_log2 = LR > 8 ? 4 : LR > 4 ? 3 : LR > 2 ? 2 : 1, LW = 1 << lw_log2;
+    const int points = LW > COLUMN ? LW : COLUMN;   // of a column
+    const int c = (int)threadIdx.x >> lw_log2, lx = c & (g.TX - 1), ly = (c >> g.tx_log2) * points;
+    const int x = tpos.tx * g.TX + lx, y = tpos.ty * g.TY + ly;
+    const int count = (c < TP / points && x < g.W) ? min(points, g.H - y) : 0;
+    if (count <= 0) return;
+    for (int h = (int)threadIdx.x & (LW - 1); h < LR; h += LW) {
+        const uint2* sp = splat_s + ly * g.TX + lx;
+        const float* in = in_s + ly * row_step + lx * point_step + 4 * h;
+        const int left = C - 4 * h;   // channels from here on; then the homogeneous one, then padding
+        Sum acc[PD + 1];
+        u32 cur[PD + 1];
+#pragma unroll
+        for (int r = 0; r <= PD; r++) {
+            acc[r].start(hdr);
+            acc[r].clear();
+            cur[r] = sp[r * TP].x;
+        }
+#pragma unroll 2
+        for (int i = 0; i < count; i++, in += row_step, sp += g.TX) {
+            float4 q = make_float4(left == 0 ? 1.f : 0.f, left == 1 ? 1.f : 0.f, left == 2 ? 1.f : 0.f, left == 3 ? 1.f : 0.f);
+            if (left > 0) q.x = in[0];
+            if (left > 1) q.y = in[1];
+            if (left > 2) q.z = in[2];
+            if (left > 3) q.w = in[3];
+#pragma unroll
+            for (int r = 0; r <= PD; r++) {
+                const uint2 vw = sp[r * TP];
+                if (vw.x != cur[r]) {
+                    acc[r].flush(v0 + (size_t)cur[r] * VP + 4 * h);
+                    acc[r].clear();
+                    cur[r] = vw.x;
+                }
+                acc[r].add(__uint_as_float(vw.y), q);
+            }
+        }
+        let_next_kernel_start();   // what is left of this thread's work: its last rows
+#pragma unroll
+        for (int r = 0; r <= PD; r++) acc[r].flush(v0 + (size_t)cur[r] * VP + 4 * h);
+    }
+}
+
 // Five CTAs per SM (47-48 registers, no spills; with the sort's counters the five CTAs take nearly all of an
 // SM's shared memory): 4 % faster than four at 16 items, and 2048 tiles (two items) take three waves, not four.
 template <int PD, int VD, bool PRE, typename Sum, typename V>
@@ -366,6 +495,8 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
     const int base = info.x, nloc = info.y;
+    // (up to 64 floats a row: a column of as many points as lanes fits the tile)
+    const bool columns = PD <= WIDE_COLUMNS_PD && LR <= 16 && in_columns<PD>(g, nloc);
 
     int item, pix;
     const bool valid = tile_point(g, tpos, tid, item, pix);
@@ -374,7 +505,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     // latency overlaps that of the tile's entry range above
     float w[PD + 1];
     int l[PD + 1];
-    if constexpr (!PRE) {
+    if (!PRE || columns) {
         const u16* rec_tile = rec + (size_t)tile * SPLATS;
         const float* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
@@ -382,16 +513,17 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
             l[r] = valid ? rec_tile[r * TP + tid] : 0;
             w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
         }
-        for (int i = tid; i < nloc; i += TP) cur_s[i] = 0;
     }
+    if (!PRE && !columns)
+        for (int i = tid; i < nloc; i += TP) cur_s[i] = 0;
     if ((PRE || bulk_ok) && tid == 0) mbar_init(&bar, 1);
     const int nvalid = __syncthreads_count(valid);
     const int total = nvalid * (PD + 1);
     // PRE: the tile's sorted splats arrive by one bulk copy, already in the windowed form the loop below reads
-    constexpr unsigned REC_BYTES = PRE ? (unsigned)(sizeof(uint2) * SR::SORTED) : 0u;
+    const unsigned rec_bytes = PRE && !columns ? (unsigned)(sizeof(uint2) * SR::SORTED) : 0u;
     if ((PRE || bulk_ok) && tid == 0) {
-        mbar_expect_tx(&bar, REC_BYTES + (bulk_ok ? (unsigned)nvalid * C * 4u : 0u));
-        if constexpr (PRE) bulk_load(sorted_s, srec + (size_t)tile * SR::SORTED, REC_BYTES, &bar);
+        mbar_expect_tx(&bar, rec_bytes + (bulk_ok ? (unsigned)nvalid * C * 4u : 0u));
+        if (rec_bytes) bulk_load(sorted_s, srec + (size_t)tile * SR::SORTED, rec_bytes, &bar);
     }
 
     // Staging.  Bulk form: every tile row's block (TX points x C floats, contiguous in memory) lands
@@ -427,10 +559,14 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
         }
     }
 
-    if constexpr (!PRE) SplatCommon<PD>::template sort_splats<WL>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
+    if constexpr (!PRE) {
+        if (!columns) SplatCommon<PD>::template sort_splats<WL>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
+    }
     // did this thread see the copies complete within the bounded wait
     const bool arrived = (PRE || bulk_ok) ? mbar_wait(&bar, 0) : true;
-    if (bulk_ok) {
+    if (bulk_ok && columns) {
+        // a column's points are read where they landed
+    } else if (bulk_ok) {
         // elements a lane reads before the first of them is written: the whole tile row (TX <= 16) where its size is
         // known, else four at a time (an element moves towards the region's start and the elements after it lie
         // behind its old place, so a trip never overwrites what a later one reads)
@@ -490,6 +626,17 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     wait_for_previous_kernel();
     if (call_failed(hdr)) return;   // a failure of the index stage
 
+    if constexpr (PD <= WIDE_COLUMNS_PD) {
+        if (columns) {
+#pragma unroll
+            for (int r = 0; r <= PD; r++)
+                sorted_s[r * TP + tid] = make_uint2(valid ? list_ref[base + l[r]] : 0u, __float_as_uint(w[r]));
+            __syncthreads();
+            splat_wide_columns<PD, Sum>(g, tpos, hdr, in_s + (bulk_ok ? land : 0), bulk_ok ? C : VP, g.TX * VP, sorted_s, v0, C, VP);
+            return;
+        }
+    }
+
     // (two lanes at least, so that a window starts on an even splat)
     const int lw_log2 = LR > 16 ? 5 : LR > 8 ? 4 : LR > 4 ? 3 : LR > 2 ? 2 : 1;
     const int LW = 1 << lw_log2, wl = LW * (PD + 1);   // lanes of a window, its splats
@@ -498,7 +645,8 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     if (first < end) {
         for (int h = tid & (LW - 1); h < LR; h += LW) {
             const float4* in4 = reinterpret_cast<const float4*>(in_s) + h;
-            Sum acc(hdr);
+            Sum acc;
+            acc.start(hdr);
             acc.clear();
             int cur = (int)(sorted_s[Cfg<PD>::srec_slot(first)].x >> 16);
             u32 vcur = list_ref[base + cur];   // vertex of the running entry, fetched when the run starts
