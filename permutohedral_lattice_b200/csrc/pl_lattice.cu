@@ -454,7 +454,9 @@ static int launch_splat(const Geom& g, const float* input, Header* hdr, const in
 template <int PD, int VP, int CT = 0>
 static int launch_slice(const Geom& g, float* output, const Header* hdr, const int2* tile_info, const u16* rec,
                         const float* rec_w, const u32* list_ref, const float* vsrc, int vd, Watch watch, cudaStream_t st) {
-    if constexpr (VP > 0) {
+    if constexpr (VP == 4) {
+        PL_LAUNCH_AFTER(OV_SLICE, (slice_points<PD, CT>), tile_grid(g), Cfg<PD>::TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, watch);
+    } else if constexpr (VP > 0) {
         int rows_cap = (40 * 1024) / (SliceFast<PD, VP>::RS * 4);
         if (rows_cap > Cfg<PD>::SPLATS) rows_cap = Cfg<PD>::SPLATS;
         const size_t smem = SliceFast<PD, VP>::bytes(rows_cap);
@@ -482,7 +484,8 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
 #define PL_SLICE_FOR(PD_, vd, ...)                              \
     ((vd) == 22            ? launch_slice<PD_, 24, 21>(__VA_ARGS__) \
      : (vd) == 4           ? launch_slice<PD_, 4, 3>(__VA_ARGS__)   \
-     : padded_vd(vd) == 4  ? launch_slice<PD_, 4>(__VA_ARGS__)  \
+     : (vd) == 3           ? launch_slice<PD_, 4, 2>(__VA_ARGS__)   \
+     : (vd) == 2           ? launch_slice<PD_, 4, 1>(__VA_ARGS__)   \
      : padded_vd(vd) == 8  ? launch_slice<PD_, 8>(__VA_ARGS__)  \
      : padded_vd(vd) == 12 ? launch_slice<PD_, 12>(__VA_ARGS__) \
      : padded_vd(vd) == 16 ? launch_slice<PD_, 16>(__VA_ARGS__) \
