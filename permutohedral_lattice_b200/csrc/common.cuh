@@ -109,7 +109,8 @@ __device__ __forceinline__ void report_late(const Watch& w, const Header* hdr) {
 struct Layout {   // byte offsets into the workspace
     size_t tile_info, rec, rec_w, srec, list_keys, list_ref, vid, vkeys, table, nbr, v0, v1, v64, total;
     u64 max_entries;   // capacity of entry- and vertex-indexed arrays
-    u64 table_slots;   // allocated slots (power of two)
+    u64 table_slots;   // allocated slots (power of two): of 16 bytes where a slot holds the key (Cfg::KEY_SLOTS), else of 8
+    u64 index_words;   // 32-bit words of the table's region that direct indexing may use
 };
 
 template <int KW>
@@ -120,6 +121,7 @@ struct alignas((KW % 2 == 0) ? 16 : 8) Key {
 template <int PD>
 struct Cfg {
     static constexpr int KW = (PD + 1 + 3) / 4;          // 16-bit fields: PD coordinates + item
+    static constexpr bool KEY_SLOTS = PD <= 5;           // a key and an index fit 16 bytes: see KeySlot
     static constexpr int TP = (PD <= 8) ? 256 : 128;     // points per tile = threads per CTA
     static constexpr int SPLATS = TP * (PD + 1);
     // 16-bit slots of the tile's hash: at least 2.5 per splat

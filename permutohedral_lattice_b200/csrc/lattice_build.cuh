@@ -517,6 +517,8 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 // or, where the call kept a sketch of the lattice's size, at least four times the vertices it tells of (twice
 // as many cost the probe chains of insert_entries more than the smaller table gained it).
 // ---------------------------------------------------------------------------------------------
+constexpr u64 KEY_SLOTS_WHOLE = 1ull << 21;   // 32 MB
+template <bool KEY_SLOTS>
 __global__ void __launch_bounds__(256)
 clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift) {
     after_previous_kernel();
@@ -544,6 +546,10 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
         if (clear > (1u << SKETCH_LOG2) / 64) {
             const float sampled = -(float)(1 << SKETCH_LOG2) * logf((float)clear * (1.f / (1 << SKETCH_LOG2)));
             u64 slots = (u64)(4.f * sampled * (float)(1u << sketch_shift));
+            // four a vertex spare more probes than the larger table costs while it stays in L2 beside everything else; a
+            // table of keys beyond 32 MB has two a vertex at least (us a call, four / two a vertex: 1024x1024 grey by RGB,
+            // forward + backward, 17 MB at four, 325 / 337; 16 x 512x512 x 21, 67 MB at four, 1857 / 1824)
+            if (KEY_SLOTS && slots > KEY_SLOTS_WHOLE) slots = slots / 2 > KEY_SLOTS_WHOLE ? slots / 2 : KEY_SLOTS_WHOLE;
             const u64 least = 1ull << (sketch_shift + 11);
             slots = slots < least ? least : slots;
             need = slots < need ? slots : need;
@@ -552,7 +558,7 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
     u32 lg = 10;
     while (lg < max_log2 && (1ull << lg) < need) lg++;
     const u32 filter_log2 =
-        (lg >= FILTER_MIN_LOG2 && lg < max_log2) ? min(lg + FILTER_BITS_LOG2, FILTER_MAX_LOG2) : 0u;
+        (!KEY_SLOTS && lg >= FILTER_MIN_LOG2 && lg < max_log2) ? min(lg + FILTER_BITS_LOG2, FILTER_MAX_LOG2) : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         hdr->table_log2 = lg;
         hdr->filter_log2 = filter_log2;
@@ -563,8 +569,10 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
             filter[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     const u64 cap = 1ull << lg;
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (u64)gridDim.x * blockDim.x)
-        table[i] = EMPTY_SLOT;
+    for (u64 i = grid_thread(); i < cap; i += grid_threads()) {
+        if constexpr (KEY_SLOTS) reinterpret_cast<ulonglong2*>(table)[i] = make_ulonglong2(EMPTY_SLOT, EMPTY_SLOT);
+        else table[i] = EMPTY_SLOT;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -709,6 +717,88 @@ insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>
     }
 }
 
+// Table of keys (pd up to 5): a slot of 16 bytes holds the key itself, four fields in its first word, the others above
+// the index in its second, so that a lookup is one access to a random sector and not one to the slot and one to the key
+// it names: the index kernels run at the rate of such accesses.  link_neighbours on 800x1200 x 3: 34.5 -> 30.1 us, on
+// 16 x 512x512: 69 -> 63 (a neighbour that is there costs one access and not two); insert_entries a few per cent, where
+// entries come in duplicates whose key was in L2 already.
+struct alignas(16) KeySlot { u64 first, rest; };   // rest: other fields << 32 | index (as in a slot of 8 bytes); all ones: empty
+__device__ __forceinline__ KeySlot load_slot(const KeySlot* p) {   // from L2, in one piece
+    KeySlot s;
+    asm volatile("{\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%2];\n\tmov.b128 {%0, %1}, v;\n\t}"
+                 : "=l"(s.first), "=l"(s.rest)
+                 : "l"(p)
+                 : "memory");
+    return s;
+}
+// Writes the key to an empty slot; what was there.
+__device__ __forceinline__ KeySlot claim_slot(KeySlot* p, u64 first, u64 rest) {
+    KeySlot s;
+    asm volatile("{\n\t.reg .b128 empty, mine, was;\n\tmov.b128 empty, {%3, %3};\n\tmov.b128 mine, {%4, %5};\n\t"
+                 "atom.relaxed.gpu.global.cas.b128 was, [%2], empty, mine;\n\tmov.b128 {%0, %1}, was;\n\t}"
+                 : "=l"(s.first), "=l"(s.rest)
+                 : "l"(p), "l"(EMPTY_SLOT), "l"(first), "l"(rest)
+                 : "memory");
+    return s;
+}
+template <int PD>
+__device__ __forceinline__ u32 key_rest(const Key<Cfg<PD>::KW>& k) {
+    constexpr int KW = Cfg<PD>::KW;
+    return KW > 1 ? (u32)k.w[KW - 1] : 0u;
+}
+
+// insert_entries into a table of keys.  The index in a slot is that of the creating entry, then (its round ended) of
+// the vertex.
+template <int PD>
+__global__ void __launch_bounds__(256)
+insert_keys(Header* hdr, KeySlot* __restrict__ table, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
+            u32* __restrict__ list_ref, u32* __restrict__ vid, Key<Cfg<PD>::KW>* __restrict__ vkeys, VertexInit vi) {
+    after_previous_kernel();
+    constexpr int KW = Cfg<PD>::KW;
+    __shared__ InsertRound rd;
+    if (threadIdx.x == 0) rd.count = 0;
+    if (call_failed(hdr)) return;   // (its barrier also publishes rd.count)
+    const u32 T = hdr->num_entries;
+    const u32 mask = (u32)((1ull << hdr->table_log2) - 1);
+    const u32 stride = gridDim.x * 256u;
+    for (u32 start = blockIdx.x * 256u; start < T;) {
+        for (int c = 0; c < INSERT_CHUNKS && start < T; c++, start += stride) {
+            const u32 t = start + threadIdx.x;
+            bool winner = false;
+            u32 s = 0;
+            if (t < T) {
+                const Key<KW> k = list_keys[t];
+                const u64 first = k.w[0];
+                const u32 rest = key_rest<PD>(k);
+                u32 ref = 0xFFFFFFFFu;
+                s = (u32)hash_key<KW>(k) & mask;
+                for (u64 it = 0; it <= mask; it++) {
+                    KeySlot cur = load_slot(table + s);
+                    if ((u32)cur.rest == 0xFFFFFFFFu) {
+                        cur = claim_slot(table + s, first, ((u64)rest << 32) | t);
+                        if ((u32)cur.rest == 0xFFFFFFFFu) {
+                            ref = t;
+                            winner = true;
+                            break;
+                        }
+                    }
+                    if (cur.first == first && (u32)(cur.rest >> 32) == rest) { ref = (u32)cur.rest; break; }
+                    s = (s + 1) & mask;
+                }
+                if (ref == 0xFFFFFFFFu) {
+                    atomicOr(&hdr->status, 1u << PL_INTERNAL_ERROR);
+                    ref = t;
+                }
+                list_ref[t] = ref;   // owning entry, or (VERTEX_FLAG set) the vertex itself
+            }
+            round_add_winner(rd, winner, t, s);
+        }
+        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 v) {
+            reinterpret_cast<u32*>(table)[4 * (u64)slot + 2] = VERTEX_FLAG | v;   // the index: the key stays
+        });
+    }
+}
+
 // entry -> vertex: after the insert launch list_ref[t] names the entry that owns t's key; the link launch
 // turns that into the owner's vertex index (first loop of link_neighbours / link_neighbours_direct).
 __device__ __forceinline__ void resolve_entries(const Header* hdr, u32* __restrict__ list_ref,
@@ -775,6 +865,31 @@ __device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mas
         }
     }
 }
+// The same in a table of keys.
+template <int PD, int A>
+__device__ __forceinline__ void link_axis(const KeySlot* __restrict__ table, u32 mask,
+                                          const Key<Cfg<PD>::KW>* __restrict__ vkeys, u32 M, int* __restrict__ nbr,
+                                          u64 max_entries) {
+    constexpr int KW = Cfg<PD>::KW;
+    int* __restrict__ nbr_axis = nbr + 2 * (u64)A * max_entries;
+    for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < M; v += gridDim.x * blockDim.x) {
+        Key<KW> k = vkeys[v];
+        u32 s = (u32)mix_hash(linear_hash<KW>(k) + axis_hash<PD>(A)) & mask;
+#pragma unroll
+        for (int j = 0; j < KW; j++) k.w[j] += axis_word<PD>(A, j);
+        for (u64 it = 0; it <= mask; it++) {
+            const ulonglong2 cur = __ldg(reinterpret_cast<const ulonglong2*>(table + s));
+            if ((u32)cur.y == 0xFFFFFFFFu) break;
+            if (cur.x == k.w[0] && (u32)(cur.y >> 32) == key_rest<PD>(k)) {
+                const u32 u = (u32)cur.y & ~VERTEX_FLAG;
+                nbr_axis[2 * (u64)v] = (int)u;
+                nbr_axis[2 * (u64)u + 1] = (int)v;
+                break;
+            }
+            s = (s + 1) & mask;
+        }
+    }
+}
 template <int PD, int A>
 struct LinkAxis {   // link_axis of the axis this block works on, chosen once per block
     template <typename... Args>
@@ -802,9 +917,13 @@ link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restr
         const u64 quads = (u64)M * (zero_row_bytes / 16);
         for (u64 i = grid_thread(); i < quads; i += grid_threads()) rows[i] = make_uint4(0u, 0u, 0u, 0u);
     }
-    const u32 filter_log2 = hdr->filter_log2;
-    const u32* filter = filter_log2 ? filter_words(table, max_log2, filter_log2) : nullptr;
-    LinkAxis<PD, 0>::run((int)blockIdx.y, table, mask, filter, (1u << filter_log2) - 1u, vkeys, M, nbr, max_entries);
+    if constexpr (Cfg<PD>::KEY_SLOTS) {
+        LinkAxis<PD, 0>::run((int)blockIdx.y, reinterpret_cast<const KeySlot*>(table), (u32)mask, vkeys, M, nbr, max_entries);
+    } else {
+        const u32 filter_log2 = hdr->filter_log2;
+        const u32* filter = filter_log2 ? filter_words(table, max_log2, filter_log2) : nullptr;
+        LinkAxis<PD, 0>::run((int)blockIdx.y, table, mask, filter, (1u << filter_log2) - 1u, vkeys, M, nbr, max_entries);
+    }
 }
 
 }  // namespace pl

@@ -29,6 +29,7 @@
 // Device code lives in the headers included below (one translation unit); this file holds the host
 // side: geometry and workspace layout, launches, and the extern "C" entry points.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -284,7 +285,11 @@ static int make_layout(Layout& L, const Geom& g, int pd, int vd, int64_t max_ent
     L.max_entries = E;
     u64 slots = 1024;
     while (slots < 2 * E) slots <<= 1;
+    // A table of keys (pd up to 5) has slots of 16 bytes and lies where the second buffer of value rows does: nothing
+    // reads the table once the neighbours are linked, nothing touches those rows before the first blur pass.
+    const bool key_slots = pd <= 5;
     L.table_slots = slots;
+    L.index_words = 2 * slots;
     const size_t tile_splats = (size_t)tp_of(pd) * (pd + 1);
     size_t off = align_up(HEADER_BYTES);
     L.tile_info = off; off += align_up(sizeof(int2) * (size_t)g.num_tiles);
@@ -296,12 +301,21 @@ static int make_layout(Layout& L, const Geom& g, int pd, int vd, int64_t max_ent
     L.list_ref = off;  off += align_up(sizeof(u32) * E);
     L.vid = off;       off += align_up(sizeof(u32) * E);
     L.vkeys = off;     off += align_up(sizeof(u64) * kw_of(pd) * E);
-    L.table = off;     off += align_up(sizeof(u64) * slots);
+    L.table = off;     off += key_slots ? 0 : align_up(sizeof(u64) * slots);
     L.nbr = off;       off += align_up(sizeof(int) * 2 * (size_t)(pd + 1) * E);
     const size_t row_bytes = real_bytes == 8 ? sizeof(double) * (size_t)padded_vd_f64(vd)
                                              : sizeof(float) * (size_t)padded_vd(vd);
     L.v0 = off;        off += align_up(row_bytes * E);
-    L.v1 = off;        off += align_up(row_bytes * E);
+    L.v1 = off;
+    if (key_slots) {
+        L.table = L.v1;
+        // Rows of one float4 are shorter than the slots of 16 bytes.  The scratch without allocation has a fixed size
+        // and takes what it always took: with half the slots, still one an entry, where it would be too small.
+        if (!with_sorted && off + align_up(2 * sizeof(u64) * slots) > PL_STATIC_SCRATCH_BYTES) L.table_slots = slots / 2;
+        off += align_up(std::max(row_bytes * (size_t)E, (size_t)(2 * sizeof(u64) * L.table_slots)));
+    } else {
+        off += align_up(row_bytes * E);
+    }
     L.v64 = off;       // deterministic mode sums (float calls only)
     if (real_bytes == 4 && with_fixed_point) off += align_up(sizeof(long long) * (size_t)padded_vd(vd) * E);
     L.total = off;
@@ -316,7 +330,7 @@ static int g_direct_index_enabled = 1;
 static bool make_direct(Direct& d, const Geom& g, int pd, const Layout& L) {
     memset(&d, 0, sizeof(d));
     if (!g_direct_index_enabled || g.from_positions || g.R != 0 || pd != g.n_sdims) return false;
-    return direct_bounds(d, pd, g.sdims, g.spatial_std, g.scale, g.batch, 2 * L.table_slots);
+    return direct_bounds(d, pd, g.sdims, g.spatial_std, g.scale, g.batch, L.index_words);
 }
 
 // Launch grid of the tile kernels (see this_tile).
@@ -543,7 +557,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
 
     // insert_entries overlaps clear_table only while the table can stay in L2 (64 MB of slots): behind a
     // clear_table that itself overlaps build_tiles it cost calls with large tables 4-25 % (pd 16: 30 -> 37 ms)
-    const bool small_table = L.table_slots <= (1ull << 23);
+    const bool small_table = L.index_words <= (1ull << 24);
     if (phases & PH_BUILD) {
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
         if (phases & PH_APPLY) {
@@ -585,8 +599,11 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             vinit.rows = nullptr;
             // (behind the build that also sorts the splats the overlap measured slower: 1.66 against 1.61 ms for
             // a build and two applies)
-            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
-            PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
+            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+            if constexpr (Cfg<PD>::KEY_SLOTS)
+                PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
+            else
+                PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
                                                       L.max_entries, zrows, vinit.row_bytes, watch);
         }
@@ -669,7 +686,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     int table_log2 = 0;
     while ((1ull << table_log2) < L.table_slots) table_log2++;
     const int vp = padded_vd_f64(vd);
-    const bool small_table = L.table_slots <= (1ull << 23);   // (as for float)
+    const bool small_table = L.index_words <= (1ull << 24);   // (as for float)
 
     PL_LAUNCH((build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
     // spatial-only calls index their vertices directly, as the float calls do (the key bounds hold for
@@ -696,8 +713,11 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     if (small) {
         PL_LAUNCH_AFTER(OV_CLEAR, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, watch);
     } else if (!use_direct) {
-        PL_LAUNCH_AFTER(OV_CLEAR, (clear_table), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
-        PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
+        PL_LAUNCH_AFTER(OV_CLEAR, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+        if constexpr (Cfg<PD>::KEY_SLOTS)
+            PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
+        else
+            PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
         PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   nullptr, 0u, watch);
     }

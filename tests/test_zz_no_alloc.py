@@ -132,3 +132,21 @@ def test_stats_of_the_built_in_scratch_take_any_form_of_device(device):
     for d in (device, torch.device(device) if device is not None else None):
         st = plb.lattice_stats(None, device=d)
         assert st.device_status == capi.PL_OK and st.num_entries > 0
+
+
+def test_noalloc_takes_what_it_took_with_half_the_slots():
+    """A table of keys needs more than the scratch has left for narrow rows just below its size: half the slots then, one
+    an entry, here nearly all of them vertices."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    from permutohedral_lattice_b200 import capi
+    rng = np.random.default_rng(11)
+    img = torch.from_numpy(rng.random((1, 304, 252, 3), dtype=np.float32)).cuda()
+    rc, got = _call_noalloc(img, img, [304, 252], True, 0.5, 0.01, 1.0, False)
+    assert rc == capi.PL_OK
+    st = plb.lattice_stats(None)
+    assert st.device_status == capi.PL_OK and st.num_entries > 400000 and st.table_slots == 1 << 19
+    want, ws, _ = plb.lattice_filter_raw(img, img, True, 0.5, 0.01, max_entries=0)
+    st = plb.lattice_stats(ws)
+    assert st.table_slots == 1 << 20 or st.table_slots >= 2 * st.num_vertices
+    assert float((got - want).norm() / want.norm()) <= REL_L2_TOL
