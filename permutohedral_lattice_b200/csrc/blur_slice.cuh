@@ -82,7 +82,11 @@ struct SliceFast {
     static size_t bytes(int rows_cap) { return region(rows_cap) + sizeof(int) * TP; }
     // CTAs per SM asked of the compiler: what the row, the weights and the entry numbers of a point leave room for
     static constexpr int NEED = VP + 2 * (PD + 1);
-    static constexpr int CTAS = TP != 256 ? (VP > 24 ? 6 : 8) : NEED <= 36 ? 5 : NEED <= 52 ? 4 : 3;
+    // Up to pd 3 the kernel waits for memory and not for shared memory's conflicts: a sixth CTA, 40 registers, for rows that
+    // leave it room (8 x 512x512 x 21, pd 2: 63 -> 58 us)
+    static constexpr bool SIX = PD <= 3 && NEED <= 30;
+    static constexpr int CTAS = TP != 256 ? (VP > 24 ? 6 : 8) : SIX ? 6 : NEED <= 36 ? 5 : NEED <= 52 ? 4 : 3;
+    static constexpr int ROWS_BYTES = (SIX ? 35 : 40) * 1024;   // of cached rows: so many CTAs fit the shared memory too
 };
 
 // CT: the channels where they are fixed at compile time, else 0 (VP - 4 <= C < VP, a few registers more).
