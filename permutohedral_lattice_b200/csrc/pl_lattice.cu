@@ -9,19 +9,21 @@
 //   clear_table     sizes the global hash table (on the device) from the entry count or, in larger calls, from
 //                   build_tiles' sketch of the vertices, and clears it and the filter in front of it.
 //   insert_entries  one CAS per entry into the table; the first entry of a key owns a new vertex, whose
-//                   neighbour slots the same launch initialises.
+//                   neighbour slots the same launch initialises.  Up to pd 5 insert_keys, into slots that hold the key.
 //   link_neighbours entry -> vertex index; value rows zeroed; then the +-1 neighbours of every vertex along each
 //                   of the pd+1 axes: one table lookup per vertex and axis fills both directions.
 //   splat_tiles     one CTA per tile: input block staged in shared memory (bulk async copies), splats
-//                   sorted by entry, runs summed in registers, vector reductions into the vertex rows.
+//                   sorted by entry, runs summed in registers, vector reductions into the vertex rows.  Tiles with
+//                   few entries, up to pd 4: columns of points instead of the sort.
 //   blur_axis       pd+1 launches: V'[v] = (V[n1] + 2 V[v] + V[n2]) / 4, Jacobi, ping-pong buffers.
 //   slice_tiles     one CTA per tile: the tile's vertex rows staged in shared memory, each point
-//                   interpolates, divides by the homogeneous channel and writes its output row.
+//                   interpolates, divides by the homogeneous channel and writes its output row.  Rows of one
+//                   float4 (slice_points): straight from global memory.
 //
 // Small lattices take one launch for the three index kernels and one for all blur passes (small.cuh); spatial-only calls
 // index their vertices without hashing (direct_index.cuh).
 //
-// A table slot is one 64-bit word: 32-bit hash tag | index of the entry that created the vertex, which becomes the
+// A table slot is one 64-bit word (beyond pd 5; else see KeySlot): 32-bit hash tag | index of the entry that created the vertex, which becomes the
 // vertex's own index when the creator's round ends.  Full keys are compared through the entry list, which a previous
 // launch has completely written, or through the vertex's key, so there are no locks, no waiting and no duplicate
 // vertices.  All device loops are bounded.

@@ -1,5 +1,6 @@
 // Splat stage: per-tile sort of the splats by entry and segmented reduction into the vertex rows
-// (a thread per window of narrow rows, a group of lanes per window of wider ones; float and fixed-point sums).
+// (a thread per window of narrow rows, a group of lanes per window of wider ones; float and fixed-point sums); tiles with
+// few entries by columns of points, unsorted.
 #pragma once
 #include <type_traits>
 #include "common.cuh"
