@@ -139,8 +139,8 @@ int pl_lattice_apply_f32(float* output, const float* input, int n_input_channels
  * This entry point has no counterpart in the reference.
  *  - It calls no cudaMalloc / cudaFree and no allocating library routine.
  *  - A call that needs more than PL_STATIC_SCRATCH_BYTES (what pl_workspace_bytes says, less 8 bytes and a
- *    little for each of the batch * n * (pd + 1) splats, whose sorted order only a kept lattice stores)
- *    and cannot do with the half of a table of keys (pd up to 5)
+ *    little for each of the batch * n * (pd + 1) splats, whose sorted order only a kept lattice stores, and,
+ *    for rows of up to 3 channels and pd up to 5, less what hash slots of 8 instead of 16 bytes save)
  *    returns PL_WORKSPACE_TOO_SMALL before launching anything (pl_last_cuda_error then holds the two sizes);
  *    a smaller max_entries shrinks the need.  Whether the lattice stayed within that max_entries is
  *    known only on the device: read it with pl_lattice_stats(NULL, &stats, stream) and check

@@ -109,7 +109,8 @@ __device__ __forceinline__ void report_late(const Watch& w, const Header* hdr) {
 struct Layout {   // byte offsets into the workspace
     size_t tile_info, rec, rec_w, srec, list_keys, list_ref, vid, vkeys, table, nbr, v0, v1, v64, total;
     u64 max_entries;   // capacity of entry- and vertex-indexed arrays
-    u64 table_slots;   // allocated slots (power of two): of 16 bytes where a slot holds the key (Cfg::KEY_SLOTS), else of 8
+    u64 table_slots;   // allocated slots (power of two)
+    bool key_slots;    // they hold the key and take 16 bytes (see KeySlot); else 8
     u64 index_words;   // 32-bit words of the table's region that direct indexing may use
 };
 

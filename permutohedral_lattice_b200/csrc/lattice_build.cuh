@@ -901,7 +901,7 @@ struct LinkAxis {   // link_axis of the axis this block works on, chosen once pe
     }
 };
 
-template <int PD>
+template <int PD, bool KEY_SLOTS>
 __global__ void __launch_bounds__(256)
 link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restrict__ list_ref,
                 const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys, int* __restrict__ nbr,
@@ -917,7 +917,7 @@ link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restr
         const u64 quads = (u64)M * (zero_row_bytes / 16);
         for (u64 i = grid_thread(); i < quads; i += grid_threads()) rows[i] = make_uint4(0u, 0u, 0u, 0u);
     }
-    if constexpr (Cfg<PD>::KEY_SLOTS) {
+    if constexpr (KEY_SLOTS) {
         LinkAxis<PD, 0>::run((int)blockIdx.y, reinterpret_cast<const KeySlot*>(table), (u32)mask, vkeys, M, nbr, max_entries);
     } else {
         const u32 filter_log2 = hdr->filter_log2;

@@ -287,10 +287,8 @@ static int make_layout(Layout& L, const Geom& g, int pd, int vd, int64_t max_ent
     L.max_entries = E;
     u64 slots = 1024;
     while (slots < 2 * E) slots <<= 1;
-    // A table of keys (pd up to 5) has slots of 16 bytes and lies where the second buffer of value rows does: nothing
-    // reads the table once the neighbours are linked, nothing touches those rows before the first blur pass.
-    const bool key_slots = pd <= 5;
     L.table_slots = slots;
+    L.key_slots = pd <= 5;
     L.index_words = 2 * slots;
     const size_t tile_splats = (size_t)tp_of(pd) * (pd + 1);
     size_t off = align_up(HEADER_BYTES);
@@ -303,18 +301,21 @@ static int make_layout(Layout& L, const Geom& g, int pd, int vd, int64_t max_ent
     L.list_ref = off;  off += align_up(sizeof(u32) * E);
     L.vid = off;       off += align_up(sizeof(u32) * E);
     L.vkeys = off;     off += align_up(sizeof(u64) * kw_of(pd) * E);
-    L.table = off;     off += key_slots ? 0 : align_up(sizeof(u64) * slots);
+    L.table = off;     off += L.key_slots ? 0 : align_up(sizeof(u64) * slots);
     L.nbr = off;       off += align_up(sizeof(int) * 2 * (size_t)(pd + 1) * E);
     const size_t row_bytes = real_bytes == 8 ? sizeof(double) * (size_t)padded_vd_f64(vd)
                                              : sizeof(float) * (size_t)padded_vd(vd);
     L.v0 = off;        off += align_up(row_bytes * E);
     L.v1 = off;
-    if (key_slots) {
+    if (L.key_slots) {
+        // The table lies where the second buffer of value rows does: nothing reads the table once the neighbours are
+        // linked, nothing touches those rows before the first blur pass.  Rows of one float4 are shorter than the slots
+        // of 16 bytes.  The scratch without allocation has a fixed size and takes what it always took: with slots of 8
+        // bytes where it would be too small, never with fewer than two an entry (a lookup that finds nothing walks 2.5
+        // slots of a table half full, 35 at a load of 0.88 and thousands close to 1).
         L.table = L.v1;
-        // Rows of one float4 are shorter than the slots of 16 bytes.  The scratch without allocation has a fixed size
-        // and takes what it always took: with half the slots, still one an entry, where it would be too small.
-        if (!with_sorted && off + align_up(2 * sizeof(u64) * slots) > PL_STATIC_SCRATCH_BYTES) L.table_slots = slots / 2;
-        off += align_up(std::max(row_bytes * (size_t)E, (size_t)(2 * sizeof(u64) * L.table_slots)));
+        if (!with_sorted && off + align_up(2 * sizeof(u64) * slots) > PL_STATIC_SCRATCH_BYTES) L.key_slots = false;
+        off += align_up(std::max(row_bytes * (size_t)E, (size_t)((L.key_slots ? 2 : 1) * sizeof(u64) * slots)));
     } else {
         off += align_up(row_bytes * E);
     }
@@ -601,13 +602,23 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             vinit.rows = nullptr;
             // (behind the build that also sorts the splats the overlap measured slower: 1.66 against 1.61 ms for
             // a build and two applies)
-            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
-            if constexpr (Cfg<PD>::KEY_SLOTS)
-                PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
-            else
-                PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
-            PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
-                                                      L.max_entries, zrows, vinit.row_bytes, watch);
+            auto hash_index = [&](auto keys_in_slots) -> int {
+                constexpr bool KEYS = decltype(keys_in_slots)::value;
+                PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+                if constexpr (KEYS)
+                    PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
+                else
+                    PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
+                PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD, KEYS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
+                                                          L.max_entries, zrows, vinit.row_bytes, watch);
+                return PL_OK;
+            };
+            if constexpr (Cfg<PD>::KEY_SLOTS) {
+                if (L.key_slots) PL_TRY(hash_index(std::true_type{}));
+                else PL_TRY(hash_index(std::false_type{}));
+            } else {
+                PL_TRY(hash_index(std::false_type{}));
+            }
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[2], st));
     } else {
@@ -720,7 +731,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
         else
             PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
-        PL_LAUNCH((link_neighbours<PD>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
+        PL_LAUNCH((link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   nullptr, 0u, watch);
     }
     PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
