@@ -187,6 +187,20 @@ __device__ __forceinline__ bool key_equal(const Key<KW>& a, const Key<KW>& b) {
     return eq;
 }
 
+// Words that CTAs of one launch read, claim and write while others do: every such access is relaxed at GPU scope and of
+// the whole word, since a narrower one beside a compare-and-swap of all of it would be a data race.
+__device__ __forceinline__ u64 load_relaxed(const u64* p) {
+    u64 v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_relaxed(u64* p, u64 v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void store_relaxed(u32* p, u32 v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 // Key read straight from L2 (no L1): for data that another CTA of the SAME launch may have written.
 template <int KW>
 __device__ __forceinline__ Key<KW> load_key_l2(const Key<KW>* p) {

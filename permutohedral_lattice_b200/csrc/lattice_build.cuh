@@ -619,7 +619,7 @@ __device__ __forceinline__ void round_add_winner(InsertRound& rd, bool winner, u
 // Ends a round: numbers its winners (consecutive vertex indices), writes vid and the vertex-ordered keys,
 // initialises the new vertices, and re-labels the winners' table slots with the vertex index, so that a
 // lookup ends at the slot (tag, vertex) and the vertex's key instead of walking entry -> owner -> vertex.
-// `relabel` writes the slot (hash table: 64-bit slots; direct index: 32-bit slots).  Called by all threads.
+// `relabel` writes the slot, whole, that entry t claimed for vertex v.  Called by all threads.
 template <int KW, typename Relabel>
 __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const Key<KW>* __restrict__ list_keys,
                                              u32* __restrict__ vid, Key<KW>* __restrict__ vkeys,
@@ -634,7 +634,7 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
         vkeys[v] = list_keys[t];
     }
     if (tot) __threadfence();   // a key is visible before its slot says "vertex v"
-    for (u32 i = threadIdx.x; i < tot; i += 256) relabel(rd.slot[i], base + i);
+    for (u32 i = threadIdx.x; i < tot; i += 256) relabel(rd.slot[i], rd.t[i], base + i);
     if (tot) {
         int2* nb = reinterpret_cast<int2*>(vi.nbr);
         for (int a = 0; a <= vi.pd; a++)
@@ -681,7 +681,7 @@ insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>
                 for (u64 it = 0; it <= mask; it++) {
                     // slots and vertex keys change during this launch: read them from L2, never from an
                     // L1 line that may predate another CTA's write
-                    u64 cur = __ldcg(&table[s]);
+                    u64 cur = load_relaxed(&table[s]);
                     if (cur == EMPTY_SLOT) {
                         cur = atomicCAS(&table[s], EMPTY_SLOT, mine);
                         if (cur == EMPTY_SLOT) {
@@ -711,8 +711,8 @@ insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>
             }
             round_add_winner(rd, winner, t, (u32)my_slot);
         }
-        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 v) {
-            reinterpret_cast<u32*>(table)[2 * (u64)slot] = VERTEX_FLAG | v;   // the low word: the tag stays
+        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 t, u32 v) {
+            store_relaxed(table + slot, (hash_key<KW>(list_keys[t]) & 0xFFFFFFFF00000000ull) | VERTEX_FLAG | v);
         });
     }
 }
@@ -730,6 +730,10 @@ __device__ __forceinline__ KeySlot load_slot(const KeySlot* p) {   // from L2, i
                  : "l"(p)
                  : "memory");
     return s;
+}
+__device__ __forceinline__ void store_slot(KeySlot* p, u64 first, u64 rest) {
+    asm volatile("{\n\t.reg .b128 v;\n\tmov.b128 v, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "l"(first), "l"(rest)
+                 : "memory");
 }
 // Writes the key to an empty slot; what was there.
 __device__ __forceinline__ KeySlot claim_slot(KeySlot* p, u64 first, u64 rest) {
@@ -750,7 +754,7 @@ __device__ __forceinline__ u32 key_rest(const Key<Cfg<PD>::KW>& k) {
 // insert_entries into a table of keys.  The index in a slot is that of the creating entry, then (its round ended) of
 // the vertex.
 template <int PD>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 8)   // as many as it is launched with
 insert_keys(Header* hdr, KeySlot* __restrict__ table, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
             u32* __restrict__ list_ref, u32* __restrict__ vid, Key<Cfg<PD>::KW>* __restrict__ vkeys, VertexInit vi) {
     after_previous_kernel();
@@ -793,8 +797,9 @@ insert_keys(Header* hdr, KeySlot* __restrict__ table, const Key<Cfg<PD>::KW>* __
             }
             round_add_winner(rd, winner, t, s);
         }
-        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 v) {
-            reinterpret_cast<u32*>(table)[4 * (u64)slot + 2] = VERTEX_FLAG | v;   // the index: the key stays
+        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 t, u32 v) {
+            const Key<KW> k = list_keys[t];
+            store_slot(table + slot, k.w[0], ((u64)key_rest<PD>(k) << 32) | VERTEX_FLAG | v);
         });
     }
 }
