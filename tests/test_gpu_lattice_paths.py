@@ -157,17 +157,30 @@ def test_small_lattices_give_the_bits_of_wide_ones(pd, n, gpu, oracle):
     gpu.assert_outputs_close(got, oracle.filter(val[0], pos[0], structure=False).out, "pd %d" % pd)
 
 
-def test_filter_in_front_of_a_large_table(gpu, oracle):
-    """2.9 M vertices in a table of 2^23 slots, half of what the workspace has room for: the lookups pass the filter."""
+def _large_table(gpu, oracle, width, guide):
+    """Word 8 of the header: the filter's bits, as a logarithm (0: none)."""
+    import torch
     rng = np.random.default_rng(73)
-    ref = np.repeat(rng.random((1, 1024, 360, 3), dtype=np.float32), 2, 2)
-    inp = rng.random((1, 1024, 720, 1), dtype=np.float32)
-    want, items = oracle.lattice_filter(inp, ref, True, 3.0, 0.05, 1.0, False, structure=True)
-    out, ws, call, _, rt = gpu.run_op(inp, ref, True, 3.0, 0.05, 1.0, False, max_entries=0)
+    ref = np.repeat(rng.random((1, 1024, width // 2, guide), dtype=np.float32), 2, 2)
+    inp = rng.random((1, 1024, width, 1), dtype=np.float32)
+    theta = 0.05 if guide == 3 else 0.1
+    want, items = oracle.lattice_filter(inp, ref, True, 3.0, theta, 1.0, False, structure=True)
+    out, ws, call, _, rt = gpu.run_op(inp, ref, True, 3.0, theta, 1.0, False, max_entries=0)
     st, (vk, vi, pv, pw) = gpu.export_op(ws, call, rt)
     assert st.table_slots == 1 << 23
     gpu.assert_structure_equal(vk, vi, pv, pw, items, "large table")
     gpu.assert_outputs_close(out.cpu().numpy(), want, "large table")
+    return int(ws[:64].view(torch.int32)[8])
+
+
+def test_filter_in_front_of_a_large_table(gpu, oracle):
+    """pd 6: 2.8 M vertices in a table of 2^23 slots, half of what the workspace has room for: the lookups pass the filter."""
+    assert _large_table(gpu, oracle, 600, 4) == 26
+
+
+def test_large_table_of_keys(gpu, oracle):
+    """pd 5: 2.9 M vertices in a table of 2^23 slots that hold the key, which has no filter."""
+    assert _large_table(gpu, oracle, 720, 3) == 0
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
