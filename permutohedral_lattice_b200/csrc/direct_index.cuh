@@ -78,8 +78,8 @@ insert_direct(Header* hdr, Direct d, u32* __restrict__ table, const Key<Cfg<PD>:
             }
             round_add_winner(rd, winner, t, (u32)s);
         }
-        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi,
-                         [&](u32 slot, u32, u32 v) { store_relaxed(table + slot, VERTEX_FLAG | v); });
+        finish_round<false, KW>(hdr, rd, list_keys, vid, vkeys, vi,
+                                [&](u32 slot, const Key<KW>&, u32 v) { store_relaxed(table + slot, VERTEX_FLAG | v); });
     }
 }
 

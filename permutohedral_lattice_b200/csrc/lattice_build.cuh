@@ -619,8 +619,9 @@ __device__ __forceinline__ void round_add_winner(InsertRound& rd, bool winner, u
 // Ends a round: numbers its winners (consecutive vertex indices), writes vid and the vertex-ordered keys,
 // initialises the new vertices, and re-labels the winners' table slots with the vertex index, so that a
 // lookup ends at the slot (tag, vertex) and the vertex's key instead of walking entry -> owner -> vertex.
-// `relabel` writes the slot, whole, that entry t claimed for vertex v.  Called by all threads.
-template <int KW, typename Relabel>
+// `relabel` writes the slot, whole, that a key claimed for vertex v: BEHIND_KEYS with the upper half of the key's hash, when
+// the keys of the round are visible, which lookups of this launch compare (tagged slots); else with the key.  Called by all threads.
+template <bool BEHIND_KEYS, int KW, typename Relabel>
 __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const Key<KW>* __restrict__ list_keys,
                                              u32* __restrict__ vid, Key<KW>* __restrict__ vkeys,
                                              const VertexInit& vi, Relabel relabel) {
@@ -630,11 +631,16 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
     const u32 base = rd.base, tot = rd.count;
     for (u32 i = threadIdx.x; i < tot; i += 256) {
         const u32 t = rd.t[i], v = base + i;
+        const Key<KW> k = list_keys[t];
         vid[t] = v;
-        vkeys[v] = list_keys[t];
+        vkeys[v] = k;
+        if constexpr (BEHIND_KEYS) rd.t[i] = (u32)(hash_key<KW>(k) >> 32);   // (read again by this thread alone)
+        else relabel(rd.slot[i], k, v);
     }
-    if (tot) __threadfence();   // a key is visible before its slot says "vertex v"
-    for (u32 i = threadIdx.x; i < tot; i += 256) relabel(rd.slot[i], rd.t[i], base + i);
+    if constexpr (BEHIND_KEYS) {
+        if (tot) __threadfence();   // a key is visible before its slot says "vertex v"
+        for (u32 i = threadIdx.x; i < tot; i += 256) relabel(rd.slot[i], rd.t[i], base + i);
+    }
     if (tot) {
         int2* nb = reinterpret_cast<int2*>(vi.nbr);
         for (int a = 0; a <= vi.pd; a++)
@@ -711,8 +717,8 @@ insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>
             }
             round_add_winner(rd, winner, t, (u32)my_slot);
         }
-        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 t, u32 v) {
-            store_relaxed(table + slot, (hash_key<KW>(list_keys[t]) & 0xFFFFFFFF00000000ull) | VERTEX_FLAG | v);
+        finish_round<true, KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 tag, u32 v) {
+            store_relaxed(table + slot, ((u64)tag << 32) | VERTEX_FLAG | v);
         });
     }
 }
@@ -797,8 +803,7 @@ insert_keys(Header* hdr, KeySlot* __restrict__ table, const Key<Cfg<PD>::KW>* __
             }
             round_add_winner(rd, winner, t, s);
         }
-        finish_round<KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, u32 t, u32 v) {
-            const Key<KW> k = list_keys[t];
+        finish_round<false, KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, const Key<KW>& k, u32 v) {
             store_slot(table + slot, k.w[0], ((u64)key_rest<PD>(k) << 32) | VERTEX_FLAG | v);
         });
     }
