@@ -418,7 +418,24 @@ struct SplatRows {
 // with an odd number of channels never meet on a shared-memory bank.  Channel 0 of point (lx, ly) lies at
 // ly row_step + lx point_step; `splat_s` holds the vertex and weight of every splat.  8 x 512x512 x 21, pd 2: 99 -> 75 us.
 // (Running sums of four remainders are what the registers of five CTAs an SM hold.)
-constexpr int WIDE_COLUMNS_PD = 3;
+// Columns meet more runs than the sorted list's windows, each flushed once.  For a float sum that is one reduction of 16
+// bytes a lane, for a fixed-point sum four of 8 bytes.  Fixed-point sums in columns or sorted, us a splat of 8 x 512x512, pd 2,
+// by channels, with 5 and with 15 splats an entry: 1-3 channels 99 / 122 and 84 / 112; 4 channels 139 / 146 and 101 / 123;
+// 6 channels 168 / 153 and 116 / 128; with 8 splats an entry 10 channels 1.03, 21 channels 1.29 times the sort's time.  pd 3:
+// 0.9 to 2.3 times its time, 21 channels 1.5 to 4.  In a kept lattice, whose splats are sorted already: 1-3 channels 87 / 101 from 8
+// splats an entry on, 4-6 channels 1.0 to 1.1 times, beyond pd 2 never faster.  Hence: pd 2 only, and there rows of one float4, or of two
+// from 4 pd splats an entry on and if the call would have to sort.
+constexpr int WIDE_COLUMNS_PD = 3, FIXED_COLUMNS_PD = 2;
+template <int PD, bool PRE, typename Sum>
+struct WideColumns {
+    static constexpr bool FIXED = !std::is_same<Sum, FloatSum>::value;
+    static constexpr bool EVER = PD <= (FIXED ? FIXED_COLUMNS_PD : WIDE_COLUMNS_PD);
+    __device__ static __forceinline__ bool take(const Geom& g, int entries, int LR) {
+        if (!EVER) return false;
+        if (FIXED) return LR <= (PRE ? 1 : 2) && in_columns<PD>(g, LR * entries);
+        return LR <= 16 && in_columns<PD>(g, entries);   // (up to 64 floats a row: a column of as many points as lanes fits the tile)
+    }
+};
 template <int PD, typename Sum, typename V>
 __device__ __forceinline__ void splat_wide_columns(const Geom& g, const TilePos& tpos, const Header* hdr,
                                                    const float* in_s, int point_step, int row_step, const uint2* splat_s,
@@ -496,8 +513,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
     const int base = info.x, nloc = info.y;
-    // (up to 64 floats a row: a column of as many points as lanes fits the tile)
-    const bool columns = PD <= WIDE_COLUMNS_PD && LR <= 16 && in_columns<PD>(g, nloc);
+    const bool columns = WideColumns<PD, PRE, Sum>::take(g, nloc, LR);
 
     int item, pix;
     const bool valid = tile_point(g, tpos, tid, item, pix);
@@ -627,7 +643,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     wait_for_previous_kernel();
     if (call_failed(hdr)) return;   // a failure of the index stage
 
-    if constexpr (PD <= WIDE_COLUMNS_PD) {
+    if constexpr (WideColumns<PD, PRE, Sum>::EVER) {
         if (columns) {
 #pragma unroll
             for (int r = 0; r <= PD; r++)
