@@ -31,6 +31,7 @@ struct Geom {
     float spatial_std, feature_std;
     float spatial_rcp, feature_rcp;   // correctly rounded reciprocals of the two (host-computed)
     int rcp_div;            // 1: divide through the reciprocals (exact for these operands), 0: IEEE divide
+    int calm_entries;       // entries of a tile up to which its points hardly change entry in disorder (see ColumnsSample)
     int from_positions;     // 1: features are read from a positions array
     float scale[MAX_PD];    // host-computed scale factors (double arithmetic rounded to float)
     // T = double calls: the same three in double
@@ -49,7 +50,8 @@ struct Header {   // first 256 bytes of the workspace
     u32 sorted;        // 1: the lattice was built for reuse and holds every tile's splats sorted by entry
     u32 filter_log2;   // bits of the vertex filter behind the table, as a logarithm; 0: none (see FILTER_BITS_LOG2)
     u32 reported;      // status bits that the call's watch has told the host of (see Watch)
-    u32 pad[54];
+    u32 calm_entries;  // of the Geom that the lattice was built with
+    u32 pad[53];
 };
 
 // Sketch of the lattice's size, behind the header (zeroed with it): a bitmap in which build_tiles sets one bit

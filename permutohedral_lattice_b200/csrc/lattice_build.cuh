@@ -230,6 +230,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     if (tile == 0 && tid == 0) {
         hdr->capacity = max_entries;
         hdr->sorted = SORTED ? 1u : 0u;
+        hdr->calm_entries = (u32)g.calm_entries;
     }
 
     int item, pix, po, py, px;

@@ -270,6 +270,10 @@ static int make_geom(Geom& g, int batch, int n, int pd, int n_sdims, const int* 
     g.num_tiles = (int)total;
     g.tx_log2 = 0;
     while ((1 << g.tx_log2) < g.TX) g.tx_log2++;
+    // Under a guide that is flat, a tile of 16 x 16 points has about (pd + 1) (1 + 0.7 * 16 / spatial_std)^2 entries (0.6 to
+    // 0.8 for 0.7 with pd 2 to 4, spatial_std 1.5 to 25, from the oracle's lattices): half as many again.
+    const double std_abs = std::fabs((double)spatial_std), across = 1.0 + (std_abs > 1e-3 ? 11.2 / std_abs : 1e4);
+    g.calm_entries = (int)std::min(1.5 * (pd + 1) * across * across, 65536.0);
     g.grid3 = (g.tiles_y <= 65535 && (long long)batch * g.outer <= 65535) ? 1 : 0;
     scale_factors(pd, g.scale);
     return PL_OK;

@@ -152,6 +152,37 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
 // 13 splats 164 / 167, 36 splats (few vertices, which all tiles add to) 158 / 138.  Hence: up to pd 4, from 2 pd splats an
 // entry on.  Tiles of points in one dimension have no columns.
 constexpr int COLUMN = 8, COLUMNS_PD = 4;
+// Few entries are not enough where a noisy guide sends neighbouring points to one and another of them: a column then meets
+// a run nearly every point, and all tiles add to few vertices.  So tiles that have more entries
+// than one under a flat guide would (Geom::calm_entries) are sampled for changes of entry from one row to the next.  A smooth guide, or none, gives 3 to 7 changes an entry, whatever its scale, noise 9 to 24.
+// Columns or sorted, us a splat: 4 x 512x512 guided by one channel, 2 channels, 12 changes 27 / 35, 15 changes 41 / 48, 18
+// changes 73 / 72, 23 changes 74 / 51; guided by two channels, 7 changes 31 / 39, 9 and 13 changes 51 / 35 and 42 / 39; two
+// noisy volumes of 96x128x128, 5 changes 84 / 96, 13 changes 275 / 190.  Rows of 21 channels: 12 changes 53 / 61, 15 changes
+// 64 / 62, 18 changes 94 / 62, 23 changes 109 / 61, and volumes with 4 changes but fewer than 12 entries a tile 148 / 119.
+// With pd 2 there is no guide.  Every warp looks at the same 64 pairs of points, so that all agree without a barrier;
+// it costs those tiles 4 to 7 %.  (All tiles sampled cost the splat of smooth volumes 7 %; all points of every second
+// row, counted over the CTA, 4 to 20 %; counted by build_tiles, that 3 to 6 %.)
+template <int PD>
+struct ColumnsSample {
+    static constexpr bool TAKEN = PD == 3 || PD == 4;
+    static constexpr int NARROW = PD == 4 ? 8 : 16, WIDE = 12;   // changes an entry, at most
+    __device__ static __forceinline__ bool smooth(const Geom& g, const TilePos& tpos, const Header* hdr,
+                                                  const u16* __restrict__ rec, int entries, int most) {   // TX <= 16
+        if (!TAKEN || entries <= (int)hdr->calm_entries) return true;
+        const u16* rec_tile = rec + (size_t)tpos.tile * Cfg<PD>::SPLATS + (threadIdx.x & 31);
+        u32 e[4];   // of 32 points each, two rows of 16 or more shorter ones, in four remainders
+#pragma unroll
+        for (int k = 0; k < 4; k++) e[k] = rec_tile[(k % (PD + 1)) * Cfg<PD>::TP + 64 * k];
+        int changes = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int row = (64 * k + ((int)threadIdx.x & 31)) >> g.tx_log2;
+            const u32 above = __shfl_up_sync(0xFFFFFFFFu, e[k], g.TX);
+            changes += __popc(__ballot_sync(0xFFFFFFFFu, (row & 1) && tpos.ty * g.TY + row < g.H && e[k] != above));
+        }
+        return 4 * (PD + 1) * changes <= most * entries;
+    }
+};
 template <int PD>
 __device__ __forceinline__ bool in_columns(const Geom& g, int entries) {
     return PD <= COLUMNS_PD && g.TX <= 16 && 2 * PD * entries <= Cfg<PD>::SPLATS;
@@ -229,8 +260,9 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     const int tid = threadIdx.x, tile = tpos.tile;
     const int2 info = tile_info[tile];
     const int base = info.x, nloc = info.y;
+    using CS = ColumnsSample<PD>;
     if constexpr (PD <= COLUMNS_PD) {
-        if (in_columns<PD>(g, nloc)) {
+        if (in_columns<PD>(g, nloc) && CS::smooth(g, tpos, hdr, rec, nloc, CS::NARROW)) {
             splat_columns<PD, VD>(g, tpos, base, input, rec + (size_t)tile * SPLATS, rec_w + (size_t)tile * SPLATS,
                                   list_ref, v0);
             let_next_kernel_start();
@@ -433,6 +465,7 @@ struct WideColumns {
     __device__ static __forceinline__ bool take(const Geom& g, int entries, int LR) {
         if (!EVER) return false;
         if (FIXED) return LR <= (PRE ? 1 : 2) && in_columns<PD>(g, LR * entries);
+        if (PD == 3 && entries < 12) return false;
         return LR <= 16 && in_columns<PD>(g, entries);   // (up to 64 floats a row: a column of as many points as lanes fits the tile)
     }
 };
@@ -513,7 +546,15 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
     const int base = info.x, nloc = info.y;
-    const bool columns = WideColumns<PD, PRE, Sum>::take(g, nloc, LR);
+    using CS = ColumnsSample<PD>;
+    constexpr bool SAMPLED = CS::TAKEN && WideColumns<PD, PRE, Sum>::EVER;
+    bool columns = WideColumns<PD, PRE, Sum>::take(g, nloc, LR);   // (so far; then by the sample)
+    auto look_at_sample = [&]() {
+        if constexpr (SAMPLED) {
+            if (columns) columns = CS::smooth(g, tpos, hdr, rec, nloc, CS::WIDE);
+        }
+    };
+    if constexpr (PRE) look_at_sample();   // which decides what is loaded
 
     int item, pix;
     const bool valid = tile_point(g, tpos, tid, item, pix);
@@ -531,7 +572,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
             w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
         }
     }
-    if (!PRE && !columns)
+    if (!PRE)
         for (int i = tid; i < nloc; i += TP) cur_s[i] = 0;
     if ((PRE || bulk_ok) && tid == 0) mbar_init(&bar, 1);
     const int nvalid = __syncthreads_count(valid);
@@ -577,6 +618,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
     }
 
     if constexpr (!PRE) {
+        look_at_sample();   // (from L1 by now, and behind the staging, whose copies it does not hold up)
         if (!columns) SplatCommon<PD>::template sort_splats<WL>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
     }
     // did this thread see the copies complete within the bounded wait

@@ -16,7 +16,7 @@ def gpu():
     return gpu_helpers
 
 
-def _check(gpu, oracle, shape, channels, r, theta, seed):
+def _check(gpu, oracle, shape, channels, r, theta, seed, noise=0.0):
     import torch
     import permutohedral_lattice_b200 as plb
     from conftest import bits
@@ -26,6 +26,7 @@ def _check(gpu, oracle, shape, channels, r, theta, seed):
     if r:
         ref = np.zeros((2,) + shape + (r,), np.float32)
         ref[..., :] = (np.arange(shape[-1]) // 9 % 3 * np.float32(0.4))[..., None]
+        ref += np.float32(noise) * rng.standard_normal(ref.shape).astype(np.float32)
     wide = rng.standard_normal((2,) + shape + (max(channels),)).astype(np.float32)
     rt = None if ref is None else torch.from_numpy(ref).cuda()
     args = (bool(r), theta, 0.3, theta)
@@ -56,3 +57,11 @@ def test_images_without_guide(shape, theta, gpu, oracle):
 @pytest.mark.parametrize("shape,r", [((33, 45), 1), ((70, 1), 1), ((3, 9, 20), 0), ((3, 17, 33), 1), ((2, 40, 5), 1)])
 def test_guides_and_volumes(shape, r, theta, gpu, oracle):
     _check(gpu, oracle, shape, [1, 2, 3, 4, 7, 12, 21, 64], r, theta, 6)
+
+
+@pytest.mark.parametrize("noise", [0.1, 0.4])
+@pytest.mark.parametrize("shape,r", [((33, 45), 1), ((40, 3), 1), ((3, 17, 33), 1), ((20, 37), 2)])
+def test_noisy_guides(shape, r, noise, gpu, oracle):
+    """Few entries (theta 40), between which the noise sends neighbouring points: both sides of the rule on changes of entry
+    from row to row."""
+    _check(gpu, oracle, shape, [1, 2, 3, 5, 21, 64], r, 40.0, 7, noise)
