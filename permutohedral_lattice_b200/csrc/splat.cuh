@@ -147,11 +147,32 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
 // PD + 1 times, from L1 after the first, neighbouring threads on neighbouring points.
 // Bound by its reductions and the latency of its loads.  Two volumes of 111x128x120 points, 20 splats an entry: 106 -> 83 us
 // (the sort kept the LSU pipe at 82 %).
-// In columns or sorted, us a call: pd 2, 21 channels, 2.4 splats an entry 354 / 352, 4.8 210 / 218, 14.7 128 / 139; pd 2, 2
-// channels, 2.4 splats 279 / 285, 14.7 114 / 126; pd 4, 9.6 splats 177 / 184, 42 splats 159 / 171; pd 5, 8 splats 201 / 197,
-// 13 splats 164 / 167, 36 splats (few vertices, which all tiles add to) 158 / 138.  Hence: up to pd 4, from 2 pd splats an
-// entry on.  Tiles of points in one dimension have no columns.
-constexpr int COLUMN = 8, COLUMNS_PD = 4;
+// Where (us a splat, columns / sorted): rows of more than one float4 from 2 pd splats an entry on (8 x 512x512, pd 2, 21 channels,
+// 4.8 splats 95 / 110, 14.7 splats 76 / 98); narrow ones as NarrowColumns says.  pd 5, us a call: 8 splats an entry 201 / 197, 36
+// splats 158 / 138: up to pd 4.  Tiles of points in one dimension, which are all there are with pd 1, have no columns.
+constexpr int COLUMN = 8;
+template <int PD>
+__device__ __forceinline__ bool in_columns(const Geom& g, int entries, int least) {   // least: splats an entry
+    return g.TX <= 16 && least * entries <= Cfg<PD>::SPLATS;
+}
+// Rows of one float4, VD - 1 channels.  Sorted tiles want the 32 registers of eight CTAs an SM (pd 2 and 3; also pd 4 in a kept
+// lattice), columns of four points ahead want 40: with those, and 24 to 56 bytes spilled, sorted tiles took 10 to 17 % longer (pd 2, 1
+// channel, 3.5 splats an entry 41 -> 48 us; 36 -> 42 in a kept lattice).  Two points ahead fit 32 registers (up to 8 bytes
+// spilled).  pd 4 sorts with 40 registers anyway.  With two channels, four points ahead gain more in columns than they cost
+// sorted tiles (pd 2, 14.7 splats an entry 37 us, two ahead 41, sorted 45; 3.5 splats, sorted with six CTAs 49, with eight 43;
+// pd 3, 12.6 splats 43, two ahead 45, sorted 50; kept lattices only at pd 2).
+// From how many splats an entry on, us a splat, columns / sorted: pd 2, 1 channel, 8 splats 47 / 39, 14.7 splats 43 / 43, 38 splats 39
+// / 49; 2 channels, 8 splats 42 / 43; 3 channels, 14.7 splats 44 / 47.  pd 3, 1 and 3 channels, 6.6 splats 1.06 to 1.12 of the
+// sort's time, 12.6 splats 0.92 to 0.96; 2 channels, 6.6 splats 1.00, 8.9 splats 0.93.  pd 4, 9.8 splats 0.88 to 1.04, 20 splats 0.82 to
+// 0.96.  Kept lattices, sorted already: pd 2 and 3 with 2 channels from 8 and 10 splats on, with 1 and 3 channels 1.03 to 1.10 at
+// 15 splats, 0.91 to 1.09 beyond 26; pd 4 never faster.
+template <int PD, int VD, bool PRE>
+struct NarrowColumns {
+    static constexpr bool EVER = PD >= 2 && PD <= (PRE ? 3 : 4);
+    static constexpr int AHEAD = PD == 4 || (VD == 3 && (PD == 2 || !PRE)) ? 4 : 2;
+    static constexpr int CTAS = !EVER ? 0 : AHEAD == 4 ? 6 : 8;
+    static constexpr int LEAST = AHEAD == 4 ? 8 : !PRE ? (PD == 2 ? 12 : 10) : VD == 3 ? 10 : 24;
+};
 // Few entries are not enough where a noisy guide sends neighbouring points to one and another of them: a column then meets
 // a run nearly every point, and all tiles add to few vertices.  So tiles that have more entries
 // than one under a flat guide would (Geom::calm_entries) are sampled for changes of entry from one row to the next.  A smooth guide, or none, gives 3 to 7 changes an entry, whatever its scale, noise 9 to 24.
@@ -183,16 +204,12 @@ struct ColumnsSample {
         return 4 * (PD + 1) * changes <= most * entries;
     }
 };
-template <int PD>
-__device__ __forceinline__ bool in_columns(const Geom& g, int entries) {
-    return PD <= COLUMNS_PD && g.TX <= 16 && 2 * PD * entries <= Cfg<PD>::SPLATS;
-}
-template <int PD, int VD>
+template <int PD, int VD, int AHEAD>
 __device__ __forceinline__ void splat_columns(const Geom& g, const TilePos& tpos, int base,
                                               const float* __restrict__ input, const u16* __restrict__ rec_tile,
                                               const float* __restrict__ recw_tile,
                                               const u32* __restrict__ list_ref, float* __restrict__ v0) {
-    constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3, COLUMNS = TP / COLUMN, AHEAD = 4;
+    constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3, COLUMNS = TP / COLUMN;
     for (int i = threadIdx.x; i < (PD + 1) * COLUMNS; i += TP) {
         const int r = i / COLUMNS, c = i % COLUMNS;
         const int lx = c & (g.TX - 1), ly = (c >> g.tx_log2) * COLUMN;
@@ -239,13 +256,14 @@ __device__ __forceinline__ void splat_columns(const Geom& g, const TilePos& tpos
 }
 
 template <int PD, int VD, bool PRE>
-__global__ void __launch_bounds__(Cfg<PD>::TP, PD <= COLUMNS_PD ? 6 : 0)
+__global__ void __launch_bounds__(Cfg<PD>::TP, NarrowColumns<PD, VD, PRE>::CTAS)
 splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
                  const u16* __restrict__ rec, const float* __restrict__ rec_w, const uint2* __restrict__ srec,
                  const u32* __restrict__ list_ref, float* __restrict__ v0, int bulk_ok) {
     wait_for_previous_kernel();
     constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, C = VD - 1, VP = (VD + 3) & ~3;
     using SF = SplatFast<PD, VD, PRE>;
+    using NC = NarrowColumns<PD, VD, PRE>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* in_s = reinterpret_cast<float*>(smem_raw);                                       // [TP][C]
     uint2* sorted_s = reinterpret_cast<uint2*>(smem_raw + SF::IN_BYTES);                    // [SORTED]
@@ -261,9 +279,9 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     const int2 info = tile_info[tile];
     const int base = info.x, nloc = info.y;
     using CS = ColumnsSample<PD>;
-    if constexpr (PD <= COLUMNS_PD) {
-        if (in_columns<PD>(g, nloc) && CS::smooth(g, tpos, hdr, rec, nloc, CS::NARROW)) {
-            splat_columns<PD, VD>(g, tpos, base, input, rec + (size_t)tile * SPLATS, rec_w + (size_t)tile * SPLATS,
+    if constexpr (NC::EVER) {
+        if (in_columns<PD>(g, nloc, NC::LEAST) && CS::smooth(g, tpos, hdr, rec, nloc, CS::NARROW)) {
+            splat_columns<PD, VD, NC::AHEAD>(g, tpos, base, input, rec + (size_t)tile * SPLATS, rec_w + (size_t)tile * SPLATS,
                                   list_ref, v0);
             let_next_kernel_start();
             return;
@@ -461,12 +479,12 @@ constexpr int WIDE_COLUMNS_PD = 3, FIXED_COLUMNS_PD = 2;
 template <int PD, bool PRE, typename Sum>
 struct WideColumns {
     static constexpr bool FIXED = !std::is_same<Sum, FloatSum>::value;
-    static constexpr bool EVER = PD <= (FIXED ? FIXED_COLUMNS_PD : WIDE_COLUMNS_PD);
+    static constexpr bool EVER = PD >= 2 && PD <= (FIXED ? FIXED_COLUMNS_PD : WIDE_COLUMNS_PD);
     __device__ static __forceinline__ bool take(const Geom& g, int entries, int LR) {
         if (!EVER) return false;
-        if (FIXED) return LR <= (PRE ? 1 : 2) && in_columns<PD>(g, LR * entries);
+        if (FIXED) return LR <= (PRE ? 1 : 2) && in_columns<PD>(g, LR * entries, 2 * PD);
         if (PD == 3 && entries < 12) return false;
-        return LR <= 16 && in_columns<PD>(g, entries);   // (up to 64 floats a row: a column of as many points as lanes fits the tile)
+        return LR <= 16 && in_columns<PD>(g, entries, 2 * PD);   // (up to 64 floats a row: a column of as many points as lanes fits the tile)
     }
 };
 template <int PD, typename Sum, typename V>
