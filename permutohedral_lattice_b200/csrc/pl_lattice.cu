@@ -478,7 +478,7 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
     if constexpr (VP == 4) {
         PL_LAUNCH_AFTER(OV_SLICE, (slice_points<PD, CT>), tile_grid(g), Cfg<PD>::TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, watch);
     } else if constexpr (VP > 0) {
-        int rows_cap = SliceFast<PD, VP>::ROWS_BYTES / (SliceFast<PD, VP>::RS * 4);
+        int rows_cap = SliceFast<PD, VP, CT>::ROWS_BYTES / (SliceFast<PD, VP>::RS * 4);
         if (rows_cap > Cfg<PD>::SPLATS) rows_cap = Cfg<PD>::SPLATS;
         const size_t smem = SliceFast<PD, VP>::bytes(rows_cap);
         PL_TRY((ensure_dynamic_smem<slice_tiles_fast<PD, VP, CT>>(smem)));
