@@ -62,9 +62,9 @@ blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restri
 // ---------------------------------------------------------------------------------------------
 // slice_tiles (src/PermutohedralLatticeCPU.h:333-352: float multiply-then-add per remainder in
 // ascending order, reciprocal of the homogeneous channel in double, one multiply per channel).
-// The tile's vertex rows are staged once in shared memory.
+// Rows of one float4: slice_points, below.  Of wider ones the tile's are staged once in shared memory.
 //
-// Fast form (rows of VP floats, VP known at compile time; up to 32): one thread per point interpolates the whole
+// Fast form (rows of VP floats, VP known at compile time; 8 to 32): one thread per point interpolates the whole
 // row in registers (float4 reads of the cached rows, row stride padded against bank conflicts), the
 // output block is assembled in shared memory and leaves by bulk asynchronous copies when its rows
 // are 16-byte aligned.

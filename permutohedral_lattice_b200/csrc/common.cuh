@@ -68,7 +68,8 @@ constexpr u64 SKETCH_MIN_ENTRIES = 1ull << 18;   // below, a table sized by entr
 // a vertex).  It lies at the end of the table's region, which has room for it whenever the table uses at most half of
 // that, and is kept for tables of 2^FILTER_MIN_LOG2 slots (64 MB) and more; beyond 2^FILTER_MAX_LOG2 bits (32 MB) it
 // would not stay in L2 itself.  1 M points with 16 features: 2133 ->
-// 2044 us a call; with a table of 32 MB, which stays in L2, it cost a call on 16 x 512x512 x 21 one per cent.
+// 2044 us a call; with a table of 32 MB, which stays in L2, it cost one per cent (16 x 512x512 x 21, while pd 5 still had
+// slots of 8 bytes).  Tables whose slots hold the key have none: a lookup there is one access anyway.
 constexpr u32 FILTER_BITS_LOG2 = 3, FILTER_MIN_LOG2 = 23, FILTER_MAX_LOG2 = 28;
 __device__ __forceinline__ u32* filter_words(u64* table, u32 max_log2, u32 filter_log2) {
     return reinterpret_cast<u32*>(table + (1ull << max_log2)) - (1ull << (filter_log2 - 5));

@@ -256,7 +256,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 #pragma unroll
         for (int r = 0; r <= PD; r++) recw_tile[r * TP + tid] = w[r];
         // COMPACT: a point's own key is formed by steps, that of a splat it is compared with from the stored ranks.
-        // Where the ranks are no permutation the two differ.
+        // The two are the same once the ranks are a permutation.
         if constexpr (COMPACT) settle_ranks<PD>(s);
         k.start(s);
         if constexpr (COMPACT) {
@@ -335,8 +335,9 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     if constexpr (COMPACT) {
         // The open splats, a few in a hundred, are put in a list and the rounds run over that.  Looked for among all 17
         // splats of a point, most warps had one or another of every remainder and went through hash and comparison
-        // for each: with it and the keys by steps 350 -> 286 us on 1 M points.  (With six splats a point, whose keys lie in shared memory as they are, the list and its barriers
-        // cost more than they saved: 160 -> 170 us on 16 x 512x512, pd 5.)
+        // for each: with it and the keys by steps 350 -> 286 us on 1 M points.  (With six splats a point, whose keys lie
+        // in shared memory as they are, the list and its barriers cost more than they saved: 160 -> 170 us on 16 x
+        // 512x512, pd 5.)
         u16* const list = lidx_s;
         __syncthreads();   // the slots kept there have been read
         if (open) {
@@ -516,7 +517,8 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 // ---------------------------------------------------------------------------------------------
 // clear_table: table capacity chosen on the device, a power of two: at least twice the entries (at least 1024),
 // or, where the call kept a sketch of the lattice's size, at least four times the vertices it tells of (twice
-// as many cost the probe chains of insert_entries more than the smaller table gained it).
+// as many cost the probe chains of insert_entries more than the smaller table gained it), in a table of keys beyond
+// 32 MB at least twice.
 // ---------------------------------------------------------------------------------------------
 constexpr u64 KEY_SLOTS_WHOLE = 1ull << 21;   // 32 MB
 template <bool KEY_SLOTS>
@@ -564,10 +566,12 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
         hdr->table_log2 = lg;
         hdr->filter_log2 = filter_log2;
     }
-    if (filter_log2) {
-        uint4* filter = reinterpret_cast<uint4*>(filter_words(table, max_log2, filter_log2));
-        for (u64 i = grid_thread(); i < (1ull << (filter_log2 - 7)); i += grid_threads())
-            filter[i] = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (!KEY_SLOTS) {
+        if (filter_log2) {
+            uint4* filter = reinterpret_cast<uint4*>(filter_words(table, max_log2, filter_log2));
+            for (u64 i = grid_thread(); i < (1ull << (filter_log2 - 7)); i += grid_threads())
+                filter[i] = make_uint4(0u, 0u, 0u, 0u);
+        }
     }
     const u64 cap = 1ull << lg;
     for (u64 i = grid_thread(); i < cap; i += grid_threads()) {

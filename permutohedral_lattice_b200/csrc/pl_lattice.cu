@@ -562,8 +562,9 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     int table_log2 = 0;
     while ((1ull << table_log2) < L.table_slots) table_log2++;
 
-    // insert_entries overlaps clear_table only while the table can stay in L2 (64 MB of slots): behind a
-    // clear_table that itself overlaps build_tiles it cost calls with large tables 4-25 % (pd 16: 30 -> 37 ms)
+    // The insert overlaps clear_table only in regions of up to 64 MB of 8-byte slots (pd up to 5: 2^23 slots too, 128 MB, of
+    // which the device uses what the vertices ask for): behind a clear_table that itself overlaps build_tiles it cost
+    // calls with large tables 4-25 % (pd 16: 30 -> 37 ms)
     const bool small_table = L.index_words <= (1ull << 24);
     if (phases & PH_BUILD) {
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
