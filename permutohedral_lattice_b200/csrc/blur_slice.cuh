@@ -82,13 +82,14 @@ struct SliceFast {
     static size_t bytes(int rows_cap) { return region(rows_cap) + sizeof(int) * TP; }
     // CTAs per SM asked of the compiler: what the row, the weights and the entry numbers of a point leave room for
     static constexpr int NEED = VP + 2 * (PD + 1);
-    // With pd 2 and 3 the kernel waits for memory and not for shared memory's conflicts: a sixth CTA, 40 registers, for rows
-    // that leave it room.  us a slice, six / five CTAs, by channels: 16 x 512x512, pd 2, 2.4 and 14.7 splats an entry, 4 channels 106
-    // / 102 and 76 / 83, 10 channels 141 / 159 and 94 / 106, 15 channels (8 bytes spilled) 156 / 152 and 104 / 115, 19 channels 166 / 186 and 119 / 129,
-    // 21 channels, known at compile time (16 bytes), 183 / 185 and 121 / 131; 4 x 64x128x128, pd 3, 1.3 and 6.6 splats, 4 channels 166 / 153 and
-    // 94 / 99, 10 channels 202 / 222 and 117 / 127, 15 channels (16 bytes) 268 / 237 and 125 / 126, 19 channels (12 bytes) 360 / 331 and
-    // 134 / 148: tiles of few splats an entry lose up to an eighth, all others gain a tenth.  20 to 23 channels known at run time only would spill
-    // 48 bytes and gain nothing (2.4 splats 188 / 176).
+    // With pd 2 and 3 the kernel waits for memory and not for shared memory's conflicts: a sixth CTA, 40 registers,
+    // for rows that leave it room.  us a slice, six / five CTAs, by channels: 16 x 512x512, pd 2, 2.4 and 14.7 splats
+    // an entry, 4 channels 106 / 102 and 76 / 83, 10 channels 141 / 159 and 94 / 106, 15 channels (8 bytes spilled)
+    // 156 / 152 and 104 / 115, 19 channels 166 / 186 and 119 / 129, 21 channels, known at compile time (16 bytes),
+    // 183 / 185 and 121 / 131; 4 x 64x128x128, pd 3, 1.3 and 6.6 splats, 4 channels 166 / 153 and 94 / 99, 10
+    // channels 202 / 222 and 117 / 127, 15 channels (16 bytes) 268 / 237 and 125 / 126, 19 channels (12 bytes) 360 /
+    // 331 and 134 / 148: tiles of few splats an entry lose up to an eighth, all others gain a tenth.  20 to 23
+    // channels known at run time only would spill 48 bytes and gain nothing (2.4 splats 188 / 176).
     static constexpr bool SIX = (PD == 2 || PD == 3) && NEED <= (CT ? 30 : 28);
     static constexpr int CTAS = TP != 256 ? (VP > 24 ? 6 : 8) : SIX ? 6 : NEED <= 36 ? 5 : NEED <= 52 ? 4 : 3;
     static constexpr int ROWS_BYTES = (SIX ? 35 : 40) * 1024;   // of cached rows: so many CTAs fit the shared memory too

@@ -145,27 +145,28 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
 // vertices, so that walking down a column of COLUMN points meets about as few runs as the sorted list cut into windows
 // does, and needs no sort.  One thread a column and remainder; nothing goes through shared memory: a point's row is read
 // PD + 1 times, from L1 after the first, neighbouring threads on neighbouring points.
-// Bound by its reductions and the latency of its loads.  Two volumes of 111x128x120 points, 20 splats an entry: 106 -> 83 us
-// (the sort kept the LSU pipe at 82 %).
-// Where (us a splat, columns / sorted): rows of more than one float4 from 2 pd splats an entry on (8 x 512x512, pd 2, 21 channels,
-// 4.8 splats 95 / 110, 14.7 splats 76 / 98); narrow ones as NarrowColumns says.  pd 5, us a call: 8 splats an entry 201 / 197, 36
-// splats 158 / 138: up to pd 4.  Tiles of points in one dimension, which are all there are with pd 1, have no columns.
+// Bound by the latency of its loads (most stalls are for them; its reductions are none, L2 is at 34 %).  Two volumes of
+// 111x128x120 points, 20 splats an entry: 106 -> 83 us (the sort kept the LSU pipe at 82 %).
+// Where (us a splat, columns / sorted): rows of more than one float4 from 2 pd splats an entry on (8 x 512x512, pd 2,
+// 21 channels, 4.8 splats 95 / 110, 14.7 splats 76 / 98); narrow ones as NarrowColumns says.  pd 5, us a call: 8
+// splats an entry 201 / 197, 36 splats 158 / 138: up to pd 4.  Tiles of points in one dimension, which are all there are with pd 1, have no columns.
 constexpr int COLUMN = 8;
 template <int PD>
 __device__ __forceinline__ bool in_columns(const Geom& g, int entries, int least) {   // least: splats an entry
     return g.TX <= 16 && least * entries <= Cfg<PD>::SPLATS;
 }
-// Rows of one float4, VD - 1 channels.  Sorted tiles want the 32 registers of eight CTAs an SM (pd 2 and 3; also pd 4 in a kept
-// lattice), columns of four points ahead want 40: with those, and 24 to 56 bytes spilled, sorted tiles took 10 to 17 % longer (pd 2, 1
-// channel, 3.5 splats an entry 41 -> 48 us; 36 -> 42 in a kept lattice).  Two points ahead fit 32 registers (up to 8 bytes
-// spilled).  pd 4 sorts with 40 registers anyway.  With two channels, four points ahead gain more in columns than they cost
-// sorted tiles (pd 2, 14.7 splats an entry 37 us, two ahead 41, sorted 45; 3.5 splats, sorted with six CTAs 49, with eight 43;
-// pd 3, 12.6 splats 43, two ahead 45, sorted 50; kept lattices only at pd 2).
-// From how many splats an entry on, us a splat, columns / sorted: pd 2, 1 channel, 8 splats 47 / 39, 14.7 splats 43 / 43, 38 splats 39
-// / 49; 2 channels, 8 splats 42 / 43; 3 channels, 14.7 splats 44 / 47.  pd 3, 1 and 3 channels, 6.6 splats 1.06 to 1.12 of the
-// sort's time, 12.6 splats 0.92 to 0.96; 2 channels, 6.6 splats 1.00, 8.9 splats 0.93.  pd 4, 9.8 splats 0.88 to 1.04, 20 splats 0.82 to
-// 0.96.  Kept lattices, sorted already: pd 2 and 3 with 2 channels from 8 and 10 splats on, with 1 and 3 channels 1.03 to 1.10 at
-// 15 splats, 0.91 to 1.09 beyond 26; pd 4 never faster.
+// Rows of one float4, VD - 1 channels.  Sorted tiles want the 32 registers of eight CTAs an SM (pd 2 and 3; also pd 4
+// in a kept lattice), columns of four points ahead want 40: with those, and 24 to 56 bytes spilled, sorted tiles took
+// 10 to 17 % longer (pd 2, 1 channel, 3.5 splats an entry 41 -> 48 us; 36 -> 42 in a kept lattice).  Two points ahead
+// fit 32 registers (up to 8 bytes spilled).  pd 4 sorts with 40 registers anyway.  With two channels, four points
+// ahead gain more in columns than they cost sorted tiles (pd 2, 14.7 splats an entry 37 us, two ahead 41, sorted 45;
+// 3.5 splats, sorted with six CTAs 49, with eight 43; pd 3, 12.6 splats 43, two ahead 45, sorted 50; kept lattices
+// only at pd 2).  From how many splats an entry on, us a splat, columns / sorted: pd 2, 1 channel, 8 splats 47 / 39,
+// 14.7 splats 43 / 43, 38 splats 39 / 49; 2 channels, 8 splats 42 / 43; 3 channels, 14.7 splats 44 / 47.  pd 3, 1 and
+// 3 channels, 6.6 splats 1.06 to 1.12 of the sort's time, 12.6 splats 0.92 to 0.96; 2 channels, 6.6 splats 1.00, 8.9
+// splats 0.93.  pd 4, 9.8 splats 0.88 to 1.04, 20 splats 0.82 to 0.96.  Kept lattices, sorted already: pd 2 and 3
+// with 2 channels from 8 and 10 splats on, with 1 and 3 channels 1.03 to 1.10 at 15 splats, 0.91 to 1.09 beyond 26;
+// pd 4 never faster.
 template <int PD, int VD, bool PRE>
 struct NarrowColumns {
     static constexpr bool EVER = PD >= 2 && PD <= (PRE ? 3 : 4);
@@ -173,13 +174,14 @@ struct NarrowColumns {
     static constexpr int CTAS = !EVER ? 0 : AHEAD == 4 ? 6 : 8;
     static constexpr int LEAST = AHEAD == 4 ? 8 : !PRE ? (PD == 2 ? 12 : 10) : VD == 3 ? 10 : 24;
 };
-// Few entries are not enough where a noisy guide sends neighbouring points to one and another of them: a column then meets
-// a run nearly every point, and all tiles add to few vertices.  So tiles that have more entries
-// than one under a flat guide would (Geom::calm_entries) are sampled for changes of entry from one row to the next.  A smooth guide, or none, gives 3 to 7 changes an entry, whatever its scale, noise 9 to 24.
-// Columns or sorted, us a splat: 4 x 512x512 guided by one channel, 2 channels, 12 changes 27 / 35, 15 changes 41 / 48, 18
-// changes 73 / 72, 23 changes 74 / 51; guided by two channels, 7 changes 31 / 39, 9 and 13 changes 51 / 35 and 42 / 39; two
-// noisy volumes of 96x128x128, 5 changes 84 / 96, 13 changes 275 / 190.  Rows of 21 channels: 12 changes 53 / 61, 15 changes
-// 64 / 62, 18 changes 94 / 62, 23 changes 109 / 61, and volumes with 4 changes but fewer than 12 entries a tile 148 / 119.
+// Few entries are not enough where a noisy guide sends neighbouring points to one and another of them: a column then
+// meets a run nearly every point, and all tiles add to few vertices.  So tiles that have more entries than one under
+// a flat guide would (Geom::calm_entries) are sampled for changes of entry from one row to the next.  A smooth guide,
+// or none, gives 3 to 7 changes an entry, whatever its scale, noise 9 to 24.  Columns or sorted, us a splat: 4 x
+// 512x512 guided by one channel, 2 channels, 12 changes 27 / 35, 15 changes 41 / 48, 18 changes 73 / 72, 23 changes
+// 74 / 51; guided by two channels, 7 changes 31 / 39, 9 and 13 changes 51 / 35 and 42 / 39; two noisy volumes of
+// 96x128x128, 5 changes 84 / 96, 13 changes 275 / 190.  Rows of 21 channels: 12 changes 53 / 61, 15 changes 64 / 62,
+// 18 changes 94 / 62, 23 changes 109 / 61, and volumes with 4 changes but fewer than 12 entries a tile 148 / 119.
 // With pd 2 there is no guide.  Every warp looks at the same 64 pairs of points, so that all agree without a barrier;
 // it costs those tiles 4 to 7 %.  (All tiles sampled cost the splat of smooth volumes 7 %; all points of every second
 // row, counted over the CTA, 4 to 20 %; counted by build_tiles, that 3 to 6 %.)
@@ -462,19 +464,20 @@ struct SplatRows {
     }
 };
 
-// Walking columns of points (see splat_columns) for rows of more than one float4, up to pd = WIDE_COLUMNS_PD: a group of
-// lanes per column, as below, with the running sums of all PD + 1 remainders, so that a point's row is read once instead
-// of PD + 1 times and neither sorted nor spread to padded rows: lanes read single floats, and four neighbouring columns
-// with an odd number of channels never meet on a shared-memory bank.  Channel 0 of point (lx, ly) lies at
-// ly row_step + lx point_step; `splat_s` holds the vertex and weight of every splat.  8 x 512x512 x 21, pd 2: 99 -> 75 us.
-// (Running sums of four remainders are what the registers of five CTAs an SM hold.)
-// Columns meet more runs than the sorted list's windows, each flushed once.  For a float sum that is one reduction of 16
-// bytes a lane, for a fixed-point sum four of 8 bytes.  Fixed-point sums in columns or sorted, us a splat of 8 x 512x512, pd 2,
-// by channels, with 5 and with 15 splats an entry: 1-3 channels 99 / 122 and 84 / 112; 4 channels 139 / 146 and 101 / 123;
-// 6 channels 168 / 153 and 116 / 128; with 8 splats an entry 10 channels 1.03, 21 channels 1.29 times the sort's time.  pd 3:
-// 0.9 to 2.3 times its time, 21 channels 1.5 to 4.  In a kept lattice, whose splats are sorted already: 1-3 channels 87 / 101 from 8
-// splats an entry on, 4-6 channels 1.0 to 1.1 times, beyond pd 2 never faster.  Hence: pd 2 only, and there rows of one float4, or of two
-// from 4 pd splats an entry on and if the call would have to sort.
+// Walking columns of points (see splat_columns) for rows of more than one float4, up to pd = WIDE_COLUMNS_PD: a group
+// of lanes per column, as below, with the running sums of all PD + 1 remainders, so that a point's row is read once
+// instead of PD + 1 times and neither sorted nor spread to padded rows: lanes read single floats, and four
+// neighbouring columns with an odd number of channels never meet on a shared-memory bank.  Channel 0 of point (lx,
+// ly) lies at ly row_step + lx point_step; `splat_s` holds the vertex and weight of every splat.  8 x 512x512 x 21,
+// pd 2: 99 -> 75 us.  (Running sums of four remainders are what the registers of five CTAs an SM hold.) Columns meet
+// more runs than the sorted list's windows, each flushed once.  For a float sum that is one reduction of 16 bytes a
+// lane, for a fixed-point sum four of 8 bytes.  Fixed-point sums in columns or sorted, us a splat of 8 x 512x512, pd
+// 2, by channels, with 5 and with 15 splats an entry: 1-3 channels 99 / 122 and 84 / 112; 4 channels 139 / 146 and
+// 101 / 123; 6 channels 168 / 153 and 116 / 128; with 8 splats an entry 10 channels 1.03, 21 channels 1.29 times the
+// sort's time.  pd 3: 0.9 to 2.3 times its time, 21 channels 1.5 to 4.  In a kept lattice, whose splats are sorted
+// already: 1-3 channels 87 / 101 from 8 splats an entry on, 4-6 channels 1.0 to 1.1 times, beyond pd 2 never faster.
+// Hence: pd 2 only, and there rows of one float4, or of two from 4 pd splats an entry on and if the call would have
+// to sort.
 constexpr int WIDE_COLUMNS_PD = 3, FIXED_COLUMNS_PD = 2;
 template <int PD, bool PRE, typename Sum>
 struct WideColumns {
@@ -484,7 +487,8 @@ struct WideColumns {
         if (!EVER) return false;
         if (FIXED) return LR <= (PRE ? 1 : 2) && in_columns<PD>(g, LR * entries, 2 * PD);
         if (PD == 3 && entries < 12) return false;
-        return LR <= 16 && in_columns<PD>(g, entries, 2 * PD);   // (up to 64 floats a row: a column of as many points as lanes fits the tile)
+        // (up to 64 floats a row: a column of as many points as lanes fits the tile)
+        return LR <= 16 && in_columns<PD>(g, entries, 2 * PD);
     }
 };
 template <int PD, typename Sum, typename V>
