@@ -312,9 +312,9 @@ __device__ __forceinline__ void load_features(const Geom& g, const float* __rest
                     c = y;
                 } else if (g.n_sdims == 1) {
                     c = x;
-                } else {
-                    c = rest % g.sdims[i];
-                    rest /= g.sdims[i];
+                } else {   // (what is left for the first dimension lies inside it: a volume's plane needs no division)
+                    c = i ? rest % g.sdims[i] : rest;
+                    if (i) rest /= g.sdims[i];
                 }
                 const float a = small_int_to_float(c);
                 f[i] = g.rcp_div ? div_by_rcp(a, g.spatial_std, g.spatial_rcp) : PL_FDIV(a, g.spatial_std);
@@ -348,8 +348,8 @@ __device__ __forceinline__ void load_features(const Geom& g, const double* __res
                 } else if (g.n_sdims == 1) {
                     c = x;
                 } else {
-                    c = rest % g.sdims[i];
-                    rest /= g.sdims[i];
+                    c = i ? rest % g.sdims[i] : rest;
+                    if (i) rest /= g.sdims[i];
                 }
                 f[i] = __ddiv_rn((double)c, g.spatial_std_d);
             }

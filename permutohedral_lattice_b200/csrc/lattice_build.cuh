@@ -155,17 +155,15 @@ struct TileKeys {
     __device__ __forceinline__ u32 hash(int id, int r, u32 seed) const {
         u32 k[CW];
         load(id, r, k);
+        return hash(k, seed);
+    }
+    __device__ static __forceinline__ u32 hash(const u32 (&k)[CW], u32 seed) {
         u32 h = seed;
 #pragma unroll
         for (int j = 0; j < CW; j++) h += k[j] * (u32)(hash_factor(j + 8) >> 32 | 1u);
         return h;
     }
     // the key as the global list holds it
-    __device__ __forceinline__ Key<Cfg<PD>::KW> global_key(int id, int r, int item) const {
-        u32 k[CW];
-        load(id, r, k);
-        return global_key(k, item);
-    }
     __device__ static __forceinline__ Key<Cfg<PD>::KW> global_key(const u32 (&k)[CW], int item) {
         constexpr int KW = Cfg<PD>::KW;
         Key<KW> out;
@@ -179,6 +177,16 @@ struct TileKeys {
         return out;
     }
 };
+
+// Sets the bit of a key, of tile hash h, in the sketch if the key is sampled (sketch_shift < 0: no sketch).
+__device__ __forceinline__ void add_to_sketch(Header* hdr, u32 h, int sketch_shift) {
+    if (sketch_shift < 0) return;
+    const u32 x = (h ^ (h >> 15)) * 0x9E3779B1u;
+    if ((x >> 1) < (0x80000000u >> sketch_shift)) {
+        const u32 bit = (h ^ (x << 7)) * 0x85EBCA77u >> (32 - SKETCH_LOG2);
+        atomicOr(reinterpret_cast<u32*>(hdr + 1) + (bit >> 5), 1u << (bit & 31u));
+    }
+}
 
 constexpr u32 TILE_SEED = 0x2C1B3C6Du;    // times the item: keys of different items sample independently
 constexpr int TILE_ROUNDS = 8;            // of the tile's de-duplication
@@ -269,7 +277,6 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
                                         ((u32)s.rank[4 * j + 2] << 16) | ((u32)s.rank[4 * j + 3] << 24);
         }
         const u32 seed = (u32)item * TILE_SEED;
-        u32* sketch = reinterpret_cast<u32*>(hdr + 1);
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
             if (r > 0) k.step(r);
@@ -279,13 +286,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             slots_s[slot] = (u16)(r * TP + tid);
             if constexpr (COMPACT) lidx_s[r * TP + tid] = (u16)slot;   // (there are no entry numbers yet)
             else slot2[r / 2] |= slot << (16 * (r & 1));
-            if (sketch_shift >= 0) {
-                const u32 x = (h ^ (h >> 15)) * 0x9E3779B1u;
-                if ((x >> 1) < (0x80000000u >> sketch_shift)) {
-                    const u32 bit = (h ^ (x << 7)) * 0x85EBCA77u >> (32 - SKETCH_LOG2);
-                    atomicOr(sketch + (bit >> 5), 1u << (bit & 31u));
-                }
-            }
+            if constexpr (COMPACT) add_to_sketch(hdr, h, sketch_shift);   // (else once an entry, below)
         }
     }
     __syncthreads();
@@ -364,8 +365,8 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             if (!__syncthreads_or((int)todo)) break;
         }
     } else {
-        for (int round = 1; round <= TILE_ROUNDS; round++) {
-            if (!__syncthreads_or((int)open)) break;
+        for (int round = 1;; round++) {   // (left behind the barrier, when nobody reads a slot any more)
+            if (!__syncthreads_or((int)open) || round > TILE_ROUNDS) break;
             if (open) {
 #pragma unroll
                 for (int r = 0; r <= PD; r++)
@@ -391,6 +392,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     // entries grouped by warp).  Per warp ONE shared-memory atomic instruction: lane r adds the warp's
     // number of new remainder-r entries to counter r.  The index stored now is relative to the
     // remainder's segment; the segment starts are known after the barrier.
+    unsigned char* owner_s = reinterpret_cast<unsigned char*>(slots_s) + 4 * SPLATS;   // [SPLATS], in the dead hash too: see below
     int* run_s = reinterpret_cast<int*>(slots_s);   // SORTED: the tile hash is dead, its memory counts the splats of every entry
     if constexpr (SORTED) {
         static_assert(sizeof(int) * SPLATS <= sizeof(u16) * Cfg<PD>::LS, "the counters fit the hash's memory");
@@ -400,19 +402,22 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     {
         const int lane = tid & 31;
         unsigned owners[PD + 1];
-        int mine = 0;
+        unsigned mine = 0;
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
             owners[r] = __ballot_sync(0xFFFFFFFFu, valid && get_rep(r) == r * TP + tid);
-            mine = (lane == r) ? __popc(owners[r]) : mine;
+            mine = (lane == r) ? owners[r] : mine;
         }
         int first = 0;
-        if (lane <= PD && mine) first = atomicAdd(&cnt_s[lane], mine);
+        if (lane <= PD && mine) first = atomicAdd(&cnt_s[lane], __popc(mine));
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
             const int first_r = __shfl_sync(0xFFFFFFFFu, first, r);
-            if ((owners[r] >> lane) & 1u)
-                lidx_s[r * TP + tid] = (u16)(first_r + __popc(owners[r] & ((1u << lane) - 1u)));
+            if ((owners[r] >> lane) & 1u) {
+                const int at = first_r + __popc(owners[r] & ((1u << lane) - 1u));
+                lidx_s[r * TP + tid] = (u16)at;
+                if constexpr (!COMPACT) owner_s[r * TP + at] = (unsigned char)tid;
+            }
         }
     }
     __syncthreads();
@@ -453,14 +458,33 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     __syncthreads();
     if constexpr (!SORTED) let_next_kernel_start();   // what is left of this tile: its keys
     const int base = base_s;
-    if (valid && base >= 0) {
-#pragma unroll (COMPACT ? 1 : PD + 1)
-        for (int r = 0; r <= PD; r++) {
-            const int me = r * TP + tid;
-            if (get_rep(r) == me)
-                list_keys[(size_t)base + (seg[r] + lidx_s[me])] =
-                    COMPACT ? TileKeys<PD>::global_key(k.w, item) : keys.global_key(me, r, item);
-            if (COMPACT && r < PD) k.step(r + 1);
+    if constexpr (COMPACT) {
+        if (valid && base >= 0) {
+#pragma unroll 1
+            for (int r = 0; r <= PD; r++) {
+                const int me = r * TP + tid;
+                if (rep_s[me] == me) list_keys[(size_t)base + (seg[r] + lidx_s[me])] = TileKeys<PD>::global_key(k.w, item);
+                if (r < PD) k.step(r + 1);
+            }
+        }
+    } else if (base >= 0) {
+        // A thread an entry: its key, from the splat that owner_s names, and its bit in the sketch.  A tile has fewer
+        // entries than threads, mostly; done by every splat that represents one, the same cost every warp a branch
+        // a remainder, and the sketch a hash a splat.  With this and the cheaper floor and wrap of find_simplex, us a
+        // call, forward + backward: two volumes of 111x128x120 549 -> 517, 1024x1024 grey by RGB 325 -> 309, 16 x 512x512
+        // x 21 1823 -> 1794; 800x1200 x 3, forward, 188 -> 180.
+        for (int e = tid; e < cnt; e += TP) {
+            int r = 0, first = 0;
+#pragma unroll
+            for (int q = 1; q <= PD; q++) {
+                r = e >= seg[q] ? q : r;
+                first = e >= seg[q] ? seg[q] : first;
+            }
+            const int id = r * TP + owner_s[r * TP + e - first];
+            u32 kw[Cfg<PD>::CW];
+            keys.load(id, r, kw);
+            list_keys[(size_t)base + e] = TileKeys<PD>::global_key(kw, item);
+            add_to_sketch(hdr, TileKeys<PD>::hash(kw, (u32)item * TILE_SEED), sketch_shift);
         }
     }
     if constexpr (SORTED && !is_double<R>::value) {

@@ -51,6 +51,16 @@ namespace pl {
 // 1.5 * 2^23: adding it to |x| < 2^22 leaves the nearest integer in the low mantissa bits.
 #define PL_ROUND_MAGIC 12582912.0f
 
+// floor(v) for |v| < 2^22.
+PL_HD float magic_floor(float v) {
+#ifdef __CUDA_ARCH__
+    return PL_FSUB(__fadd_rd(v, PL_ROUND_MAGIC), PL_ROUND_MAGIC);   // the sum rounded down: no comparison with v
+#else
+    const float fl = PL_FSUB(PL_FADD(v, PL_ROUND_MAGIC), PL_ROUND_MAGIC);   // nearest integer
+    return (fl > v) ? PL_FSUB(fl, 1.0f) : fl;
+#endif
+}
+
 // Integer value of a float that holds an integer of magnitude below 2^22 (no conversion unit).
 PL_HD int exact_int(float x) { return PL_F2BITS(PL_FADD(x, PL_ROUND_MAGIC)) - 0x4B400000; }
 
@@ -156,16 +166,17 @@ PL_HD void find_simplex(const float* pos, const float* scale, Simplex<PD>& s) {
     float cells = 0.f;   // sum of the coordinates' cell numbers: small integers, exact
 #pragma unroll
     for (int i = 0; i <= PD; i++) {
-        const float v = PL_FMUL(s.el[i], inv_f);
-        float fl = PL_FSUB(PL_FADD(v, PL_ROUND_MAGIC), PL_ROUND_MAGIC);   // nearest integer
-        fl = (fl > v) ? PL_FSUB(fl, 1.0f) : fl;                          // -> floor
+        const float fl = magic_floor(PL_FMUL(s.el[i], inv_f));
         const float down = PL_FMUL(fl, (float)(PD + 1));                 // exact: small integers
         const float up = PL_FADD(down, (float)(PD + 1));
         const bool take_up = PL_FSUB(up, s.el[i]) < PL_FSUB(s.el[i], down);
         s.rem0f[i] = take_up ? up : down;
-        cells = PL_FADD(cells, take_up ? PL_FADD(fl, 1.0f) : fl);
+        cells = PL_FADD(cells, fl);
+        if (take_up) cells = PL_FADD(cells, 1.0f);
     }
     const int sum = exact_int(cells);
+    const int cell = sum < 0 ? PD + 1 : -(PD + 1);   // what a coordinate outside 0..PD moves by, below
+    const float cell_f = sum < 0 ? (float)(PD + 1) : -(float)(PD + 1);
 
     // Rank of a residual: how many of the others are larger, equal ones in index order.  rank[j] starts as if
     // all earlier ones were.
@@ -186,10 +197,11 @@ PL_HD void find_simplex(const float* pos, const float* scale, Simplex<PD>& s) {
     }
 #pragma unroll
     for (int i = 0; i <= PD; i++) {
-        // wrap into 0..PD: +1 cell when below, -1 cell when above (selects, no branches)
-        const bool below = s.rank[i] < 0, above = s.rank[i] > PD;
-        s.rank[i] += below ? PD + 1 : above ? -(PD + 1) : 0;
-        s.rem0f[i] = PL_FADD(s.rem0f[i], below ? (float)(PD + 1) : above ? -(float)(PD + 1) : 0.f);
+        // wrap into 0..PD: +1 cell when below, -1 cell when above.  A rank is sum plus 0..PD, so that the sign of
+        // sum says which of the two a point can meet at all.
+        const bool outside = (unsigned)s.rank[i] > (unsigned)PD;
+        if (outside) s.rank[i] += cell;
+        if (outside) s.rem0f[i] = PL_FADD(s.rem0f[i], cell_f);
     }
 }
 
