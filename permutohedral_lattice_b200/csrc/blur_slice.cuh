@@ -12,15 +12,33 @@ namespace pl {
 // then the rows.  So the pair of the next trip is fetched together with the rows of this one, and a thread goes on
 // to its next row without dividing (a 64-bit quotient a trip before).  16 x 512x512 x 21,
 // forward + backward (12 passes): 1872 -> 1842 us; 1 M points with 16 features (17 passes): 2048 -> 2014.
+// Rows of floats are mixed in floats, pairs an instruction, with what the two sums round off added at the end: the
+// exact sum rounded once, as in doubles (none of 60 M random triples differ; below 2^-124 a quarter loses its last bits).
+// Doubles took three conversions up and one down a
+// value, sixteen of a warp's a cycle and SM, more than half of a pass: 16 x 512x512 x 21 1790 -> 1764 us, 8 x 512x512 x 21
+// by position alone (pd 2) 438 -> 431, 1 M points with 16 features 1968 -> 1943.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ double mix3(double a, double b, double c) {
     return __fma_rn(0.25, c, __fma_rn(0.5, b, PL_DMUL(0.25, a)));
 }
-__device__ __forceinline__ float mix3(float a, float b, float c) {
-    return (float)mix3((double)a, (double)b, (double)c);
+// Sum of two pairs of floats, and what its rounding left out (Knuth's two-sum, six additions, two of them an instruction).
+__device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& rest) {
+    const float2 s = add2(a, b), from_b = sub2(s, a);
+    rest = add2(sub2(a, sub2(s, from_b)), sub2(b, from_b));
+    return s;
+}
+__device__ __forceinline__ float2 mix3(float2 a, float2 b, float2 c) {
+    float2 r1, r2;
+    const float2 s = two_sum(mul2(a, make_float2(0.25f, 0.25f)), mul2(c, make_float2(0.25f, 0.25f)), r1);
+    const float2 t = two_sum(s, mul2(b, make_float2(0.5f, 0.5f)), r2);
+    const float2 r = add2(r1, r2);
+    // (an infinite sum leaves NaN out, which the maximum drops; finite rests it leaves as they are)
+    return add2(t, make_float2(fmaxf(r.x, -3.402823466e38f), fmaxf(r.y, -3.402823466e38f)));
 }
 __device__ __forceinline__ float4 mix_rows(float4 a, float4 b, float4 c) {
-    return make_float4(mix3(a.x, b.x, c.x), mix3(a.y, b.y, c.y), mix3(a.z, b.z, c.z), mix3(a.w, b.w, c.w));
+    const float2 lo = mix3(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
+    const float2 hi = mix3(make_float2(a.z, a.w), make_float2(b.z, b.w), make_float2(c.z, c.w));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 __device__ __forceinline__ double2 mix_rows(double2 a, double2 b, double2 c) {
     return make_double2(mix3(a.x, b.x, c.x), mix3(a.y, b.y, c.y));
