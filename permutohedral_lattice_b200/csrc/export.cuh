@@ -57,10 +57,9 @@ export_points(Geom g, const Header* hdr, const int2* __restrict__ tile_info, con
     }
 }
 
-template <int PD>
-__global__ void export_vertices(const Header* hdr, const Key<Cfg<PD>::KW>* __restrict__ vkeys, long long max_vertices,
+template <int PD, int KW>
+__global__ void export_vertices(const Header* hdr, const Key<KW>* __restrict__ vkeys, long long max_vertices,
                                 int16_t* __restrict__ vertex_keys, int32_t* __restrict__ vertex_item) {
-    constexpr int KW = Cfg<PD>::KW;
     if (hdr->status != 0) return;
     const u32 M = hdr->num_vertices;
     for (u64 v = (u64)blockIdx.x * blockDim.x + threadIdx.x; v < M && v < (u64)max_vertices;
@@ -70,7 +69,7 @@ __global__ void export_vertices(const Header* hdr, const Key<Cfg<PD>::KW>* __res
 #pragma unroll
             for (int i = 0; i < PD; i++) vertex_keys[v * PD + i] = (int16_t)(key_get<KW>(k, i) ^ 0x8000);
         }
-        if (vertex_item) vertex_item[v] = (int32_t)key_get<KW>(k, PD);
+        if (vertex_item) vertex_item[v] = KW * 4 > PD ? (int32_t)key_get<KW>(k, KW * 4 > PD ? PD : 0) : 0;
     }
 }
 

@@ -164,8 +164,8 @@ struct TileKeys {
         return h;
     }
     // the key as the global list holds it
-    __device__ static __forceinline__ Key<Cfg<PD>::KW> global_key(const u32 (&k)[CW], int item) {
-        constexpr int KW = Cfg<PD>::KW;
+    template <int KW>
+    __device__ static __forceinline__ Key<KW> global_key(const u32 (&k)[CW], int item) {
         Key<KW> out;
 #pragma unroll
         for (int j = 0; j < KW; j++) {
@@ -173,7 +173,7 @@ struct TileKeys {
             const u32 hi = (2 * j + 1 < CW) ? k[2 * j + 1 < CW ? 2 * j + 1 : 0] : 0u;
             out.w[j] = (u64)lo | ((u64)hi << 32);
         }
-        key_set<KW>(out, PD, (u16)item);
+        if constexpr (KW * 4 > PD) key_set<KW>(out, PD, (u16)item);
         return out;
     }
 };
@@ -212,11 +212,12 @@ constexpr int TILE_ROUNDS = 8;            // of the tile's de-duplication
 // It costs this kernel a quarter more time and saves every splat a fifth: worth it from the second
 // splat on, which is why the one-call filter does not ask for it.
 // sketch_shift < 0: no sketch of the lattice's size (see SKETCH_LOG2).
-template <int PD, typename R = float, bool SORTED = false>
+// KW: words of a key (see Cfg).
+template <int PD, typename R = float, bool SORTED = false, int KW = Cfg<PD>::KW>
 __global__ void __launch_bounds__(Cfg<PD>::TP, (PD <= 5 && !is_double<R>::value) ? 6 : (Cfg<PD>::COMPACT && !is_double<R>::value) ? 5 : 1)
 build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ reference,
             Header* hdr, int2* __restrict__ tile_info, u16* __restrict__ rec, R* __restrict__ rec_w,
-            uint2* __restrict__ srec, Key<Cfg<PD>::KW>* __restrict__ list_keys, u32 max_entries, int sketch_shift) {
+            uint2* __restrict__ srec, Key<KW>* __restrict__ list_keys, u32 max_entries, int sketch_shift) {
     wait_for_previous_kernel();
     constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS, LSLOG = Cfg<PD>::LSLOG;
     constexpr bool COMPACT = Cfg<PD>::COMPACT;
@@ -463,7 +464,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 #pragma unroll 1
             for (int r = 0; r <= PD; r++) {
                 const int me = r * TP + tid;
-                if (rep_s[me] == me) list_keys[(size_t)base + (seg[r] + lidx_s[me])] = TileKeys<PD>::global_key(k.w, item);
+                if (rep_s[me] == me) list_keys[(size_t)base + (seg[r] + lidx_s[me])] = TileKeys<PD>::template global_key<KW>(k.w, item);
                 if (r < PD) k.step(r + 1);
             }
         }
@@ -483,7 +484,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
             const int id = r * TP + owner_s[r * TP + e - first];
             u32 kw[Cfg<PD>::CW];
             keys.load(id, r, kw);
-            list_keys[(size_t)base + e] = TileKeys<PD>::global_key(kw, item);
+            list_keys[(size_t)base + e] = TileKeys<PD>::template global_key<KW>(kw, item);
             add_to_sketch(hdr, TileKeys<PD>::hash(kw, (u32)item * TILE_SEED), sketch_shift);
         }
     }
@@ -545,6 +546,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 // 32 MB at least twice.
 // ---------------------------------------------------------------------------------------------
 constexpr u64 KEY_SLOTS_WHOLE = 1ull << 21;   // 32 MB
+constexpr u64 TAG_SLOTS_WHOLE = 1ull << 23;   // 64 MB
 template <bool KEY_SLOTS>
 __global__ void __launch_bounds__(256)
 clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift) {
@@ -575,8 +577,11 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
             u64 slots = (u64)(4.f * sampled * (float)(1u << sketch_shift));
             // four a vertex spare more probes than the larger table costs while it stays in L2 beside everything else; a
             // table of keys beyond 32 MB has two a vertex at least (us a call, four / two a vertex: 1024x1024 grey by RGB,
-            // forward + backward, 17 MB at four, 325 / 337; 16 x 512x512 x 21, 67 MB at four, 1857 / 1824)
-            if (KEY_SLOTS && slots > KEY_SLOTS_WHOLE) slots = slots / 2 > KEY_SLOTS_WHOLE ? slots / 2 : KEY_SLOTS_WHOLE;
+            // forward + backward, 17 MB at four, 325 / 337; 16 x 512x512 x 21, 67 MB at four, 1857 / 1824.  So has
+            // a tagged one beyond 64 MB (1 M points, pd 16, 134 / 67 MB with keys of one sector: insert 454 / 404 us, link
+            // 670 / 578, clear 31 / 18; 4 x 300x300 points 1775 / 1447 us a call)
+            constexpr u64 WHOLE = KEY_SLOTS ? KEY_SLOTS_WHOLE : TAG_SLOTS_WHOLE;
+            if (slots > WHOLE) slots = slots / 2 > WHOLE ? slots / 2 : WHOLE;
             const u64 least = 1ull << (sketch_shift + 11);
             slots = slots < least ? least : slots;
             need = slots < need ? slots : need;
@@ -872,12 +877,11 @@ __host__ __device__ constexpr u64 axis_hash(int a) {          // and to its line
     for (int j = 0; j < Cfg<PD>::KW; j++) h += axis_word<PD>(a, j) * hash_factor(j);
     return h;
 }
-template <int PD, int A>
+template <int PD, int KW, int A>
 __device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mask, const u32* __restrict__ filter,
                                           u32 filter_mask,
-                                          const Key<Cfg<PD>::KW>* __restrict__ vkeys, u32 M, int* __restrict__ nbr,
+                                          const Key<KW>* __restrict__ vkeys, u32 M, int* __restrict__ nbr,
                                           u64 max_entries) {
-    constexpr int KW = Cfg<PD>::KW;
     int* __restrict__ nbr_axis = nbr + 2 * (u64)A * max_entries;
     for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < M; v += gridDim.x * blockDim.x) {
         Key<KW> k = vkeys[v];
@@ -905,11 +909,10 @@ __device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mas
     }
 }
 // The same in a table of keys.
-template <int PD, int A>
+template <int PD, int KW, int A>
 __device__ __forceinline__ void link_axis(const KeySlot* __restrict__ table, u32 mask,
-                                          const Key<Cfg<PD>::KW>* __restrict__ vkeys, u32 M, int* __restrict__ nbr,
+                                          const Key<KW>* __restrict__ vkeys, u32 M, int* __restrict__ nbr,
                                           u64 max_entries) {
-    constexpr int KW = Cfg<PD>::KW;
     int* __restrict__ nbr_axis = nbr + 2 * (u64)A * max_entries;
     for (u32 v = blockIdx.x * blockDim.x + threadIdx.x; v < M; v += gridDim.x * blockDim.x) {
         Key<KW> k = vkeys[v];
@@ -929,21 +932,21 @@ __device__ __forceinline__ void link_axis(const KeySlot* __restrict__ table, u32
         }
     }
 }
-template <int PD, int A>
+template <int PD, int KW, int A>
 struct LinkAxis {   // link_axis of the axis this block works on, chosen once per block
     template <typename... Args>
     __device__ static __forceinline__ void run(int axis, Args... args) {
         if (axis == A)
-            link_axis<PD, A>(args...);
+            link_axis<PD, KW, A>(args...);
         else if constexpr (A < PD)
-            LinkAxis<PD, A + 1>::run(axis, args...);
+            LinkAxis<PD, KW, A + 1>::run(axis, args...);
     }
 };
 
-template <int PD, bool KEY_SLOTS>
+template <int PD, bool KEY_SLOTS, int KW = Cfg<PD>::KW>
 __global__ void __launch_bounds__(256)
 link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restrict__ list_ref,
-                const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys, int* __restrict__ nbr,
+                const u32* __restrict__ vid, const Key<KW>* __restrict__ vkeys, int* __restrict__ nbr,
                 u64 max_entries, void* zero_rows_ptr, u32 zero_row_bytes, Watch watch) {
     after_previous_kernel();
     report_to(watch, hdr);
@@ -957,11 +960,11 @@ link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restr
         for (u64 i = grid_thread(); i < quads; i += grid_threads()) rows[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     if constexpr (KEY_SLOTS) {
-        LinkAxis<PD, 0>::run((int)blockIdx.y, reinterpret_cast<const KeySlot*>(table), (u32)mask, vkeys, M, nbr, max_entries);
+        LinkAxis<PD, KW, 0>::run((int)blockIdx.y, reinterpret_cast<const KeySlot*>(table), (u32)mask, vkeys, M, nbr, max_entries);
     } else {
         const u32 filter_log2 = hdr->filter_log2;
         const u32* filter = filter_log2 ? filter_words(table, max_log2, filter_log2) : nullptr;
-        LinkAxis<PD, 0>::run((int)blockIdx.y, table, mask, filter, (1u << filter_log2) - 1u, vkeys, M, nbr, max_entries);
+        LinkAxis<PD, KW, 0>::run((int)blockIdx.y, table, mask, filter, (1u << filter_log2) - 1u, vkeys, M, nbr, max_entries);
     }
 }
 

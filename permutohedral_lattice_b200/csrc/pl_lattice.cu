@@ -526,11 +526,12 @@ static bool small_blur(const Layout& L, u32 vpr) { return L.max_entries * vpr <=
 
 enum { PH_BUILD = 1, PH_APPLY = 2 };   // halves of a call: lattice structure / values through it
 
-template <int PD>
+// KW: words of a key.
+template <int PD, int KW>
 static int run_filter(const Geom& g, float* output, const float* input, const float* positions,
                       const float* reference, int vd, int reverse, int mode, void* workspace,
                       const Layout& L, cudaStream_t st, int phases = PH_BUILD | PH_APPLY) {
-    constexpr int KW = Cfg<PD>::KW, TP = Cfg<PD>::TP;
+    constexpr int TP = Cfg<PD>::TP;
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     Header* hdr = reinterpret_cast<Header*>(ws);
     int2* tile_info = reinterpret_cast<int2*>(ws + L.tile_info);
@@ -556,7 +557,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     if (g.num_tiles == 0) return PL_OK;
     const Watch watch = (phases & PH_BUILD) ? take_watch(st) : Watch{nullptr, 0u};
 
-    PL_TRY((ensure_dynamic_smem<build_tiles<PD, float>>(Cfg<PD>::build_smem(false))));
+    PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, false, KW>>(Cfg<PD>::build_smem(false))));
     const int sms = num_sms();
     const int wide = sms * 8;
     int table_log2 = 0;
@@ -569,11 +570,11 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     if (phases & PH_BUILD) {
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
         if (phases & PH_APPLY) {
-            PL_LAUNCH((build_tiles<PD, float, false>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr,
+            PL_LAUNCH((build_tiles<PD, float, false, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr,
                                                                          tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         } else {
-            PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, true>>(Cfg<PD>::build_smem(true))));
-            PL_LAUNCH((build_tiles<PD, float, true>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
+            PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, true, KW>>(Cfg<PD>::build_smem(true))));
+            PL_LAUNCH((build_tiles<PD, float, true, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[1], st));
@@ -600,7 +601,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         const bool small = !use_direct && small_index(L);
         PL_COUNT_LAUNCHES(small ? 2 : 4);   // build_tiles and the launches of the index stage
         if (small) {
-            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, watch);
+            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD, KW>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, watch);
         } else if (!use_direct) {
             // the value rows are zeroed by the link launch, whose lookups leave the memory system idle
             void* zrows = vinit.rows;
@@ -614,7 +615,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
                     PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
                 else
                     PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
-                PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD, KEYS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
+                PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
                                                           L.max_entries, zrows, vinit.row_bytes, watch);
                 return PL_OK;
             };
@@ -758,12 +759,15 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     return PL_OK;
 }
 
-template <int PD, typename R>
+// Whose keys hold no item (float calls; see Cfg::KW_ALONE): the same for whoever reads the workspace later.
+static bool batch_of_one(const Geom& g) { return g.batch == 1; }
+
+template <int PD, typename R, int KW>
 static int run_export(const Geom& g, const R* positions, const R* reference, const void* workspace,
                       const Layout& L, long long max_vertices, int16_t* vertex_keys,
                       int32_t* vertex_item, int32_t* pixel_vertex, R* pixel_weight,
                       cudaStream_t st) {
-    constexpr int KW = Cfg<PD>::KW, TP = Cfg<PD>::TP;
+    constexpr int TP = Cfg<PD>::TP;
     const unsigned char* ws = static_cast<const unsigned char*>(workspace);
     const Header* hdr = reinterpret_cast<const Header*>(ws);
     if (g.num_tiles == 0) return PL_OK;
@@ -773,7 +777,7 @@ static int run_export(const Geom& g, const R* positions, const R* reference, con
             reinterpret_cast<const R*>(ws + L.rec_w), reinterpret_cast<const u32*>(ws + L.list_ref),
             pixel_vertex, pixel_weight);
     if (vertex_keys || vertex_item)
-        export_vertices<PD><<<num_sms() * 4, 256, 0, st>>>(
+        export_vertices<PD, KW><<<num_sms() * 4, 256, 0, st>>>(
             hdr, reinterpret_cast<const Key<KW>*>(ws + L.vkeys), max_vertices, vertex_keys, vertex_item);
     PL_CUDA(cudaGetLastError());
     return PL_OK;
@@ -802,7 +806,7 @@ static int filter_common(const Geom& g, float* output, const float* input, const
     int rc = make_layout(L, g, pd, vd, max_entries, 4, mode == PL_MODE_DETERMINISTIC, with_sorted);
     if (rc != PL_OK) return rc;
     if (workspace_bytes < L.total) return PL_WORKSPACE_TOO_SMALL;
-#define CALL(P) run_filter<P>(g, output, input, positions, reference, vd, reverse, mode, workspace, L, st, phases)
+#define CALL(P) (batch_of_one(g) ? run_filter<P, Cfg<P>::KW_ALONE> : run_filter<P, Cfg<P>::KW>)(g, output, input, positions, reference, vd, reverse, mode, workspace, L, st, phases)
     PL_DISPATCH_PD(pd, CALL)
 #undef CALL
 }
@@ -1171,7 +1175,7 @@ int pl_export_lattice_f64(const void* workspace, const double* positions, const 
     Layout L;
     rc = make_layout(L, g, pd, vd, max_entries, 8);
     if (rc != PL_OK) return rc;
-#define CALL(P) run_export<P, double>(g, positions, reference, workspace, L, (long long)max_vertices, vertex_keys, \
+#define CALL(P) run_export<P, double, Cfg<P>::KW>(g, positions, reference, workspace, L, (long long)max_vertices, vertex_keys, \
                                       vertex_item, pixel_vertex, pixel_weight, (cudaStream_t)stream)
     PL_DISPATCH_PD(pd, CALL)
 #undef CALL
@@ -1364,7 +1368,7 @@ int pl_export_lattice(const void* workspace, const float* positions, const float
     Layout L;
     rc = make_layout(L, g, pd, vd, max_entries);
     if (rc != PL_OK) return rc;
-#define CALL(P) run_export<P, float>(g, positions, reference, workspace, L, (long long)max_vertices, vertex_keys, \
+#define CALL(P) (batch_of_one(g) ? run_export<P, float, Cfg<P>::KW_ALONE> : run_export<P, float, Cfg<P>::KW>)(g, positions, reference, workspace, L, (long long)max_vertices, vertex_keys, \
                                      vertex_item, pixel_vertex, pixel_weight, (cudaStream_t)stream)
     PL_DISPATCH_PD(pd, CALL)
 #undef CALL

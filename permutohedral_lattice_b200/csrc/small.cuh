@@ -23,12 +23,11 @@ __device__ __forceinline__ void cluster_sync() {
 
 // clear_table, insert_entries and link_neighbours.  What another CTA wrote in an earlier phase is read from L2.  A
 // table slot names the entry that created it throughout: its key in list_keys is older than this launch.
-template <int PD>
+template <int PD, int KW = Cfg<PD>::KW>
 __global__ void __cluster_dims__(SMALL_CTAS, 1, 1) __launch_bounds__(SMALL_THREADS)
-index_small(Header* hdr, u64* table, u32 max_log2, const Key<Cfg<PD>::KW>* __restrict__ list_keys, u32* list_ref,
-            u32* vid, Key<Cfg<PD>::KW>* vkeys, VertexInit vi, Watch watch) {
+index_small(Header* hdr, u64* table, u32 max_log2, const Key<KW>* __restrict__ list_keys, u32* list_ref,
+            u32* vid, Key<KW>* vkeys, VertexInit vi, Watch watch) {
     after_previous_kernel();
-    constexpr int KW = Cfg<PD>::KW;
     const u32 tid = blockIdx.x * SMALL_THREADS + threadIdx.x, threads = SMALL_CTAS * SMALL_THREADS;
     if (call_failed(hdr)) {   // the same answer in every CTA: nothing sets the status before the first barrier
         report_to(watch, hdr);
