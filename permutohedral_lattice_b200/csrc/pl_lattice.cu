@@ -516,13 +516,43 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
      : padded_vd(vd) == 32 ? launch_slice<PD_, 32>(__VA_ARGS__) \
                            : launch_slice<PD_, 0>(__VA_ARGS__))
 
-// Which calls take the one-cluster kernels of small.cuh, by the bounds the host knows.
-// RGB calls one after another, wide -> one cluster, us a call: 33x45, 573 entries 43 -> 34; 48x56, 806 entries 43 -> 36;
-// 8910 entries, all vertices, 59 -> 67; 16128 of them 73 -> 108: the two lines cross at about 6700 entries.  The blur
-// alone, all vertices: 8910 rows of one piece 58 -> 62, 16128 of them 73 -> 78, so one piece a thread at most.
-constexpr u64 SMALL_ENTRIES = 6144, SMALL_ITEMS = SMALL_CTAS * SMALL_THREADS;
-static bool small_index(const Layout& L) { return L.max_entries <= SMALL_ENTRIES; }
-static bool small_blur(const Layout& L, u32 vpr) { return L.max_entries * vpr <= SMALL_ITEMS; }
+// Which calls take the kernels of small.cuh, by the bounds the host knows.  The index as far as its shared memory goes: 3074 entries
+// 17.8 (one cluster on global memory) -> 9.4 us, 7017 entries 20.7 -> 17, as long as the three wide launches by then.
+static bool small_index(const Layout& L) { return L.max_entries <= SMALL_MAX_ENTRIES; }
+// A cluster for every 16 bytes of a row, as many as the GPU takes at once (two CTAs an SM while a thread has one vertex, else
+// one), or twice as many of the small ones.  Six passes, us, wide / in one launch, by the bound: 4096, 1 float4 a row 15 / 7, 3
+// float4 14 / 9; 12000, 1 float4 15 / 12; 30000, 6 float4 15 / 14.6, and five launches less for the host, which such calls
+// wait for: 2 x 100x100 x 21, forward + backward, 170 / 146 us.
+constexpr int SMALL_PIECES = 4;   // vertices a thread of blur_small, at most
+static bool small_blur(const Layout& L, u32 vpr) {
+    const u64 one_each = SMALL_CTAS * SMALL_THREADS;
+    return L.max_entries <= one_each ? vpr <= 64 : L.max_entries <= SMALL_PIECES * one_each && vpr <= 16;
+}
+template <int PD, int KW>
+static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
+                              const VertexInit& vinit, Watch watch, bool overlap, cudaStream_t st) {
+    const u32 entries = (u32)L.max_entries;
+    const size_t smem = SmallIndex<PD>::bytes(entries);
+    PL_TRY((ensure_dynamic_smem<index_small<PD, KW>>(smem)));
+    // a thread for every axis and vertex, up to 64 CTAs
+    const u32 ctas = std::max(8u, std::min(64u, (entries * (PD + 1) + SMALL_THREADS - 1) / SMALL_THREADS));
+    PL_CUDA(launch_kernel(overlap, index_small<PD, KW>, dim3(ctas), dim3(SMALL_THREADS), smem, st, hdr, list_keys, list_ref, vkeys, vinit, (u32)smem, watch));
+    return PL_OK;
+}
+template <typename V, int PIECES>
+static int launch_small_blur_as(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
+    const size_t smem = sizeof(V) * 2 * PIECES * SMALL_THREADS;
+    PL_TRY((ensure_dynamic_smem<blur_small<V, PIECES>>(smem)));
+    PL_LAUNCH_AFTER(OV_BLUR, (blur_small<V, PIECES>), SMALL_CTAS * vpr, SMALL_THREADS, smem, st, hdr, nbr, L.max_entries, v, vpr, axes, reverse);
+    return PL_OK;
+}
+template <typename V>
+static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
+    const u64 pieces = (L.max_entries + SMALL_CTAS * SMALL_THREADS - 1) / (SMALL_CTAS * SMALL_THREADS);   // a thread
+    return pieces <= 1   ? launch_small_blur_as<V, 1>(hdr, nbr, L, v, vpr, axes, reverse, st)
+           : pieces <= 2 ? launch_small_blur_as<V, 2>(hdr, nbr, L, v, vpr, axes, reverse, st)
+                         : launch_small_blur_as<V, SMALL_PIECES>(hdr, nbr, L, v, vpr, axes, reverse, st);
+}
 
 enum { PH_BUILD = 1, PH_APPLY = 2 };   // halves of a call: lattice structure / values through it
 
@@ -601,7 +631,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         const bool small = !use_direct && small_index(L);
         PL_COUNT_LAUNCHES(small ? 2 : 4);   // build_tiles and the launches of the index stage
         if (small) {
-            PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (index_small<PD, KW>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, watch);
+            PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, (phases & PH_APPLY) != 0, st)));
         } else if (!use_direct) {
             // the value rows are zeroed by the link launch, whose lookups leave the memory system idle
             void* zrows = vinit.rows;
@@ -656,9 +686,8 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     float* dst = v1;
     const u32 qpr = (u32)padded_vd(vd) / 4;
     if (small_blur(L, qpr)) {
-        PL_LAUNCH_AFTER(OV_BLUR, (blur_small<float4>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, nbr, L.max_entries, reinterpret_cast<float4*>(v0), reinterpret_cast<float4*>(v1), qpr, PD + 1, reverse);
+        PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, st));
         PL_COUNT_LAUNCHES(1);
-        if (PD % 2 == 0) src = v1;   // an odd number of passes
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * L.max_entries * 2;
@@ -730,7 +759,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     }
     const bool small = !use_direct && small_index(L);
     if (small) {
-        PL_LAUNCH_AFTER(OV_CLEAR, (index_small<PD>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, watch);
+        PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, true, st)));
     } else if (!use_direct) {
         PL_LAUNCH_AFTER(OV_CLEAR, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         if constexpr (Cfg<PD>::KEY_SLOTS)
@@ -746,8 +775,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* dst = v1;
     const bool one_blur = small_blur(L, (u32)vp / 2);
     if (one_blur) {
-        PL_LAUNCH_AFTER(OV_BLUR, (blur_small<double2>), SMALL_CTAS, SMALL_THREADS, 0, st, hdr, nbr, L.max_entries, reinterpret_cast<double2*>(v0), reinterpret_cast<double2*>(v1), (u32)vp / 2, PD + 1, reverse);
-        if (PD % 2 == 0) src = v1;   // an odd number of passes
+        PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<double2*>(v0), (u32)vp / 2, PD + 1, reverse, st));
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);

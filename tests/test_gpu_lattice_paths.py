@@ -133,8 +133,8 @@ def test_calls_of_several_widths_from_several_threads(dtype, gpu):
 
 @pytest.mark.parametrize("pd,n", [(1, 8200), (2, 5470), (3, 4100), (5, 2735), (8, 1825), (16, 970)])
 def test_small_lattices_give_the_bits_of_wide_ones(pd, n, gpu, oracle):
-    """A bound of 6144 entries is the largest that takes the one-cluster index, and with it rows of one quad take
-    the one-cluster blur (8192 quads), wider ones the passes one by one.  Deterministic sums make small and wide comparable."""
+    """A bound of 6144 entries takes the index and the blur of small lattices, the worst case the wide index and, beyond its
+    limits, the passes one by one.  Deterministic sums make small and wide comparable."""
     import torch
     import permutohedral_lattice_b200 as plb
     rng = np.random.default_rng(79)
