@@ -183,9 +183,9 @@ static cudaError_t launch_kernel(bool overlap, void (*kernel)(Params...), dim3 g
 // slower at 16 items: link_neighbours
 // after insert_entries (index stage 0.175 -> 0.181 ms; in small calls it gains or loses 0.5 %) and the first
 // blur pass after the splat (2.09).
-enum { OV_BLUR = 1, OV_INSERT = 2, OV_SPLAT = 4, OV_BLUR0 = 8, OV_SLICE = 16, OV_CLEAR = 32, OV_LINK = 64 };
+enum { OV_BLUR = 1, OV_INSERT = 2, OV_SPLAT = 4, OV_BLUR0 = 8, OV_SLICE = 16, OV_CLEAR = 32, OV_LINK = 64, OV_BUILD = 128 };
 #ifndef PL_OVERLAP
-#define PL_OVERLAP (OV_BLUR | OV_INSERT | OV_SPLAT | OV_SLICE | OV_CLEAR)
+#define PL_OVERLAP (OV_BLUR | OV_INSERT | OV_SPLAT | OV_SLICE | OV_CLEAR | OV_BUILD)
 #endif
 #define PL_LAUNCH_AFTER(which, kernel, grid, block, smem, st, ...) \
     PL_CUDA(launch_kernel((PL_OVERLAP & (which)) != 0, kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
@@ -554,6 +554,13 @@ static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L,
                          : launch_small_blur_as<V, SMALL_PIECES>(hdr, nbr, L, v, vpr, axes, reverse, st);
 }
 
+// The header's counters and, in calls that keep one, the sketch behind it.
+static int clear_header_of(Header* hdr, int sketch_shift, cudaStream_t st) {
+    PL_LAUNCH((clear_header), 1, 256, 0, st, hdr, (u32)((sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header)) / 16));
+    PL_COUNT_LAUNCHES(1);
+    return PL_OK;
+}
+
 enum { PH_BUILD = 1, PH_APPLY = 2 };   // halves of a call: lattice structure / values through it
 
 // KW: words of a key.
@@ -583,7 +590,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     cudaEvent_t* ev = g_stage_events;
     g_stage_events = nullptr;
     if (ev) PL_CUDA(cudaEventRecord(ev[0], st));
-    if (phases & PH_BUILD) PL_CUDA(cudaMemsetAsync(hdr, 0, sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header), st));
+    if (phases & PH_BUILD) PL_TRY(clear_header_of(hdr, sketch_shift, st));
     if (g.num_tiles == 0) return PL_OK;
     const Watch watch = (phases & PH_BUILD) ? take_watch(st) : Watch{nullptr, 0u};
 
@@ -598,13 +605,15 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     // calls with large tables 4-25 % (pd 16: 30 -> 37 ms)
     const bool small_table = L.index_words <= (1ull << 24);
     if (phases & PH_BUILD) {
+        // (beyond pd 8 the build has to wait for the header at its start, and launched beside it took 112 -> 128 us)
+        constexpr int beside_clear = Cfg<PD>::COMPACT ? 0 : OV_BUILD;
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
         if (phases & PH_APPLY) {
-            PL_LAUNCH((build_tiles<PD, float, false, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr,
+            PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, false, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr,
                                                                          tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         } else {
             PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, true, KW>>(Cfg<PD>::build_smem(true))));
-            PL_LAUNCH((build_tiles<PD, float, true, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
+            PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, true, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[1], st));
@@ -724,7 +733,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* v1 = reinterpret_cast<double*>(ws + L.v1);
 
     const int sketch_shift = sketch_shift_of(L.max_entries);
-    PL_CUDA(cudaMemsetAsync(hdr, 0, sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header), st));
+    PL_TRY(clear_header_of(hdr, sketch_shift, st));
     if (g.num_tiles == 0) return PL_OK;
     const Watch watch = take_watch(st);
     PL_TRY((ensure_dynamic_smem<build_tiles<PD, double>>(Cfg<PD>::build_smem(false))));
@@ -736,7 +745,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     const int vp = padded_vd_f64(vd);
     const bool small_table = L.index_words <= (1ull << 24);   // (as for float)
 
-    PL_LAUNCH((build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
+    PL_LAUNCH_AFTER(Cfg<PD>::COMPACT ? 0 : OV_BUILD, (build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
     // spatial-only calls index their vertices directly, as the float calls do (the key bounds hold for
     // either arithmetic: the margin is far wider than any rounding)
     Direct direct;
