@@ -207,6 +207,18 @@ int pl_crf_update_f32(float* q_out, const float* unaries, const float* q_bilater
                       const float* compatibility, float bilateral_weight, float spatial_weight,
                       int64_t n_points, int n_labels, void* stream);
 
+/* One mean-field step of a CRF with the Potts model through two lattices that pl_lattice_build_f32 left in their
+ * workspaces, `bilateral` (reference image of n_reference_channels) and spatial-only, of the same batch and spatial_dims and
+ * built for n_labels + 1 values at least: both filters of q and pl_crf_update_f32 without a compatibility matrix, the same
+ * values up to the order of the sums, in fewer launches and without the filtered distributions in memory.  *_entries: the
+ * max_entries of each build.  PL_UNSUPPORTED_DIMS: not two spatial dimensions with three reference channels, fewer
+ * than 4 or more than 31 labels, or more tiles than a grid of both lattices holds; the two applies and pl_crf_update_f32
+ * take those.  A lattice that failed fills q_out with NaN.  No counterpart in the reference. */
+int pl_crf_step_f32(float* q_out, const float* q, const float* unaries, float bilateral_weight, float spatial_weight,
+                    int n_labels, int batch, int n_spatial_dims, const int* spatial_dims, int n_reference_channels,
+                    void* bilateral_workspace, size_t bilateral_bytes, int64_t bilateral_entries,
+                    void* spatial_workspace, size_t spatial_bytes, int64_t spatial_entries, void* stream);
+
 /* Number of kernels the library has launched in this process so far (filter stages and pl_crf_update_f32;
  * memsets, copies and event records are not counted).  The difference across a region is the number
  * of kernels that region launched.  No counterpart in the reference. */

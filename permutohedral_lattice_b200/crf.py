@@ -13,12 +13,13 @@ guide image I[B, *S, R]:
 
 Both lattices depend on the image only: they are built once (`Lattice`) and applied in every iteration.
 Everything after the two filters (weights, compatibility product, unaries, softmax) is one fused kernel,
-pl_crf_update_f32: one read of Qb, Qs and U and one write of Q per iteration.
+pl_crf_update_f32: one read of Qb, Qs and U and one write of Q per iteration.  For the Potts model on RGB images with 4 to 31
+labels the whole iteration is pl_crf_step_f32: each stage of both filters in one launch, the update in the slice.
 """
 import torch
 
 from . import capi
-from .lattice_filter import Lattice, _stream_handle
+from .lattice_filter import Lattice, _OnDevice, _check_tensor, _float32_only, _stream_handle
 
 
 class DenseCRF:
@@ -43,6 +44,10 @@ class DenseCRF:
         if unaries.dtype != torch.float32 or not unaries.is_cuda:
             raise TypeError("unaries must be a float32 CUDA tensor")
         unaries = unaries.contiguous()
+        if self.compatibility is None:
+            out = self._fused_step(q, unaries)
+            if out is not None:
+                return out
         qb = self.bilateral.apply(q)
         qs = self.spatial.apply(q)
         out = torch.empty_like(qb)
@@ -52,6 +57,29 @@ class DenseCRF:
                 out.data_ptr(), unaries.data_ptr(), qb.data_ptr(), qs.data_ptr(),
                 0 if self.compatibility is None else self.compatibility.data_ptr(), self.bilateral_weight,
                 self.spatial_weight, n_points, self.n_labels, _stream_handle(out.device)), "pl_crf_update_f32")
+        return out
+
+    def _fused_step(self, q, unaries):
+        """The whole step by pl_crf_step_f32, or None where that takes another number of dimensions or labels."""
+        a, s = self.bilateral, self.spatial
+        call = a.call
+        if a.workspace is None or s.workspace is None:
+            return None
+        _check_tensor(q, "input_image")
+        _float32_only(q, "Lattice (build once, apply many times)")
+        if tuple(q.shape[:-1]) != (call.batch,) + tuple(call.sdims):
+            raise ValueError("input_image does not have the lattice's batch and spatial shape")
+        q = q.contiguous()
+        out = torch.empty_like(q)
+        with _OnDevice(a.device):
+            rc = capi.lib().pl_crf_step_f32(
+                out.data_ptr(), q.data_ptr(), unaries.data_ptr(), self.bilateral_weight, self.spatial_weight,
+                self.n_labels, call.batch, len(call.sdims), call.c_sdims, call.r, a.workspace.data_ptr(),
+                a.workspace.numel(), a.max_entries, s.workspace.data_ptr(), s.workspace.numel(), s.max_entries,
+                _stream_handle(a.device))
+        if rc == capi.PL_UNSUPPORTED_DIMS:
+            return None
+        capi.check(rc, "pl_crf_step_f32")
         return out
 
     def infer(self, unaries, iterations=5):

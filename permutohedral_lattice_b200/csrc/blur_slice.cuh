@@ -45,17 +45,16 @@ __device__ __forceinline__ double2 mix_rows(double2 a, double2 b, double2 c) {
 }
 
 template <typename V>
-__global__ void __launch_bounds__(256, 8)
-blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst,
-          u32 vpr /* V per row */) {
+__device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src,
+                                          V* __restrict__ dst, u32 vpr /* V per row */, u32 block, u32 blocks) {
     // Passes after the first overlap the tail of the pass before (see after_previous_kernel).  The vertex count
     // and the neighbour table are older than any blur pass: a thread's first pair of neighbours is fetched
     // before the wait, so that one of the two dependent loads of its first row is off the critical path.
     const u32 M = hdr->num_vertices;
     const u64 items = (u64)M * vpr;
     const int2* __restrict__ nb = reinterpret_cast<const int2*>(nbr_axis);
-    const u32 stride = gridDim.x * blockDim.x, dv = stride / vpr, dj = stride - dv * vpr;
-    u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+    const u32 stride = blocks * blockDim.x, dv = stride / vpr, dj = stride - dv * vpr;
+    u64 e = (u64)block * blockDim.x + threadIdx.x;
     u32 v = (u32)e / vpr, j = (u32)e - v * vpr;   // item e is V j of vertex v's row (the first e fits 32 bits)
     int2 n = (v < M) ? __ldg(nb + v) : make_int2(-1, -1);
     after_previous_kernel();
@@ -75,6 +74,11 @@ blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restri
         dst[e] = mix_rows(a, b, c);
         e += stride;
     }
+}
+template <typename V>
+__global__ void __launch_bounds__(256, 8)
+blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst, u32 vpr) {
+    blur_rows<V>(hdr, nbr_axis, src, dst, vpr, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -112,6 +116,71 @@ struct SliceFast {
     static constexpr int CTAS = TP != 256 ? (VP > 24 ? 6 : 8) : SIX ? 6 : NEED <= 36 ? 5 : NEED <= 52 ? 4 : 3;
     static constexpr int ROWS_BYTES = (SIX ? 35 : 40) * 1024;   // of cached rows: so many CTAs fit the shared memory too
 };
+
+// The tile's vertex rows, `nrows` of them, on their way to shared memory.  CH copies per thread and trip: first the vertex
+// numbers of all CH rows (independent loads, in flight together with the record loads before them), then the asynchronous
+// copies that depend on them; interleaving them one by one would put a full memory latency between consecutive copies.
+template <int PD, int VP>
+__device__ __forceinline__ void stage_rows(float* rows_s, int nrows, const u32* __restrict__ list_ref, int base, const float4* v4) {
+    constexpr int TP = Cfg<PD>::TP, QPR = VP / 4, RS = SliceFast<PD, VP>::RS, CH = 8;
+    const int total = nrows * QPR;
+    for (int i0 = threadIdx.x; i0 < total; i0 += CH * TP) {
+        u32 vtx[CH];
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            const int i = i0 + c * TP;
+            vtx[c] = (i < total) ? list_ref[base + i / QPR] : 0u;
+        }
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            const int i = i0 + c * TP;
+            if (i < total) {
+                const int lrow = i / QPR, q = i - lrow * QPR;
+                cp_async16(rows_s + lrow * RS + 4 * q, v4 + (size_t)vtx[c] * QPR + q);
+            }
+        }
+    }
+}
+
+// A point's row: its pd + 1 vertex rows, weighted.
+template <int PD, int VP>
+__device__ __forceinline__ void mix_rows_of_point(float (&acc)[VP], bool valid, const int (&l)[PD + 1], const float (&w)[PD + 1],
+                                                  const float* rows_s, int nrows, int cnt, int rows_cap,
+                                                  const u32* __restrict__ list_ref, int base, const float4* v4) {
+    constexpr int QPR = VP / 4, RS = SliceFast<PD, VP>::RS;
+#pragma unroll
+    for (int j = 0; j < VP; j++) acc[j] = 0.f;
+    if (valid && cnt <= rows_cap) {
+        // every row of the tile is cached (the usual case): plain shared-memory reads
+#pragma unroll
+        for (int r = 0; r <= PD; r++) {
+            const float4* row = reinterpret_cast<const float4*>(rows_s + l[r] * RS);
+#pragma unroll
+            for (int q = 0; q < QPR; q++) {
+                const float4 x = row[q];
+                acc[4 * q] = PL_FADD(acc[4 * q], PL_FMUL(w[r], x.x));
+                acc[4 * q + 1] = PL_FADD(acc[4 * q + 1], PL_FMUL(w[r], x.y));
+                acc[4 * q + 2] = PL_FADD(acc[4 * q + 2], PL_FMUL(w[r], x.z));
+                acc[4 * q + 3] = PL_FADD(acc[4 * q + 3], PL_FMUL(w[r], x.w));
+            }
+        }
+    } else if (valid) {
+        // a tile with more entries than the cache holds: the rest comes straight from global memory
+#pragma unroll
+        for (int r = 0; r <= PD; r++) {
+            const float4* row = (l[r] < nrows) ? reinterpret_cast<const float4*>(rows_s + l[r] * RS)
+                                               : v4 + (size_t)list_ref[base + l[r]] * QPR;
+#pragma unroll
+            for (int q = 0; q < QPR; q++) {
+                const float4 x = row[q];
+                acc[4 * q] = PL_FADD(acc[4 * q], PL_FMUL(w[r], x.x));
+                acc[4 * q + 1] = PL_FADD(acc[4 * q + 1], PL_FMUL(w[r], x.y));
+                acc[4 * q + 2] = PL_FADD(acc[4 * q + 2], PL_FMUL(w[r], x.z));
+                acc[4 * q + 3] = PL_FADD(acc[4 * q + 3], PL_FMUL(w[r], x.w));
+            }
+        }
+    }
+}
 
 // CT: the channels where they are fixed at compile time, else 0 (VP - 4 <= C < VP, a few registers more).
 template <int PD, int VP, int CT>
@@ -154,64 +223,11 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
         w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
     }
     wait_for_previous_kernel();
-    // Row staging, CH copies per thread and trip: first the vertex numbers of all CH rows (independent
-    // loads, in flight together with the record loads above), then the asynchronous copies that depend on
-    // them; interleaving them one by one would put a full memory latency between consecutive copies.
-    {
-        constexpr int CH = 8;
-        const int total = nrows * QPR;
-        for (int i0 = tid; i0 < total; i0 += CH * TP) {
-            u32 vtx[CH];
-#pragma unroll
-            for (int c = 0; c < CH; c++) {
-                const int i = i0 + c * TP;
-                vtx[c] = (i < total) ? list_ref[base + i / QPR] : 0u;
-            }
-#pragma unroll
-            for (int c = 0; c < CH; c++) {
-                const int i = i0 + c * TP;
-                if (i < total) {
-                    const int lrow = i / QPR, q = i - lrow * QPR;
-                    cp_async16(rows_s + lrow * RS + 4 * q, v4 + (size_t)vtx[c] * QPR + q);
-                }
-            }
-        }
-    }
+    stage_rows<PD, VP>(rows_s, nrows, list_ref, base, v4);
     cp_async_wait_all();
     __syncthreads();
     float acc[VP];
-#pragma unroll
-    for (int j = 0; j < VP; j++) acc[j] = 0.f;
-    if (valid && cnt <= rows_cap) {
-        // every row of the tile is cached (the usual case): plain shared-memory reads
-#pragma unroll
-        for (int r = 0; r <= PD; r++) {
-            const float4* row = reinterpret_cast<const float4*>(rows_s + l[r] * RS);
-#pragma unroll
-            for (int q = 0; q < QPR; q++) {
-                const float4 x = row[q];
-                acc[4 * q] = PL_FADD(acc[4 * q], PL_FMUL(w[r], x.x));
-                acc[4 * q + 1] = PL_FADD(acc[4 * q + 1], PL_FMUL(w[r], x.y));
-                acc[4 * q + 2] = PL_FADD(acc[4 * q + 2], PL_FMUL(w[r], x.z));
-                acc[4 * q + 3] = PL_FADD(acc[4 * q + 3], PL_FMUL(w[r], x.w));
-            }
-        }
-    } else if (valid) {
-        // a tile with more entries than the cache holds: the rest comes straight from global memory
-#pragma unroll
-        for (int r = 0; r <= PD; r++) {
-            const float4* row = (l[r] < nrows) ? reinterpret_cast<const float4*>(rows_s + l[r] * RS)
-                                               : v4 + (size_t)list_ref[base + l[r]] * QPR;
-#pragma unroll
-            for (int q = 0; q < QPR; q++) {
-                const float4 x = row[q];
-                acc[4 * q] = PL_FADD(acc[4 * q], PL_FMUL(w[r], x.x));
-                acc[4 * q + 1] = PL_FADD(acc[4 * q + 1], PL_FMUL(w[r], x.y));
-                acc[4 * q + 2] = PL_FADD(acc[4 * q + 2], PL_FMUL(w[r], x.z));
-                acc[4 * q + 3] = PL_FADD(acc[4 * q + 3], PL_FMUL(w[r], x.w));
-            }
-        }
-    }
+    mix_rows_of_point<PD, VP>(acc, valid, l, w, rows_s, nrows, cnt, rows_cap, list_ref, base, v4);
     __syncthreads();   // every cached row has been read: the output block may overwrite them
     if (valid) {
         const int last = C - (VP - 4);   // channels in the row's last quad; the next one is the homogeneous channel

@@ -242,12 +242,11 @@ __host__ __device__ constexpr u64 coord_ones(int j) {
 struct TilePos {
     int tile, item, o, ty, tx;
 };
-__device__ __forceinline__ TilePos this_tile(const Geom& g) {
+__device__ __forceinline__ TilePos tile_at(const Geom& g, int x, int z) {   // CTA (x, blockIdx.y, z)
     TilePos t;
     if (g.grid3) {
-        t.tx = blockIdx.x;
+        t.tx = x;
         t.ty = blockIdx.y;
-        const int z = blockIdx.z;
         if (g.outer == 1) {
             t.item = z;
             t.o = 0;
@@ -257,7 +256,7 @@ __device__ __forceinline__ TilePos this_tile(const Geom& g) {
         }
         t.tile = (z * g.tiles_y + t.ty) * g.tiles_x + t.tx;
     } else {
-        t.tile = blockIdx.x;
+        t.tile = x;
         t.item = t.tile / g.tiles_per_item;
         int r = t.tile - t.item * g.tiles_per_item;
         const int per_plane = g.tiles_x * g.tiles_y;
@@ -268,6 +267,8 @@ __device__ __forceinline__ TilePos this_tile(const Geom& g) {
     }
     return t;
 }
+
+__device__ __forceinline__ TilePos this_tile(const Geom& g) { return tile_at(g, blockIdx.x, blockIdx.z); }
 
 // Point handled by thread `tid` of the tile: item, point index inside the item, validity; the long
 // form also gives the point's position (outer index, row, column).

@@ -799,6 +799,86 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
 // Whose keys hold no item (float calls; see Cfg::KW_ALONE): the same for whoever reads the workspace later.
 static bool batch_of_one(const Geom& g) { return g.batch == 1; }
 
+// A mean-field step through two kept lattices (crf.cuh).
+static LatticeRows lattice_rows(void* workspace, const Layout& L) {
+    unsigned char* ws = static_cast<unsigned char*>(workspace);
+    LatticeRows l;
+    l.hdr = reinterpret_cast<Header*>(ws);
+    l.tile_info = reinterpret_cast<const int2*>(ws + L.tile_info);
+    l.rec = reinterpret_cast<const u16*>(ws + L.rec);
+    l.rec_w = reinterpret_cast<const float*>(ws + L.rec_w);
+    l.srec = reinterpret_cast<const uint2*>(ws + L.srec);
+    l.list_ref = reinterpret_cast<const u32*>(ws + L.list_ref);
+    l.nbr = reinterpret_cast<const int*>(ws + L.nbr);
+    l.max_entries = L.max_entries;
+    l.v0 = reinterpret_cast<float*>(ws + L.v0);
+    l.v1 = reinterpret_cast<float*>(ws + L.v1);
+    return l;
+}
+template <int PDA, int PDS, int VD>
+static int launch_crf_splat(const Geom& g, const float* q, const LatticeRows& a, const LatticeRows& s, int vd, cudaStream_t st) {
+    const size_t smem = std::max(SplatRows<PDA, VD, true>::bytes(vd), SplatRows<PDS, VD, true>::bytes(vd));
+    PL_TRY((ensure_dynamic_smem<crf_splat<PDA, PDS, VD>>(smem, true)));
+    dim3 grid = tile_grid(g);
+    (g.grid3 ? grid.z : grid.x) *= 2;
+    PL_LAUNCH_AFTER(OV_SPLAT, (crf_splat<PDA, PDS, VD>), grid, Cfg<PDA>::TP, smem, st, g, q, a, s, vd, bulk_staging_ok(g, q, vd) ? 1 : 0);
+    return PL_OK;
+}
+template <int PDA, int PDS, int VP, int CT = 0>
+static int launch_crf_slices(const Geom& g, float* q_out, const float* unaries, const LatticeRows& a, const LatticeRows& s,
+                             const float* va, const float* vs, float wa, float ws, int labels, cudaStream_t st) {
+    const size_t smem = CrfSlices<PDA, PDS, VP>::bytes(labels);
+    PL_TRY((ensure_dynamic_smem<crf_slices<PDA, PDS, VP, CT>>(smem)));
+    // (an even number of labels is spread to an odd stride, which a bulk copy cannot do)
+    const bool bulk_in = (labels & 1) && bulk_rows_ok(g, unaries, labels), bulk_out = bulk_rows_ok(g, q_out, labels);
+    PL_LAUNCH_AFTER(OV_SLICE, (crf_slices<PDA, PDS, VP, CT>), tile_grid(g), Cfg<PDA>::TP, smem, st, g, q_out, unaries, a, s, va, vs, wa, ws, labels, bulk_in ? 1 : 0, bulk_out ? 1 : 0);
+    return PL_OK;
+}
+template <int PDA, int PDS>
+static int run_crf_step(const Geom& g, float* q_out, const float* q, const float* unaries, float wa, float wsp, int labels,
+                        void* ws_a, const Layout& LA, void* ws_s, const Layout& LS, cudaStream_t st) {
+    const LatticeRows a = lattice_rows(ws_a, LA), s = lattice_rows(ws_s, LS);
+    const int vd = labels + 1, vp = padded_vd(vd), wide = num_sms() * 8;
+    const u32 quads = (u32)vp / 4;
+    PL_LAUNCH_AFTER(OV_CLEAR, (crf_zero_rows), dim3(wide / 2, 2), 256, 0, st, a, s, quads);
+    PL_TRY((vd == 22 ? launch_crf_splat<PDA, PDS, 22>(g, q, a, s, vd, st) : launch_crf_splat<PDA, PDS, 0>(g, q, a, s, vd, st)));
+    // small lattices have all their passes in one launch each; else a launch a pass, both as long as S has some left
+    const bool small_a = small_blur(LA, quads), small_s = small_blur(LS, quads);
+    const float *va = a.v0, *vs = s.v0;
+    int launches = 3;
+    if (small_s) {
+        PL_TRY(launch_small_blur(s.hdr, s.nbr, LS, reinterpret_cast<float4*>(s.v0), quads, PDS + 1, 0, st));
+        launches++;
+    }
+    if (small_a) {
+        PL_TRY(launch_small_blur(a.hdr, a.nbr, LA, reinterpret_cast<float4*>(a.v0), quads, PDA + 1, 0, st));
+        launches++;
+    }
+    for (int step = 0; step <= std::max(PDA, PDS); step++) {
+        const bool pass_a = !small_a && step <= PDA, pass_s = !small_s && step <= PDS;
+        if (!pass_a && !pass_s) continue;
+        const bool first = step == 0 && !small_a && !small_s;
+        const LatticeRows& one = pass_a ? a : s;
+        PL_LAUNCH_AFTER(first ? OV_BLUR0 : OV_BLUR, (crf_blur), dim3(pass_a && pass_s ? wide / 2 : wide, pass_a && pass_s ? 2 : 1), 256, 0, st, one, s, step, quads);
+        launches++;
+        if (pass_a) va = (step & 1) ? a.v0 : a.v1;
+        if (pass_s) vs = (step & 1) ? s.v0 : s.v1;
+    }
+    PL_COUNT_LAUNCHES(launches);
+#define PL_CRF_SLICES(VP_, ...) launch_crf_slices<PDA, PDS, VP_, ##__VA_ARGS__>(g, q_out, unaries, a, s, va, vs, wa, wsp, labels, st)
+    PL_TRY((labels == 21 ? PL_CRF_SLICES(24, 21)
+            : vp == 8    ? PL_CRF_SLICES(8)
+            : vp == 12   ? PL_CRF_SLICES(12)
+            : vp == 16   ? PL_CRF_SLICES(16)
+            : vp == 20   ? PL_CRF_SLICES(20)
+            : vp == 24   ? PL_CRF_SLICES(24)
+            : vp == 28   ? PL_CRF_SLICES(28)
+                         : PL_CRF_SLICES(32)));
+#undef PL_CRF_SLICES
+    PL_CUDA(cudaGetLastError());
+    return PL_OK;
+}
+
 template <int PD, typename R, int KW>
 static int run_export(const Geom& g, const R* positions, const R* reference, const void* workspace,
                       const Layout& L, long long max_vertices, int16_t* vertex_keys,
@@ -1216,6 +1296,35 @@ int pl_export_lattice_f64(const void* workspace, const double* positions, const 
                                       vertex_item, pixel_vertex, pixel_weight, (cudaStream_t)stream)
     PL_DISPATCH_PD(pd, CALL)
 #undef CALL
+}
+
+int pl_crf_step_f32(float* q_out, const float* q, const float* unaries, float bilateral_weight, float spatial_weight,
+                    int n_labels, int batch, int n_spatial_dims, const int* spatial_dims, int n_reference_channels,
+                    void* bilateral_workspace, size_t bilateral_bytes, int64_t bilateral_entries, void* spatial_workspace,
+                    size_t spatial_bytes, int64_t spatial_entries, void* stream) {
+    if (n_labels < 1 || batch < 0 || batch > 65535 || n_spatial_dims < 1 || n_spatial_dims > MAX_SDIMS || !spatial_dims ||
+        n_reference_channels < 0)
+        return PL_INVALID_ARGUMENT;
+    if (n_spatial_dims != 2 || n_reference_channels != 3 || n_labels < 4 || n_labels > 31) return PL_UNSUPPORTED_DIMS;
+    const int pda = n_spatial_dims + n_reference_channels, pds = n_spatial_dims, vd = n_labels + 1;
+    long long n = 1;
+    for (int i = 0; i < n_spatial_dims; i++) {
+        if (spatial_dims[i] < 0) return PL_INVALID_ARGUMENT;
+        n *= spatial_dims[i];
+        if (n > 0x7FFFFFFFll) return PL_INVALID_ARGUMENT;
+    }
+    if (batch == 0 || n == 0) return PL_OK;
+    if (!q_out || !q || !unaries || !bilateral_workspace || !spatial_workspace) return PL_INVALID_ARGUMENT;
+    Geom g;
+    PL_TRY(make_geom(g, batch, (int)n, pda, n_spatial_dims, spatial_dims, n_reference_channels, 1.f, 1.f, false));
+    const dim3 grid = tile_grid(g);
+    if (g.grid3 ? grid.z > 32767u : grid.x > 0x3FFFFFFFu) return PL_UNSUPPORTED_DIMS;   // twice as many in one launch
+    Layout LA, LS;
+    PL_TRY(make_layout(LA, g, pda, vd, bilateral_entries));
+    PL_TRY(make_layout(LS, g, pds, vd, spatial_entries));
+    if (bilateral_bytes < LA.total || spatial_bytes < LS.total) return PL_WORKSPACE_TOO_SMALL;
+    return run_crf_step<5, 2>(g, q_out, q, unaries, bilateral_weight, spatial_weight, n_labels, bilateral_workspace, LA,
+                              spatial_workspace, LS, (cudaStream_t)stream);
 }
 
 int pl_crf_update_f32(float* q_out, const float* unaries, const float* q_bilateral, const float* q_spatial,

@@ -539,13 +539,11 @@ __device__ __forceinline__ void splat_wide_columns(const Geom& g, const TilePos&
     }
 }
 
-// Five CTAs per SM (47-48 registers, no spills; with the sort's counters the five CTAs take nearly all of an
-// SM's shared memory): 4 % faster than four at 16 items, and 2048 tiles (two items) take three waves, not four.
 template <int PD, int VD, bool PRE, typename Sum, typename V>
-__global__ void __launch_bounds__(Cfg<PD>::TP, std::is_same<Sum, FloatSum>::value ? 5 : 4)
-splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
-                 const u16* __restrict__ rec, const float* __restrict__ rec_w, const uint2* __restrict__ srec,
-                 const u32* __restrict__ list_ref, V* __restrict__ v0, int vd, int bulk_ok) {
+__device__ __forceinline__ void splat_rows(const Geom& g, const TilePos& tpos, const float* __restrict__ input, Header* hdr,
+                                           const int2* __restrict__ tile_info, const u16* __restrict__ rec,
+                                           const float* __restrict__ rec_w, const uint2* __restrict__ srec,
+                                           const u32* __restrict__ list_ref, V* __restrict__ v0, int vd, int bulk_ok) {
     // Launched to overlap the tail of the kernel before it (link_neighbours, or zero_rows in an apply): all
     // that the staging and the sort read (the input, the records and tile ranges of build_tiles, whose
     // failures are final by now) is older than that kernel, so they run before the wait; the window loop,
@@ -564,7 +562,6 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
         wait_for_previous_kernel();
         return;
     }
-    const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
     const int base = info.x, nloc = info.y;
@@ -760,6 +757,16 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
             if constexpr (ONE) break;
         }
     }
+}
+
+// Five CTAs per SM (47-48 registers, no spills; with the sort's counters the five CTAs take nearly all of an
+// SM's shared memory): 4 % faster than four at 16 items, and 2048 tiles (two items) take three waves, not four.
+template <int PD, int VD, bool PRE, typename Sum, typename V>
+__global__ void __launch_bounds__(Cfg<PD>::TP, std::is_same<Sum, FloatSum>::value ? 5 : 4)
+splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int2* __restrict__ tile_info,
+                 const u16* __restrict__ rec, const float* __restrict__ rec_w, const uint2* __restrict__ srec,
+                 const u32* __restrict__ list_ref, V* __restrict__ v0, int vd, int bulk_ok) {
+    splat_rows<PD, VD, PRE, Sum, V>(g, this_tile(g), input, hdr, tile_info, rec, rec_w, srec, list_ref, v0, vd, bulk_ok);
 }
 
 // ---------------------------------------------------------------------------------------------
