@@ -142,15 +142,18 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
 }
 
 // A tile with few entries for its splats (a volume, a smooth guide): points next to one another mostly share their
-// vertices, so that walking down a column of COLUMN points meets about as few runs as the sorted list cut into windows
-// does, and needs no sort.  One thread a column and remainder; nothing goes through shared memory: a point's row is read
-// PD + 1 times, from L1 after the first, neighbouring threads on neighbouring points.
+// vertices, so that walking down a piece of a column of points meets about as few runs as the sorted list cut into windows
+// does, and needs no sort.  One thread a piece and remainder; nothing goes through shared memory: a point's row is read
+// PD + 1 times, from L1 after the first, neighbouring threads on neighbouring points.  Sixteen points are cut into as many
+// pieces as give every thread one (5, 4 and 3 with pd 2, 3 and 4).
 // Bound by the latency of its loads (most stalls are for them; its reductions are none, L2 is at 34 %).  Two volumes of
-// 111x128x120 points, 20 splats an entry: 106 -> 83 us (the sort kept the LSU pipe at 82 %).
+// 111x128x120 points, 20 splats an entry: sorted 106 us (LSU pipe at 82 %), in columns of eight points, which left 3 of 8 warps
+// without work, 87, so 83.  us a call, eight points / so: 16 x 512x512 x 1 without a guide 208 / 186, x 3 198 / 189; 96x128x128 x
+// 1 without a guide, forward + backward, 207 / 200.  (The figures below are those of eight points.)
 // Where (us a splat, columns / sorted): rows of more than one float4 from 2 pd splats an entry on (8 x 512x512, pd 2,
 // 21 channels, 4.8 splats 95 / 110, 14.7 splats 76 / 98); narrow ones as NarrowColumns says.  pd 5, us a call: 8
 // splats an entry 201 / 197, 36 splats 158 / 138: up to pd 4.  Tiles of points in one dimension, which are all there are with pd 1, have no columns.
-constexpr int COLUMN = 8;
+constexpr int COLUMN = 8;   // points of a column, wide rows
 template <int PD>
 __device__ __forceinline__ bool in_columns(const Geom& g, int entries, int least) {   // least: splats an entry
     return g.TX <= 16 && least * entries <= Cfg<PD>::SPLATS;
@@ -170,9 +173,9 @@ __device__ __forceinline__ bool in_columns(const Geom& g, int entries, int least
 template <int PD, int VD, bool PRE>
 struct NarrowColumns {
     static constexpr bool EVER = PD >= 2 && PD <= (PRE ? 3 : 4);
-    static constexpr int AHEAD = PD == 4 || (VD == 3 && (PD == 2 || !PRE)) ? 4 : 2;
-    static constexpr int CTAS = !EVER ? 0 : AHEAD == 4 ? 6 : 8;
-    static constexpr int LEAST = AHEAD == 4 ? 8 : !PRE ? (PD == 2 ? 12 : 10) : VD == 3 ? 10 : 24;
+    static constexpr int AHEAD = PD == 4 ? 3 : VD == 3 && (PD == 2 || !PRE) ? 4 : 2;
+    static constexpr int CTAS = !EVER ? 0 : AHEAD >= 3 ? 6 : 8;
+    static constexpr int LEAST = AHEAD >= 3 ? 8 : !PRE ? (PD == 2 ? 12 : 10) : VD == 3 ? 10 : 24;
 };
 // Few entries are not enough where a noisy guide sends neighbouring points to one and another of them: a column then
 // meets a run nearly every point, and all tiles add to few vertices.  So tiles that have more entries than one under
@@ -211,50 +214,49 @@ __device__ __forceinline__ void splat_columns(const Geom& g, const TilePos& tpos
                                               const float* __restrict__ input, const u16* __restrict__ rec_tile,
                                               const float* __restrict__ recw_tile,
                                               const u32* __restrict__ list_ref, float* __restrict__ v0) {
-    constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3, COLUMNS = TP / COLUMN;
-    for (int i = threadIdx.x; i < (PD + 1) * COLUMNS; i += TP) {
-        const int r = i / COLUMNS, c = i % COLUMNS;
-        const int lx = c & (g.TX - 1), ly = (c >> g.tx_log2) * COLUMN;
-        const int x = tpos.tx * g.TX + lx, y = tpos.ty * g.TY + ly;
-        const int rows = x < g.W ? min(COLUMN, g.H - y) : 0;
-        if (rows <= 0) continue;
-        const u16* rp = rec_tile + r * TP + ly * g.TX + lx;
-        const float* wp = recw_tile + r * TP + ly * g.TX + lx;
-        const float* in = input + ((size_t)tpos.item * g.n + ((size_t)tpos.o * g.H + y) * g.W + x) * C;
-        const size_t step = (size_t)g.W * C;
-        float acc[VP];
+    constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3;
+    constexpr int PIECES = TP / (16 * (PD + 1)), ALL = 16 * PIECES;   // of 16 points of a column; of a tile (TX columns of 256 / TX points)
+    const int r = (int)threadIdx.x / ALL, c = (int)threadIdx.x % ALL, lx = c & (g.TX - 1), s = c >> g.tx_log2, k = s % PIECES;
+    const int from = 16 * k / PIECES, ly = s / PIECES * 16 + from;
+    const int x = tpos.tx * g.TX + lx, y = tpos.ty * g.TY + ly;
+    const int rows = r <= PD && x < g.W ? min(16 * (k + 1) / PIECES - from, g.H - y) : 0;
+    if (rows <= 0) return;
+    const u16* rp = rec_tile + r * TP + ly * g.TX + lx;
+    const float* wp = recw_tile + r * TP + ly * g.TX + lx;
+    const float* in = input + ((size_t)tpos.item * g.n + ((size_t)tpos.o * g.H + y) * g.W + x) * C;
+    const size_t step = (size_t)g.W * C;
+    float acc[VP];
 #pragma unroll
-        for (int j = 0; j < VP; j++) acc[j] = 0.f;
-        u32 cur = list_ref[base + rp[0]];
+    for (int j = 0; j < VP; j++) acc[j] = 0.f;
+    u32 cur = list_ref[base + rp[0]];
 #pragma unroll 1
-        for (int k0 = 0; k0 < rows; k0 += AHEAD) {   // AHEAD points' loads in flight
-            u32 v[AHEAD];
-            float w[AHEAD], xv[AHEAD][C];
+    for (int k0 = 0; k0 < rows; k0 += AHEAD) {   // AHEAD points' loads in flight
+        u32 v[AHEAD];
+        float w[AHEAD], xv[AHEAD][C];
 #pragma unroll
-            for (int k = 0; k < AHEAD; k++) {
-                const bool there = k0 + k < rows;
-                v[k] = there ? rp[(k0 + k) * g.TX] : 0u;
-                w[k] = there ? wp[(k0 + k) * g.TX] : 0.f;
+        for (int k = 0; k < AHEAD; k++) {
+            const bool there = k0 + k < rows;
+            v[k] = there ? rp[(k0 + k) * g.TX] : 0u;
+            w[k] = there ? wp[(k0 + k) * g.TX] : 0.f;
 #pragma unroll
-                for (int j = 0; j < C; j++) xv[k][j] = there ? __ldg(in + (size_t)(k0 + k) * step + j) : 0.f;
-            }
+            for (int j = 0; j < C; j++) xv[k][j] = there ? __ldg(in + (size_t)(k0 + k) * step + j) : 0.f;
+        }
 #pragma unroll
-            for (int k = 0; k < AHEAD; k++) v[k] = (k0 + k < rows) ? list_ref[base + v[k]] : cur;
+        for (int k = 0; k < AHEAD; k++) v[k] = (k0 + k < rows) ? list_ref[base + v[k]] : cur;
 #pragma unroll
-            for (int k = 0; k < AHEAD; k++) {
-                if (k0 + k < rows) {
-                    if (v[k] != cur) {
-                        flush_row<VP>(v0 + (size_t)cur * VP, acc);
-                        cur = v[k];
-                    }
-#pragma unroll
-                    for (int j = 0; j < C; j++) acc[j] = PL_FMA(w[k], xv[k][j], acc[j]);
-                    acc[C] = PL_FADD(acc[C], w[k]);
+        for (int k = 0; k < AHEAD; k++) {
+            if (k0 + k < rows) {
+                if (v[k] != cur) {
+                    flush_row<VP>(v0 + (size_t)cur * VP, acc);
+                    cur = v[k];
                 }
+#pragma unroll
+                for (int j = 0; j < C; j++) acc[j] = PL_FMA(w[k], xv[k][j], acc[j]);
+                acc[C] = PL_FADD(acc[C], w[k]);
             }
         }
-        flush_row<VP>(v0 + (size_t)cur * VP, acc);
     }
+    flush_row<VP>(v0 + (size_t)cur * VP, acc);
 }
 
 template <int PD, int VD, bool PRE>
