@@ -207,6 +207,10 @@ int pl_crf_update_f32(float* q_out, const float* unaries, const float* q_bilater
                       const float* compatibility, float bilateral_weight, float spatial_weight,
                       int64_t n_points, int n_labels, void* stream);
 
+/* What an inference starts from: q_out = softmax over labels of -unaries ([n_points][n_labels] arrays; up to 128
+ * labels).  No counterpart in the reference. */
+int pl_crf_start_f32(float* q_out, const float* unaries, int64_t n_points, int n_labels, void* stream);
+
 /* One mean-field step of a CRF with the Potts model through two lattices that pl_lattice_build_f32 left in their
  * workspaces, `bilateral` (reference image of n_reference_channels) and spatial-only, of the same batch and spatial_dims and
  * built for n_labels + 1 values at least: both filters of q and pl_crf_update_f32 without a compatibility matrix, the same

@@ -26,7 +26,7 @@ EXPORTED_SYMBOLS = [
     "pl_export_lattice", "pl_profile_next_call", "pl_lattice_filter_f32_noalloc",
     "pl_lattice_build_f32", "pl_lattice_build_positions_f32", "pl_lattice_apply_f32",
     "pl_workspace_bytes_f64", "pl_compute_positions_f64", "pl_filter_f64", "pl_lattice_filter_f64",
-    "pl_export_lattice_f64", "pl_debug_direct_index", "pl_crf_update_f32", "pl_crf_step_f32", "pl_launch_count",
+    "pl_export_lattice_f64", "pl_debug_direct_index", "pl_crf_update_f32", "pl_crf_step_f32", "pl_crf_start_f32", "pl_launch_count",
     "pl_direct_index_min_entries", "pl_watch_next_call", "pl_cancel_watch", "pl_await_watched_call",
     "pl_watched_calls_status",
 ]
@@ -90,6 +90,7 @@ def lib():
         L.pl_debug_direct_index.argtypes = [i]
         L.pl_direct_index_min_entries.argtypes = [i, i, ip, f, ctypes.POINTER(ctypes.c_int64)]
         L.pl_crf_update_f32.argtypes = [vp, vp, vp, vp, vp, f, f, i64, i, vp]
+        L.pl_crf_start_f32.argtypes = [vp, vp, i64, i, vp]
         L.pl_crf_step_f32.argtypes = [vp, vp, vp, f, f, i, i, i, ip, i, vp, ctypes.c_size_t, i64, vp, ctypes.c_size_t, i64, vp]
         L.pl_profile_next_call.argtypes = [ctypes.POINTER(ctypes.c_void_p)]
         L.pl_watch_next_call.argtypes = [vp]

@@ -82,9 +82,22 @@ class DenseCRF:
         capi.check(rc, "pl_crf_step_f32")
         return out
 
+    @staticmethod
+    def _start(unaries):
+        """softmax(-unaries), in one kernel where pl_crf_start_f32 takes them."""
+        if not unaries.is_cuda or unaries.dtype != torch.float32 or unaries.requires_grad or unaries.dim() < 1 \
+                or not 1 <= unaries.shape[-1] <= 128:
+            return torch.softmax(-unaries, dim=-1)
+        u = unaries.contiguous()
+        q = torch.empty_like(u)
+        with _OnDevice(u.device):
+            capi.check(capi.lib().pl_crf_start_f32(q.data_ptr(), u.data_ptr(), u.numel() // u.shape[-1], u.shape[-1],
+                                                   _stream_handle(u.device)), "pl_crf_start_f32")
+        return q
+
     def infer(self, unaries, iterations=5):
         """Q after `iterations` mean-field updates, starting from softmax(-unaries)."""
-        q = torch.softmax(-unaries, dim=-1)
+        q = self._start(unaries)
         for _ in range(int(iterations)):
             q = self.step(q, unaries)
         return q

@@ -25,6 +25,8 @@ __host__ __forceinline__ size_t crf_smem_bytes(int tpb, int L) {
 // LT > 0: Potts model with the label count fixed at compile time (a point's rows then live in registers:
 // one shared-memory read and one write per value); LT == 0: any count, any compatibility (rows stay in
 // shared memory).
+// qb == nullptr: no message yet, the distributions that an inference starts from (softmax of -unaries; as torch
+// operations a negation and a softmax, 21 us on 375x500 x 21, so 11).
 template <int TPB, int LT>
 __global__ void __launch_bounds__(TPB)
 crf_update(float* __restrict__ q_out, const float* __restrict__ unaries, const float* __restrict__ qb,
@@ -47,7 +49,7 @@ crf_update(float* __restrict__ q_out, const float* __restrict__ unaries, const f
     {
         int p = tid / L, j = tid - p * L;
         for (int e = tid; e < total; e += TPB) {
-            m_s[p * LS + j] = PL_FADD(PL_FMUL(wb, qb[g0 + e]), PL_FMUL(ws, qs[g0 + e]));
+            m_s[p * LS + j] = qb ? PL_FADD(PL_FMUL(wb, qb[g0 + e]), PL_FMUL(ws, qs[g0 + e])) : 0.f;
             z_s[p * LS + j] = -unaries[g0 + e];
             p += DP;
             j += DJ;

@@ -796,6 +796,31 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     return PL_OK;
 }
 
+// crf_update, or without messages (crf.cuh) the start of an inference.
+static int launch_crf_update(float* q_out, const float* unaries, const float* q_bilateral, const float* q_spatial,
+                             const float* compatibility, float bilateral_weight, float spatial_weight, int64_t n_points,
+                             int n_labels, cudaStream_t st) {
+    const int tpb = n_labels <= 32 ? 256 : 128;
+    const size_t smem = crf_smem_bytes(tpb, n_labels);
+    const long long blocks = (n_points + tpb - 1) / tpb;
+    if (blocks > 0x7FFFFFFFll) return PL_INVALID_ARGUMENT;
+#define PL_CRF_LAUNCH(TPB, LT)                                                                                   \
+    do {                                                                                                         \
+        PL_TRY((ensure_dynamic_smem<crf_update<TPB, LT>>(smem)));                                                \
+        crf_update<TPB, LT><<<(unsigned)blocks, TPB, smem, st>>>(q_out, unaries, q_bilateral, q_spatial,         \
+                                                                 compatibility, bilateral_weight, spatial_weight, \
+                                                                 n_points, n_labels);                            \
+    } while (0)
+    // Potts model at the label count of the benchmark's CRF (20 classes + background): rows in registers
+    if (n_labels == 21 && !compatibility) PL_CRF_LAUNCH(256, 21);
+    else if (n_labels <= 32) PL_CRF_LAUNCH(256, 0);
+    else PL_CRF_LAUNCH(128, 0);
+    PL_COUNT_LAUNCHES(1);
+#undef PL_CRF_LAUNCH
+    PL_CUDA(cudaGetLastError());
+    return PL_OK;
+}
+
 // Whose keys hold no item (float calls; see Cfg::KW_ALONE): the same for whoever reads the workspace later.
 static bool batch_of_one(const Geom& g) { return g.batch == 1; }
 
@@ -1334,26 +1359,16 @@ int pl_crf_update_f32(float* q_out, const float* unaries, const float* q_bilater
     if (n_labels > 128) return PL_UNSUPPORTED_DIMS;
     if (n_points == 0) return PL_OK;
     if (!q_out || !unaries || !q_bilateral || !q_spatial) return PL_INVALID_ARGUMENT;
-    cudaStream_t st = (cudaStream_t)stream;
-    const int tpb = n_labels <= 32 ? 256 : 128;
-    const size_t smem = crf_smem_bytes(tpb, n_labels);
-    const long long blocks = (n_points + tpb - 1) / tpb;
-    if (blocks > 0x7FFFFFFFll) return PL_INVALID_ARGUMENT;
-#define PL_CRF_LAUNCH(TPB, LT)                                                                                   \
-    do {                                                                                                         \
-        PL_TRY((ensure_dynamic_smem<crf_update<TPB, LT>>(smem)));                                                \
-        crf_update<TPB, LT><<<(unsigned)blocks, TPB, smem, st>>>(q_out, unaries, q_bilateral, q_spatial,         \
-                                                                 compatibility, bilateral_weight, spatial_weight, \
-                                                                 n_points, n_labels);                            \
-    } while (0)
-    // Potts model at the label count of the benchmark's CRF (20 classes + background): rows in registers
-    if (n_labels == 21 && !compatibility) PL_CRF_LAUNCH(256, 21);
-    else if (n_labels <= 32) PL_CRF_LAUNCH(256, 0);
-    else PL_CRF_LAUNCH(128, 0);
-    PL_COUNT_LAUNCHES(1);
-#undef PL_CRF_LAUNCH
-    PL_CUDA(cudaGetLastError());
-    return PL_OK;
+    return launch_crf_update(q_out, unaries, q_bilateral, q_spatial, compatibility, bilateral_weight, spatial_weight, n_points,
+                             n_labels, (cudaStream_t)stream);
+}
+
+int pl_crf_start_f32(float* q_out, const float* unaries, int64_t n_points, int n_labels, void* stream) {
+    if (n_points < 0 || n_labels < 1) return PL_INVALID_ARGUMENT;
+    if (n_labels > 128) return PL_UNSUPPORTED_DIMS;
+    if (n_points == 0) return PL_OK;
+    if (!q_out || !unaries) return PL_INVALID_ARGUMENT;
+    return launch_crf_update(q_out, unaries, nullptr, nullptr, nullptr, 0.f, 0.f, n_points, n_labels, (cudaStream_t)stream);
 }
 
 unsigned long long pl_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }

@@ -77,3 +77,17 @@ def test_step_through_a_failed_lattice_is_nan_and_bad_shapes_are_refused(plb):
         crf.step(q.double(), u)
     crf.spatial.workspace[8:12] = torch.tensor([1 << capi.PL_CAPACITY_EXCEEDED, 0, 0, 0], dtype=torch.uint8, device="cuda")
     assert torch.isnan(crf.step(q, u)).all()
+
+
+@pytest.mark.parametrize("n_points,labels", [(1, 1), (255, 2), (257, 21), (1000, 32), (130, 33), (129, 128), (40, 129)])
+def test_inference_starts_from_the_softmax_of_the_unaries(plb, n_points, labels):
+    import torch
+    g = torch.Generator().manual_seed(labels)
+    u = (5.0 * torch.randn((1, n_points, labels), generator=g)).cuda()
+    want = torch.softmax(-u.double(), -1)
+    for x in (u, u.transpose(0, 1).contiguous().transpose(0, 1)):
+        q = plb.DenseCRF._start(x)
+        assert q.shape == u.shape and float((q - want).abs().max()) <= 1e-6      # an exponential and a quotient
+    assert torch.equal(plb.DenseCRF._start(u.cpu()), torch.softmax(-u.cpu(), -1))
+    assert plb.DenseCRF._start(u.double()).dtype == torch.float64
+    assert plb.DenseCRF._start(u[:, :0]).numel() == 0
