@@ -8,9 +8,30 @@ namespace pl {
 
 // The header and the sketch before a call.  A kernel and not a memset, so that build_tiles can start beside it (the gap between a memset and the
 // build, 3 to 4 us a call: 8 x 512x512 x 21, pd 2, forward + backward, 431 -> 425; 512x512 x 3 in double 188.5 -> 185.5).
-__global__ void __launch_bounds__(256) clear_header(Header* hdr, u32 quads) {
+// It also clears (to ones: empty slots) what the index stage needs where the host knows how much that may be, the direct index
+// or the table of a call without a sketch, so that no launch between the build and the insert has to: us a call, 2 x
+// 48x64 x 3 52 / 46, 4 x 180x240 x 3 60 / 57, 60x70 x 2 without a guide 32 / 28.  (By build_tiles, a share a tile, it cost calls without any
+// 0.7 %.)
+struct ClearTable {
+    uint4* table;       // null: a launch of its own does
+    u32 quads;          // 16 bytes each
+    u32 direct_log2;    // direct indexing: the logarithm of its slots; 0: a hash table
+};
+constexpr u32 CLEAR_QUADS = 1u << 19;   // 8 MB, at most
+__global__ void __launch_bounds__(256) clear_header(Header* hdr, u32 quads, ClearTable clear) {
     after_previous_kernel();
-    for (u32 i = threadIdx.x; i < quads; i += 256) reinterpret_cast<uint4*>(hdr)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (blockIdx.x == 0) {
+        for (u32 i = threadIdx.x; i < quads; i += 256) reinterpret_cast<uint4*>(hdr)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (clear.direct_log2) {
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                hdr->direct = 1;
+                hdr->table_log2 = clear.direct_log2;
+            }
+        }
+    }
+    for (u32 i = blockIdx.x * 256 + threadIdx.x; i < clear.quads; i += gridDim.x * 256)
+        clear.table[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -635,6 +656,16 @@ struct VertexInit {
 // created a vertex) are collected in shared memory and numbered with ONE atomic on the global vertex
 // counter.  One atomic per chunk, all on the same address, was what bounded this launch.
 constexpr int INSERT_CHUNKS = 8;
+
+// The table's size in calls whose clear_header cleared all that the table may take: by the entries, here; else clear_table
+// has chosen it (see there).  By all threads of an insert launch alike; one of them tells the lookups after it.
+__device__ __forceinline__ u32 table_log2_of(Header* hdr, u32 entries, u32 max_log2, bool cleared) {
+    if (!cleared) return hdr->table_log2;
+    u32 lg = 10;
+    while (lg < max_log2 && (1ull << lg) < 2ull * entries) lg++;
+    if (blockIdx.x == 0 && threadIdx.x == 0) hdr->table_log2 = lg;
+    return lg;
+}
 constexpr u32 VERTEX_FLAG = 0x80000000u;   // low word of a table slot: vertex index (set) or entry index (clear)
 
 struct InsertRound {
@@ -704,13 +735,13 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
 template <int KW>
 __global__ void __launch_bounds__(256)
 insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>* __restrict__ list_keys,
-               u32* __restrict__ list_ref, u32* __restrict__ vid, Key<KW>* __restrict__ vkeys, VertexInit vi) {
+               u32* __restrict__ list_ref, u32* __restrict__ vid, Key<KW>* __restrict__ vkeys, VertexInit vi, bool cleared) {
     after_previous_kernel();
     __shared__ InsertRound rd;
     if (threadIdx.x == 0) rd.count = 0;
     if (call_failed(hdr)) return;   // (its barrier also publishes rd.count)
     const u32 T = hdr->num_entries;
-    const u64 mask = (1ull << hdr->table_log2) - 1;
+    const u64 mask = (1ull << table_log2_of(hdr, T, max_log2, cleared)) - 1;
     const u32 filter_log2 = hdr->filter_log2;
     u32* filter = filter_log2 ? filter_words(table, max_log2, filter_log2) : nullptr;
     const u32 stride = gridDim.x * 256u;
@@ -803,15 +834,15 @@ __device__ __forceinline__ u32 key_rest(const Key<Cfg<PD>::KW>& k) {
 // the vertex.
 template <int PD>
 __global__ void __launch_bounds__(256, 8)   // as many as it is launched with
-insert_keys(Header* hdr, KeySlot* __restrict__ table, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
-            u32* __restrict__ list_ref, u32* __restrict__ vid, Key<Cfg<PD>::KW>* __restrict__ vkeys, VertexInit vi) {
+insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
+            u32* __restrict__ list_ref, u32* __restrict__ vid, Key<Cfg<PD>::KW>* __restrict__ vkeys, VertexInit vi, bool cleared) {
     after_previous_kernel();
     constexpr int KW = Cfg<PD>::KW;
     __shared__ InsertRound rd;
     if (threadIdx.x == 0) rd.count = 0;
     if (call_failed(hdr)) return;   // (its barrier also publishes rd.count)
     const u32 T = hdr->num_entries;
-    const u32 mask = (u32)((1ull << hdr->table_log2) - 1);
+    const u32 mask = (u32)((1ull << table_log2_of(hdr, T, max_log2, cleared)) - 1);
     const u32 stride = gridDim.x * 256u;
     for (u32 start = blockIdx.x * 256u; start < T;) {
         for (int c = 0; c < INSERT_CHUNKS && start < T; c++, start += stride) {

@@ -340,6 +340,18 @@ static bool make_direct(Direct& d, const Geom& g, int pd, const Layout& L) {
     return direct_bounds(d, pd, g.sdims, g.spatial_std, g.scale, g.batch, L.index_words);
 }
 
+// What clear_header clears for the index stage (see ClearTable): the direct index, or the hash table of a call that keeps no
+// sketch, whose size its bound gives.  A small lattice's table lies elsewhere.
+static ClearTable table_to_clear(const Direct* direct, const Layout& L, void* table, int sketch_shift, bool small) {
+    ClearTable c = {nullptr, 0u, 0u};
+    const u64 bytes = direct ? sizeof(u32) * direct->slots : (L.key_slots ? 16ull : 8ull) * L.table_slots;
+    if (small || (!direct && sketch_shift >= 0) || bytes > 16ull * CLEAR_QUADS) return c;
+    c.table = static_cast<uint4*>(table);
+    c.quads = (u32)((bytes + 15) / 16);   // (regions are 256-byte aligned: so is the end)
+    if (direct) while ((1ull << c.direct_log2) < direct->slots || c.direct_log2 == 0) c.direct_log2++;
+    return c;
+}
+
 // Launch grid of the tile kernels (see this_tile).
 static dim3 tile_grid(const Geom& g) {
     if (g.grid3) return dim3((unsigned)g.tiles_x, (unsigned)g.tiles_y, (unsigned)(g.batch * g.outer));
@@ -555,8 +567,9 @@ static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L,
 }
 
 // The header's counters and, in calls that keep one, the sketch behind it.
-static int clear_header_of(Header* hdr, int sketch_shift, cudaStream_t st) {
-    PL_LAUNCH((clear_header), 1, 256, 0, st, hdr, (u32)((sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header)) / 16));
+static int clear_header_of(Header* hdr, int sketch_shift, const ClearTable& clear, cudaStream_t st) {
+    const unsigned ctas = std::min(1u + clear.quads / 1024u, 2u * (unsigned)num_sms());
+    PL_LAUNCH((clear_header), ctas, 256, 0, st, hdr, (u32)((sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header)) / 16), clear);
     PL_COUNT_LAUNCHES(1);
     return PL_OK;
 }
@@ -590,7 +603,15 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     cudaEvent_t* ev = g_stage_events;
     g_stage_events = nullptr;
     if (ev) PL_CUDA(cudaEventRecord(ev[0], st));
-    if (phases & PH_BUILD) PL_TRY(clear_header_of(hdr, sketch_shift, st));
+    Direct direct;
+    bool use_direct = false, small = false, cleared = false;
+    if (phases & PH_BUILD) {
+        if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
+        small = !use_direct && small_index(L);
+        const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, L, table, sketch_shift, small);
+        cleared = clear.table != nullptr;
+        PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));
+    }
     if (g.num_tiles == 0) return PL_OK;
     const Watch watch = (phases & PH_BUILD) ? take_watch(st) : Watch{nullptr, 0u};
 
@@ -605,6 +626,8 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     // calls with large tables 4-25 % (pd 16: 30 -> 37 ms)
     const bool small_table = L.index_words <= (1ull << 24);
     if (phases & PH_BUILD) {
+        // what the insert overlaps: clear_table (see above), or the build itself
+        const int before_insert = cleared ? ((phases & PH_APPLY) ? OV_CLEAR : 0) : small_table ? OV_INSERT : 0;
         // (beyond pd 8 the build has to wait for the header at its start, and launched beside it took 112 -> 128 us)
         constexpr int beside_clear = Cfg<PD>::COMPACT ? 0 : OV_BUILD;
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
@@ -617,9 +640,6 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[1], st));
-        Direct direct;
-        bool use_direct = false;
-        if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
         // a new vertex's neighbour slots and (when this call also applies) its value row are initialised
         // by the launch that creates it
         VertexInit vinit;
@@ -631,14 +651,13 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         if constexpr (PD <= MAX_SDIMS) {
             if (use_direct) {
                 u32* table32 = reinterpret_cast<u32*>(table);
-                PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
-                PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
+                if (!cleared) PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
+                PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
                 PL_LAUNCH_AFTER(OV_LINK, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
                                                                  L.max_entries, watch);
             }
         }
-        const bool small = !use_direct && small_index(L);
-        PL_COUNT_LAUNCHES(small ? 2 : 4);   // build_tiles and the launches of the index stage
+        PL_COUNT_LAUNCHES(small ? 2 : cleared ? 3 : 4);   // build_tiles and the launches of the index stage
         if (small) {
             PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, (phases & PH_APPLY) != 0, st)));
         } else if (!use_direct) {
@@ -649,11 +668,11 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
             // a build and two applies)
             auto hash_index = [&](auto keys_in_slots) -> int {
                 constexpr bool KEYS = decltype(keys_in_slots)::value;
-                PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+                if (!cleared) PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
                 if constexpr (KEYS)
-                    PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
+                    PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
                 else
-                    PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
+                    PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
                 PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
                                                           L.max_entries, zrows, vinit.row_bytes, watch);
                 return PL_OK;
@@ -733,7 +752,15 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* v1 = reinterpret_cast<double*>(ws + L.v1);
 
     const int sketch_shift = sketch_shift_of(L.max_entries);
-    PL_TRY(clear_header_of(hdr, sketch_shift, st));
+    // spatial-only calls index their vertices directly, as the float calls do (the key bounds hold for
+    // either arithmetic: the margin is far wider than any rounding)
+    Direct direct;
+    bool use_direct = false;
+    if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
+    const bool small = !use_direct && small_index(L);
+    const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, L, table, sketch_shift, small);
+    const bool cleared = clear.table != nullptr;
+    PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));
     if (g.num_tiles == 0) return PL_OK;
     const Watch watch = take_watch(st);
     PL_TRY((ensure_dynamic_smem<build_tiles<PD, double>>(Cfg<PD>::build_smem(false))));
@@ -744,13 +771,9 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     while ((1ull << table_log2) < L.table_slots) table_log2++;
     const int vp = padded_vd_f64(vd);
     const bool small_table = L.index_words <= (1ull << 24);   // (as for float)
+    const int before_insert = cleared ? OV_CLEAR : small_table ? OV_INSERT : 0;
 
     PL_LAUNCH_AFTER(Cfg<PD>::COMPACT ? 0 : OV_BUILD, (build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
-    // spatial-only calls index their vertices directly, as the float calls do (the key bounds hold for
-    // either arithmetic: the margin is far wider than any rounding)
-    Direct direct;
-    bool use_direct = false;
-    if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
     u32* table32 = reinterpret_cast<u32*>(table);
     VertexInit vinit;
     vinit.nbr = nbr;
@@ -760,21 +783,20 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     vinit.row_bytes = (u32)vp * 8u;
     if constexpr (PD <= MAX_SDIMS) {
         if (use_direct) {
-            PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
-            PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
+            if (!cleared) PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
+            PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH((link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
                                                              L.max_entries, watch);
         }
     }
-    const bool small = !use_direct && small_index(L);
     if (small) {
         PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, true, st)));
     } else if (!use_direct) {
-        PL_LAUNCH_AFTER(OV_CLEAR, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+        if (!cleared) PL_LAUNCH_AFTER(OV_CLEAR, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         if constexpr (Cfg<PD>::KEY_SLOTS)
-            PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), list_keys, list_ref, vid, vkeys, vinit);
+            PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
         else
-            PL_LAUNCH_AFTER(small_table ? OV_INSERT : 0, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit);
+            PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
         PL_LAUNCH((link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   nullptr, 0u, watch);
     }
@@ -791,7 +813,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         double* tmp = src; src = dst; dst = tmp;
     }
     PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
-    PL_COUNT_LAUNCHES((small ? 2 : 4) + 1 + (one_blur ? 1 : PD + 1) + 1);   // build and index; splat; blur; slice
+    PL_COUNT_LAUNCHES((small ? 2 : cleared ? 3 : 4) + 1 + (one_blur ? 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;
 }
