@@ -81,6 +81,62 @@ blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restri
     blur_rows<V>(hdr, nbr_axis, src, dst, vpr, blockIdx.x, gridDim.x);
 }
 
+// Two passes in one launch, along axes a and then b: a thread mixes the row that pass b needs of its vertex and of that one's
+// two neighbours, from nine rows in all, and what pass a would have stored is rounded as it would have been: the same bits.
+// All indices are older than the splat and are fetched before the wait, so that a pair of passes waits for rows once.  A
+// pass of a lattice whose items (16 bytes of a row) fit the GPU's threads about once takes its launch and one round trip to
+// L2, whatever it does; larger ones are bound by their rows, of which this reads half as many again.
+// us a call: 4 x 180x240 x 3 59 -> 54, 512x512 x 3 in double, forward + backward, 185 -> 179, a CRF of 2 x 200x200 x 5 219 ->
+// 192; 900 k vertices of one float4 239 -> 254, which is why it ends at PAIR_ITEMS (see blur_in_pairs).
+// nbr_b null: pass a alone.
+constexpr int PAIR_CTAS = 5;
+constexpr u64 PAIR_ITEMS = 1000000, PAIR_ITEMS_WORST = 300000;   // by the bound, by one that is the worst case
+template <typename V>
+__device__ __forceinline__ void blur_pair_rows(const Header* hdr, const int* __restrict__ nbr_a, const int* __restrict__ nbr_b,
+                                               const V* __restrict__ src, V* __restrict__ dst, u32 vpr, u32 block, u32 blocks) {
+    const u32 M = hdr->num_vertices, items = M * vpr, stride = blocks * blockDim.x;
+    const int2* __restrict__ na = reinterpret_cast<const int2*>(nbr_a);
+    const int2* __restrict__ nb = reinterpret_cast<const int2*>(nbr_b);
+    u32 e = block * blockDim.x + threadIdx.x, v = e / vpr, j = e - v * vpr;
+    int u[3];      // the vertex and its neighbours along b
+    int2 n[3];     // theirs along a
+    auto look_up = [&]() {
+        int2 beside = make_int2(-1, -1);
+        if (v < M && nb) beside = __ldg(nb + v);
+        u[0] = v < M ? (int)v : -1;
+        u[1] = beside.x;
+        u[2] = beside.y;
+#pragma unroll
+        for (int k = 0; k < 3; k++) n[k] = u[k] >= 0 ? __ldg(na + u[k]) : make_int2(-1, -1);
+    };
+    look_up();
+    after_previous_kernel();
+    if (hdr->status != 0) return;
+    const V zero = {};
+    while (e < items) {
+        V lo[3], mid[3], hi[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            mid[k] = u[k] >= 0 ? src[(u32)u[k] * vpr + j] : zero;
+            lo[k] = n[k].x >= 0 ? src[(u32)n[k].x * vpr + j] : zero;
+            hi[k] = n[k].y >= 0 ? src[(u32)n[k].y * vpr + j] : zero;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) mid[k] = mix_rows(lo[k], mid[k], hi[k]);
+        dst[e] = nb ? mix_rows(mid[1], mid[0], mid[2]) : mid[0];
+        e += stride;
+        v = e / vpr;
+        j = e - v * vpr;
+        if (e < items) look_up();
+    }
+}
+template <typename V>
+__global__ void __launch_bounds__(256, PAIR_CTAS)
+blur_pair(const Header* hdr, const int* __restrict__ nbr_a, const int* __restrict__ nbr_b, const V* __restrict__ src,
+          V* __restrict__ dst, u32 vpr) {
+    blur_pair_rows<V>(hdr, nbr_a, nbr_b, src, dst, vpr, blockIdx.x, gridDim.x);
+}
+
 // ---------------------------------------------------------------------------------------------
 // slice_tiles (src/PermutohedralLatticeCPU.h:333-352: float multiply-then-add per remainder in
 // ascending order, reciprocal of the homogeneous channel in double, one multiply per channel).

@@ -174,6 +174,18 @@ crf_splat(Geom g, const float* __restrict__ input, LatticeRows a, LatticeRows s,
         splat_rows<PDS, VD, true, FloatSum, float>(g, tpos, input, s.hdr, s.tile_info, s.rec, s.rec_w, s.srec, s.list_ref, s.v0, vd, bulk_ok);
 }
 
+// Passes 2 `pair` and 2 pair + 1 of both (S: as many as it has; see blur_pair_rows), from v0 to v1 in even pairs.
+template <int PDA, int PDS>
+__global__ void __launch_bounds__(256, PAIR_CTAS)
+crf_blur_pair(LatticeRows a, LatticeRows s, int only, int pair, u32 quads) {
+    const bool second = only ? only == 2 : blockIdx.y != 0;
+    const LatticeRows& l = second ? s : a;
+    const float4* src = reinterpret_cast<const float4*>((pair & 1) ? l.v1 : l.v0);
+    float4* dst = reinterpret_cast<float4*>((pair & 1) ? l.v0 : l.v1);
+    const int* nbr = l.nbr + 4 * (u64)pair * l.max_entries;
+    blur_pair_rows<float4>(l.hdr, nbr, 2 * pair + 1 <= (second ? PDS : PDA) ? nbr + 2 * l.max_entries : nullptr, src, dst, quads, blockIdx.x, gridDim.x);
+}
+
 // Pass `step` of both: A's rows go from v0 to v1 in even passes, S's too.
 __global__ void __launch_bounds__(256, 8)
 crf_blur(LatticeRows a, LatticeRows s, int step, u32 quads) {

@@ -540,6 +540,14 @@ static bool small_blur(const Layout& L, u32 vpr) {
     const u64 one_each = SMALL_CTAS * SMALL_THREADS;
     return L.max_entries <= one_each ? vpr <= 64 : L.max_entries <= SMALL_PIECES * one_each && vpr <= 16;
 }
+// Two passes a launch (see blur_pair_rows), by what the bound says of the vertices: it is 1.5 times the entries or more, of which
+// a half at most are vertices, usually, unless it is the worst case, which lattices of points with nothing in common
+// need and fill.  us a call, a pass / two a launch: bounds of 393 k x 2 items, 115 k vertices (512x512 x 3 in double, forward
+// + backward) 185 / 179; worst cases filled by vertices: 240 k 99.3 / 98.2, 470 k 142 / 144, 960 k 239 / 254.
+static bool blur_in_pairs(const Geom& g, int pd, const Layout& L, u32 vpr) {
+    const bool worst = L.max_entries >= (u64)g.batch * (u64)g.n * (u64)(pd + 1);
+    return L.max_entries * vpr <= (worst ? PAIR_ITEMS_WORST : PAIR_ITEMS);
+}
 template <int PD, int KW>
 static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
                               const VertexInit& vinit, Watch watch, bool overlap, cudaStream_t st) {
@@ -716,6 +724,14 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     if (small_blur(L, qpr)) {
         PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, st));
         PL_COUNT_LAUNCHES(1);
+    } else if (blur_in_pairs(g, PD, L, qpr)) {
+        for (int step = 0; step <= PD; step += 2) {
+            const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
+            const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
+            PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_pair<float4>), sms * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
+            std::swap(src, dst);
+            PL_COUNT_LAUNCHES(1);
+        }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * L.max_entries * 2;
@@ -804,16 +820,23 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
                                                                       list_ref, v0, vd);
     double* src = v0;
     double* dst = v1;
-    const bool one_blur = small_blur(L, (u32)vp / 2);
+    const bool one_blur = small_blur(L, (u32)vp / 2), pairs = blur_in_pairs(g, PD, L, (u32)vp / 2);
     if (one_blur) {
         PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<double2*>(v0), (u32)vp / 2, PD + 1, reverse, st));
+    } else if (pairs) {
+        for (int step = 0; step <= PD; step += 2) {
+            const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
+            const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
+            PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+            std::swap(src, dst);
+        }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
     PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
-    PL_COUNT_LAUNCHES((small ? 2 : cleared ? 3 : 4) + 1 + (one_blur ? 1 : PD + 1) + 1);   // build and index; splat; blur; slice
+    PL_COUNT_LAUNCHES((small ? 2 : cleared ? 3 : 4) + 1 + (one_blur ? 1 : pairs ? PD / 2 + 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;
 }
@@ -901,7 +924,17 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
         PL_TRY(launch_small_blur(a.hdr, a.nbr, LA, reinterpret_cast<float4*>(a.v0), quads, PDA + 1, 0, st));
         launches++;
     }
-    for (int step = 0; step <= std::max(PDA, PDS); step++) {
+    const bool pairs = blur_in_pairs(g, PDA, LA, quads) && blur_in_pairs(g, PDS, LS, quads);
+    for (int pair = 0; pairs && pair <= std::max(PDA, PDS) / 2; pair++) {
+        const bool pass_a = !small_a && 2 * pair <= PDA, pass_s = !small_s && 2 * pair <= PDS, both = pass_a && pass_s;
+        if (!pass_a && !pass_s) continue;
+        const bool first = pair == 0 && !small_a && !small_s;
+        PL_LAUNCH_AFTER(first ? OV_BLUR0 : OV_BLUR, (crf_blur_pair<PDA, PDS>), dim3(num_sms() * PAIR_CTAS / (both ? 2 : 1), both ? 2 : 1), 256, 0, st, a, s, both ? 0 : pass_a ? 1 : 2, pair, quads);
+        launches++;
+        if (pass_a) va = (pair & 1) ? a.v0 : a.v1;
+        if (pass_s) vs = (pair & 1) ? s.v0 : s.v1;
+    }
+    for (int step = 0; !pairs && step <= std::max(PDA, PDS); step++) {
         const bool pass_a = !small_a && step <= PDA, pass_s = !small_s && step <= PDS;
         if (!pass_a && !pass_s) continue;
         const bool first = step == 0 && !small_a && !small_s;
