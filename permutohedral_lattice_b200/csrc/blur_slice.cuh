@@ -254,14 +254,9 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     float* rows_s = reinterpret_cast<float*>(smem_raw);                                         // [rows_cap][RS]
     float* out_s = reinterpret_cast<float*>(smem_raw);                                          // [TP][C], later
     int* prow_s = reinterpret_cast<int*>(smem_raw + SliceFast<PD, VP>::region(rows_cap));       // [TP]
-    if (call_failed(hdr)) {
-        poison_tile_output(g, output, C);
-        report_late(watch, hdr);
-        wait_for_previous_kernel();
-        return;
-    }
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
+    const u32 status = hdr->status;   // final by now, the same in every thread; one round trip with all that follows
     const int2 info = tile_info[tile];
     const int base = info.x, cnt = info.y;
     const int nrows = min(cnt, rows_cap);
@@ -277,6 +272,12 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     for (int r = 0; r <= PD; r++) {
         l[r] = valid ? rec_tile[r * TP + tid] : 0;
         w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
+    }
+    if (status != 0) {
+        poison_tile_output(g, output, C);
+        report_late(watch, hdr);
+        wait_for_previous_kernel();
+        return;
     }
     wait_for_previous_kernel();
     stage_rows<PD, VP>(rows_s, nrows, list_ref, base, v4);
@@ -343,21 +344,16 @@ __device__ __forceinline__ float4 load_row(const float4* p) {   // never moved a
     return x;
 }
 template <int PD, int C>
-__global__ void __launch_bounds__(Cfg<PD>::TP)
+__global__ void __launch_bounds__(Cfg<PD>::TP, PD < 5 || (PD == 5 && C == 1) ? 8 : 1)   // (32 registers)
 slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* __restrict__ tile_info,
              const u16* __restrict__ rec, const float* __restrict__ rec_w, const u32* __restrict__ list_ref,
              const float* __restrict__ vsrc, Watch watch) {
     // (what is read before the wait is older than any blur pass, as in slice_tiles_fast)
     constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS;
-    if (hdr->status != 0) {   // final by now: the same in every thread
-        poison_tile_output(g, output, C);
-        report_late(watch, hdr);
-        wait_for_previous_kernel();
-        return;
-    }
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x;
-    const u32* ref = list_ref + tile_info[tpos.tile].x;
+    const u32 status = hdr->status;   // final by now: the same in every thread
+    const int base = tile_info[tpos.tile].x;
     int item, pix;
     const bool valid = tile_point(g, tpos, tid, item, pix);
     const size_t at = (size_t)tpos.tile * SPLATS + tid;
@@ -367,6 +363,13 @@ slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* 
     for (int r = 0; r <= PD; r++) v[r] = valid ? rec[at + r * TP] : 0;
 #pragma unroll
     for (int r = 0; r <= PD; r++) w[r] = valid ? rec_w[at + r * TP] : 0.f;
+    if (status != 0) {
+        poison_tile_output(g, output, C);
+        report_late(watch, hdr);
+        wait_for_previous_kernel();
+        return;
+    }
+    const u32* ref = list_ref + base;
 #pragma unroll
     for (int r = 0; r <= PD; r++) v[r] = valid ? ref[v[r]] : 0u;
     wait_for_previous_kernel();

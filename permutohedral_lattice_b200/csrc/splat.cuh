@@ -276,11 +276,11 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     int* cur_s = reinterpret_cast<int*>(vid_s + SPLATS);                                    // [SPLATS], only without PRE
     __shared__ int wsum_s[32];
     __shared__ __align__(8) u64 bar;
-    if (call_failed(hdr)) return;
-    if (PRE && !lattice_is_sorted(hdr)) return;
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
-    const int2 info = tile_info[tile];
+    const int2 info = tile_info[tile];   // (in flight with the status)
+    if (call_failed(hdr)) return;
+    if (PRE && !lattice_is_sorted(hdr)) return;
     const int base = info.x, nloc = info.y;
     using CS = ColumnsSample<PD>;
     if constexpr (NC::EVER) {
