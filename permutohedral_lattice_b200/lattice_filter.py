@@ -6,6 +6,7 @@ reverse)` has the arguments, defaults, shapes and gradient of the `LatticeFilter
 device memory and streams only, every computation happens in libpl_lattice.so through its C ABI.
 """
 import ctypes
+import functools
 
 import torch
 from torch.autograd import forward_ad
@@ -285,7 +286,7 @@ class _Plan:
     def __init__(self, device, call, dtype):
         if not capi.lib().pl_supported(call.pd, call.vd):
             raise capi.PlError(capi.PL_UNSUPPORTED_DIMS, "lattice_filter(pd=%d, vd=%d)" % (call.pd, call.vd))
-        self.call, self.dtype = call, dtype
+        self.call, self.dtype, self.f32 = call, dtype, dtype == torch.float32
         self.kind = _kind(device, call)
         self.worst = call.batch * call.n * (call.pd + 1)
         self.floor = _direct_index_floor(call) if call.batch and call.n else 0
@@ -383,6 +384,37 @@ def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha
                     raise capi.PlError(st.device_status, "lattice_filter (device)")
     call.max_entries = max_entries     # what pl_export_lattice must be told again
     return out, ws, call
+
+
+def _filter(input_image, reference_image, bilateral, theta_alpha, theta_beta, theta_gamma, reverse, mode):
+    """lattice_filter_raw's output, by the short way where that call would only look things up: contiguous tensors on the
+    current device whose plan is known, a reference that a verified call of this kind just used, and a workspace that is
+    there.  Anything else, errors above all, goes the long way.  (A call on a small image waits for the host: 8 us of
+    Python a call the long way, 5 the short one; a gradient took 15 us less: 40x50 x 2 136 -> 120 us, 3 x 200x150 x 1 146 -> 134.)"""
+    x, ref = input_image, reference_image if bilateral else None
+    index = torch.cuda.current_device() if x.is_cuda else -1
+    if x.is_cuda and x.get_device() == index and x.is_contiguous() and (ref is None or (
+            ref.is_cuda and ref.get_device() == index and ref.dtype == x.dtype and ref.is_contiguous())):
+        plan = _plans.get((index, x.dtype, x.shape, None if ref is None else ref.shape, bilateral, theta_alpha, theta_beta,
+                           theta_gamma))
+        if plan is not None and (plan.f32 or mode == "atomic"):
+            call, known = plan.call, _verified.get(plan.kind)
+            if known is not None and known[0] == _identity(ref, call.batch):
+                bound, stream = known[1], torch._C._cuda_getCurrentRawStream(index)
+                ws = _workspaces.get((index, stream))
+                if ws is not None and ws.numel() >= plan.bytes(bound, mode):
+                    out = torch.empty_like(x)
+                    head = (out.data_ptr(), x.data_ptr(), 0 if ref is None else ref.data_ptr(), call.batch,
+                            len(call.sdims), call.c_sdims, call.c, call.r, call.bilateral, *call.theta,
+                            bool(reverse), ws.data_ptr(), ws.numel(), bound)
+                    if plan.f32:
+                        rc = capi.lib().pl_lattice_filter_f32(*head, capi.MODES[mode], stream)
+                    else:
+                        rc = capi.lib().pl_lattice_filter_f64(*head, stream)
+                    if rc != capi.PL_OK:
+                        capi.check(rc, "pl_lattice_filter_f32" if plan.f32 else "pl_lattice_filter_f64")
+                    return out
+    return lattice_filter_raw(input_image, reference_image, bilateral, theta_alpha, theta_beta, theta_gamma, reverse, mode)[0]
 
 
 def lattice_stats(workspace, stream=None, device=None):
@@ -516,9 +548,7 @@ class _LatticeFilterFunction(torch.autograd.Function):
                 reverse, mode):
         ctx.args = (bilateral, theta_alpha, theta_beta, theta_gamma, mode)
         ctx.save_for_backward(reference_image)
-        out, _, _ = lattice_filter_raw(input_image, reference_image, bilateral, theta_alpha,
-                                       theta_beta, theta_gamma, reverse, mode)
-        return out
+        return _filter(input_image, reference_image, bilateral, theta_alpha, theta_beta, theta_gamma, reverse, mode)
 
     @staticmethod
     def backward(ctx, grad):
@@ -526,8 +556,7 @@ class _LatticeFilterFunction(torch.autograd.Function):
         # to the upstream gradient with reverse=True; the reference image gets zeros.
         (reference_image,) = ctx.saved_tensors
         bilateral, theta_alpha, theta_beta, theta_gamma, mode = ctx.args
-        g, _, _ = lattice_filter_raw(grad, reference_image, bilateral, theta_alpha, theta_beta,
-                                     theta_gamma, True, mode)
+        g = _filter(grad, reference_image, bilateral, theta_alpha, theta_beta, theta_gamma, True, mode)
         ref_grad = torch.zeros_like(reference_image) if ctx.needs_input_grad[1] else None
         return g, ref_grad, None, None, None, None, None, None
 
@@ -545,7 +574,7 @@ def lattice_filter(input_image, reference_image, bilateral=True, theta_alpha=1.0
             reference_image is not None and reference_image.requires_grad))):
         # nothing to differentiate: the autograd function would only add its own cost (a tenth of a small call)
         if not reuse_lattice:
-            return lattice_filter_raw(input_image, reference_image, bool(bilateral), *thetas, bool(reverse), mode)[0]
+            return _filter(input_image, reference_image, bool(bilateral), *thetas, bool(reverse), mode)
         return Lattice(reference_image, tuple(input_image.shape[:-1]), bool(bilateral), *thetas,
                        max_channels=input_image.shape[-1], mode=mode).apply(input_image, bool(reverse), mode)
     fn = _LatticeFilterReuseFunction if reuse_lattice else _LatticeFilterFunction
@@ -563,8 +592,13 @@ def _watched_by_torch():
     return _is_tracing() or forward_ad._current_level >= 0 or _functorch_level() is not None or _is_compiling()
 
 
+@functools.lru_cache(maxsize=1024)
+def _float_as_attr(v):
+    return ctypes.c_float(v).value
+
+
 def _as_attr(v):
-    return ctypes.c_float(float(v)).value
+    return _float_as_attr(v) if type(v) is float else ctypes.c_float(float(v)).value
 
 
 def compute_positions(reference_image, spatial_dims, spatial_std, feature_std, dtype=None):
