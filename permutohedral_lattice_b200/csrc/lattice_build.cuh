@@ -576,6 +576,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 // ---------------------------------------------------------------------------------------------
 constexpr u64 KEY_SLOTS_WHOLE = 1ull << 21;   // 32 MB
 constexpr u64 TAG_SLOTS_WHOLE = 1ull << 23;   // 64 MB
+constexpr u64 TAG_SLOTS_MOST = 1ull << 25;    // beyond, half as many would not stay in L2 either
 template <bool KEY_SLOTS>
 __global__ void __launch_bounds__(256)
 clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift) {
@@ -608,9 +609,10 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
             // table of keys beyond 32 MB has two a vertex at least (us a call, four / two a vertex: 1024x1024 grey by RGB,
             // forward + backward, 17 MB at four, 325 / 337; 16 x 512x512 x 21, 67 MB at four, 1857 / 1824.  So has
             // a tagged one beyond 64 MB (1 M points, pd 16, 134 / 67 MB with keys of one sector: insert 454 / 404 us, link
-            // 670 / 578, clear 31 / 18; 4 x 300x300 points 1775 / 1447 us a call)
+            // 670 / 578, clear 31 / 18; 4 x 300x300 points 1775 / 1447 us a call), up to 256 MB (8 M points, 16 M vertices, 13.5 / 13.8 ms
+            // of index)
             constexpr u64 WHOLE = KEY_SLOTS ? KEY_SLOTS_WHOLE : TAG_SLOTS_WHOLE;
-            if (slots > WHOLE) slots = slots / 2 > WHOLE ? slots / 2 : WHOLE;
+            if (slots > WHOLE && (KEY_SLOTS || slots <= TAG_SLOTS_MOST)) slots = slots / 2 > WHOLE ? slots / 2 : WHOLE;
             const u64 least = 1ull << (sketch_shift + 11);
             slots = slots < least ? least : slots;
             need = slots < need ? slots : need;

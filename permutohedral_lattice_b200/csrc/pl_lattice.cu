@@ -2,11 +2,12 @@
 //
 // Pipeline of one call (whole batch in every launch, nothing synchronises with the host):
 //
+//   clear_header    zeroes the counters; in calls without a sketch, and with direct indexing, clears the table too.
 //   build_tiles     one CTA per tile of TP points: features -> enclosing simplex -> pd+1 vertex keys
 //                   per point; the tile's keys are de-duplicated in a shared-memory hash; the
 //                   distinct keys become a contiguous run of "entries" in a global list and every
 //                   splat records the 16-bit index of its entry inside the tile.
-//   clear_table     sizes the global hash table (on the device) from the entry count or, in larger calls, from
+//   clear_table     calls with a sketch: sizes the global hash table (on the device) from the entry count or from
 //                   build_tiles' sketch of the vertices, and clears it and the filter in front of it.
 //   insert_entries  one CAS per entry into the table; the first entry of a key owns a new vertex, whose
 //                   neighbour slots the same launch initialises.  Up to pd 5 insert_keys, into slots that hold the key.
@@ -15,7 +16,8 @@
 //   splat_tiles     one CTA per tile: input block staged in shared memory (bulk async copies), splats
 //                   sorted by entry, runs summed in registers, vector reductions into the vertex rows.  Tiles with
 //                   few entries, up to pd 4: columns of points instead of the sort.
-//   blur_axis       pd+1 launches: V'[v] = (V[n1] + 2 V[v] + V[n2]) / 4, Jacobi, ping-pong buffers.
+//   blur_axis       pd+1 launches: V'[v] = (V[n1] + 2 V[v] + V[n2]) / 4, Jacobi, ping-pong buffers.  Medium-sized
+//                   lattices: two passes a launch (blur_pair).
 //   slice_tiles     one CTA per tile: the tile's vertex rows staged in shared memory, each point
 //                   interpolates, divides by the homogeneous channel and writes its output row.  Rows of one
 //                   float4 (slice_points): straight from global memory.

@@ -389,8 +389,8 @@ def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha
 def _filter(input_image, reference_image, bilateral, theta_alpha, theta_beta, theta_gamma, reverse, mode):
     """lattice_filter_raw's output, by the short way where that call would only look things up: contiguous tensors on the
     current device whose plan is known, a reference that a verified call of this kind just used, and a workspace that is
-    there.  Anything else, errors above all, goes the long way.  (A call on a small image waits for the host: 8 us of
-    Python a call the long way, 5 the short one; a gradient took 15 us less: 40x50 x 2 136 -> 120 us, 3 x 200x150 x 1 146 -> 134.)"""
+    there.  Anything else, errors above all, goes the long way.  (A call on a small image waits for the host: 9.0 us
+    of Python the long way, 6.4 the short one; forward + backward of 40x50 x 2 136 -> 120 us, of 3 x 200x150 x 1 146 -> 134.)"""
     x, ref = input_image, reference_image if bilateral else None
     index = torch.cuda.current_device() if x.is_cuda else -1
     if x.is_cuda and x.get_device() == index and x.is_contiguous() and (ref is None or (

@@ -1,5 +1,5 @@
 """Bounds at which a call takes another route and must give the same bits (deterministic sums): two blur passes a launch or
-one, the table cleared with the header or by a launch of its own, for hash tables and for the direct index."""
+one, rows mixed in floats or (more than 5,000,000 float4 of them) in doubles, the table cleared with the header or by a launch of its own, for hash tables and for the direct index."""
 import numpy as np
 import pytest
 
@@ -37,6 +37,19 @@ def test_pairs_of_passes_give_the_bits_of_single_ones(plb, pd):
     single = plb.filter_positions(x64, p64, max_entries=worst)[0].clone()
     pairs = plb.filter_positions(x64, p64, max_entries=worst - 1)[0].clone()
     assert float((single - pairs).norm() / single.norm()) <= 1e-12      # double sums in varying order
+
+
+def test_rows_mixed_in_doubles_give_the_bits_of_floats(plb):
+    """The same first channels beside 68 others: 330,000 rows of 18 float4, or of one."""
+    import torch
+    g = torch.Generator().manual_seed(3)
+    pos = (60 * torch.randn((1, 60000, 5), generator=g)).cuda()
+    x = torch.rand((1, 60000, 71), generator=g).cuda()          # below 1: the same fixed-point grid for both
+    for reverse in (False, True):
+        wide, ws = plb.filter_positions(x, pos, reverse, "deterministic", max_entries=0)
+        assert plb.lattice_stats(ws).num_vertices * 18 > 5000000
+        narrow, _ = plb.filter_positions(x[..., :3].contiguous(), pos, reverse, "deterministic", max_entries=0)
+        assert torch.equal(wide[..., :3], narrow)
 
 
 @pytest.mark.parametrize("pd", [1, 3, 5, 7, 16])
