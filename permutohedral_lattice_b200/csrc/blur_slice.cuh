@@ -359,7 +359,8 @@ __device__ __forceinline__ float4 load_row(const float4* p) {   // never moved a
     return x;
 }
 template <int PD, int C>
-__global__ void __launch_bounds__(Cfg<PD>::TP, PD < 5 || (PD == 5 && C == 1) ? 8 : 1)   // (32 registers)
+// (CTAs an SM: left alone the compiler takes up to 91 registers at pd 16; 8 M points there 0.46 / 0.41 ms)
+__global__ void __launch_bounds__(Cfg<PD>::TP, Cfg<PD>::COMPACT || (PD == 5 && C > 1) ? 7 : PD > 5 ? 5 : 8)
 slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* __restrict__ tile_info,
              const u16* __restrict__ rec, const float* __restrict__ rec_w, const u32* __restrict__ list_ref,
              const float* __restrict__ vsrc, Watch watch) {
@@ -376,7 +377,7 @@ slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* 
         report_late(watch, hdr);
         wait_for_previous_kernel();
     };
-    if (Cfg<PD>::COMPACT && status != 0) return stop();   // (asked for first: 8 M points at pd 16, 0.41 / 0.46 ms)
+    if (Cfg<PD>::COMPACT && status != 0) return stop();
     const size_t at = (size_t)tpos.tile * SPLATS + tid;
     float w[PD + 1];
     u32 v[PD + 1];
