@@ -19,7 +19,7 @@ labels the whole iteration is pl_crf_step_f32: each stage of both filters in one
 import torch
 
 from . import capi
-from .lattice_filter import Lattice, _OnDevice, _check_tensor, _float32_only, _stream_handle
+from .lattice_filter import Lattice, _OnDevice, _check_tensor, _float32_only, _stream_handle, _watched_by_torch
 
 
 class DenseCRF:
@@ -84,8 +84,10 @@ class DenseCRF:
 
     @staticmethod
     def _start(unaries):
-        """softmax(-unaries), in one kernel where pl_crf_start_f32 takes them."""
-        if not unaries.is_cuda or unaries.dtype != torch.float32 or unaries.requires_grad or unaries.dim() < 1 \
+        """softmax(-unaries), in one kernel where pl_crf_start_f32 takes them and torch does not follow them: a tracer,
+        a transform or a tensor of another class would not see the kernel, torch's softmax they do."""
+        if type(unaries) is not torch.Tensor or _watched_by_torch() or not unaries.is_cuda \
+                or unaries.dtype != torch.float32 or unaries.requires_grad or unaries.dim() < 1 \
                 or not 1 <= unaries.shape[-1] <= 128:
             return torch.softmax(-unaries, dim=-1)
         u = unaries.contiguous()

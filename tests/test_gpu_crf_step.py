@@ -91,3 +91,27 @@ def test_inference_starts_from_the_softmax_of_the_unaries(plb, n_points, labels)
     assert torch.equal(plb.DenseCRF._start(u.cpu()), torch.softmax(-u.cpu(), -1))
     assert plb.DenseCRF._start(u.double()).dtype == torch.float64
     assert plb.DenseCRF._start(u[:, :0]).numel() == 0
+
+
+def test_inference_starts_from_torchs_softmax_where_torch_follows_the_unaries(plb):
+    """Forward mode, vmap, jvp and tracers used to go through torch.softmax: none of them sees a kernel launched by ctypes."""
+    import torch
+    from torch.autograd import forward_ad
+    g = torch.Generator().manual_seed(7)
+    u, v, t = (torch.randn((1, 6, 7, 5), generator=g).cuda() for _ in range(3))
+    start = plb.DenseCRF._start
+
+    def softmax(x):
+        return torch.softmax(-x, -1)
+
+    with forward_ad.dual_level():
+        q = forward_ad.unpack_dual(start(forward_ad.make_dual(u, t)))
+        want = forward_ad.unpack_dual(softmax(forward_ad.make_dual(u, t)))
+        assert torch.equal(q.primal, want.primal) and torch.equal(q.tangent, want.tangent)
+    assert torch.equal(torch.func.vmap(start)(torch.stack([u, v])), softmax(torch.stack([u, v])))
+    got, want = torch.func.jvp(start, (u,), (t,)), torch.func.jvp(softmax, (u,), (t,))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    traced = torch.jit.trace(start, (u,), check_trace=False)
+    assert torch.equal(traced(v), softmax(v))
+    crf, _, unaries = _case(plb, (1, 30, 30), 5)
+    assert torch.equal(torch.func.vmap(lambda x: crf.infer(x, 0))(unaries[None]), softmax(unaries)[None])
