@@ -12,48 +12,48 @@ namespace pl {
 // then the rows.  So the pair of the next trip is fetched together with the rows of this one, and a thread goes on
 // to its next row without dividing (a 64-bit quotient a trip before).  16 x 512x512 x 21,
 // forward + backward (12 passes): 1872 -> 1842 us; 1 M points with 16 features (17 passes): 2048 -> 2014.
-// Rows of floats are mixed in floats, pairs an instruction, with what the two sums round off added at the end: the
-// exact sum rounded once, as in doubles (none of 60 M random triples differ; below 2^-124 a quarter loses its last bits).
-// Doubles took three conversions up and one down a
-// value, sixteen of a warp's a cycle and SM, more than half of a pass: 16 x 512x512 x 21 1790 -> 1764 us, 8 x 512x512 x 21
-// by position alone (pd 2) 438 -> 431, 1 M points with 16 features 1968 -> 1943.
+// The sums are in double throughout.  What that costs is the conversions, three up and one down a value and sixteen of a warp's a
+// cycle and SM, more than half of a pass; so the way up is a move of bits (see moved) where it is faster.  us a call, conversions / moves:
+// 16 x 512x512 x 21 1779 / 1766, 375x500 x 21, five steps of a CRF, 442 / 421, 8 x 512x512 x 21 by position alone (pd 2) 428 / 424,
+// 1 M points with 16 features 1705 / 1698.  (Floats with the sums' rounding errors added at the end took 1759, 409, 422 and 1691; they are not
+// the same bits where the errors' sum fits no float.)
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ double mix3(double a, double b, double c) {
     return __fma_rn(0.25, c, __fma_rn(0.5, b, PL_DMUL(0.25, a)));
 }
-// Sum of two pairs of floats, and what its rounding left out (Knuth's two-sum, six additions, two of them an instruction).
-__device__ __forceinline__ float2 two_sum(float2 a, float2 b, float2& rest) {
-    const float2 s = add2(a, b), from_b = sub2(s, a);
-    rest = add2(sub2(a, sub2(s, from_b)), sub2(b, from_b));
-    return s;
-}
-__device__ __forceinline__ float2 mix3(float2 a, float2 b, float2 c) {
-    float2 r1, r2;
-    const float2 s = two_sum(mul2(a, make_float2(0.25f, 0.25f)), mul2(c, make_float2(0.25f, 0.25f)), r1);
-    const float2 t = two_sum(s, mul2(b, make_float2(0.5f, 0.5f)), r2);
-    const float2 r = add2(r1, r2);
-    // (an infinite sum leaves NaN out, which the maximum drops; finite rests it leaves as they are)
-    return add2(t, make_float2(fmaxf(r.x, -3.402823466e38f), fmaxf(r.y, -3.402823466e38f)));
-}
+__device__ __forceinline__ float mix3(float a, float b, float c) { return (float)mix3((double)a, (double)b, (double)c); }
 __device__ __forceinline__ float4 mix_rows(float4 a, float4 b, float4 c) {
-    const float2 lo = mix3(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
-    const float2 hi = mix3(make_float2(a.z, a.w), make_float2(b.z, b.w), make_float2(c.z, c.w));
-    return make_float4(lo.x, lo.y, hi.x, hi.y);
-}
-// Rows that do not stay in L2 (8 x 1 M points at pd 16, 260 MB of them: 1.91 / 2.47 ms the passes of a call in doubles / floats)
-// are mixed in doubles; the bits are the same.
-constexpr u64 FLOAT_ITEMS = 5000000;
-__device__ __forceinline__ float mix3_in_double(float a, float b, float c) {
-    return (float)mix3((double)a, (double)b, (double)c);
-}
-__device__ __forceinline__ float4 mix_rows_in_double(float4 a, float4 b, float4 c) {
-    return make_float4(mix3_in_double(a.x, b.x, c.x), mix3_in_double(a.y, b.y, c.y), mix3_in_double(a.z, b.z, c.z),
-                       mix3_in_double(a.w, b.w, c.w));
+    return make_float4(mix3(a.x, b.x, c.x), mix3(a.y, b.y, c.y), mix3(a.z, b.z, c.z), mix3(a.w, b.w, c.w));
 }
 __device__ __forceinline__ double2 mix_rows(double2 a, double2 b, double2 c) {
     return make_double2(mix3(a.x, b.x, c.x), mix3(a.y, b.y, c.y));
 }
-__device__ __forceinline__ double2 mix_rows_in_double(double2 a, double2 b, double2 c) { return mix_rows(a, b, c); }
+// A finite float as a double 2^896 times smaller: its bits as they are, three places down.  The double's exponent counts on
+// from 0 as the float's did, and subnormal floats become subnormal doubles.  (Infinities and NaN would become numbers.)
+__device__ __forceinline__ double moved(float x) {
+    const long long w = (long long)__float_as_int(x) << 29;   // the sign four times over, of which the double has the first
+    return __hiloint2double((int)(w >> 32) & 0x8FFFFFFF, (int)w);
+}
+// The same products as mix3's, exact as there (2^896 / 4 and 2^896 / 2 times the moved numbers): the same sums and bits.
+__device__ __forceinline__ float mix3_moved(float a, float b, float c) {
+    return (float)__fma_rn(0x1p894, moved(c), __fma_rn(0x1p895, moved(b), PL_DMUL(0x1p894, moved(a))));
+}
+__device__ __forceinline__ float4 mix_rows_moved(float4 a, float4 b, float4 c) {
+    return make_float4(mix3_moved(a.x, b.x, c.x), mix3_moved(a.y, b.y, c.y), mix3_moved(a.z, b.z, c.z),
+                       mix3_moved(a.w, b.w, c.w));
+}
+__device__ __forceinline__ double2 mix_rows_moved(double2 a, double2 b, double2 c) { return mix_rows(a, b, c); }
+// z stays zero as long as all numbers given were finite, else it is NaN: which of the two mixes may be taken.
+__device__ __forceinline__ void look_for_finite(float2& z, float4 x) {
+    const float2 zero = make_float2(0.f, 0.f);
+    z = fma2(make_float2(x.z, x.w), zero, fma2(make_float2(x.x, x.y), zero, z));
+}
+__device__ __forceinline__ void look_for_finite(float2&, double2) {}
+__device__ __forceinline__ bool all_finite(float2 z) { return PL_FADD(z.x, z.y) == 0.f; }
+
+// Beyond so many pieces of 16 bytes the rows do not stay in L2, and conversions are as fast as moves or faster: 8 x 512x512 x 21
+// of a noisy lattice (20 M pieces) 3768 / 3841 us a call.
+constexpr u64 MOVED_ITEMS = 5000000;
 
 template <typename V>
 __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src,
@@ -87,8 +87,15 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
             e += stride;
         }
     };
-    if (items <= FLOAT_ITEMS) rows([](V a, V b, V c) { return mix_rows(a, b, c); });
-    else rows([](V a, V b, V c) { return mix_rows_in_double(a, b, c); });
+    auto moving = [](V a, V b, V c) {
+        float2 z = make_float2(0.f, 0.f);
+        look_for_finite(z, a);
+        look_for_finite(z, b);
+        look_for_finite(z, c);
+        return all_finite(z) ? mix_rows_moved(a, b, c) : mix_rows(a, b, c);
+    };
+    if (items <= MOVED_ITEMS) rows(moving);
+    else rows([](V a, V b, V c) { return mix_rows(a, b, c); });
 }
 template <typename V>
 __global__ void __launch_bounds__(256, 8)
@@ -103,8 +110,9 @@ blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restri
 // L2, whatever it does; larger ones are bound by their rows, of which this reads half as many again.
 // us a call: 4 x 180x240 x 3 59 -> 54, 512x512 x 3 in double, forward + backward, 185 -> 179, a CRF of 2 x 200x200 x 5 219 ->
 // 192; 900 k vertices of one float4 239 -> 254, which is why it ends at PAIR_ITEMS (see blur_in_pairs).
-// nbr_b null: pass a alone.
-constexpr int PAIR_CTAS = 5;
+// nbr_b null: pass a alone.  Four CTAs an SM, with five the mixes spill 64 bytes: 1024x1024 grey by RGB, forward + backward, 317.8 -> 312.0
+// us, a CRF of 2 x 200x200 x 5 199.1 -> 189.2.
+constexpr int PAIR_CTAS = 4;
 constexpr u64 PAIR_ITEMS = 1000000, PAIR_ITEMS_WORST = 300000;   // by the bound, by one that is the worst case
 template <typename V>
 __device__ __forceinline__ void blur_pair_rows(const Header* hdr, const int* __restrict__ nbr_a, const int* __restrict__ nbr_b,
@@ -136,9 +144,23 @@ __device__ __forceinline__ void blur_pair_rows(const Header* hdr, const int* __r
             lo[k] = n[k].x >= 0 ? src[(u32)n[k].x * vpr + j] : zero;
             hi[k] = n[k].y >= 0 ? src[(u32)n[k].y * vpr + j] : zero;
         }
+        float2 z = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int k = 0; k < 3; k++) mid[k] = mix_rows(lo[k], mid[k], hi[k]);
-        dst[e] = nb ? mix_rows(mid[1], mid[0], mid[2]) : mid[0];
+        for (int k = 0; k < 3; k++) {
+            look_for_finite(z, lo[k]);
+            look_for_finite(z, mid[k]);
+            look_for_finite(z, hi[k]);
+        }
+        if (all_finite(z)) {   // (and so is what pass a makes of them)
+#pragma unroll
+            for (int k = 0; k < 3; k++) mid[k] = mix_rows_moved(lo[k], mid[k], hi[k]);
+            if (nb) mid[0] = mix_rows_moved(mid[1], mid[0], mid[2]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; k++) mid[k] = mix_rows(lo[k], mid[k], hi[k]);
+            if (nb) mid[0] = mix_rows(mid[1], mid[0], mid[2]);
+        }
+        dst[e] = mid[0];
         e += stride;
         v = e / vpr;
         j = e - v * vpr;

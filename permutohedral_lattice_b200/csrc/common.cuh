@@ -409,8 +409,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     return *reinterpret_cast<float2*>(&d);
 }
 
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, make_float2(-1.f, -1.f), a); }
-
 // Vector reduction into global memory (sm_90+): one L2 operation per 16 bytes.
 __device__ __forceinline__ void red_add_v4(float* addr, float4 v) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v.x), "f"(v.y), "f"(v.z),

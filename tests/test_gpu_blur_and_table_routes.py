@@ -1,5 +1,5 @@
 """Bounds at which a call takes another route and must give the same bits (deterministic sums): two blur passes a launch or
-one, rows mixed in floats or (more than 5,000,000 float4 of them) in doubles, the table cleared with the header or by a launch of its own, for hash tables and for the direct index."""
+one, rows made doubles by moves of bits or (more than 5,000,000 float4 of them) by conversions, the table cleared with the header or by a launch of its own, for hash tables and for the direct index."""
 import numpy as np
 import pytest
 
@@ -39,12 +39,13 @@ def test_pairs_of_passes_give_the_bits_of_single_ones(plb, pd):
     assert float((single - pairs).norm() / single.norm()) <= 1e-12      # double sums in varying order
 
 
-def test_rows_mixed_in_doubles_give_the_bits_of_floats(plb):
-    """The same first channels beside 68 others: 330,000 rows of 18 float4, or of one."""
+def test_rows_mixed_by_moves_give_the_bits_of_conversions(plb):
+    """The same first channels beside 68 others: 330,000 rows of 18 float4, or of one.  Both signs, thirty binades."""
     import torch
     g = torch.Generator().manual_seed(3)
     pos = (60 * torch.randn((1, 60000, 5), generator=g)).cuda()
     x = torch.rand((1, 60000, 71), generator=g).cuda()          # below 1: the same fixed-point grid for both
+    x *= torch.exp2(-30 * torch.rand((1, 60000, 71), generator=g)).cuda() * (torch.randint(0, 2, (1, 60000, 71), generator=g) * 2 - 1).cuda()
     for reverse in (False, True):
         wide, ws = plb.filter_positions(x, pos, reverse, "deterministic", max_entries=0)
         assert plb.lattice_stats(ws).num_vertices * 18 > 5000000

@@ -59,7 +59,7 @@ def test_blur_around_its_limits(bound, channels, dtype, gpu, oracle):
 
 
 def test_blur_keeps_infinite_rows_infinite(gpu):
-    """A float sum that is infinite has no finite rest: it stays infinite, and other channels stay what they are."""
+    """An infinite row stays infinite, and other channels stay what they are."""
     import torch
     import permutohedral_lattice_b200 as plb
     rng = np.random.default_rng(89)
