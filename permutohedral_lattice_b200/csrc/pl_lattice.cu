@@ -485,10 +485,18 @@ static int launch_splat(const Geom& g, const float* input, Header* hdr, const in
                      : launch_splat_as<PD, VD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v0, vd, st);
 }
 
+// Whether the slice of wide rows overlaps the last blur pass (OV_SLICE or 0).  With fewer tiles than SMs not: of a grid that starts
+// while the pass leaves the GPU, four or five CTAs go to the first SMs that become free, and the others stay idle (12 k vertices of 2000
+// points at pd 5, 21 channels: the slice 25 / 8 us, the call 88 / 74).  The small blur leaves most SMs free for it.  Narrow rows read
+// too little for it to matter: the plain launch costs them 1 to 2 us.
+static int slice_overlap(const Geom& g, bool after_small_blur) {
+    return after_small_blur || g.num_tiles >= num_sms() ? OV_SLICE : 0;
+}
+
 // slice for rows of VP floats (CT > 0: of CT channels), or (VP = 0) of more than 32.
 template <int PD, int VP, int CT = 0>
 static int launch_slice(const Geom& g, float* output, const Header* hdr, const int2* tile_info, const u16* rec,
-                        const float* rec_w, const u32* list_ref, const float* vsrc, int vd, Watch watch, cudaStream_t st) {
+                        const float* rec_w, const u32* list_ref, const float* vsrc, int vd, Watch watch, int overlap, cudaStream_t st) {
     if constexpr (VP == 4) {
         PL_LAUNCH_AFTER(OV_SLICE, (slice_points<PD, CT>), tile_grid(g), Cfg<PD>::TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, watch);
     } else if constexpr (VP > 0) {
@@ -496,14 +504,14 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
         if (rows_cap > Cfg<PD>::SPLATS) rows_cap = Cfg<PD>::SPLATS;
         const size_t smem = SliceFast<PD, VP>::bytes(rows_cap);
         PL_TRY((ensure_dynamic_smem<slice_tiles_fast<PD, VP, CT>>(smem)));
-        PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_fast<PD, VP, CT>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, vd - 1, rows_cap, bulk_rows_ok(g, output, vd - 1) ? 1 : 0, watch);
+        PL_LAUNCH_AFTER(overlap, (slice_tiles_fast<PD, VP, CT>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, vd - 1, rows_cap, bulk_rows_ok(g, output, vd - 1) ? 1 : 0, watch);
     } else {
         const int rows_cap = rows_cap_for(PD, vd);
         const size_t fixed = sizeof(float) * Cfg<PD>::TP * SliceCfg<PD>::PW + sizeof(int) * Cfg<PD>::TP;
         const size_t smem = sizeof(float) * (size_t)rows_cap * padded_vd(vd) + fixed;
         if (smem > 200 * 1024) return PL_UNSUPPORTED_DIMS;
         PL_TRY((ensure_dynamic_smem<slice_tiles_generic<PD>>(smem)));
-        PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_generic<PD>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w,
+        PL_LAUNCH_AFTER(overlap, (slice_tiles_generic<PD>), tile_grid(g), Cfg<PD>::TP, smem, st, g, output, hdr, tile_info, rec, rec_w,
                                                                         list_ref, vsrc, vd, rows_cap, watch);
     }
     return PL_OK;
@@ -533,22 +541,28 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
 // Which calls take the kernels of small.cuh, by the bounds the host knows.  The index as far as its shared memory goes: 3074 entries
 // 17.8 (one cluster on global memory) -> 9.4 us, 7017 entries 20.7 -> 17, as long as the three wide launches by then.
 static bool small_index(const Layout& L) { return L.max_entries <= SMALL_MAX_ENTRIES; }
+// Whether a bound is the worst case, which lattices of points with nothing in common need and fill.  Other bounds are 1.5 times the
+// entries or more, of which a half at most are vertices, usually.
+static bool worst_case(const Geom& g, int pd, const Layout& L) { return L.max_entries >= (u64)g.batch * (u64)g.n * (u64)(pd + 1); }
 // A cluster for every 16 bytes of a row, as many as the GPU takes at once (two CTAs an SM while a thread has one vertex, else
-// one), or twice as many of the small ones.  Six passes, us, wide / in one launch, by the bound: 4096, 1 float4 a row 15 / 7, 3
-// float4 14 / 9; 12000, 1 float4 15 / 12; 30000, 6 float4 15 / 14.6, and five launches less for the host, which such calls
-// wait for: 2 x 100x100 x 21, forward + backward, 170 / 146 us.
+// one), or twice as many of the small ones.  Six passes, us, wide (a pass a launch) / in one launch, by the bound: 4096, 1 float4 a row 15 /
+// 7, 3 float4 14 / 9; 12000, 1 float4 15 / 12; 30000, 6 float4 15 / 14.6, and five launches less for the host, which such calls
+// wait for: 2 x 100x100 x 21, forward + backward, 170 / 146 us.  That is with a third of the bound or less in vertices.  Bounds of the worst
+// case may be all vertices, up to 22 k of them on eight SMs: us a call, two passes a launch / in one, 3 channels, pd 4, 12 k vertices 45 / 47,
+// 21 k 49 / 60; pd 8, 9 k 57 / 62, 18 k 58 / 75; pd 16, 10 k 83 / 92; pd 2, without a guide, 11 k 27.6 / 26.9, 24 k 31 / 42; pd 2, 1.1 k of
+// 9 k 42 / 38.  So they go on to a vertex a thread, up to pd 2 to two.
 constexpr int SMALL_PIECES = 4;   // vertices a thread of blur_small, at most
-static bool small_blur(const Layout& L, u32 vpr) {
+static bool small_blur(const Geom& g, int pd, const Layout& L, u32 vpr) {
     const u64 one_each = SMALL_CTAS * SMALL_THREADS;
-    return L.max_entries <= one_each ? vpr <= 64 : L.max_entries <= SMALL_PIECES * one_each && vpr <= 16;
+    if (L.max_entries <= one_each) return vpr <= 64;
+    const int pieces = !worst_case(g, pd, L) ? SMALL_PIECES : pd <= 2 ? 2 : 1;
+    return L.max_entries <= pieces * one_each && vpr <= 16;
 }
-// Two passes a launch (see blur_pair_rows), by what the bound says of the vertices: it is 1.5 times the entries or more, of which
-// a half at most are vertices, usually, unless it is the worst case, which lattices of points with nothing in common
-// need and fill.  us a call, a pass / two a launch: bounds of 393 k x 2 items, 115 k vertices (512x512 x 3 in double, forward
-// + backward) 185 / 179; worst cases filled by vertices: 240 k 99.3 / 98.2, 470 k 142 / 144, 960 k 239 / 254.
+// Two passes a launch (see blur_pair_rows), by what the bound says of the vertices.  us a call, a pass / two a launch: bounds
+// of 393 k x 2 items, 115 k vertices (512x512 x 3 in double, forward + backward) 185 / 179; worst cases filled by vertices: 240 k
+// 99.3 / 98.2, 470 k 142 / 144, 960 k 239 / 254.
 static bool blur_in_pairs(const Geom& g, int pd, const Layout& L, u32 vpr) {
-    const bool worst = L.max_entries >= (u64)g.batch * (u64)g.n * (u64)(pd + 1);
-    return L.max_entries * vpr <= (worst ? PAIR_ITEMS_WORST : PAIR_ITEMS);
+    return L.max_entries * vpr <= (worst_case(g, pd, L) ? PAIR_ITEMS_WORST : PAIR_ITEMS);
 }
 template <int PD, int KW>
 static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
@@ -723,7 +737,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     float* src = v0;
     float* dst = v1;
     const u32 qpr = (u32)padded_vd(vd) / 4;
-    if (small_blur(L, qpr)) {
+    if (small_blur(g, PD, L, qpr)) {
         PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, st));
         PL_COUNT_LAUNCHES(1);
     } else if (blur_in_pairs(g, PD, L, qpr)) {
@@ -742,7 +756,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         PL_COUNT_LAUNCHES(1);
     }
     if (ev) PL_CUDA(cudaEventRecord(ev[4], st));
-    rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch, st);
+    rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch, slice_overlap(g, small_blur(g, PD, L, qpr)), st);
     if (rc != PL_OK) return rc;
     if (ev) PL_CUDA(cudaEventRecord(ev[5], st));
     PL_CUDA(cudaGetLastError());
@@ -822,7 +836,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
                                                                       list_ref, v0, vd);
     double* src = v0;
     double* dst = v1;
-    const bool one_blur = small_blur(L, (u32)vp / 2), pairs = blur_in_pairs(g, PD, L, (u32)vp / 2);
+    const bool one_blur = small_blur(g, PD, L, (u32)vp / 2), pairs = blur_in_pairs(g, PD, L, (u32)vp / 2);
     if (one_blur) {
         PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<double2*>(v0), (u32)vp / 2, PD + 1, reverse, st));
     } else if (pairs) {
@@ -898,12 +912,12 @@ static int launch_crf_splat(const Geom& g, const float* q, const LatticeRows& a,
 }
 template <int PDA, int PDS, int VP, int CT = 0>
 static int launch_crf_slices(const Geom& g, float* q_out, const float* unaries, const LatticeRows& a, const LatticeRows& s,
-                             const float* va, const float* vs, float wa, float ws, int labels, cudaStream_t st) {
+                             const float* va, const float* vs, float wa, float ws, int labels, bool blurred_small, cudaStream_t st) {
     const size_t smem = CrfSlices<PDA, PDS, VP>::bytes(labels);
     PL_TRY((ensure_dynamic_smem<crf_slices<PDA, PDS, VP, CT>>(smem)));
     // (an even number of labels is spread to an odd stride, which a bulk copy cannot do)
     const bool bulk_in = (labels & 1) && bulk_rows_ok(g, unaries, labels), bulk_out = bulk_rows_ok(g, q_out, labels);
-    PL_LAUNCH_AFTER(OV_SLICE, (crf_slices<PDA, PDS, VP, CT>), tile_grid(g), Cfg<PDA>::TP, smem, st, g, q_out, unaries, a, s, va, vs, wa, ws, labels, bulk_in ? 1 : 0, bulk_out ? 1 : 0);
+    PL_LAUNCH_AFTER(slice_overlap(g, blurred_small), (crf_slices<PDA, PDS, VP, CT>), tile_grid(g), Cfg<PDA>::TP, smem, st, g, q_out, unaries, a, s, va, vs, wa, ws, labels, bulk_in ? 1 : 0, bulk_out ? 1 : 0);
     return PL_OK;
 }
 template <int PDA, int PDS>
@@ -915,7 +929,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     PL_LAUNCH_AFTER(OV_CLEAR, (crf_zero_rows), dim3(wide / 2, 2), 256, 0, st, a, s, quads);
     PL_TRY((vd == 22 ? launch_crf_splat<PDA, PDS, 22>(g, q, a, s, vd, st) : launch_crf_splat<PDA, PDS, 0>(g, q, a, s, vd, st)));
     // small lattices have all their passes in one launch each; else a launch a pass, both as long as S has some left
-    const bool small_a = small_blur(LA, quads), small_s = small_blur(LS, quads);
+    const bool small_a = small_blur(g, PDA, LA, quads), small_s = small_blur(g, PDS, LS, quads);
     const float *va = a.v0, *vs = s.v0;
     int launches = 3;
     if (small_s) {
@@ -947,7 +961,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
         if (pass_s) vs = (step & 1) ? s.v0 : s.v1;
     }
     PL_COUNT_LAUNCHES(launches);
-#define PL_CRF_SLICES(VP_, ...) launch_crf_slices<PDA, PDS, VP_, ##__VA_ARGS__>(g, q_out, unaries, a, s, va, vs, wa, wsp, labels, st)
+#define PL_CRF_SLICES(VP_, ...) launch_crf_slices<PDA, PDS, VP_, ##__VA_ARGS__>(g, q_out, unaries, a, s, va, vs, wa, wsp, labels, small_a && small_s, st)
     PL_TRY((labels == 21 ? PL_CRF_SLICES(24, 21)
             : vp == 8    ? PL_CRF_SLICES(8)
             : vp == 12   ? PL_CRF_SLICES(12)

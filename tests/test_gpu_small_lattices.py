@@ -1,7 +1,7 @@
 """The index of small lattices in shared memory and their blur in clusters, around the sizes where the wide kernels take over:
 by the bound on the entries (10240) for the index; for the blur 1, 2 and 4 vertices a thread of a cluster (bounds of 8192,
-16384, 32768) and the number of clusters, one for 16 bytes of a row (64, which only rows of doubles reach; beyond 8192
-entries 16)."""
+16384, 32768; where the bound is the worst case 1, up to pd 2 2) and the number of clusters, one for 16 bytes of a row (64, which
+only rows of doubles reach; beyond 8192 entries 16)."""
 import numpy as np
 import pytest
 
@@ -56,6 +56,35 @@ def test_blur_around_its_limits(bound, channels, dtype, gpu, oracle):
         # 32-bit sums of some tens of products in another order, as elsewhere; in 64 bits the same, 2^29 times finer
         rel = np.linalg.norm(out[0].cpu().numpy() - want) / np.linalg.norm(want)
         assert rel <= (1e-5 if dtype == "float32" else 1e-12), (pd, rel)
+
+
+@pytest.mark.parametrize("bound,channels", [(8193, 3), (8193, 63), (16384, 7), (16385, 3), (32768, 12), (32769, 12)])
+@pytest.mark.parametrize("pd", [2, 5, 16])
+def test_blur_of_bounds_below_the_worst_case(bound, channels, pd, gpu):
+    """Every point twice: a bound of half the worst case, all of it vertices.  The bits of a lattice with room for the worst."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(97)
+    n = bound // (pd + 1)
+    pos = torch.from_numpy(np.repeat((rng.standard_normal((1, n, pd)) * 60).astype(np.float32), 2, 1)).cuda()
+    x = torch.from_numpy(rng.random((1, 2 * n, channels), dtype=np.float32)).cuda()
+    for reverse in (False, True):
+        got = plb.filter_positions(x, pos, reverse, "deterministic", max_entries=bound)[0].clone()
+        want = plb.filter_positions(x, pos, reverse, "deterministic", max_entries=2 * n * (pd + 1))[0]
+        assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1500, 2000, 3600])
+def test_slice_of_few_tiles_behind_wide_passes(n, gpu, oracle):
+    """Fewer tiles than SMs, worst-case bounds beyond the small blur: the slice of wide rows is launched plainly."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(101)
+    pos = (rng.standard_normal((1, n, 5)) * 6).astype(np.float32)
+    for channels in (5, 21, 33):
+        val = rng.random((1, n, channels), dtype=np.float32)
+        out, _ = plb.filter_positions(torch.from_numpy(val).cuda(), torch.from_numpy(pos).cuda(), max_entries=0)
+        gpu.assert_outputs_close(out.cpu().numpy(), oracle.filter(val[0], pos[0]).out[None], "%d channels" % channels)
 
 
 def test_blur_keeps_infinite_rows_infinite(gpu):
