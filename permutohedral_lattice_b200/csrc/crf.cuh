@@ -133,7 +133,7 @@ crf_update(float* __restrict__ q_out, const float* __restrict__ unaries, const f
 
 // ---------------------------------------------------------------------------------------------
 // A whole mean-field step of a CRF whose two lattices, appearance (A) and smoothness (S), have tiles of the same points:
-// each stage of both in one launch, and the update in the slice.  On one image the stages are small kernels, bound by their
+// each stage of both in one launch (the blur passes of large lattices one after the other), and the update in the slice.  On one image the stages are small kernels, bound by their
 // launches and by nearly empty last waves: apart, a step is 17 launches, and the filtered distributions go through memory
 // once more each way.  375x500 x 21: 98 -> 65 us a step; 2 x 200x200 x 5, five steps and both builds, 360 -> 220.
 // ---------------------------------------------------------------------------------------------
@@ -186,13 +186,13 @@ crf_blur_pair(LatticeRows a, LatticeRows s, int only, int pair, u32 quads) {
     blur_pair_rows<float4>(l.hdr, nbr, 2 * pair + 1 <= (second ? PDS : PDA) ? nbr + 2 * l.max_entries : nullptr, src, dst, quads, blockIdx.x, gridDim.x);
 }
 
-// Pass `step` of both: A's rows go from v0 to v1 in even passes, S's too.
+// A pass of both, blockIdx.y 0 and 1.  (The fields of each by themselves; choosing between two LatticeRows spilled 40 bytes in place of
+// 8: 8 x 512x512 x 21 of noisy images 2266 -> 2076 us a step.)
 __global__ void __launch_bounds__(256, 8)
-crf_blur(LatticeRows a, LatticeRows s, int step, u32 quads) {
-    const LatticeRows& l = blockIdx.y ? s : a;
-    const float4* src = reinterpret_cast<const float4*>((step & 1) ? l.v1 : l.v0);
-    float4* dst = reinterpret_cast<float4*>((step & 1) ? l.v0 : l.v1);
-    blur_rows<float4>(l.hdr, l.nbr + 2 * (u64)step * l.max_entries, src, dst, quads, blockIdx.x, gridDim.x);
+crf_blur(const Header* hdr_a, const int* nbr_a, const float4* src_a, float4* dst_a, const Header* hdr_s, const int* nbr_s,
+         const float4* src_s, float4* dst_s, u32 quads) {
+    const bool second = blockIdx.y != 0;
+    blur_rows<float4>(second ? hdr_s : hdr_a, second ? nbr_s : nbr_a, second ? src_s : src_a, second ? dst_s : dst_a, quads, blockIdx.x, gridDim.x);
 }
 
 // Both slices and the update of a Potts model (see crf_update, whose arithmetic this is).  A thread a point: the tile's rows

@@ -920,6 +920,11 @@ static int launch_crf_slices(const Geom& g, float* q_out, const float* unaries, 
     PL_LAUNCH_AFTER(slice_overlap(g, blurred_small), (crf_slices<PDA, PDS, VP, CT>), tile_grid(g), Cfg<PDA>::TP, smem, st, g, q_out, unaries, a, s, va, vs, wa, ws, labels, bulk_in ? 1 : 0, bulk_out ? 1 : 0);
     return PL_OK;
 }
+// Pass by pass both lattices in one launch, as long as their rows may stay in L2 together: by the bounds, in pieces of 16 bytes.  us a step,
+// together / one after the other: 375x500 x 21 (2.5 M) 66.3 / 71.5; 2 x 500x640 x 21 (9 M) 152.5 / 157.6; 4 x 512x512 x 21 (14 M) 265 / 271; 4 x
+// 512x512 x 5 of noisy images (19 M) 208 / 212; 8 x 512x512 x 21 (26 M) 497 / 498; of noisy ones 2 x 512x512 x 21 (28 M) 468 / 450, 8 x
+// 512x512 x 12 (45 M) 920 / 866, 2000x3000 x 10 (75 M and more) 2051 / 1869, 8 x 512x512 x 21 (113 M) 2076 / 1872.
+constexpr u64 CRF_TOGETHER = 20000000;
 template <int PDA, int PDS>
 static int run_crf_step(const Geom& g, float* q_out, const float* q, const float* unaries, float wa, float wsp, int labels,
                         void* ws_a, const Layout& LA, void* ws_s, const Layout& LS, cudaStream_t st) {
@@ -950,15 +955,41 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
         if (pass_a) va = (pair & 1) ? a.v0 : a.v1;
         if (pass_s) vs = (pair & 1) ? s.v0 : s.v1;
     }
-    for (int step = 0; !pairs && step <= std::max(PDA, PDS); step++) {
-        const bool pass_a = !small_a && step <= PDA, pass_s = !small_s && step <= PDS;
-        if (!pass_a && !pass_s) continue;
-        const bool first = step == 0 && !small_a && !small_s;
-        const LatticeRows& one = pass_a ? a : s;
-        PL_LAUNCH_AFTER(first ? OV_BLUR0 : OV_BLUR, (crf_blur), dim3(pass_a && pass_s ? wide / 2 : wide, pass_a && pass_s ? 2 : 1), 256, 0, st, one, s, step, quads);
-        launches++;
-        if (pass_a) va = (step & 1) ? a.v0 : a.v1;
-        if (pass_s) vs = (step & 1) ? s.v0 : s.v1;
+    // a pass of one lattice, from v0 to v1 in even passes
+    struct Pass {
+        const int* nbr;
+        const float4* src;
+        float4* dst;
+    };
+    auto pass_of = [](const LatticeRows& l, int step) {
+        float4* const v[2] = {reinterpret_cast<float4*>(l.v0), reinterpret_cast<float4*>(l.v1)};
+        return Pass{l.nbr + 2 * (u64)step * l.max_entries, v[step & 1], v[1 - (step & 1)]};
+    };
+    bool first_pass = !small_a && !small_s;   // right behind the splat
+    auto rest_of = [&](const LatticeRows& l, int step, int pd, const float*& v) -> int {   // from pass `step` on
+        for (; step <= pd; step++) {
+            const Pass p = pass_of(l, step);
+            PL_LAUNCH_AFTER(first_pass ? OV_BLUR0 : OV_BLUR, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads);
+            first_pass = false;
+            launches++;
+            v = reinterpret_cast<const float*>(p.dst);
+        }
+        return PL_OK;
+    };
+    if (!pairs) {
+        int step = 0;
+        if (!small_a && !small_s && (LA.max_entries + LS.max_entries) * quads <= CRF_TOGETHER) {
+            for (; step <= std::min(PDA, PDS); step++) {
+                const Pass p = pass_of(a, step), q2 = pass_of(s, step);
+                PL_LAUNCH_AFTER(first_pass ? OV_BLUR0 : OV_BLUR, (crf_blur), dim3(wide / 2, 2), 256, 0, st, a.hdr, p.nbr, p.src, p.dst, s.hdr, q2.nbr, q2.src, q2.dst, quads);
+                first_pass = false;
+                launches++;
+                va = reinterpret_cast<const float*>(p.dst);
+                vs = reinterpret_cast<const float*>(q2.dst);
+            }
+        }
+        if (!small_a) PL_TRY(rest_of(a, step, PDA, va));
+        if (!small_s) PL_TRY(rest_of(s, step, PDS, vs));
     }
     PL_COUNT_LAUNCHES(launches);
 #define PL_CRF_SLICES(VP_, ...) launch_crf_slices<PDA, PDS, VP_, ##__VA_ARGS__>(g, q_out, unaries, a, s, va, vs, wa, wsp, labels, small_a && small_s, st)

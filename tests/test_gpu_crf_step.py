@@ -57,6 +57,14 @@ def test_step_through_lattices_of_any_size(plb, theta):
         assert float((crf.step(q, u) - want).abs().max()) <= 2e-5
 
 
+@pytest.mark.parametrize("shape,labels", [((1, 500, 500), 21), ((1, 700, 700), 21), ((2, 700, 700), 8)])
+def test_step_with_passes_together_and_one_after_the_other(plb, shape, labels):
+    """Noisy images: bounds of the worst case, 14, 26 and 26 million pieces of 16 bytes in both lattices."""
+    crf, q, u = _case(plb, shape, labels, theta=(1.5, 0.02, 0.4))
+    got = crf._fused_step(q, u)
+    assert float((got - _apart(crf, q, u)).abs().max()) <= 2e-5
+
+
 def test_steps_that_are_left_to_the_separate_calls(plb):
     import torch
     for shape, labels, channels in (((1, 30, 30), 3, 3), ((1, 30, 30), 32, 3), ((1, 30, 30), 5, 1), ((1, 9, 12, 14), 5, 1)):
