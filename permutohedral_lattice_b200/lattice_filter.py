@@ -627,6 +627,18 @@ def compute_positions(reference_image, spatial_dims, spatial_std, feature_std, d
     return pos
 
 
+@functools.lru_cache(maxsize=256)
+def _positions_workspace_bytes(batch, n, pd, vd, bound, f64, mode):
+    """What pl_workspace_bytes says of a positions call: asked once a size, as _Plan does for filter calls."""
+    nbytes = ctypes.c_size_t(0)
+    if f64:
+        rc = capi.lib().pl_workspace_bytes_f64(batch, n, pd, vd, 0, None, bound, ctypes.byref(nbytes))
+    else:
+        rc = capi.lib().pl_workspace_bytes(batch, n, pd, vd, 0, None, bound, capi.MODES[mode], ctypes.byref(nbytes))
+    capi.check(rc, "pl_workspace_bytes")
+    return nbytes.value
+
+
 def filter_positions(input_values, positions, reverse=False, mode="atomic", max_entries=None,
                      check=None, workspace=None, out=None, info=None):
     """The LatticeFilter functor (src/LatticeFilterKernel.h:28-38) on [batch, n, C] values at
@@ -655,14 +667,8 @@ def filter_positions(input_values, positions, reverse=False, mode="atomic", max_
         stream = _stream_handle(x.device)
 
         def launch(bound):
-            nbytes = ctypes.c_size_t(0)
-            if f64:
-                rc = capi.lib().pl_workspace_bytes_f64(batch, n, pd, vd, 0, None, int(bound), ctypes.byref(nbytes))
-            else:
-                rc = capi.lib().pl_workspace_bytes(batch, n, pd, vd, 0, None, int(bound), capi.MODES[mode],
-                                                   ctypes.byref(nbytes))
-            capi.check(rc, "pl_workspace_bytes")
-            w = workspace if workspace is not None else _workspace(x.device, stream, nbytes.value)
+            nbytes = _positions_workspace_bytes(batch, n, pd, vd, int(bound), f64, mode)
+            w = workspace if workspace is not None else _workspace(x.device, stream, nbytes)
             head = (out.data_ptr(), x.data_ptr(), p.data_ptr(), batch, n, pd, vd, int(bool(reverse)),
                     w.data_ptr(), w.numel(), int(bound))
             if f64:
