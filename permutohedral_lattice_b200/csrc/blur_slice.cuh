@@ -109,7 +109,7 @@ blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restri
 // pass of a lattice whose items (16 bytes of a row) fit the GPU's threads about once takes its launch and one round trip to
 // L2, whatever it does; larger ones are bound by their rows, of which this reads half as many again.
 // us a call: 4 x 180x240 x 3 59 -> 54, 512x512 x 3 in double, forward + backward, 185 -> 179, a CRF of 2 x 200x200 x 5 219 ->
-// 192; 900 k vertices of one float4 239 -> 254, which is why it ends at PAIR_ITEMS (see blur_in_pairs).
+// 189; 900 k vertices of one float4 239 -> 254, which is why it ends at PAIR_ITEMS (see blur_in_pairs).
 // nbr_b null: pass a alone.  Four CTAs an SM, with five the mixes spill 64 bytes: 1024x1024 grey by RGB, forward + backward, 317.8 -> 312.0
 // us, a CRF of 2 x 200x200 x 5 199.1 -> 189.2.
 constexpr int PAIR_CTAS = 4;

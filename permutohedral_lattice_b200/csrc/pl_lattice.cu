@@ -548,14 +548,14 @@ static bool worst_case(const Geom& g, int pd, const Layout& L) { return L.max_en
 // one), or twice as many of the small ones.  Six passes, us, wide (a pass a launch) / in one launch, by the bound: 4096, 1 float4 a row 15 /
 // 7, 3 float4 14 / 9; 12000, 1 float4 15 / 12; 30000, 6 float4 15 / 14.6, and five launches less for the host, which such calls
 // wait for: 2 x 100x100 x 21, forward + backward, 170 / 146 us.  That is with a third of the bound or less in vertices.  Bounds of the worst
-// case may be all vertices, up to 22 k of them on eight SMs: us a call, two passes a launch / in one, 3 channels, pd 4, 12 k vertices 45 / 47,
-// 21 k 49 / 60; pd 8, 9 k 57 / 62, 18 k 58 / 75; pd 16, 10 k 83 / 92; pd 2, without a guide, 11 k 27.6 / 26.9, 24 k 31 / 42; pd 2, 1.1 k of
-// 9 k 42 / 38.  So they go on to a vertex a thread, up to pd 2 to two.
+// case may be all vertices, up to 32 k of them on eight SMs, and go on to two vertices a thread: us a call, two passes a launch / in one, 3
+// channels, pd 4, 12 k vertices 45 / 47, 21 k 49 / 60; pd 8, 9 k 57 / 62, 18 k 58 / 75; pd 16, 10 k 83 / 92, 25 k 86 / 116; without a guide 24 k
+// 31 / 42; few vertices, bounds of 9000 and 10000, pd 5 30 / 27, pd 4 30 / 26.6, pd 2 42 / 38.
 constexpr int SMALL_PIECES = 4;   // vertices a thread of blur_small, at most
 static bool small_blur(const Geom& g, int pd, const Layout& L, u32 vpr) {
     const u64 one_each = SMALL_CTAS * SMALL_THREADS;
     if (L.max_entries <= one_each) return vpr <= 64;
-    const int pieces = !worst_case(g, pd, L) ? SMALL_PIECES : pd <= 2 ? 2 : 1;
+    const int pieces = worst_case(g, pd, L) ? 2 : SMALL_PIECES;
     return L.max_entries <= pieces * one_each && vpr <= 16;
 }
 // Two passes a launch (see blur_pair_rows), by what the bound says of the vertices.  us a call, a pass / two a launch: bounds

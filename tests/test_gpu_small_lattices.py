@@ -1,6 +1,6 @@
 """The index of small lattices in shared memory and their blur in clusters, around the sizes where the wide kernels take over:
 by the bound on the entries (10240) for the index; for the blur 1, 2 and 4 vertices a thread of a cluster (bounds of 8192,
-16384, 32768; where the bound is the worst case 1, up to pd 2 2) and the number of clusters, one for 16 bytes of a row (64, which
+16384, 32768; where the bound is the worst case 1 and 2) and the number of clusters, one for 16 bytes of a row (64, which
 only rows of doubles reach; beyond 8192 entries 16)."""
 import numpy as np
 import pytest
