@@ -37,12 +37,6 @@ __device__ __forceinline__ bool direct_slot(const Direct& d, const Key<Cfg<PD>::
 __global__ void clear_direct(Header* hdr, u32* __restrict__ table, u64 slots) {
     after_previous_kernel();
     if (hdr->status != 0) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        u32 lg = 0;
-        while ((1ull << lg) < slots) lg++;
-        hdr->table_log2 = lg;
-        hdr->direct = 1;
-    }
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += (u64)gridDim.x * blockDim.x)
         table[i] = DIRECT_EMPTY;
 }
@@ -58,6 +52,12 @@ insert_direct(Header* hdr, Direct d, u32* __restrict__ table, const Key<Cfg<PD>:
     __shared__ InsertRound rd;
     if (threadIdx.x == 0) rd.count = 0;
     if (call_failed(hdr)) return;   // (its barrier also publishes rd.count)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // (here, whoever cleared the index: not of a call that failed before it)
+        u32 lg = 0;
+        while ((1ull << lg) < d.slots) lg++;
+        hdr->table_log2 = lg;
+        hdr->direct = 1;
+    }
     const u32 T = hdr->num_entries;
     const u32 stride = gridDim.x * 256u;
     for (u32 start = blockIdx.x * 256u; start < T;) {

@@ -13,23 +13,14 @@ namespace pl {
 // 48x64 x 3 52 / 46, 4 x 180x240 x 3 60 / 57, 60x70 x 2 without a guide 32 / 28.  (By build_tiles, a share a tile, it cost calls without any
 // 0.7 %.)
 struct ClearTable {
-    uint4* table;       // null: a launch of its own does
-    u32 quads;          // 16 bytes each
-    u32 direct_log2;    // direct indexing: the logarithm of its slots; 0: a hash table
+    uint4* table;   // null: a launch of its own does
+    u32 quads;      // 16 bytes each
 };
 constexpr u32 CLEAR_QUADS = 1u << 19;   // 8 MB, at most
 __global__ void __launch_bounds__(256) clear_header(Header* hdr, u32 quads, ClearTable clear) {
     after_previous_kernel();
-    if (blockIdx.x == 0) {
+    if (blockIdx.x == 0)
         for (u32 i = threadIdx.x; i < quads; i += 256) reinterpret_cast<uint4*>(hdr)[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (clear.direct_log2) {
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                hdr->direct = 1;
-                hdr->table_log2 = clear.direct_log2;
-            }
-        }
-    }
     for (u32 i = blockIdx.x * 256 + threadIdx.x; i < clear.quads; i += gridDim.x * 256)
         clear.table[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
 }

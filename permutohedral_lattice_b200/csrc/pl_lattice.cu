@@ -345,12 +345,11 @@ static bool make_direct(Direct& d, const Geom& g, int pd, const Layout& L) {
 // What clear_header clears for the index stage (see ClearTable): the direct index, or the hash table of a call that keeps no
 // sketch, whose size its bound gives.  A small lattice's table lies elsewhere.
 static ClearTable table_to_clear(const Direct* direct, const Layout& L, void* table, int sketch_shift, bool small) {
-    ClearTable c = {nullptr, 0u, 0u};
+    ClearTable c = {nullptr, 0u};
     const u64 bytes = direct ? sizeof(u32) * direct->slots : (L.key_slots ? 16ull : 8ull) * L.table_slots;
     if (small || (!direct && sketch_shift >= 0) || bytes > 16ull * CLEAR_QUADS) return c;
     c.table = static_cast<uint4*>(table);
     c.quads = (u32)((bytes + 15) / 16);   // (regions are 256-byte aligned: so is the end)
-    if (direct) while ((1ull << c.direct_log2) < direct->slots || c.direct_log2 == 0) c.direct_log2++;
     return c;
 }
 

@@ -108,3 +108,18 @@ def test_spatial_only_lattice_reuse(gpu, oracle):
         want = oracle.lattice_filter(inp, None, False, 1.0, 1.0, 3.0, reverse)
         got = lat.apply(torch.from_numpy(inp).cuda(), reverse=reverse)
         gpu.assert_outputs_close(got.cpu().numpy(), want, "reuse")
+
+
+@pytest.mark.parametrize("shape,theta,bound", [((512, 512), 3.0, 40000), ((1500, 1500), 1.0, 2200000)])
+def test_a_call_that_outgrew_its_bound_reports_no_index(gpu, shape, theta, bound):
+    """The index, cleared with the header (1 MB) or by a launch of its own (29 MB), is not built by a call that failed before."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    x = torch.rand((1,) + shape + (1,), device="cuda")
+    for dtype in (torch.float32, torch.float64):
+        out, ws, _ = plb.lattice_filter_raw(x.to(dtype), None, False, 1.0, 1.0, theta, max_entries=bound, check=False)
+        st = plb.lattice_stats(ws)
+        assert st.device_status == plb.capi.PL_CAPACITY_EXCEEDED and torch.isnan(out).all()
+        assert st.direct_index == 0 and st.table_slots == 1
+        out, ws, _ = plb.lattice_filter_raw(x.to(dtype), None, False, 1.0, 1.0, theta, max_entries=2 * bound)
+        assert plb.lattice_stats(ws).direct_index == 1 and torch.isfinite(out).all()
