@@ -17,6 +17,7 @@ struct ClearTable {
     u32 quads;      // 16 bytes each
 };
 constexpr u32 CLEAR_QUADS = 1u << 19;   // 8 MB, at most
+static_assert(2 * SKETCH_MIN_ENTRIES <= CLEAR_QUADS, "the largest table of a call without a sketch, slots of 16 bytes");
 __global__ void __launch_bounds__(256) clear_header(Header* hdr, u32 quads, ClearTable clear) {
     after_previous_kernel();
     if (blockIdx.x == 0)
@@ -560,11 +561,16 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 }
 
 // ---------------------------------------------------------------------------------------------
-// clear_table: table capacity chosen on the device, a power of two: at least twice the entries (at least 1024),
-// or, where the call kept a sketch of the lattice's size, at least four times the vertices it tells of (twice
-// as many cost the probe chains of insert_entries more than the smaller table gained it), in a table of keys beyond
-// 32 MB at least twice.
+// Table capacity, chosen on the device, a power of two: at least twice the entries (at least 1024), in calls that keep a sketch of
+// the lattice's size at least four times the vertices it tells of if that is less (twice as many cost the probe chains of insert_entries
+// more than the smaller table gained it), in a table of keys beyond 32 MB at least twice.
+// clear_table: calls with a sketch (clear_header has cleared the table of all others).
 // ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ u32 log2_of_slots(u64 need, u32 max_log2) {
+    u32 lg = 10;
+    while (lg < max_log2 && (1ull << lg) < need) lg++;
+    return lg;
+}
 constexpr u64 KEY_SLOTS_WHOLE = 1ull << 21;   // 32 MB
 constexpr u64 TAG_SLOTS_WHOLE = 1ull << 23;   // 64 MB
 constexpr u64 TAG_SLOTS_MOST = 1ull << 25;    // beyond, half as many would not stay in L2 either
@@ -575,7 +581,7 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
     if (hdr->status != 0) return;
     __shared__ u32 bits_s[8];
     u64 need = 2ull * hdr->num_entries;
-    if (sketch_shift >= 0 && need > (1ull << (sketch_shift + 10))) {
+    if (need > (1ull << (sketch_shift + 10))) {
         const uint4* sketch = reinterpret_cast<const uint4*>(hdr + 1);
         u32 bits = 0;
 #pragma unroll
@@ -609,8 +615,7 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
             need = slots < need ? slots : need;
         }
     }
-    u32 lg = 10;
-    while (lg < max_log2 && (1ull << lg) < need) lg++;
+    const u32 lg = log2_of_slots(need, max_log2);
     const u32 filter_log2 =
         (!KEY_SLOTS && lg >= FILTER_MIN_LOG2 && lg < max_log2) ? min(lg + FILTER_BITS_LOG2, FILTER_MAX_LOG2) : 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -654,8 +659,7 @@ constexpr int INSERT_CHUNKS = 8;
 // has chosen it (see there).  By all threads of an insert launch alike; one of them tells the lookups after it.
 __device__ __forceinline__ u32 table_log2_of(Header* hdr, u32 entries, u32 max_log2, bool cleared) {
     if (!cleared) return hdr->table_log2;
-    u32 lg = 10;
-    while (lg < max_log2 && (1ull << lg) < 2ull * entries) lg++;
+    const u32 lg = log2_of_slots(2ull * entries, max_log2);
     if (blockIdx.x == 0 && threadIdx.x == 0) hdr->table_log2 = lg;
     return lg;
 }
