@@ -301,6 +301,18 @@ class _Plan:
             nbytes = self._bytes[key] = self.call.workspace_bytes(bound, self.dtype, mode)
         return nbytes
 
+    def launch(self, out, x, ref, reverse, mode, ws, bound, stream):
+        """The call itself, on contiguous tensors of this geometry with their device current."""
+        c = self.call
+        head = (out.data_ptr(), x.data_ptr(), 0 if ref is None else ref.data_ptr(), c.batch, len(c.sdims), c.c_sdims,
+                c.c, c.r, c.bilateral, *c.theta, bool(reverse), ws.data_ptr(), ws.numel(), bound)
+        if self.f32:
+            rc = capi.lib().pl_lattice_filter_f32(*head, capi.MODES[mode], stream)
+        else:
+            rc = capi.lib().pl_lattice_filter_f64(*head, stream)
+        if rc != capi.PL_OK:
+            capi.check(rc, "pl_lattice_filter_f32" if self.f32 else "pl_lattice_filter_f64")
+
 
 _plans = {}        # arguments of a call that fix its geometry -> _Plan; emptied when it has grown to MOST_PLANS
 MOST_PLANS = 256
@@ -348,7 +360,6 @@ def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha
         out = torch.empty_like(x)
     if call.batch == 0 or call.n == 0:
         return out, None, call
-    L = capi.lib()
     stream = _stream_handle(x.device)
     owner = stream if workspace_owner is None else workspace_owner
 
@@ -356,16 +367,7 @@ def lattice_filter_raw(input_image, reference_image, bilateral=True, theta_alpha
         ws = workspace
         if ws is None:
             ws = _workspace(x.device, owner, plan.bytes(bound, mode))
-        head = (out.data_ptr(), x.data_ptr(), 0 if ref is None else ref.data_ptr(), call.batch,
-                len(call.sdims), call.c_sdims, call.c, call.r, call.bilateral,
-                call.theta[0], call.theta[1], call.theta[2], bool(reverse), ws.data_ptr(),
-                ws.numel(), bound)
-        if f64:
-            rc = L.pl_lattice_filter_f64(*head, stream)
-        else:
-            rc = L.pl_lattice_filter_f32(*head, capi.MODES[mode], stream)
-        if rc != capi.PL_OK:
-            capi.check(rc, "pl_lattice_filter_f64" if f64 else "pl_lattice_filter_f32")
+        plan.launch(out, x, ref, reverse, mode, ws, bound, stream)
         return ws
 
     with _OnDevice(x.device):
@@ -398,21 +400,13 @@ def _filter(input_image, reference_image, bilateral, theta_alpha, theta_beta, th
         plan = _plans.get((index, x.dtype, x.shape, None if ref is None else ref.shape, bilateral, theta_alpha, theta_beta,
                            theta_gamma))
         if plan is not None and (plan.f32 or mode == "atomic"):
-            call, known = plan.call, _verified.get(plan.kind)
-            if known is not None and known[0] == _identity(ref, call.batch):
+            known = _verified.get(plan.kind)
+            if known is not None and known[0] == _identity(ref, plan.call.batch):
                 bound, stream = known[1], torch._C._cuda_getCurrentRawStream(index)
                 ws = _workspaces.get((index, stream))
                 if ws is not None and ws.numel() >= plan.bytes(bound, mode):
                     out = torch.empty_like(x)
-                    head = (out.data_ptr(), x.data_ptr(), 0 if ref is None else ref.data_ptr(), call.batch,
-                            len(call.sdims), call.c_sdims, call.c, call.r, call.bilateral, *call.theta,
-                            bool(reverse), ws.data_ptr(), ws.numel(), bound)
-                    if plan.f32:
-                        rc = capi.lib().pl_lattice_filter_f32(*head, capi.MODES[mode], stream)
-                    else:
-                        rc = capi.lib().pl_lattice_filter_f64(*head, stream)
-                    if rc != capi.PL_OK:
-                        capi.check(rc, "pl_lattice_filter_f32" if plan.f32 else "pl_lattice_filter_f64")
+                    plan.launch(out, x, ref, reverse, mode, ws, bound, stream)
                     return out
     return lattice_filter_raw(input_image, reference_image, bilateral, theta_alpha, theta_beta, theta_gamma, reverse, mode)[0]
 
