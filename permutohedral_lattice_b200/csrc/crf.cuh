@@ -135,7 +135,8 @@ crf_update(float* __restrict__ q_out, const float* __restrict__ unaries, const f
 // A whole mean-field step of a CRF whose two lattices, appearance (A) and smoothness (S), have tiles of the same points:
 // each stage of both in one launch (the blur passes of large lattices one after the other), and the update in the slice.  On one image the stages are small kernels, bound by their
 // launches and by nearly empty last waves: apart, a step is 17 launches, and the filtered distributions go through memory
-// once more each way.  375x500 x 21: 98 -> 65 us a step; 2 x 200x200 x 5, five steps and both builds, 360 -> 220.
+// once more each way.  375x500 x 21: 98 -> 66 us a step; 2 x 200x200 x 5, five steps and both builds, 360 -> 191; 16 x 512x512 x 21 1187 -> 964,
+// 16 x 512x512 x 8 864 -> 800, 8 x 512x512 x 21 of noisy images 2013 -> 1872, 2000x3000 x 10 1988 -> 1869.
 // ---------------------------------------------------------------------------------------------
 struct LatticeRows {   // a kept lattice, as its workspace holds it
     Header* hdr;
@@ -197,7 +198,7 @@ crf_blur(const Header* hdr_a, const int* nbr_a, const float4* src_a, float4* dst
 
 // Both slices and the update of a Potts model (see crf_update, whose arithmetic this is).  A thread a point: the tile's rows
 // of A are staged, mixed and normalised, then those of S in the same memory, while the unaries arrive; the message and
-// the logits stay in registers.
+// the logits stay in registers: 80 of them, for three CTAs an SM; from rows of 16 floats on 4 to 92 bytes are spilled (48 at 21 labels).
 template <int PDA, int PDS, int VP>
 struct CrfSlices {
     static constexpr int TP = Cfg<PDA>::TP, RS = VP + 4;

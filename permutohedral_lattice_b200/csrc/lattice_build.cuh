@@ -7,7 +7,8 @@
 namespace pl {
 
 // The header and the sketch before a call.  A kernel and not a memset, so that build_tiles can start beside it (the gap between a memset and the
-// build, 3 to 4 us a call: 8 x 512x512 x 21, pd 2, forward + backward, 431 -> 425; 512x512 x 3 in double 188.5 -> 185.5).
+// build, 3 to 4 us a call: 8 x 512x512 x 21, pd 2, forward + backward, 431 -> 425; 512x512 x 3 in double 188.5 -> 185.5).  The host needs a
+// microsecond more for it.
 // It also clears (to ones: empty slots) what the index stage needs where the host knows how much that may be, the direct index
 // or the table of a call without a sketch, so that no launch between the build and the insert has to: us a call, 2 x
 // 48x64 x 3 52 / 46, 4 x 180x240 x 3 60 / 57, 60x70 x 2 without a guide 32 / 28.  (By build_tiles, a share a tile, it cost calls without any
