@@ -537,12 +537,17 @@ static int launch_slice(const Geom& g, float* output, const Header* hdr, const i
      : padded_vd(vd) == 32 ? launch_slice<PD_, 32>(__VA_ARGS__) \
                            : launch_slice<PD_, 0>(__VA_ARGS__))
 
-// Which calls take the kernels of small.cuh, by the bounds the host knows.  The index as far as its shared memory goes: 3074 entries
-// 17.8 (one cluster on global memory) -> 9.4 us, 7017 entries 20.7 -> 17, as long as the three wide launches by then.
-static bool small_index(const Layout& L) { return L.max_entries <= SMALL_MAX_ENTRIES; }
 // Whether a bound is the worst case, which lattices of points with nothing in common need and fill.  Other bounds are 1.5 times the
 // entries or more, of which a half at most are vertices, usually.
 static bool worst_case(const Geom& g, int pd, const Layout& L) { return L.max_entries >= (u64)g.batch * (u64)g.n * (u64)(pd + 1); }
+// Which calls take the kernels of small.cuh, by the bounds the host knows.  The index as far as its shared memory goes: 3074 entries
+// 17.8 (one cluster on global memory) -> 9.4 us, 7017 entries 20.7 -> 17, as long as the three wide launches by then.  With pd 4 and 5 an
+// entry takes 16 bytes beside the table, which is left 2.1 slots an entry at 9216 of them and 1.5 at 10240, too few: us a call, small / wide,
+// all of the bound vertices, pd 4, 9200 50 / 44, 10200 71 / 44, pd 5 52 / 47 and 66 / 47 (few of them: 24 / 27); other pd 41 / 40 to 93 / 87 at
+// 10200.  So bounds of the worst case end there.
+static bool small_index(const Geom& g, int pd, const Layout& L) {
+    return L.max_entries <= (worst_case(g, pd, L) && (pd == 4 || pd == 5) ? 9216u : SMALL_MAX_ENTRIES);
+}
 // A cluster for every 16 bytes of a row, as many as the GPU takes at once (two CTAs an SM while a thread has one vertex, else
 // one), or twice as many of the small ones.  Six passes, us, wide (a pass a launch) / in one launch, by the bound: 4096, 1 float4 a row 15 /
 // 7, 3 float4 14 / 9; 12000, 1 float4 15 / 12; 30000, 6 float4 15 / 14.6, and five launches less for the host, which such calls
@@ -630,7 +635,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     bool use_direct = false, small = false, cleared = false;
     if (phases & PH_BUILD) {
         if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
-        small = !use_direct && small_index(L);
+        small = !use_direct && small_index(g, PD, L);
         const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, L, table, sketch_shift, small);
         cleared = clear.table != nullptr;
         PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));
@@ -788,7 +793,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     Direct direct;
     bool use_direct = false;
     if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
-    const bool small = !use_direct && small_index(L);
+    const bool small = !use_direct && small_index(g, PD, L);
     const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, L, table, sketch_shift, small);
     const bool cleared = clear.table != nullptr;
     PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));

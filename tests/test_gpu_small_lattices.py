@@ -1,5 +1,5 @@
 """The index of small lattices in shared memory and their blur in clusters, around the sizes where the wide kernels take over:
-by the bound on the entries (10240) for the index; for the blur 1, 2 and 4 vertices a thread of a cluster (bounds of 8192,
+by the bound on the entries (10240; pd 4 and 5 9216 where that is the worst case) for the index; for the blur 1, 2 and 4 vertices a thread of a cluster (bounds of 8192,
 16384, 32768; where the bound is the worst case 1 and 2) and the number of clusters, one for 16 bytes of a row (64, which
 only rows of doubles reach; beyond 8192 entries 16)."""
 import numpy as np
@@ -37,6 +37,27 @@ def test_index_around_its_largest_bound(pd, spread, bound, batch, gpu, oracle):
     vk, vi, pv, pw = plb.export_lattice(ws, st, batch, n, pd, 3, positions=pt)
     gpu.assert_structure_equal(vk, vi, pv, pw, items, "pd %d" % pd)
     gpu.assert_outputs_close(out.cpu().numpy(), np.stack([o.out for o in items]), "pd %d" % pd)
+
+
+@pytest.mark.parametrize("pd", [2, 4, 5, 8])
+@pytest.mark.parametrize("bound,twice", [(9216, False), (9217, False), (MOST, True)])
+def test_index_with_its_table_at_its_fullest(pd, bound, twice, gpu, oracle):
+    """All keys distinct: as many entries as the bound has room for, of the worst case or (every point twice) of half of it."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    rng = np.random.default_rng(81)
+    n = bound // (pd + 1)
+    pos = (rng.standard_normal((1, n, pd)) * 60).astype(np.float32)
+    if twice:
+        pos = np.repeat(pos, 2, 1)
+    val = rng.random((1, pos.shape[1], 2), dtype=np.float32)
+    pt, xt = torch.from_numpy(pos).cuda(), torch.from_numpy(val).cuda()
+    item = oracle.filter(val[0], pos[0])
+    out, ws = plb.filter_positions(xt, pt, max_entries=bound)
+    st = plb.lattice_stats(ws)
+    vk, vi, pv, pw = plb.export_lattice(ws, st, 1, pos.shape[1], pd, 3, positions=pt)
+    gpu.assert_structure_equal(vk, vi, pv, pw, [item], "pd %d" % pd)
+    gpu.assert_outputs_close(out.cpu().numpy(), item.out[None], "pd %d" % pd)
 
 
 @pytest.mark.parametrize("bound,channels", [(2048, 127), (2048, 130), (8192, 3), (8192, 16), (8193, 63), (8193, 64), (16384, 7),
