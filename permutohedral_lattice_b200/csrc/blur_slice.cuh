@@ -1,5 +1,6 @@
 // Blur passes over the vertex rows and the slice stage (interpolate, normalise, write out).
 #pragma once
+#include <type_traits>
 #include "common.cuh"
 
 namespace pl {
@@ -87,15 +88,19 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
             e += stride;
         }
     };
-    auto moving = [](V a, V b, V c) {
-        float2 z = make_float2(0.f, 0.f);
-        look_for_finite(z, a);
-        look_for_finite(z, b);
-        look_for_finite(z, c);
-        return all_finite(z) ? mix_rows_moved(a, b, c) : mix_rows(a, b, c);
-    };
-    if (items <= MOVED_ITEMS) rows(moving);
-    else rows([](V a, V b, V c) { return mix_rows(a, b, c); });
+    if constexpr (std::is_same<V, float4>::value) {
+        if (items <= MOVED_ITEMS) {
+            rows([](V a, V b, V c) {
+                float2 z = make_float2(0.f, 0.f);
+                look_for_finite(z, a);
+                look_for_finite(z, b);
+                look_for_finite(z, c);
+                return all_finite(z) ? mix_rows_moved(a, b, c) : mix_rows(a, b, c);
+            });
+            return;
+        }
+    }
+    rows([](V a, V b, V c) { return mix_rows(a, b, c); });
 }
 template <typename V>
 __global__ void __launch_bounds__(256, 8)
