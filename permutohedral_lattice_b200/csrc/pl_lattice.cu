@@ -486,7 +486,7 @@ static int launch_splat(const Geom& g, const float* input, Header* hdr, const in
 
 // Whether the slice of wide rows overlaps the last blur pass (OV_SLICE or 0).  With fewer tiles than SMs not: of a grid that starts
 // while the pass leaves the GPU, four or five CTAs go to the first SMs that become free, and the others stay idle (12 k vertices of 2000
-// points at pd 5, 21 channels: the slice 25 / 8 us, the call 88 / 74).  The small blur leaves most SMs free for it.  Narrow rows read
+// points at pd 5, 21 channels: the slice 25 / 8 us, the call 88 / 74; 8 x 79x38 x 30 in double 33 / 15 and 81 / 66).  The small blur leaves most SMs free for it.  Narrow rows read
 // too little for it to matter: the plain launch costs them 1 to 2 us.
 static int slice_overlap(const Geom& g, bool after_small_blur) {
     return after_small_blur || g.num_tiles >= num_sms() ? OV_SLICE : 0;
@@ -855,7 +855,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
-    PL_LAUNCH_AFTER(OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
+    PL_LAUNCH_AFTER(vd > 4 ? slice_overlap(g, one_blur) : OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
     PL_COUNT_LAUNCHES((small ? 2 : cleared ? 3 : 4) + 1 + (one_blur ? 1 : pairs ? PD / 2 + 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;

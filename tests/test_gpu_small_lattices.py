@@ -106,6 +106,10 @@ def test_slice_of_few_tiles_behind_wide_passes(n, gpu, oracle):
         val = rng.random((1, n, channels), dtype=np.float32)
         out, _ = plb.filter_positions(torch.from_numpy(val).cuda(), torch.from_numpy(pos).cuda(), max_entries=0)
         gpu.assert_outputs_close(out.cpu().numpy(), oracle.filter(val[0], pos[0]).out[None], "%d channels" % channels)
+        # in double: sums of some tens of products in another order
+        out, _ = plb.filter_positions(torch.from_numpy(val).double().cuda(), torch.from_numpy(pos).double().cuda(), max_entries=0)
+        want = oracle.filter(val[0].astype(np.float64), pos[0].astype(np.float64), dtype=np.float64).out
+        assert np.linalg.norm(out[0].cpu().numpy() - want) / np.linalg.norm(want) <= 1e-12
 
 
 def test_blur_keeps_infinite_rows_infinite(gpu):
