@@ -145,7 +145,7 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
 // vertices, so that walking down a piece of a column of points meets about as few runs as the sorted list cut into windows
 // does, and needs no sort.  One thread a piece and remainder; nothing goes through shared memory: a point's row is read
 // PD + 1 times, from L1 after the first, neighbouring threads on neighbouring points.  Sixteen points are cut into as many
-// pieces as give every thread one (5, 4 and 3 with pd 2, 3 and 4).
+// pieces as give every thread one (5, 4 and 3 with pd 2, 3 and 4), or two where many tiles share a vertex.
 // Bound by the latency of its loads (most stalls are for them; its reductions are none, L2 is at 34 %).  Two volumes of
 // 111x128x120 points, 20 splats an entry: sorted 106 us (LSU pipe at 82 %), in columns of eight points, which left 3 of 8 warps
 // without work, 87, so 83.  us a call, eight points / so: 16 x 512x512 x 1 without a guide 208 / 186, x 3 198 / 189; 96x128x128 x
@@ -175,6 +175,10 @@ struct NarrowColumns {
     static constexpr bool EVER = PD >= 2 && PD <= (PRE ? 3 : 4);
     static constexpr int AHEAD = PD == 4 ? 3 : VD == 3 && (PD == 2 || !PRE) ? 4 : 2;
     static constexpr int CTAS = !EVER ? 0 : AHEAD >= 3 ? 6 : 8;
+    // Where a vertex is shared by more tiles (entries a vertex), what counts is how often they add to it: pieces of eight points then.  us
+    // a call, pieces of 3 to 5 points / of eight: pd 2, 3 tiles a vertex 98.7 / 101.3, 4.5 104.7 / 101.3, 21 165 / 119, 76 381 / 199; pd 3, 6.8 79.0 / 80.0,
+    // 7 to 8 195 / 204 and 35.3 / 33.7, 26 95.6 / 86.2, 111 214 / 145; pd 4, 12.5 223 / 229, 18.8 75 / 72, 78 366 / 311.
+    static constexpr u32 SHARED = PD == 2 ? 4 : PD == 3 ? 10 : 16;
     static constexpr int LEAST = AHEAD >= 3 ? 8 : !PRE ? (PD == 2 ? 12 : 10) : VD == 3 ? 10 : 24;
 };
 // Few entries are not enough where a noisy guide sends neighbouring points to one and another of them: a column then
@@ -213,13 +217,15 @@ template <int PD, int VD, int AHEAD>
 __device__ __forceinline__ void splat_columns(const Geom& g, const TilePos& tpos, int base,
                                               const float* __restrict__ input, const u16* __restrict__ rec_tile,
                                               const float* __restrict__ recw_tile,
-                                              const u32* __restrict__ list_ref, float* __restrict__ v0) {
+                                              const u32* __restrict__ list_ref, float* __restrict__ v0, bool halves) {
     constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3;
-    constexpr int PIECES = TP / (16 * (PD + 1)), ALL = 16 * PIECES;   // of 16 points of a column; of a tile (TX columns of 256 / TX points)
-    const int r = (int)threadIdx.x / ALL, c = (int)threadIdx.x % ALL, lx = c & (g.TX - 1), s = c >> g.tx_log2, k = s % PIECES;
-    const int from = 16 * k / PIECES, ly = s / PIECES * 16 + from;
+    constexpr int PIECES = TP / (16 * (PD + 1));   // of 16 points of a column, or two; a tile has TX columns of 256 / TX points
+    const int tid = threadIdx.x, r = halves ? tid / 32 : tid / (16 * PIECES), c = halves ? tid % 32 : tid % (16 * PIECES);
+    const int lx = c & (g.TX - 1), s = c >> g.tx_log2, k = halves ? s % 2 : s % PIECES;
+    const int from = halves ? 8 * k : 16 * k / PIECES, to = halves ? from + 8 : 16 * (k + 1) / PIECES;
+    const int ly = (halves ? s / 2 : s / PIECES) * 16 + from;
     const int x = tpos.tx * g.TX + lx, y = tpos.ty * g.TY + ly;
-    const int rows = r <= PD && x < g.W ? min(16 * (k + 1) / PIECES - from, g.H - y) : 0;
+    const int rows = r <= PD && x < g.W ? min(to - from, g.H - y) : 0;
     if (rows <= 0) return;
     const u16* rp = rec_tile + r * TP + ly * g.TX + lx;
     const float* wp = recw_tile + r * TP + ly * g.TX + lx;
@@ -279,6 +285,8 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile;
     const int2 info = tile_info[tile];   // (in flight with the status)
+    bool halves = false;
+    if constexpr (NC::EVER) halves = hdr->num_entries > NC::SHARED * hdr->num_vertices;
     if (call_failed(hdr)) return;
     if (PRE && !lattice_is_sorted(hdr)) return;
     const int base = info.x, nloc = info.y;
@@ -286,7 +294,7 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     if constexpr (NC::EVER) {
         if (in_columns<PD>(g, nloc, NC::LEAST) && CS::smooth(g, tpos, hdr, rec, nloc, CS::NARROW)) {
             splat_columns<PD, VD, NC::AHEAD>(g, tpos, base, input, rec + (size_t)tile * SPLATS, rec_w + (size_t)tile * SPLATS,
-                                  list_ref, v0);
+                                  list_ref, v0, halves);
             let_next_kernel_start();
             return;
         }

@@ -65,3 +65,10 @@ def test_noisy_guides(shape, r, noise, gpu, oracle):
     """Few entries (theta 40), between which the noise sends neighbouring points: both sides of the rule on changes of entry
     from row to row."""
     _check(gpu, oracle, shape, [1, 2, 3, 5, 21, 64], r, 40.0, 7, noise)
+
+
+@pytest.mark.parametrize("shape,r,theta", [((100, 120), 0, 40.0), ((97, 33), 0, 12.0), ((30, 17, 33), 0, 6.0), ((30, 17, 33), 0, 40.0),
+                                           ((40, 35, 20), 1, 20.0), ((100, 70), 1, 60.0)])
+def test_vertices_that_many_tiles_share(shape, r, theta, gpu, oracle):
+    """Narrow rows in pieces of eight points, where a vertex has more than 4 (pd 2), 10 (pd 3) or 16 (pd 4) entries."""
+    _check(gpu, oracle, shape, [1, 2, 3], r, theta, 8)
