@@ -515,14 +515,13 @@ __device__ __forceinline__ void after_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// The two halves for kernels whose grid runs in several waves (the tile kernels): they let the next kernel
-// start only when their own work is nearly done.  Released at their start, the next kernel's CTAs sat on the
-// SMs beside the tile kernel's later waves and slowed them (measured: a call 15 % slower).
+// The first half alone, for kernels whose grid runs in several waves (the tile kernels) or whose CTAs all need their slots
+// to the end (the inserts): they never release the next kernel, which then starts when the last of their CTAs has ended.
+// Released at their start, the next kernel's CTAs sat on the SMs beside the tile kernel's later waves and slowed them (a
+// call 15 % slower); released by every thread ahead of its last row, the splat still cost the dense CRF 16 x 512x512 x 21
+// a tenth (forward + backward 1764 -> 1953 us).
 __device__ __forceinline__ void wait_for_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void let_next_kernel_start() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // First point and number of valid points of tile row `ly` (the run of points that is contiguous in

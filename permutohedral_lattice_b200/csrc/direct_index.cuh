@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256)
 insert_direct(Header* hdr, Direct d, u32* __restrict__ table, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
               u32* __restrict__ list_ref, u32* __restrict__ vid, Key<Cfg<PD>::KW>* __restrict__ vkeys,
               VertexInit vi) {
-    after_previous_kernel();
+    wait_for_previous_kernel();
     constexpr int KW = Cfg<PD>::KW;
     __shared__ InsertRound rd;
     if (threadIdx.x == 0) rd.count = 0;

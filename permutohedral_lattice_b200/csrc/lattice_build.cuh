@@ -737,7 +737,7 @@ template <int KW>
 __global__ void __launch_bounds__(256)
 insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>* __restrict__ list_keys,
                u32* __restrict__ list_ref, u32* __restrict__ vid, Key<KW>* __restrict__ vkeys, VertexInit vi, bool cleared) {
-    after_previous_kernel();
+    wait_for_previous_kernel();
     __shared__ InsertRound rd;
     if (threadIdx.x == 0) rd.count = 0;
     if (call_failed(hdr)) return;   // (its barrier also publishes rd.count)
@@ -837,7 +837,7 @@ template <int PD>
 __global__ void __launch_bounds__(256, 8)   // as many as it is launched with
 insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
             u32* __restrict__ list_ref, u32* __restrict__ vid, Key<Cfg<PD>::KW>* __restrict__ vkeys, VertexInit vi, bool cleared) {
-    after_previous_kernel();
+    wait_for_previous_kernel();
     constexpr int KW = Cfg<PD>::KW;
     __shared__ InsertRound rd;
     if (threadIdx.x == 0) rd.count = 0;

@@ -177,20 +177,15 @@ static cudaError_t launch_kernel(bool overlap, void (*kernel)(Params...), dim3 g
 }
 #define PL_LAUNCH(kernel, grid, block, smem, st, ...) \
     PL_CUDA(launch_kernel(false, kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
-// Which launches overlap the tail of the kernel before them (bits of PL_OVERLAP), each measured on its own
-// (B200, 16 items / 2 items of the dense-CRF workload, ms per forward + backward step, all others as chosen):
-// the blur passes after one another 2.023 -> 2.007 / 0.353 -> 0.342; the slice after the last pass and the
-// splat after link_neighbours -> 2.002 / 0.335; clear_table after build_tiles -> 1.993 / 0.331; insert_entries
-// after clear_table -> 1.992 / 0.328 (small tables only, see run_filter).  Left plain because they measured
-// slower at 16 items: link_neighbours
-// after insert_entries (index stage 0.175 -> 0.181 ms; in small calls it gains or loses 0.5 %) and the first
-// blur pass after the splat (2.09).
-enum { OV_BLUR = 1, OV_INSERT = 2, OV_SPLAT = 4, OV_BLUR0 = 8, OV_SLICE = 16, OV_CLEAR = 32, OV_LINK = 64, OV_BUILD = 128 };
-#ifndef PL_OVERLAP
-#define PL_OVERLAP (OV_BLUR | OV_INSERT | OV_SPLAT | OV_SLICE | OV_CLEAR | OV_BUILD)
-#endif
-#define PL_LAUNCH_AFTER(which, kernel, grid, block, smem, st, ...) \
-    PL_CUDA(launch_kernel((PL_OVERLAP & (which)) != 0, kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
+// A launch that may overlap the tail of the kernel before it: all but the first of a call and those whose callers say why not.
+// What each gave when it was measured by itself, all others as they are now, us a call or step, plain / overlapped: the blur passes after one
+// another, 16 and 2 items of 512x512 x 21, 2023 / 2007 and 353 / 342; the slice after the last pass and the splat after the link 2002 and 335;
+// clear_table after the build 1993 and 331; the insert after clear_table 1992 and 328.  The link after the insert and the first
+// blur pass after the splat, which gain only where the insert and the splat release them at their end (see
+// wait_for_previous_kernel): 800x1200 x 3 176.6 / 172.3, 1024x1024 grey by RGB, forward + backward, 306.9 / 299.4, five CRF steps on
+// 375x500 x 21 427 / 411 (and 408 with the index stage of the two kept lattices), two volumes of 111x128x120 509 / 502, 8 x 512x512 x 21 without a guide 424 / 415, 16 x 512x512 x 21 1764 / 1764.
+#define PL_LAUNCH_AFTER(overlap, kernel, grid, block, smem, st, ...) \
+    PL_CUDA(launch_kernel((overlap), kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
 
 // The header and the sketch behind it.
 constexpr size_t HEADER_BYTES = sizeof(Header) + sizeof(u32) * SKETCH_WORDS;
@@ -448,7 +443,7 @@ static int launch_splat_as(const Geom& g, const float* input, Header* hdr, const
     if constexpr (VD > 0 && VD <= 4) {
         const size_t smem = SplatFast<PD, VD, PRE>::BYTES;
         PL_TRY((ensure_dynamic_smem<splat_tiles_fast<PD, VD, PRE>>(smem)));
-        PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_fast<PD, VD, PRE>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+        PL_LAUNCH_AFTER(true, (splat_tiles_fast<PD, VD, PRE>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                               srec, list_ref, v0, bulk_rows_ok(g, input, VD - 1) ? 1 : 0);
     } else {
         const size_t smem = SplatRows<PD, VD, PRE>::bytes(vd);
@@ -456,7 +451,7 @@ static int launch_splat_as(const Geom& g, const float* input, Header* hdr, const
         // five CTAs per SM need nearly all of the SM's shared memory: ask for the largest carve-out
         PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, VD, PRE, FloatSum, float>>(smem, true)));
         const bool bulk = bulk_staging_ok(g, input, vd);
-        PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_rows<PD, VD, PRE, FloatSum, float>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+        PL_LAUNCH_AFTER(true, (splat_tiles_rows<PD, VD, PRE, FloatSum, float>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                               srec, list_ref, v0, vd, bulk ? 1 : 0);
     }
     return PL_OK;
@@ -470,7 +465,7 @@ static int launch_splat_fixed(const Geom& g, const float* input, Header* hdr, co
     const size_t smem = SplatRows<PD, 0, PRE>::bytes(vd);
     PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, 0, PRE, FixedSum, long long>>(smem, true)));
     const bool bulk = bulk_staging_ok(g, input, vd);
-    PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_rows<PD, 0, PRE, FixedSum, long long>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+    PL_LAUNCH_AFTER(true, (splat_tiles_rows<PD, 0, PRE, FixedSum, long long>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                           srec, list_ref, v64, vd, bulk ? 1 : 0);
     return PL_OK;
 }
@@ -484,20 +479,20 @@ static int launch_splat(const Geom& g, const float* input, Header* hdr, const in
                      : launch_splat_as<PD, VD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v0, vd, st);
 }
 
-// Whether the slice of wide rows overlaps the last blur pass (OV_SLICE or 0).  With fewer tiles than SMs not: of a grid that starts
+// Whether the slice of wide rows overlaps the last blur pass.  With fewer tiles than SMs not: of a grid that starts
 // while the pass leaves the GPU, four or five CTAs go to the first SMs that become free, and the others stay idle (12 k vertices of 2000
 // points at pd 5, 21 channels: the slice 25 / 8 us, the call 88 / 74; 8 x 79x38 x 30 in double 33 / 15 and 81 / 66).  The small blur leaves most SMs free for it.  Narrow rows read
 // too little for it to matter: the plain launch costs them 1 to 2 us.
-static int slice_overlap(const Geom& g, bool after_small_blur) {
-    return after_small_blur || g.num_tiles >= num_sms() ? OV_SLICE : 0;
+static bool slice_overlap(const Geom& g, bool after_small_blur) {
+    return after_small_blur || g.num_tiles >= num_sms();
 }
 
 // slice for rows of VP floats (CT > 0: of CT channels), or (VP = 0) of more than 32.
 template <int PD, int VP, int CT = 0>
 static int launch_slice(const Geom& g, float* output, const Header* hdr, const int2* tile_info, const u16* rec,
-                        const float* rec_w, const u32* list_ref, const float* vsrc, int vd, Watch watch, int overlap, cudaStream_t st) {
+                        const float* rec_w, const u32* list_ref, const float* vsrc, int vd, Watch watch, bool overlap, cudaStream_t st) {
     if constexpr (VP == 4) {
-        PL_LAUNCH_AFTER(OV_SLICE, (slice_points<PD, CT>), tile_grid(g), Cfg<PD>::TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, watch);
+        PL_LAUNCH_AFTER(true, (slice_points<PD, CT>), tile_grid(g), Cfg<PD>::TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, vsrc, watch);
     } else if constexpr (VP > 0) {
         int rows_cap = SliceFast<PD, VP, CT>::ROWS_BYTES / (SliceFast<PD, VP>::RS * 4);
         if (rows_cap > Cfg<PD>::SPLATS) rows_cap = Cfg<PD>::SPLATS;
@@ -570,20 +565,20 @@ static bool blur_in_pairs(const Geom& g, int pd, const Layout& L, u32 vpr) {
 }
 template <int PD, int KW>
 static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
-                              const VertexInit& vinit, Watch watch, bool overlap, cudaStream_t st) {
+                              const VertexInit& vinit, Watch watch, cudaStream_t st) {
     const u32 entries = (u32)L.max_entries;
     const size_t smem = SmallIndex<PD>::bytes(entries);
     PL_TRY((ensure_dynamic_smem<index_small<PD, KW>>(smem)));
     // a thread for every axis and vertex, up to 64 CTAs
     const u32 ctas = std::max(8u, std::min(64u, (entries * (PD + 1) + SMALL_THREADS - 1) / SMALL_THREADS));
-    PL_CUDA(launch_kernel(overlap, index_small<PD, KW>, dim3(ctas), dim3(SMALL_THREADS), smem, st, hdr, list_keys, list_ref, vkeys, vinit, (u32)smem, watch));
+    PL_LAUNCH_AFTER(true, (index_small<PD, KW>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, (u32)smem, watch);
     return PL_OK;
 }
 template <typename V, int PIECES>
 static int launch_small_blur_as(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
     const size_t smem = sizeof(V) * 2 * PIECES * SMALL_THREADS;
     PL_TRY((ensure_dynamic_smem<blur_small<V, PIECES>>(smem)));
-    PL_LAUNCH_AFTER(OV_BLUR, (blur_small<V, PIECES>), SMALL_CTAS * vpr, SMALL_THREADS, smem, st, hdr, nbr, L.max_entries, v, vpr, axes, reverse);
+    PL_LAUNCH_AFTER(true, (blur_small<V, PIECES>), SMALL_CTAS * vpr, SMALL_THREADS, smem, st, hdr, nbr, L.max_entries, v, vpr, axes, reverse);
     return PL_OK;
 }
 template <typename V>
@@ -655,9 +650,9 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     const bool small_table = L.index_words <= (1ull << 24);
     if (phases & PH_BUILD) {
         // what the insert overlaps: clear_table (see above), or the build itself
-        const int before_insert = cleared ? ((phases & PH_APPLY) ? OV_CLEAR : 0) : small_table ? OV_INSERT : 0;
+        const bool before_insert = cleared || small_table;
         // (beyond pd 8 the build has to wait for the header at its start, and launched beside it took 112 -> 128 us)
-        constexpr int beside_clear = Cfg<PD>::COMPACT ? 0 : OV_BUILD;
+        constexpr bool beside_clear = !Cfg<PD>::COMPACT;
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
         if (phases & PH_APPLY) {
             PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, false, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr,
@@ -679,29 +674,27 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         if constexpr (PD <= MAX_SDIMS) {
             if (use_direct) {
                 u32* table32 = reinterpret_cast<u32*>(table);
-                if (!cleared) PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
+                if (!cleared) PL_LAUNCH_AFTER(true, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
                 PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
-                PL_LAUNCH_AFTER(OV_LINK, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
+                PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
                                                                  L.max_entries, watch);
             }
         }
         PL_COUNT_LAUNCHES(small ? 2 : cleared ? 3 : 4);   // build_tiles and the launches of the index stage
         if (small) {
-            PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, (phases & PH_APPLY) != 0, st)));
+            PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, st)));
         } else if (!use_direct) {
             // the value rows are zeroed by the link launch, whose lookups leave the memory system idle
             void* zrows = vinit.rows;
             vinit.rows = nullptr;
-            // (behind the build that also sorts the splats the overlap measured slower: 1.66 against 1.61 ms for
-            // a build and two applies)
             auto hash_index = [&](auto keys_in_slots) -> int {
                 constexpr bool KEYS = decltype(keys_in_slots)::value;
-                if (!cleared) PL_LAUNCH_AFTER((phases & PH_APPLY) ? OV_CLEAR : 0, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+                if (!cleared) PL_LAUNCH_AFTER(true, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
                 if constexpr (KEYS)
                     PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
                 else
                     PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
-                PL_LAUNCH_AFTER(OV_LINK, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
+                PL_LAUNCH_AFTER(true, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
                                                           L.max_entries, zrows, vinit.row_bytes, watch);
                 return PL_OK;
             };
@@ -715,7 +708,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         if (ev) PL_CUDA(cudaEventRecord(ev[2], st));
     } else {
         if (ev) { PL_CUDA(cudaEventRecord(ev[1], st)); }
-        PL_LAUNCH_AFTER(OV_CLEAR, (zero_rows), wide, 256, 0, st, hdr, v0, v64, padded_vd(vd));
+        PL_LAUNCH_AFTER(true, (zero_rows), wide, 256, 0, st, hdr, v0, v64, padded_vd(vd));
         PL_COUNT_LAUNCHES(1);
         if (ev) { PL_CUDA(cudaEventRecord(ev[2], st)); }
     }
@@ -726,11 +719,11 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     int rc = PL_OK;
     if (v64) {
         if (vd > widest_vd_fixed(PD)) return PL_UNSUPPORTED_DIMS;
-        PL_LAUNCH((absmax_kernel), wide, 256, 0, st, input, (u64)g.batch * g.n * (vd - 1), hdr);
+        PL_LAUNCH_AFTER(true, (absmax_kernel), wide, 256, 0, st, input, (u64)g.batch * g.n * (vd - 1), hdr);
         rc = (phases & PH_BUILD) ? launch_splat_fixed<PD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st)
                                  : launch_splat_fixed<PD, true>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st);
         if (rc != PL_OK) return rc;
-        PL_LAUNCH((convert_fixed), wide, 256, 0, st, hdr, v64, v0, padded_vd(vd));
+        PL_LAUNCH_AFTER(true, (convert_fixed), wide, 256, 0, st, hdr, v64, v0, padded_vd(vd));
         PL_COUNT_LAUNCHES(2);   // absmax_kernel, convert_fixed (the splat itself is counted below)
     } else {
         rc = PL_SPLAT_FOR(PD, vd, g, input, hdr, tile_info, rec, rec_w, srec, !(phases & PH_BUILD), list_ref, v0, vd, st);
@@ -748,14 +741,14 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
-            PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_pair<float4>), sms * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
+            PL_LAUNCH_AFTER(true, (blur_pair<float4>), sms * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
             std::swap(src, dst);
             PL_COUNT_LAUNCHES(1);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * L.max_entries * 2;
-        PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<float4>), wide, 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
+        PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
         float* tmp = src; src = dst; dst = tmp;
         PL_COUNT_LAUNCHES(1);
     }
@@ -807,9 +800,9 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     while ((1ull << table_log2) < L.table_slots) table_log2++;
     const int vp = padded_vd_f64(vd);
     const bool small_table = L.index_words <= (1ull << 24);   // (as for float)
-    const int before_insert = cleared ? OV_CLEAR : small_table ? OV_INSERT : 0;
+    const bool before_insert = cleared || small_table;
 
-    PL_LAUNCH_AFTER(Cfg<PD>::COMPACT ? 0 : OV_BUILD, (build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
+    PL_LAUNCH_AFTER(!Cfg<PD>::COMPACT, (build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
     u32* table32 = reinterpret_cast<u32*>(table);
     VertexInit vinit;
     vinit.nbr = nbr;
@@ -819,24 +812,24 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     vinit.row_bytes = (u32)vp * 8u;
     if constexpr (PD <= MAX_SDIMS) {
         if (use_direct) {
-            if (!cleared) PL_LAUNCH_AFTER(OV_CLEAR, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
+            if (!cleared) PL_LAUNCH_AFTER(true, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
             PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
-            PL_LAUNCH((link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
+            PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
                                                              L.max_entries, watch);
         }
     }
     if (small) {
-        PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, true, st)));
+        PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, st)));
     } else if (!use_direct) {
-        if (!cleared) PL_LAUNCH_AFTER(OV_CLEAR, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
+        if (!cleared) PL_LAUNCH_AFTER(true, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         if constexpr (Cfg<PD>::KEY_SLOTS)
             PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
         else
             PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
-        PL_LAUNCH((link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
+        PL_LAUNCH_AFTER(true, (link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   nullptr, 0u, watch);
     }
-    PL_LAUNCH_AFTER(OV_SPLAT, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
+    PL_LAUNCH_AFTER(true, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                       list_ref, v0, vd);
     double* src = v0;
     double* dst = v1;
@@ -847,15 +840,15 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
-            PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
             std::swap(src, dst);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        PL_LAUNCH_AFTER(step == 0 ? OV_BLUR0 : OV_BLUR, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
-    PL_LAUNCH_AFTER(vd > 4 ? slice_overlap(g, one_blur) : OV_SLICE, (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
+    PL_LAUNCH_AFTER(vd <= 4 || slice_overlap(g, one_blur), (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
     PL_COUNT_LAUNCHES((small ? 2 : cleared ? 3 : 4) + 1 + (one_blur ? 1 : pairs ? PD / 2 + 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;
@@ -911,7 +904,7 @@ static int launch_crf_splat(const Geom& g, const float* q, const LatticeRows& a,
     PL_TRY((ensure_dynamic_smem<crf_splat<PDA, PDS, VD>>(smem, true)));
     dim3 grid = tile_grid(g);
     (g.grid3 ? grid.z : grid.x) *= 2;
-    PL_LAUNCH_AFTER(OV_SPLAT, (crf_splat<PDA, PDS, VD>), grid, Cfg<PDA>::TP, smem, st, g, q, a, s, vd, bulk_staging_ok(g, q, vd) ? 1 : 0);
+    PL_LAUNCH_AFTER(true, (crf_splat<PDA, PDS, VD>), grid, Cfg<PDA>::TP, smem, st, g, q, a, s, vd, bulk_staging_ok(g, q, vd) ? 1 : 0);
     return PL_OK;
 }
 template <int PDA, int PDS, int VP, int CT = 0>
@@ -935,7 +928,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     const LatticeRows a = lattice_rows(ws_a, LA), s = lattice_rows(ws_s, LS);
     const int vd = labels + 1, vp = padded_vd(vd), wide = num_sms() * 8;
     const u32 quads = (u32)vp / 4;
-    PL_LAUNCH_AFTER(OV_CLEAR, (crf_zero_rows), dim3(wide / 2, 2), 256, 0, st, a, s, quads);
+    PL_LAUNCH_AFTER(true, (crf_zero_rows), dim3(wide / 2, 2), 256, 0, st, a, s, quads);
     PL_TRY((vd == 22 ? launch_crf_splat<PDA, PDS, 22>(g, q, a, s, vd, st) : launch_crf_splat<PDA, PDS, 0>(g, q, a, s, vd, st)));
     // small lattices have all their passes in one launch each; else a launch a pass, both as long as S has some left
     const bool small_a = small_blur(g, PDA, LA, quads), small_s = small_blur(g, PDS, LS, quads);
@@ -953,8 +946,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     for (int pair = 0; pairs && pair <= std::max(PDA, PDS) / 2; pair++) {
         const bool pass_a = !small_a && 2 * pair <= PDA, pass_s = !small_s && 2 * pair <= PDS, both = pass_a && pass_s;
         if (!pass_a && !pass_s) continue;
-        const bool first = pair == 0 && !small_a && !small_s;
-        PL_LAUNCH_AFTER(first ? OV_BLUR0 : OV_BLUR, (crf_blur_pair<PDA, PDS>), dim3(num_sms() * PAIR_CTAS / (both ? 2 : 1), both ? 2 : 1), 256, 0, st, a, s, both ? 0 : pass_a ? 1 : 2, pair, quads);
+        PL_LAUNCH_AFTER(true, (crf_blur_pair<PDA, PDS>), dim3(num_sms() * PAIR_CTAS / (both ? 2 : 1), both ? 2 : 1), 256, 0, st, a, s, both ? 0 : pass_a ? 1 : 2, pair, quads);
         launches++;
         if (pass_a) va = (pair & 1) ? a.v0 : a.v1;
         if (pass_s) vs = (pair & 1) ? s.v0 : s.v1;
@@ -969,12 +961,10 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
         float4* const v[2] = {reinterpret_cast<float4*>(l.v0), reinterpret_cast<float4*>(l.v1)};
         return Pass{l.nbr + 2 * (u64)step * l.max_entries, v[step & 1], v[1 - (step & 1)]};
     };
-    bool first_pass = !small_a && !small_s;   // right behind the splat
     auto rest_of = [&](const LatticeRows& l, int step, int pd, const float*& v) -> int {   // from pass `step` on
         for (; step <= pd; step++) {
             const Pass p = pass_of(l, step);
-            PL_LAUNCH_AFTER(first_pass ? OV_BLUR0 : OV_BLUR, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads);
-            first_pass = false;
+            PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads);
             launches++;
             v = reinterpret_cast<const float*>(p.dst);
         }
@@ -985,8 +975,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
         if (!small_a && !small_s && (LA.max_entries + LS.max_entries) * quads <= CRF_TOGETHER) {
             for (; step <= std::min(PDA, PDS); step++) {
                 const Pass p = pass_of(a, step), q2 = pass_of(s, step);
-                PL_LAUNCH_AFTER(first_pass ? OV_BLUR0 : OV_BLUR, (crf_blur), dim3(wide / 2, 2), 256, 0, st, a.hdr, p.nbr, p.src, p.dst, s.hdr, q2.nbr, q2.src, q2.dst, quads);
-                first_pass = false;
+                PL_LAUNCH_AFTER(true, (crf_blur), dim3(wide / 2, 2), 256, 0, st, a.hdr, p.nbr, p.src, p.dst, s.hdr, q2.nbr, q2.src, q2.dst, quads);
                 launches++;
                 va = reinterpret_cast<const float*>(p.dst);
                 vs = reinterpret_cast<const float*>(q2.dst);

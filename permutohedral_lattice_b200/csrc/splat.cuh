@@ -295,7 +295,6 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
         if (in_columns<PD>(g, nloc, NC::LEAST) && CS::smooth(g, tpos, hdr, rec, nloc, CS::NARROW)) {
             splat_columns<PD, VD, NC::AHEAD>(g, tpos, base, input, rec + (size_t)tile * SPLATS, rec_w + (size_t)tile * SPLATS,
                                   list_ref, v0, halves);
-            let_next_kernel_start();
             return;
         }
     }
@@ -382,7 +381,6 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
             acc[C] = PL_FADD(acc[C], wt);
         }
     }
-    let_next_kernel_start();   // what is left of this thread's work: its last row
     flush_row<VP>(v0 + (size_t)vid_s[cur] * VP, acc);
 }
 
@@ -543,7 +541,6 @@ __device__ __forceinline__ void splat_wide_columns(const Geom& g, const TilePos&
                 acc[r].add(__uint_as_float(vw.y), q);
             }
         }
-        let_next_kernel_start();   // what is left of this thread's work: its last rows
 #pragma unroll
         for (int r = 0; r <= PD; r++) acc[r].flush(v0 + (size_t)cur[r] * VP + 4 * h);
     }
@@ -762,7 +759,6 @@ __device__ __forceinline__ void splat_rows(const Geom& g, const TilePos& tpos, c
                 if (i < count) one(sp[i].x, sp[i].y);
                 if constexpr (ONE) break;
             }
-            let_next_kernel_start();   // what is left of this thread's work: its last row
             acc.flush(v0 + (size_t)vcur * VP + 4 * h);
             if constexpr (ONE) break;
         }
