@@ -58,7 +58,7 @@ constexpr u64 MOVED_ITEMS = 5000000;
 
 template <typename V>
 __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src,
-                                          V* __restrict__ dst, u32 vpr /* V per row */, u32 block, u32 blocks) {
+                                          V* __restrict__ dst, u32 vpr /* V per row */, u32 block, u32 blocks, u32 lattices /* of this size */) {
     // Passes after the first overlap the tail of the pass before (see after_previous_kernel).  The vertex count
     // and the neighbour table are older than any blur pass: a thread's first pair of neighbours is fetched
     // before the wait, so that one of the two dependent loads of its first row is off the critical path.
@@ -89,7 +89,7 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
         }
     };
     if constexpr (std::is_same<V, float4>::value) {
-        if (items <= MOVED_ITEMS) {
+        if (items * lattices <= MOVED_ITEMS) {
             rows([](V a, V b, V c) {
                 float2 z = make_float2(0.f, 0.f);
                 look_for_finite(z, a);
@@ -102,10 +102,11 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
     }
     rows([](V a, V b, V c) { return mix_rows(a, b, c); });
 }
+// blockIdx.y: the item, where one lattice serves several (item_v: V from one's rows to the next's).
 template <typename V>
 __global__ void __launch_bounds__(256, 8)
-blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst, u32 vpr) {
-    blur_rows<V>(hdr, nbr_axis, src, dst, vpr, blockIdx.x, gridDim.x);
+blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst, u32 vpr, u64 item_v) {
+    blur_rows<V>(hdr, nbr_axis, src + blockIdx.y * item_v, dst + blockIdx.y * item_v, vpr, blockIdx.x, gridDim.x, gridDim.y);
 }
 
 // Two passes in one launch, along axes a and then b: a thread mixes the row that pass b needs of its vertex and of that one's
@@ -175,8 +176,8 @@ __device__ __forceinline__ void blur_pair_rows(const Header* hdr, const int* __r
 template <typename V>
 __global__ void __launch_bounds__(256, PAIR_CTAS)
 blur_pair(const Header* hdr, const int* __restrict__ nbr_a, const int* __restrict__ nbr_b, const V* __restrict__ src,
-          V* __restrict__ dst, u32 vpr) {
-    blur_pair_rows<V>(hdr, nbr_a, nbr_b, src, dst, vpr, blockIdx.x, gridDim.x);
+          V* __restrict__ dst, u32 vpr, u64 item_v) {
+    blur_pair_rows<V>(hdr, nbr_a, nbr_b, src + blockIdx.y * item_v, dst + blockIdx.y * item_v, vpr, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -300,7 +301,7 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     const int tid = threadIdx.x, tile = tpos.tile;
     const u32 status = hdr->status;   // final by now, the same in every thread; one round trip with all that follows
     const int2 info = tile_info[tile];
-    const int base = info.x, cnt = info.y;
+    const int base = info.x + first_entry_of(g, tpos.item), cnt = info.y;
     const int nrows = min(cnt, rows_cap);
     const float4* v4 = reinterpret_cast<const float4*>(vsrc);
     int item, pix;
@@ -396,7 +397,7 @@ slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* 
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x;
     const u32 status = hdr->status;   // final by now: the same in every thread
-    const int base = tile_info[tpos.tile].x;
+    const int base = tile_info[tpos.tile].x + first_entry_of(g, tpos.item);
     int item, pix;
     const bool valid = tile_point(g, tpos, tid, item, pix);
     auto stop = [&]() {
@@ -460,7 +461,7 @@ slice_tiles_generic(Geom g, float* __restrict__ output, const Header* hdr, const
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
-    const int base = info.x, cnt = info.y;
+    const int base = info.x + first_entry_of(g, tpos.item), cnt = info.y;
     const int nrows = min(cnt, rows_cap);
     const float4* v4 = reinterpret_cast<const float4*>(vsrc);
     int item, pix;

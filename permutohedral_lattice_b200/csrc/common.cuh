@@ -33,6 +33,9 @@ struct Geom {
     int rcp_div;            // 1: divide through the reciprocals (exact for these operands), 0: IEEE divide
     int calm_entries;       // entries of a tile up to which its points hardly change entry in disorder (see ColumnsSample)
     int from_positions;     // 1: features are read from a positions array
+    int lattice_items;      // items that one lattice serves (see one_for_all): records and vertices are those of item 0
+    u32 item_rows;          // then: value rows (and entries) from one item's to the next's
+    u32 bound;              // then: the call's max_entries (the lattice's own is a share of it)
     float scale[MAX_PD];    // host-computed scale factors (double arithmetic rounded to float)
     // T = double calls: the same three in double
     double spatial_std_d, feature_std_d;
@@ -51,7 +54,8 @@ struct Header {   // first 256 bytes of the workspace
     u32 filter_log2;   // bits of the vertex filter behind the table, as a logarithm; 0: none (see FILTER_BITS_LOG2)
     u32 reported;      // status bits that the call's watch has told the host of (see Watch)
     u32 calm_entries;  // of the Geom that the lattice was built with
-    u32 pad[53];
+    u32 items;         // items that the lattice serves: entries and vertices are those of one of them
+    u32 pad[52];
 };
 
 // Sketch of the lattice's size, behind the header (zeroed with it): a bitmap in which build_tiles sets one bit
@@ -98,7 +102,7 @@ __device__ __forceinline__ void report_to(const Watch& w, Header* hdr) {
     if (w.words && grid_thread() == 0) {
         const u32 status = __ldcg(&hdr->status);
         hdr->reported = status;
-        store_to_host(w.words, ((u64)w.seq << 40) | ((u64)(status & 0xFFu) << 32) | (u64)hdr->num_entries);
+        store_to_host(w.words, ((u64)w.seq << 40) | ((u64)(status & 0xFFu) << 32) | (u64)(hdr->num_entries * hdr->items));
     }
 }
 // By the first thread of the grid of a slice kernel that has found the call failed.
@@ -240,7 +244,7 @@ __host__ __device__ constexpr u64 coord_ones(int j) {
 // Tile of this CTA.  Tile kernels run on a 3-D grid (tile column, tile row, item * outer + outer index)
 // whenever that fits the grid limits, so no thread divides to find its tile; else on a 1-D grid.
 struct TilePos {
-    int tile, item, o, ty, tx;
+    int tile, item, o, ty, tx;   // tile: whose records and range of entries these points have
 };
 __device__ __forceinline__ TilePos tile_at(const Geom& g, int x, int z) {   // CTA (x, blockIdx.y, z)
     TilePos t;
@@ -254,11 +258,12 @@ __device__ __forceinline__ TilePos tile_at(const Geom& g, int x, int z) {   // C
             t.item = z / g.outer;
             t.o = z - t.item * g.outer;
         }
-        t.tile = (z * g.tiles_y + t.ty) * g.tiles_x + t.tx;
+        t.tile = ((g.lattice_items > 1 ? t.o : z) * g.tiles_y + t.ty) * g.tiles_x + t.tx;
     } else {
         t.tile = x;
         t.item = t.tile / g.tiles_per_item;
         int r = t.tile - t.item * g.tiles_per_item;
+        if (g.lattice_items > 1) t.tile = r;
         const int per_plane = g.tiles_x * g.tiles_y;
         t.o = r / per_plane;
         r -= t.o * per_plane;
@@ -267,6 +272,11 @@ __device__ __forceinline__ TilePos tile_at(const Geom& g, int x, int z) {   // C
     }
     return t;
 }
+
+// Where one lattice serves several items (see one_for_all), every item has its own value rows and its own copy of the list of
+// entries, which names them, `item_rows` apart: what an item adds to its tiles' first entries.  (Added to the rows' address
+// instead, it cost the splat of narrow rows up to 28 bytes of spills, and at pd 5 an SM's sixth CTA.)
+__device__ __forceinline__ int first_entry_of(const Geom& g, int item) { return item * (int)g.item_rows; }
 
 __device__ __forceinline__ TilePos this_tile(const Geom& g) { return tile_at(g, blockIdx.x, blockIdx.z); }
 

@@ -86,16 +86,17 @@ insert_direct(Header* hdr, Direct d, u32* __restrict__ table, const Key<Cfg<PD>:
 // The "+" neighbour of vertex v along axis a (src/PermutohedralLatticeCPU.h:381-388) by one load of
 // its slot (every slot carries a vertex index by now); the same result fills that neighbour's "-" slot.
 template <int PD>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 8)
 link_neighbours_direct(Header* hdr, Direct d, const u32* __restrict__ table, u32* __restrict__ list_ref,
                        const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys,
-                       int* __restrict__ nbr, u64 max_entries, Watch watch) {
+                       int* __restrict__ nbr, u64 max_entries, ItemRows rows, Watch watch) {
     after_previous_kernel();
     report_to(watch, hdr);
     constexpr int KW = Cfg<PD>::KW;
     if (hdr->status != 0) return;
-    resolve_entries(hdr, list_ref, vid);
+    resolve_entries(hdr, list_ref, vid, rows);
     const u32 M = hdr->num_vertices;
+    zero_rows_of(rows, M, grid_thread(), grid_threads());
     const u64 items = (u64)M * (PD + 1);
     for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < items; e += (u64)gridDim.x * blockDim.x) {
         const u32 v = (u32)(e / (PD + 1));

@@ -43,16 +43,19 @@ export_points(Geom g, const Header* hdr, const int2* __restrict__ tile_info, con
     constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS;
     if (hdr->status != 0) return;
     const TilePos tpos = this_tile(g);
-    const int tid = threadIdx.x, tile = tpos.tile;
+    // (of a lattice that serves several items the records are those of the first, and the vertices counted item by item)
+    const u32 shared = hdr->items > 1 ? 1u : 0u;
+    const int tid = threadIdx.x, tile = shared ? tpos.tile % g.tiles_per_item : tpos.tile;
     int item, pix;
     if (!tile_point(g, tpos, tid, item, pix)) return;
     const int base = tile_info[tile].x;
+    const u32 first = shared * (u32)item * hdr->num_vertices;
     const u16* rec_tile = rec + (size_t)tile * SPLATS;
     const R* recw_tile = rec_w + (size_t)tile * SPLATS;
     const size_t o = ((size_t)item * g.n + pix) * (PD + 1);
 #pragma unroll
     for (int r = 0; r <= PD; r++) {
-        if (pixel_vertex) pixel_vertex[o + r] = (int32_t)list_ref[base + rec_tile[r * TP + tid]];
+        if (pixel_vertex) pixel_vertex[o + r] = (int32_t)(first + list_ref[base + rec_tile[r * TP + tid]]);
         if (pixel_weight) pixel_weight[o + r] = recw_tile[r * TP + tid];
     }
 }
@@ -61,15 +64,17 @@ template <int PD, int KW>
 __global__ void export_vertices(const Header* hdr, const Key<KW>* __restrict__ vkeys, long long max_vertices,
                                 int16_t* __restrict__ vertex_keys, int32_t* __restrict__ vertex_item) {
     if (hdr->status != 0) return;
-    const u32 M = hdr->num_vertices;
+    const u32 of_item = hdr->num_vertices, items = hdr->items;
+    const u64 M = (u64)of_item * items;
     for (u64 v = (u64)blockIdx.x * blockDim.x + threadIdx.x; v < M && v < (u64)max_vertices;
          v += (u64)gridDim.x * blockDim.x) {
-        const Key<KW> k = vkeys[v];
+        const u32 item = (u32)v / of_item;
+        const Key<KW> k = vkeys[items > 1 ? (u32)v - item * of_item : (u32)v];
         if (vertex_keys) {
 #pragma unroll
             for (int i = 0; i < PD; i++) vertex_keys[v * PD + i] = (int16_t)(key_get<KW>(k, i) ^ 0x8000);
         }
-        if (vertex_item) vertex_item[v] = KW * 4 > PD ? (int32_t)key_get<KW>(k, KW * 4 > PD ? PD : 0) : 0;
+        if (vertex_item) vertex_item[v] = items > 1 ? (int32_t)item : KW * 4 > PD ? (int32_t)key_get<KW>(k, KW * 4 > PD ? PD : 0) : 0;
     }
 }
 

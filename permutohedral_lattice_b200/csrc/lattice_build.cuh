@@ -447,9 +447,10 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
     }
     wait_for_previous_kernel();
     if (tile == 0 && tid == 0) {
-        hdr->capacity = max_entries;
+        hdr->capacity = g.lattice_items > 1 ? g.bound : max_entries;
         hdr->sorted = SORTED ? 1u : 0u;
         hdr->calm_entries = (u32)g.calm_entries;
+        hdr->items = (u32)g.lattice_items;
     }
     if (tid == 0) {
         u32 base = atomicAdd(&hdr->num_entries, (u32)cnt);
@@ -643,15 +644,31 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
 // ---------------------------------------------------------------------------------------------
 // insert_entries
 // ---------------------------------------------------------------------------------------------
+// The items that the lattice serves (1, or see one_for_all), and their value rows, to be zeroed.
+struct ItemRows {
+    u32 items, stride;   // rows, and entries, from one item's to the next's
+    uint4* rows;         // float rows, rows of doubles, or the 64-bit sums of the deterministic mode; null: none
+    u32 row_quads;       // 16 bytes each
+};
+__device__ __forceinline__ void zero_rows_of(const ItemRows& z, u32 M, u64 thread, u64 threads) {
+    if (!z.rows) return;
+    const u64 quads = (u64)M * z.row_quads;
+    for (u32 b = 0; b < z.items; b++)
+        for (u64 i = thread; i < quads; i += threads) z.rows[(u64)b * z.stride * z.row_quads + i] = make_uint4(0u, 0u, 0u, 0u);
+}
+// The vertex of entry t, and its rows, of every item.
+__device__ __forceinline__ void store_vertex_of(const ItemRows& z, u32* __restrict__ list_ref, u32 t, u32 v) {
+    list_ref[t] = v;
+    for (u32 b = 1; b < z.items; b++) list_ref[(u64)b * z.stride + t] = b * z.stride + v;
+}
+
 // What the insert launch sets up for every vertex it creates, so that no later launch has to: the
-// vertex's key (vertex order), its slots of the neighbour table ("missing") and, when `rows` is given,
-// its value row (zero).
+// vertex's key (vertex order) and its slots of the neighbour table ("missing").  (Its value row is zeroed by the link launch,
+// by streaming stores under the latency of its lookups.)
 struct VertexInit {
     int* nbr;            // [pd + 1][max_entries] pairs
     u64 max_entries;
     int pd;
-    void* rows;          // value rows to zero (float rows, or the 64-bit sums of the deterministic mode); may be null
-    u32 row_bytes;       // bytes of one such row (a multiple of 16)
 };
 
 // Entries are inserted in rounds of INSERT_CHUNKS chunks of 256: the winners of a round (entries that
@@ -719,11 +736,6 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
         int2* nb = reinterpret_cast<int2*>(vi.nbr);
         for (int a = 0; a <= vi.pd; a++)
             for (u32 i = threadIdx.x; i < tot; i += 256) nb[(u64)a * vi.max_entries + base + i] = make_int2(-1, -1);
-        if (vi.rows) {
-            uint4* rows = reinterpret_cast<uint4*>(static_cast<unsigned char*>(vi.rows) + (u64)base * vi.row_bytes);
-            const u32 quads = tot * (vi.row_bytes / 16);
-            for (u32 i = threadIdx.x; i < quads; i += 256) rows[i] = make_uint4(0u, 0u, 0u, 0u);
-        }
     }
     __syncthreads();
     if (threadIdx.x == 0) rd.count = 0;
@@ -886,11 +898,11 @@ insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cf
 // entry -> vertex: after the insert launch list_ref[t] names the entry that owns t's key; the link launch
 // turns that into the owner's vertex index (first loop of link_neighbours / link_neighbours_direct).
 __device__ __forceinline__ void resolve_entries(const Header* hdr, u32* __restrict__ list_ref,
-                                                const u32* __restrict__ vid) {
+                                                const u32* __restrict__ vid, const ItemRows& rows) {
     const u32 T = hdr->num_entries;
     for (u64 t = grid_thread(); t < T; t += grid_threads()) {
         const u32 ref = list_ref[t];
-        list_ref[t] = (ref & VERTEX_FLAG) ? (ref & ~VERTEX_FLAG) : vid[ref];
+        store_vertex_of(rows, list_ref, (u32)t, (ref & VERTEX_FLAG) ? (ref & ~VERTEX_FLAG) : vid[ref]);
     }
 }
 
@@ -987,18 +999,14 @@ template <int PD, bool KEY_SLOTS, int KW = Cfg<PD>::KW>
 __global__ void __launch_bounds__(256)
 link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restrict__ list_ref,
                 const u32* __restrict__ vid, const Key<KW>* __restrict__ vkeys, int* __restrict__ nbr,
-                u64 max_entries, void* zero_rows_ptr, u32 zero_row_bytes, Watch watch) {
+                u64 max_entries, ItemRows rows, Watch watch) {
     after_previous_kernel();
     report_to(watch, hdr);
     if (hdr->status != 0) return;
-    resolve_entries(hdr, list_ref, vid);
+    resolve_entries(hdr, list_ref, vid, rows);
     const u32 M = hdr->num_vertices;
     const u64 mask = (1ull << hdr->table_log2) - 1;
-    if (zero_rows_ptr) {   // streaming stores that overlap the latency of the lookups below
-        uint4* rows = reinterpret_cast<uint4*>(zero_rows_ptr);
-        const u64 quads = (u64)M * (zero_row_bytes / 16);
-        for (u64 i = grid_thread(); i < quads; i += grid_threads()) rows[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
+    zero_rows_of(rows, M, grid_thread(), grid_threads());   // under the latency of the lookups below
     if constexpr (KEY_SLOTS) {
         LinkAxis<PD, KW, 0>::run((int)blockIdx.y, reinterpret_cast<const KeySlot*>(table), (u32)mask, vkeys, M, nbr, max_entries);
     } else {

@@ -234,6 +234,7 @@ static int make_geom(Geom& g, int batch, int n, int pd, int n_sdims, const int* 
     g.batch = batch;
     g.n = n;
     g.from_positions = from_positions ? 1 : 0;
+    g.lattice_items = 1;
     g.n_sdims = n_sdims;
     g.R = R;
     g.spatial_std = spatial_std;
@@ -335,6 +336,25 @@ static bool make_direct(Direct& d, const Geom& g, int pd, const Layout& L) {
     memset(&d, 0, sizeof(d));
     if (!g_direct_index_enabled || g.from_positions || g.R != 0 || pd != g.n_sdims) return false;
     return direct_bounds(d, pd, g.sdims, g.spatial_std, g.scale, g.batch, L.index_words);
+}
+
+// The features of a spatial-only call are those of its grid, the same in every item: one lattice does for all, with its share of the
+// bound, and value rows for every item.  The lattice's own geometry and layout, of one item; false: the call builds a lattice of all
+// its items.  A share fits where the whole would have: entries are the same in every item.  us a call, forward + backward, an own
+// lattice each / one: 8 x 512x512 x 21 414 / 346, 16 x 512x512 x 1 399 / 217; forward, 3 x 1000x700 x 3 100 / 76, 4 x 300x200 x 5 44 / 37.5.
+static bool one_for_all(const Geom& g, const Layout& L, int pd, Geom& one, Layout& share) {
+    one = g;
+    share = L;
+    if (g.from_positions || g.R != 0 || pd != g.n_sdims || g.batch < 2 || L.max_entries < (u64)g.batch) return false;
+    share.max_entries = L.max_entries / (u64)g.batch;
+    while (share.table_slots > 1024 && share.table_slots / 2 >= 2 * share.max_entries) share.table_slots /= 2;
+    one.lattice_items = g.batch;
+    one.item_rows = (u32)share.max_entries;
+    one.bound = (u32)L.max_entries;
+    one.batch = 1;
+    one.num_tiles = one.tiles_per_item;
+    one.grid3 = (one.tiles_y <= 65535 && one.outer <= 65535) ? 1 : 0;
+    return true;
 }
 
 // What clear_header clears for the index stage (see ClearTable): the direct index, or the hash table of a call that keeps no
@@ -565,28 +585,28 @@ static bool blur_in_pairs(const Geom& g, int pd, const Layout& L, u32 vpr) {
 }
 template <int PD, int KW>
 static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
-                              const VertexInit& vinit, Watch watch, cudaStream_t st) {
+                              const VertexInit& vinit, const ItemRows& rows, Watch watch, cudaStream_t st) {
     const u32 entries = (u32)L.max_entries;
     const size_t smem = SmallIndex<PD>::bytes(entries);
     PL_TRY((ensure_dynamic_smem<index_small<PD, KW>>(smem)));
     // a thread for every axis and vertex, up to 64 CTAs
     const u32 ctas = std::max(8u, std::min(64u, (entries * (PD + 1) + SMALL_THREADS - 1) / SMALL_THREADS));
-    PL_LAUNCH_AFTER(true, (index_small<PD, KW>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, (u32)smem, watch);
+    PL_LAUNCH_AFTER(true, (index_small<PD, KW>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, rows, (u32)smem, watch);
     return PL_OK;
 }
 template <typename V, int PIECES>
-static int launch_small_blur_as(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
+static int launch_small_blur_as(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, u32 items, u64 item_v, cudaStream_t st) {
     const size_t smem = sizeof(V) * 2 * PIECES * SMALL_THREADS;
     PL_TRY((ensure_dynamic_smem<blur_small<V, PIECES>>(smem)));
-    PL_LAUNCH_AFTER(true, (blur_small<V, PIECES>), SMALL_CTAS * vpr, SMALL_THREADS, smem, st, hdr, nbr, L.max_entries, v, vpr, axes, reverse);
+    PL_LAUNCH_AFTER(true, (blur_small<V, PIECES>), dim3(SMALL_CTAS * vpr, items), SMALL_THREADS, smem, st, hdr, nbr, L.max_entries, v, vpr, axes, reverse, item_v);
     return PL_OK;
 }
 template <typename V>
-static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
+static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, u32 items, u64 item_v, cudaStream_t st) {
     const u64 pieces = (L.max_entries + SMALL_CTAS * SMALL_THREADS - 1) / (SMALL_CTAS * SMALL_THREADS);   // a thread
-    return pieces <= 1   ? launch_small_blur_as<V, 1>(hdr, nbr, L, v, vpr, axes, reverse, st)
-           : pieces <= 2 ? launch_small_blur_as<V, 2>(hdr, nbr, L, v, vpr, axes, reverse, st)
-                         : launch_small_blur_as<V, SMALL_PIECES>(hdr, nbr, L, v, vpr, axes, reverse, st);
+    return pieces <= 1   ? launch_small_blur_as<V, 1>(hdr, nbr, L, v, vpr, axes, reverse, items, item_v, st)
+           : pieces <= 2 ? launch_small_blur_as<V, 2>(hdr, nbr, L, v, vpr, axes, reverse, items, item_v, st)
+                         : launch_small_blur_as<V, SMALL_PIECES>(hdr, nbr, L, v, vpr, axes, reverse, items, item_v, st);
 }
 
 // The header's counters and, in calls that keep one, the sketch behind it.
@@ -601,10 +621,23 @@ enum { PH_BUILD = 1, PH_APPLY = 2 };   // halves of a call: lattice structure / 
 
 // KW: words of a key.
 template <int PD, int KW>
-static int run_filter(const Geom& g, float* output, const float* input, const float* positions,
+static int run_filter(const Geom& call, float* output, const float* input, const float* positions,
                       const float* reference, int vd, int reverse, int mode, void* workspace,
-                      const Layout& L, cudaStream_t st, int phases = PH_BUILD | PH_APPLY) {
+                      const Layout& whole, cudaStream_t st, int phases = PH_BUILD | PH_APPLY) {
     constexpr int TP = Cfg<PD>::TP;
+    // g, L: of the whole call; the lattice is that of `one`, within `share` of the bound (see one_for_all)
+    Geom g = call, one;
+    Layout share;
+    const bool together = phases == (PH_BUILD | PH_APPLY) && one_for_all(call, whole, PD, one, share);
+    if (together) {
+        g.lattice_items = one.lattice_items;
+        g.item_rows = one.item_rows;
+    } else {
+        one = call;
+        share = whole;
+    }
+    const Layout& L = whole;
+    const u32 items = (u32)one.lattice_items;
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     Header* hdr = reinterpret_cast<Header*>(ws);
     int2* tile_info = reinterpret_cast<int2*>(ws + L.tile_info);
@@ -622,16 +655,17 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     float* v1 = reinterpret_cast<float*>(ws + L.v1);
     long long* v64 = (mode == PL_MODE_DETERMINISTIC) ? reinterpret_cast<long long*>(ws + L.v64) : nullptr;
 
-    const int sketch_shift = sketch_shift_of(L.max_entries);
+    const int sketch_shift = sketch_shift_of(share.max_entries);
     cudaEvent_t* ev = g_stage_events;
     g_stage_events = nullptr;
     if (ev) PL_CUDA(cudaEventRecord(ev[0], st));
     Direct direct;
     bool use_direct = false, small = false, cleared = false;
     if (phases & PH_BUILD) {
-        if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
-        small = !use_direct && small_index(g, PD, L);
-        const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, L, table, sketch_shift, small);
+        if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, call, PD, L);
+        if (together) direct.slots = direct.cells;
+        small = !use_direct && small_index(one, PD, share);
+        const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, share, table, sketch_shift, small);
         cleared = clear.table != nullptr;
         PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));
     }
@@ -642,7 +676,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     const int sms = num_sms();
     const int wide = sms * 8;
     int table_log2 = 0;
-    while ((1ull << table_log2) < L.table_slots) table_log2++;
+    while ((1ull << table_log2) < share.table_slots) table_log2++;
 
     // The insert overlaps clear_table only in regions of up to 64 MB of 8-byte slots (pd up to 5: 2^23 slots too, 128 MB, of
     // which the device uses what the vertices ask for): behind a clear_table that itself overlaps build_tiles it cost
@@ -655,38 +689,38 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         constexpr bool beside_clear = !Cfg<PD>::COMPACT;
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
         if (phases & PH_APPLY) {
-            PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, false, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr,
-                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
+            PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, false, KW>), tile_grid(one), TP, Cfg<PD>::build_smem(false), st, one, positions, reference, hdr,
+                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)share.max_entries, sketch_shift);
         } else {
             PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, true, KW>>(Cfg<PD>::build_smem(true))));
             PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, true, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)L.max_entries, sketch_shift);
         }
         if (ev) PL_CUDA(cudaEventRecord(ev[1], st));
-        // a new vertex's neighbour slots and (when this call also applies) its value row are initialised
-        // by the launch that creates it
+        // a new vertex's neighbour slots are initialised by the launch that creates it, its value row (when this call also
+        // applies) by the link launch
         VertexInit vinit;
         vinit.nbr = nbr;
-        vinit.max_entries = L.max_entries;
+        vinit.max_entries = share.max_entries;
         vinit.pd = PD;
-        vinit.rows = (phases & PH_APPLY) ? (v64 ? static_cast<void*>(v64) : static_cast<void*>(v0)) : nullptr;
-        vinit.row_bytes = (u32)padded_vd(vd) * (v64 ? 8u : 4u);
+        ItemRows rows;
+        rows.items = items;
+        rows.stride = one.item_rows;
+        rows.rows = (phases & PH_APPLY) ? (v64 ? reinterpret_cast<uint4*>(v64) : reinterpret_cast<uint4*>(v0)) : nullptr;
+        rows.row_quads = (u32)padded_vd(vd) / (v64 ? 2u : 4u);
         if constexpr (PD <= MAX_SDIMS) {
             if (use_direct) {
                 u32* table32 = reinterpret_cast<u32*>(table);
                 if (!cleared) PL_LAUNCH_AFTER(true, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
                 PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
                 PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                                 L.max_entries, watch);
+                                                                 share.max_entries, rows, watch);
             }
         }
         PL_COUNT_LAUNCHES(small ? 2 : cleared ? 3 : 4);   // build_tiles and the launches of the index stage
         if (small) {
-            PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, st)));
+            PL_TRY((launch_small_index<PD, KW>(hdr, share, list_keys, list_ref, vkeys, vinit, rows, watch, st)));
         } else if (!use_direct) {
-            // the value rows are zeroed by the link launch, whose lookups leave the memory system idle
-            void* zrows = vinit.rows;
-            vinit.rows = nullptr;
             auto hash_index = [&](auto keys_in_slots) -> int {
                 constexpr bool KEYS = decltype(keys_in_slots)::value;
                 if (!cleared) PL_LAUNCH_AFTER(true, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
@@ -694,8 +728,8 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
                     PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
                 else
                     PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
-                PL_LAUNCH_AFTER(true, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
-                                                          L.max_entries, zrows, vinit.row_bytes, watch);
+                PL_LAUNCH_AFTER(true, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, share.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
+                                                          share.max_entries, rows, watch);
                 return PL_OK;
             };
             if constexpr (Cfg<PD>::KEY_SLOTS) {
@@ -716,6 +750,10 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         PL_CUDA(cudaGetLastError());
         return PL_OK;
     }
+    // the blur passes (and the conversion of the fixed-point sums): a row of blocks for every item that the lattice serves
+    const u32 qpr = (u32)padded_vd(vd) / 4;
+    const u64 item_v = (u64)one.item_rows * qpr;
+    auto rows_of_blocks = [&](int blocks) { return (unsigned)((blocks + (int)items - 1) / (int)items); };
     int rc = PL_OK;
     if (v64) {
         if (vd > widest_vd_fixed(PD)) return PL_UNSUPPORTED_DIMS;
@@ -723,7 +761,7 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
         rc = (phases & PH_BUILD) ? launch_splat_fixed<PD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st)
                                  : launch_splat_fixed<PD, true>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st);
         if (rc != PL_OK) return rc;
-        PL_LAUNCH_AFTER(true, (convert_fixed), wide, 256, 0, st, hdr, v64, v0, padded_vd(vd));
+        PL_LAUNCH_AFTER(true, (convert_fixed), dim3(rows_of_blocks(wide), items), 256, 0, st, hdr, v64, v0, padded_vd(vd), item_v * 4);
         PL_COUNT_LAUNCHES(2);   // absmax_kernel, convert_fixed (the splat itself is counted below)
     } else {
         rc = PL_SPLAT_FOR(PD, vd, g, input, hdr, tile_info, rec, rec_w, srec, !(phases & PH_BUILD), list_ref, v0, vd, st);
@@ -733,27 +771,27 @@ static int run_filter(const Geom& g, float* output, const float* input, const fl
     if (ev) PL_CUDA(cudaEventRecord(ev[3], st));
     float* src = v0;
     float* dst = v1;
-    const u32 qpr = (u32)padded_vd(vd) / 4;
-    if (small_blur(g, PD, L, qpr)) {
-        PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, st));
+    const bool one_blur = small_blur(one, PD, share, qpr * items);
+    if (one_blur) {
+        PL_TRY(launch_small_blur(hdr, nbr, share, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, items, item_v, st));
         PL_COUNT_LAUNCHES(1);
-    } else if (blur_in_pairs(g, PD, L, qpr)) {
+    } else if (blur_in_pairs(one, PD, share, qpr * items)) {
         for (int step = 0; step <= PD; step += 2) {
-            const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
-            const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<float4>), sms * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
+            const int* nb = nbr + (size_t)(reverse ? PD - step : step) * share.max_entries * 2;
+            const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * share.max_entries * 2;
+            PL_LAUNCH_AFTER(true, (blur_pair<float4>), dim3(rows_of_blocks(sms * PAIR_CTAS), items), 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
             std::swap(src, dst);
             PL_COUNT_LAUNCHES(1);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        const int* nb = nbr + (size_t)axis * L.max_entries * 2;
-        PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
+        const int* nb = nbr + (size_t)axis * share.max_entries * 2;
+        PL_LAUNCH_AFTER(true, (blur_axis<float4>), dim3(rows_of_blocks(wide), items), 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
         float* tmp = src; src = dst; dst = tmp;
         PL_COUNT_LAUNCHES(1);
     }
     if (ev) PL_CUDA(cudaEventRecord(ev[4], st));
-    rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch, slice_overlap(g, small_blur(g, PD, L, qpr)), st);
+    rc = PL_SLICE_FOR(PD, vd, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch, slice_overlap(g, one_blur), st);
     if (rc != PL_OK) return rc;
     if (ev) PL_CUDA(cudaEventRecord(ev[5], st));
     PL_CUDA(cudaGetLastError());
@@ -808,18 +846,17 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     vinit.nbr = nbr;
     vinit.max_entries = L.max_entries;
     vinit.pd = PD;
-    vinit.rows = v0;   // rows of vp doubles
-    vinit.row_bytes = (u32)vp * 8u;
+    const ItemRows rows = {1u, 0u, reinterpret_cast<uint4*>(v0), (u32)vp / 2};   // rows of vp doubles
     if constexpr (PD <= MAX_SDIMS) {
         if (use_direct) {
             if (!cleared) PL_LAUNCH_AFTER(true, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
             PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
             PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
-                                                             L.max_entries, watch);
+                                                             L.max_entries, rows, watch);
         }
     }
     if (small) {
-        PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, watch, st)));
+        PL_TRY((launch_small_index<PD, KW>(hdr, L, list_keys, list_ref, vkeys, vinit, rows, watch, st)));
     } else if (!use_direct) {
         if (!cleared) PL_LAUNCH_AFTER(true, (clear_table<Cfg<PD>::KEY_SLOTS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
         if constexpr (Cfg<PD>::KEY_SLOTS)
@@ -827,7 +864,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         else
             PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
         PL_LAUNCH_AFTER(true, (link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
-                                                  nullptr, 0u, watch);
+                                                  rows, watch);
     }
     PL_LAUNCH_AFTER(true, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
                                                                       list_ref, v0, vd);
@@ -835,17 +872,17 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* dst = v1;
     const bool one_blur = small_blur(g, PD, L, (u32)vp / 2), pairs = blur_in_pairs(g, PD, L, (u32)vp / 2);
     if (one_blur) {
-        PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<double2*>(v0), (u32)vp / 2, PD + 1, reverse, st));
+        PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<double2*>(v0), (u32)vp / 2, PD + 1, reverse, 1, 0, st));
     } else if (pairs) {
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
             std::swap(src, dst);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
         double* tmp = src; src = dst; dst = tmp;
     }
     PL_LAUNCH_AFTER(vd <= 4 || slice_overlap(g, one_blur), (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
@@ -935,11 +972,11 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     const float *va = a.v0, *vs = s.v0;
     int launches = 3;
     if (small_s) {
-        PL_TRY(launch_small_blur(s.hdr, s.nbr, LS, reinterpret_cast<float4*>(s.v0), quads, PDS + 1, 0, st));
+        PL_TRY(launch_small_blur(s.hdr, s.nbr, LS, reinterpret_cast<float4*>(s.v0), quads, PDS + 1, 0, 1, 0, st));
         launches++;
     }
     if (small_a) {
-        PL_TRY(launch_small_blur(a.hdr, a.nbr, LA, reinterpret_cast<float4*>(a.v0), quads, PDA + 1, 0, st));
+        PL_TRY(launch_small_blur(a.hdr, a.nbr, LA, reinterpret_cast<float4*>(a.v0), quads, PDA + 1, 0, 1, 0, st));
         launches++;
     }
     const bool pairs = blur_in_pairs(g, PDA, LA, quads) && blur_in_pairs(g, PDS, LS, quads);
@@ -964,7 +1001,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     auto rest_of = [&](const LatticeRows& l, int step, int pd, const float*& v) -> int {   // from pass `step` on
         for (; step <= pd; step++) {
             const Pass p = pass_of(l, step);
-            PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads);
+            PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads, (u64)0);
             launches++;
             v = reinterpret_cast<const float*>(p.dst);
         }
@@ -1588,8 +1625,9 @@ int pl_lattice_stats(const void* workspace, pl_stats* stats, void* stream) {
     Header h;
     PL_CUDA(cudaMemcpyAsync(&h, workspace, sizeof(Header), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     PL_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    stats->num_vertices = h.num_vertices;
-    stats->num_entries = h.num_entries;
+    const u32 items = h.items > 1 ? h.items : 1;   // (see one_for_all)
+    stats->num_vertices = (int64_t)h.num_vertices * items;
+    stats->num_entries = (int64_t)h.num_entries * items;
     stats->table_slots = (int64_t)1 << h.table_log2;
     stats->device_status = PL_OK;
     for (int code = PL_INVALID_ARGUMENT; code <= PL_INTERNAL_ERROR; code++)

@@ -46,7 +46,7 @@ __device__ __forceinline__ u32 small_hash(u64 first) {
 template <int PD, int KW = Cfg<PD>::KW>
 __global__ void __launch_bounds__(SMALL_THREADS)
 index_small(Header* hdr, const Key<KW>* __restrict__ list_keys, u32* __restrict__ list_ref,
-            Key<KW>* __restrict__ vkeys, VertexInit vi, u32 smem_bytes, Watch watch) {
+            Key<KW>* __restrict__ vkeys, VertexInit vi, ItemRows rows, u32 smem_bytes, Watch watch) {
     after_previous_kernel();
     using SI = SmallIndex<PD>;
     constexpr int WARPS = SMALL_THREADS / 32, CHUNKS = SMALL_MAX_ENTRIES / SMALL_THREADS;
@@ -165,7 +165,7 @@ index_small(Header* hdr, const Key<KW>* __restrict__ list_keys, u32* __restrict_
     }
     for (u32 t = me; t < T; t += all) {
         const u32 v = table_s[slot_s[t]] >> 16;
-        list_ref[t] = v;
+        store_vertex_of(rows, list_ref, t, v);
         if (owner_s[v] == t) {
             if constexpr (SI::EXACT) {
                 Key<KW> k;
@@ -177,10 +177,7 @@ index_small(Header* hdr, const Key<KW>* __restrict__ list_keys, u32* __restrict_
             }
         }
     }
-    if (vi.rows) {
-        uint4* rows = static_cast<uint4*>(vi.rows);
-        for (u32 i = me; i < M * (vi.row_bytes / 16); i += all) rows[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
+    zero_rows_of(rows, M, me, all);
     int2* nb = reinterpret_cast<int2*>(vi.nbr);
     for (u32 i = me; i < M * (PD + 1); i += all) {
         const u32 a = i / M, v = i - a * M, t = owner_s[v];
@@ -253,14 +250,14 @@ __device__ __forceinline__ double2 load_cluster(u32 addr, u32 cta, double2) {
 }
 template <typename V, int PIECES>
 __global__ void __cluster_dims__(SMALL_CTAS, 1, 1) __launch_bounds__(SMALL_THREADS)
-blur_small(const Header* hdr, const int* __restrict__ nbr, u64 max_entries, V* v, u32 vpr, int axes, int reverse) {
+blur_small(const Header* hdr, const int* __restrict__ nbr, u64 max_entries, V* v, u32 vpr, int axes, int reverse, u64 item_v) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* const buf = reinterpret_cast<V*>(smem_raw);
     const u32 M = hdr->num_vertices;   // (older than the splat before this)
     u32 chunk_log2 = 5;
     while ((u32)SMALL_CTAS << chunk_log2 < M) chunk_log2++;
     const u32 chunk = 1u << chunk_log2, first = (blockIdx.x % SMALL_CTAS) << chunk_log2;
-    v += blockIdx.x / SMALL_CTAS;
+    v += blockIdx.x / SMALL_CTAS + blockIdx.y * item_v;
     const int2* __restrict__ nb = reinterpret_cast<const int2*>(nbr);
     auto axis = [&](int step) { return (u64)(reverse ? axes - 1 - step : step) * max_entries; };
     int2 even[PIECES], odd[PIECES];   // neighbours of vertex first + at(p) in the next pass of either kind

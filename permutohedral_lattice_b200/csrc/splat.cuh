@@ -289,7 +289,7 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     if constexpr (NC::EVER) halves = hdr->num_entries > NC::SHARED * hdr->num_vertices;
     if (call_failed(hdr)) return;
     if (PRE && !lattice_is_sorted(hdr)) return;
-    const int base = info.x, nloc = info.y;
+    const int base = info.x + first_entry_of(g, tpos.item), nloc = info.y;
     using CS = ColumnsSample<PD>;
     if constexpr (NC::EVER) {
         if (in_columns<PD>(g, nloc, NC::LEAST) && CS::smooth(g, tpos, hdr, rec, nloc, CS::NARROW)) {
@@ -571,7 +571,7 @@ __device__ __forceinline__ void splat_rows(const Geom& g, const TilePos& tpos, c
     }
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
-    const int base = info.x, nloc = info.y;
+    const int base = info.x + first_entry_of(g, tpos.item), nloc = info.y;
     using CS = ColumnsSample<PD>;
     constexpr bool SAMPLED = CS::TAKEN && WideColumns<PD, PRE, Sum>::EVER;
     bool columns = WideColumns<PD, PRE, Sum>::take(g, nloc, LR);   // (so far; then by the sample)
@@ -825,8 +825,10 @@ absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
 
 // fixed-point sums -> float rows
 __global__ void __launch_bounds__(256)
-convert_fixed(const Header* hdr, const long long* __restrict__ v64, float* __restrict__ v0, int vp) {
+convert_fixed(const Header* hdr, const long long* __restrict__ v64, float* __restrict__ v0, int vp, u64 item_cells) {
     after_previous_kernel();
+    v64 += blockIdx.y * item_cells;
+    v0 += blockIdx.y * item_cells;
     if (hdr->status != 0) return;
     const double inv = __longlong_as_double((long long)(1023 - fixed_exponent(hdr)) << 52);
     const u64 cells = (u64)hdr->num_vertices * vp;

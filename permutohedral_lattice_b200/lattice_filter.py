@@ -53,8 +53,8 @@ def release_workspaces():
 # ---------------------------------------------------------------------------------------------------
 _entries_per_item = {}   # kind of call -> largest num_entries / batch seen
 _verified = {}           # kind of call -> (identity of the reference it ran on, the bound that sufficed, weak reference)
-_pending = {}            # kind of call -> list of (event, pinned int32[3] = entries, vertices, status bits, bound, batch)
-_pinned_words = []       # pinned int32[3] buffers waiting to be used again (allocating pinned memory is slow)
+_pending = {}            # kind of call -> list of (event, pinned int32[12], the start of its workspace's header, bound, batch)
+_pinned_words = []       # pinned int32[12] buffers waiting to be used again (allocating pinned memory is slow)
 FIRST_GUESS_DIVISOR = 4
 LATE_FAILURE = "an earlier lattice filter call failed on the device after its lattice was complete; its output holds NaN"
 HEADROOM = 1.5
@@ -85,7 +85,8 @@ def _status_code(bits):
 def _look_at(kind, entry):
     """Takes a finished call's counters into account; raises if that call did not fit its bound."""
     _, host, bound, batch = entry
-    entries, _, bits = (int(v) for v in host.tolist())
+    words = host.tolist()
+    entries, bits = words[0] * max(words[11], 1), words[2]   # of one item, times the items that the lattice serves
     _pinned_words.append(host)
     code = _status_code(bits)
     if code == capi.PL_CAPACITY_EXCEEDED:
@@ -148,9 +149,9 @@ def _direct_index_floor(call):
 
 
 def _note_call(kind, ws, bound, batch, device):
-    """Queues the copy of the call's counters (first 12 bytes of the workspace) behind it."""
-    host = _pinned_words.pop() if _pinned_words else torch.empty(3, dtype=torch.int32).pin_memory()
-    host.copy_(ws[:12].view(torch.int32), non_blocking=True)
+    """Queues the copy of the call's counters (first 48 bytes of the workspace) behind it."""
+    host = _pinned_words.pop() if _pinned_words else torch.empty(12, dtype=torch.int32).pin_memory()
+    host.copy_(ws[:48].view(torch.int32), non_blocking=True)
     ev = torch.cuda.Event()
     ev.record(torch.cuda.current_stream(device))
     _pending.setdefault(kind, []).append((ev, host, bound, batch))

@@ -123,3 +123,41 @@ def test_a_call_that_outgrew_its_bound_reports_no_index(gpu, shape, theta, bound
         assert st.direct_index == 0 and st.table_slots == 1
         out, ws, _ = plb.lattice_filter_raw(x.to(dtype), None, False, 1.0, 1.0, theta, max_entries=2 * bound)
         assert plb.lattice_stats(ws).direct_index == 1 and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("shape,c,theta,batch", [
+    ((1, 1), 2, 3.0, 2),             # a single point
+    ((33, 47), 3, 3.0, 5),           # the index and the blur of small lattices
+    ((130, 150), 1, 1.5, 3),         # narrow rows, passes in pairs
+    ((200, 260), 21, 2.0, 4),        # wide rows, a pass a launch
+    ((20, 24, 31), 2, 2.0, 3),       # volumes
+    ((70, 50), 6, 0.37, 3),          # hashed: the index would not fit
+    ((4000,), 1, 5.0, 16),           # one dimension
+    ((40, 50), 70, 2.0, 2),          # rows beyond the staged ones
+])
+def test_one_lattice_for_all_items(shape, c, theta, batch, gpu):
+    """The items of a spatial-only call share a lattice: every one of them as if filtered alone, bit for bit, the counters
+    and the exported vertices as of a lattice of them all, and the bound that of the whole call."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    x = torch.randn((batch,) + shape + (c,), generator=torch.Generator("cuda").manual_seed(3), device="cuda")
+    x[:, ..., 0].view(batch, -1)[:, 0] = 6.0    # one grid of the fixed-point sums for all
+    x.clamp_(-6.0, 6.0)
+    for reverse in (False, True):
+        out, ws, call = plb.lattice_filter_raw(x, None, False, 1.0, 1.0, theta, reverse, mode="deterministic", max_entries=0)
+        st = plb.lattice_stats(ws)
+        vk, vi, pv, _ = (t.cpu().numpy() for t in gpu.export_op(ws, call, None, max_entries=0)[1])
+        for b in range(batch):
+            alone, ws1, call1 = plb.lattice_filter_raw(x[b:b + 1], None, False, 1.0, 1.0, theta, reverse, mode="deterministic",
+                                                       max_entries=0, workspace_owner="alone")
+            assert torch.equal(out[b:b + 1], alone)
+        st1 = plb.lattice_stats(ws1)
+        vk1, _, pv1, _ = (t.cpu().numpy() for t in gpu.export_op(ws1, call1, None, max_entries=0)[1])
+        assert (st.num_entries, st.num_vertices) == (batch * st1.num_entries, batch * st1.num_vertices)
+        for b in range(batch):
+            assert (vi[pv[b]] == b).all() and np.array_equal(vk[pv[b]], vk1[pv1[0]])
+    for bound, code in ((st.num_entries, 0), (st.num_entries - 1, plb.capi.PL_CAPACITY_EXCEEDED)):
+        out, ws, _ = plb.lattice_filter_raw(x, None, False, 1.0, 1.0, theta, max_entries=bound, check=False)
+        st = plb.lattice_stats(ws)
+        assert st.device_status == code and st.max_entries == bound
+        assert torch.isfinite(out).all() if code == 0 else torch.isnan(out).all()
