@@ -533,6 +533,10 @@ __device__ __forceinline__ void after_previous_kernel() {
 __device__ __forceinline__ void wait_for_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The second half alone, for a kernel that starts on what is older than the kernel before it and waits for that at its end.
+__device__ __forceinline__ void let_next_kernel_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // First point and number of valid points of tile row `ly` (the run of points that is contiguous in
 // memory); returns false if the row lies outside the item.

@@ -617,6 +617,15 @@ static int clear_header_of(Header* hdr, int sketch_shift, const ClearTable& clea
     return PL_OK;
 }
 
+// The deterministic mode's largest magnitude, beside the next kernel (see absmax_kernel).  Its CTAs use no shared memory, but are split as
+// those of the tile kernels are: an SM takes CTAs of another split only when it is empty, and nothing overlapped.  Two CTAs an SM.
+static int launch_absmax(const float* input, const Geom& g, int vd, Header* hdr, cudaStream_t st) {
+    PL_TRY((ensure_dynamic_smem<absmax_kernel>(16, true)));
+    PL_LAUNCH_AFTER(true, (absmax_kernel), num_sms() * 2, 256, 0, st, input, (u64)g.batch * g.n * (vd - 1), hdr);
+    PL_COUNT_LAUNCHES(1);
+    return PL_OK;
+}
+
 enum { PH_BUILD = 1, PH_APPLY = 2 };   // halves of a call: lattice structure / values through it
 
 // KW: words of a key.
@@ -668,6 +677,7 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, share, table, sketch_shift, small);
         cleared = clear.table != nullptr;
         PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));
+        if (v64 && (phases & PH_APPLY)) PL_TRY(launch_absmax(input, call, vd, hdr, st));
     }
     if (g.num_tiles == 0) return PL_OK;
     const Watch watch = (phases & PH_BUILD) ? take_watch(st) : Watch{nullptr, 0u};
@@ -757,12 +767,12 @@ static int run_filter(const Geom& call, float* output, const float* input, const
     int rc = PL_OK;
     if (v64) {
         if (vd > widest_vd_fixed(PD)) return PL_UNSUPPORTED_DIMS;
-        PL_LAUNCH_AFTER(true, (absmax_kernel), wide, 256, 0, st, input, (u64)g.batch * g.n * (vd - 1), hdr);
+        if (!(phases & PH_BUILD)) PL_TRY(launch_absmax(input, call, vd, hdr, st));
         rc = (phases & PH_BUILD) ? launch_splat_fixed<PD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st)
                                  : launch_splat_fixed<PD, true>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st);
         if (rc != PL_OK) return rc;
         PL_LAUNCH_AFTER(true, (convert_fixed), dim3(rows_of_blocks(wide), items), 256, 0, st, hdr, v64, v0, padded_vd(vd), item_v * 4);
-        PL_COUNT_LAUNCHES(2);   // absmax_kernel, convert_fixed (the splat itself is counted below)
+        PL_COUNT_LAUNCHES(1);   // convert_fixed (the splat itself is counted below)
     } else {
         rc = PL_SPLAT_FOR(PD, vd, g, input, hdr, tile_info, rec, rec_w, srec, !(phases & PH_BUILD), list_ref, v0, vd, st);
     }

@@ -781,9 +781,11 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
 // One pass over the input, 16 bytes a load and four loads in flight (4-byte loads one by one reached 1.9 TB/s); the up
 // to three floats before the first 16-byte boundary and after the last go one by one.  2 x 512x512 x 21, forward +
 // backward: 491 -> 466 us.
+// It runs beside the kernel after it, whose first part needs nothing of it: the lattice construction, or, in a kept lattice, the
+// splat.  Behind the link launch, where it stood alone, 2 x 512x512 x 21, forward + backward, took 414.6 us, so 408.2.
 __global__ void __launch_bounds__(256)
 absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
-    after_previous_kernel();
+    let_next_kernel_start();   // (the input is older than the kernel before this)
     u32 m = 0;
     auto take = [&](float x) { m = max(m, __float_as_uint(fabsf(x))); };
     const u64 lead = min(count, (u64)(((16u - ((u32)(uintptr_t)input & 15u)) & 15u) >> 2));
@@ -819,6 +821,7 @@ absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 1; k < 8; k++) m = max(m, m_s[k]);
+        wait_for_previous_kernel();   // which zeroes the header's word
         if (m) atomicMax(&hdr->absmax_bits, m);
     }
 }
