@@ -55,7 +55,8 @@ struct Header {   // first 256 bytes of the workspace
     u32 reported;      // status bits that the call's watch has told the host of (see Watch)
     u32 calm_entries;  // of the Geom that the lattice was built with
     u32 items;         // items that the lattice serves: entries and vertices are those of one of them
-    u32 pad[52];
+    u32 mostly_new;    // in calls with a sketch: most of the entries are vertices (see insert_keys)
+    u32 pad[51];
 };
 
 // Sketch of the lattice's size, behind the header (zeroed with it): a bitmap in which build_tiles sets one bit

@@ -9,16 +9,19 @@ namespace pl {
 // The header and the sketch before a call.  A kernel and not a memset, so that build_tiles can start beside it (the gap between a memset and the
 // build, 3 to 4 us a call: 8 x 512x512 x 21, pd 2, forward + backward, 431 -> 425; 512x512 x 3 in double 188.5 -> 185.5).  The host needs a
 // microsecond more for it.
-// It also clears (to ones: empty slots) what the index stage needs where the host knows how much that may be, the direct index
-// or the table of a call without a sketch, so that no launch between the build and the insert has to: us a call, 2 x
-// 48x64 x 3 52 / 46, 4 x 180x240 x 3 60 / 57, 60x70 x 2 without a guide 32 / 28.  (By build_tiles, a share a tile, it cost calls without any
+// It also clears (to ones: empty slots) what the index stage needs, the direct index or the whole table that the call's bound allows,
+// where that is at most 16 MB, so that no launch between the build and the insert has to, and the call keeps no sketch: us a call, 2 x
+// 48x64 x 3 52 / 46, 4 x 180x240 x 3 60 / 57, 60x70 x 2 without a guide 32 / 28, five CRF steps on
+// 375x500 x 21 with both builds 413 / 405, 512x512 x 3 in double, forward + backward, 175 / 167.  At 32 MB nothing is left of it (2 x 512x512 x 21,
+// deterministic, 407 / 406).  (By build_tiles, a share a tile, it cost calls without any
 // 0.7 %.)
 struct ClearTable {
     uint4* table;   // null: a launch of its own does
     u32 quads;      // 16 bytes each
 };
-constexpr u32 CLEAR_QUADS = 1u << 19;   // 8 MB, at most
-static_assert(2 * SKETCH_MIN_ENTRIES <= CLEAR_QUADS, "the largest table of a call without a sketch, slots of 16 bytes");
+constexpr u32 CLEAR_QUADS = 1u << 20;         // 16 MB, at most; 8 MB where the build waits for it at its start (pd 16)
+constexpr u32 CLEAR_QUADS_ALONE = 1u << 19;
+static_assert(2 * SKETCH_MIN_ENTRIES <= CLEAR_QUADS_ALONE, "the largest table of a call that is too small for a sketch, slots of 16 bytes");
 __global__ void __launch_bounds__(256) clear_header(Header* hdr, u32 quads, ClearTable clear) {
     after_previous_kernel();
     if (blockIdx.x == 0)
@@ -579,6 +582,7 @@ __device__ __forceinline__ u32 log2_of_slots(u64 need, u32 max_log2) {
 constexpr u64 KEY_SLOTS_WHOLE = 1ull << 21;   // 32 MB
 constexpr u64 TAG_SLOTS_WHOLE = 1ull << 23;   // 64 MB
 constexpr u64 TAG_SLOTS_MOST = 1ull << 25;    // beyond, half as many would not stay in L2 either
+constexpr float MOSTLY_NEW = 0.3f;            // see insert_keys
 template <bool KEY_SLOTS>
 __global__ void __launch_bounds__(256)
 clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift) {
@@ -586,6 +590,7 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
     if (hdr->status != 0) return;
     __shared__ u32 bits_s[8];
     u64 need = 2ull * hdr->num_entries;
+    bool mostly_new = false;
     if (need > (1ull << (sketch_shift + 10))) {
         const uint4* sketch = reinterpret_cast<const uint4*>(hdr + 1);
         u32 bits = 0;
@@ -606,7 +611,9 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
         const u32 clear = (1u << SKETCH_LOG2) - set;
         if (clear > (1u << SKETCH_LOG2) / 64) {
             const float sampled = -(float)(1 << SKETCH_LOG2) * logf((float)clear * (1.f / (1 << SKETCH_LOG2)));
-            u64 slots = (u64)(4.f * sampled * (float)(1u << sketch_shift));
+            const float vertices = sampled * (float)(1u << sketch_shift);
+            mostly_new = vertices >= MOSTLY_NEW * (float)hdr->num_entries;
+            u64 slots = (u64)(4.f * vertices);
             // four a vertex spare more probes than the larger table costs while it stays in L2 beside everything else; a
             // table of keys beyond 32 MB has two a vertex at least (us a call, four / two a vertex: 1024x1024 grey by RGB,
             // forward + backward, 17 MB at four, 325 / 337; 16 x 512x512 x 21, 67 MB at four, 1857 / 1824.  So has
@@ -626,6 +633,7 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         hdr->table_log2 = lg;
         hdr->filter_log2 = filter_log2;
+        hdr->mostly_new = mostly_new ? 1u : 0u;
     }
     if constexpr (!KEY_SLOTS) {
         if (filter_log2) {
@@ -845,6 +853,11 @@ __device__ __forceinline__ u32 key_rest(const Key<Cfg<PD>::KW>& k) {
 
 // insert_entries into a table of keys.  The index in a slot is that of the creating entry, then (its round ended) of
 // the vertex.
+// A compare-and-swap on a line that was just read takes longer than one on a line that was not: in a table of 32 MB a ns sees 175 loads of
+// random slots, 80 swaps, 50 times load, swap and store of an empty slot, 70 times swap and store.  So slots are claimed unseen where the sketch
+// says that MOSTLY_NEW of the entries are vertices and, in calls without one, by a warp as long as a third of what it claims is free,
+// which the first of the entries mostly are, whatever the lattice.  us a call, a
+// look first / not: 800x1200 x 3, 54 % vertices, 172 / 169.5, 1024x1024 grey by RGB, 33 %, 300 / 298.5; 16 x 512x512 x 21, 16 %, 1764 / 1791.
 template <int PD>
 __global__ void __launch_bounds__(256, 8)   // as many as it is launched with
 insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
@@ -857,37 +870,48 @@ insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cf
     const u32 T = hdr->num_entries;
     const u32 mask = (u32)((1ull << table_log2_of(hdr, T, max_log2, cleared)) - 1);
     const u32 stride = gridDim.x * 256u;
+    bool unseen = cleared || hdr->mostly_new != 0;
+    // entry t, of which slot s of the table is the first to ask; true: it has claimed slot s
+    auto insert = [&](auto unseen_too, u32 t, u32& s) -> bool {
+        const Key<KW> k = list_keys[t];
+        const u64 first = k.w[0];
+        const u32 rest = key_rest<PD>(k);
+        u32 ref = 0xFFFFFFFFu;
+        bool winner = false;
+        s = (u32)hash_key<KW>(k) & mask;
+        for (u64 it = 0; it <= mask; it++) {
+            KeySlot cur = {EMPTY_SLOT, EMPTY_SLOT};
+            if constexpr (!decltype(unseen_too)::value) cur = load_slot(table + s);
+            if ((u32)cur.rest == 0xFFFFFFFFu) {
+                cur = claim_slot(table + s, first, ((u64)rest << 32) | t);
+                if ((u32)cur.rest == 0xFFFFFFFFu) {
+                    ref = t;
+                    winner = true;
+                    break;
+                }
+            }
+            if (cur.first == first && (u32)(cur.rest >> 32) == rest) { ref = (u32)cur.rest; break; }
+            s = (s + 1) & mask;
+        }
+        if (ref == 0xFFFFFFFFu) {
+            atomicOr(&hdr->status, 1u << PL_INTERNAL_ERROR);
+            ref = t;
+        }
+        list_ref[t] = ref;   // owning entry, or (VERTEX_FLAG set) the vertex itself
+        return winner;
+    };
     for (u32 start = blockIdx.x * 256u; start < T;) {
         for (int c = 0; c < INSERT_CHUNKS && start < T; c++, start += stride) {
             const u32 t = start + threadIdx.x;
             bool winner = false;
             u32 s = 0;
-            if (t < T) {
-                const Key<KW> k = list_keys[t];
-                const u64 first = k.w[0];
-                const u32 rest = key_rest<PD>(k);
-                u32 ref = 0xFFFFFFFFu;
-                s = (u32)hash_key<KW>(k) & mask;
-                for (u64 it = 0; it <= mask; it++) {
-                    KeySlot cur = load_slot(table + s);
-                    if ((u32)cur.rest == 0xFFFFFFFFu) {
-                        cur = claim_slot(table + s, first, ((u64)rest << 32) | t);
-                        if ((u32)cur.rest == 0xFFFFFFFFu) {
-                            ref = t;
-                            winner = true;
-                            break;
-                        }
-                    }
-                    if (cur.first == first && (u32)(cur.rest >> 32) == rest) { ref = (u32)cur.rest; break; }
-                    s = (s + 1) & mask;
-                }
-                if (ref == 0xFFFFFFFFu) {
-                    atomicOr(&hdr->status, 1u << PL_INTERNAL_ERROR);
-                    ref = t;
-                }
-                list_ref[t] = ref;   // owning entry, or (VERTEX_FLAG set) the vertex itself
+            if (unseen) {
+                if (t < T) winner = insert(std::true_type{}, t, s);
+            } else {
+                if (t < T) winner = insert(std::false_type{}, t, s);
             }
             round_add_winner(rd, winner, t, s);
+            if (cleared) unseen = 3 * __popc(__ballot_sync(0xFFFFFFFFu, winner)) >= 32;
         }
         finish_round<false, KW>(hdr, rd, list_keys, vid, vkeys, vi, [&](u32 slot, const Key<KW>& k, u32 v) {
             store_slot(table + slot, k.w[0], ((u64)key_rest<PD>(k) << 32) | VERTEX_FLAG | v);

@@ -357,12 +357,12 @@ static bool one_for_all(const Geom& g, const Layout& L, int pd, Geom& one, Layou
     return true;
 }
 
-// What clear_header clears for the index stage (see ClearTable): the direct index, or the hash table of a call that keeps no
-// sketch, whose size its bound gives.  A small lattice's table lies elsewhere.
-static ClearTable table_to_clear(const Direct* direct, const Layout& L, void* table, int sketch_shift, bool small) {
+// What clear_header clears for the index stage (see ClearTable): the direct index, or all of the hash table.  A small lattice's table lies
+// elsewhere.
+static ClearTable table_to_clear(const Direct* direct, const Layout& L, void* table, bool small, bool beside_build) {
     ClearTable c = {nullptr, 0u};
     const u64 bytes = direct ? sizeof(u32) * direct->slots : (L.key_slots ? 16ull : 8ull) * L.table_slots;
-    if (small || (!direct && sketch_shift >= 0) || bytes > 16ull * CLEAR_QUADS) return c;
+    if (small || bytes > 16ull * (beside_build ? CLEAR_QUADS : CLEAR_QUADS_ALONE)) return c;
     c.table = static_cast<uint4*>(table);
     c.quads = (u32)((bytes + 15) / 16);   // (regions are 256-byte aligned: so is the end)
     return c;
@@ -612,6 +612,8 @@ static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L,
 // The header's counters and, in calls that keep one, the sketch behind it.
 static int clear_header_of(Header* hdr, int sketch_shift, const ClearTable& clear, cudaStream_t st) {
     const unsigned ctas = std::min(1u + clear.quads / 1024u, 2u * (unsigned)num_sms());
+    // (the split of the build beside it, see launch_absmax; a microsecond of the host that small calls are better without)
+    if (clear.quads > (1u << 16)) PL_TRY((ensure_dynamic_smem<clear_header>(16, true)));
     PL_LAUNCH((clear_header), ctas, 256, 0, st, hdr, (u32)((sketch_shift >= 0 ? HEADER_BYTES : sizeof(Header)) / 16), clear);
     PL_COUNT_LAUNCHES(1);
     return PL_OK;
@@ -664,7 +666,7 @@ static int run_filter(const Geom& call, float* output, const float* input, const
     float* v1 = reinterpret_cast<float*>(ws + L.v1);
     long long* v64 = (mode == PL_MODE_DETERMINISTIC) ? reinterpret_cast<long long*>(ws + L.v64) : nullptr;
 
-    const int sketch_shift = sketch_shift_of(share.max_entries);
+    int sketch_shift = -1;   // no sketch
     cudaEvent_t* ev = g_stage_events;
     g_stage_events = nullptr;
     if (ev) PL_CUDA(cudaEventRecord(ev[0], st));
@@ -674,8 +676,9 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, call, PD, L);
         if (together) direct.slots = direct.cells;
         small = !use_direct && small_index(one, PD, share);
-        const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, share, table, sketch_shift, small);
+        const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, share, table, small, !Cfg<PD>::COMPACT);
         cleared = clear.table != nullptr;
+        if (!use_direct && !small && !cleared) sketch_shift = sketch_shift_of(share.max_entries);
         PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));
         if (v64 && (phases & PH_APPLY)) PL_TRY(launch_absmax(input, call, vd, hdr, st));
     }
@@ -828,15 +831,15 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* v0 = reinterpret_cast<double*>(ws + L.v0);
     double* v1 = reinterpret_cast<double*>(ws + L.v1);
 
-    const int sketch_shift = sketch_shift_of(L.max_entries);
     // spatial-only calls index their vertices directly, as the float calls do (the key bounds hold for
     // either arithmetic: the margin is far wider than any rounding)
     Direct direct;
     bool use_direct = false;
     if constexpr (PD <= MAX_SDIMS) use_direct = make_direct(direct, g, PD, L);
     const bool small = !use_direct && small_index(g, PD, L);
-    const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, L, table, sketch_shift, small);
+    const ClearTable clear = table_to_clear(use_direct ? &direct : nullptr, L, table, small, !Cfg<PD>::COMPACT);
     const bool cleared = clear.table != nullptr;
+    const int sketch_shift = use_direct || small || cleared ? -1 : sketch_shift_of(L.max_entries);
     PL_TRY(clear_header_of(hdr, sketch_shift, clear, st));
     if (g.num_tiles == 0) return PL_OK;
     const Watch watch = take_watch(st);

@@ -87,3 +87,34 @@ def test_direct_index_cleared_with_the_header_or_by_itself(plb, batch):
         finally:
             capi.lib().pl_debug_direct_index(was)
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("pd", [3, 5, 6])
+@pytest.mark.parametrize("noise", [0.0, 0.3])
+@pytest.mark.parametrize("more", [False, True])
+def test_slots_claimed_unseen_or_not(pd, noise, more):
+    """Entries that are mostly vertices (a noisy guide) and entries that are not, in tables cleared with the header (up to
+    2^19 entries) and sized by the sketch of the lattice: every key one vertex, each item as if filtered alone."""
+    import torch
+    import permutohedral_lattice_b200 as plb
+    n = (1 << 19) // (2 * (pd + 1))                 # two items of n points have just no more than 2^19 entries
+    h, w = 128, n // 128 + (2 if more else 0)
+    gen = torch.Generator("cuda").manual_seed(pd)
+    ref = torch.linspace(0, 1, w, device="cuda").expand(2, h, w).unsqueeze(-1).repeat(1, 1, 1, pd - 2)
+    ref = (ref + noise * torch.randn(ref.shape, generator=gen, device="cuda")).contiguous()
+    x = torch.randn((2, h, w, 3), generator=gen, device="cuda").clamp_(-4, 4)
+    x[:, 0, 0, 0] = 4.0                             # one grid of the fixed-point sums for all
+    out, ws, call = plb.lattice_filter_raw(x, ref, True, 8.0, 0.1, 1.0, mode="deterministic", max_entries=0)
+    st = plb.lattice_stats(ws)
+    assert st.device_status == 0 and st.table_slots >= 2 * st.num_vertices
+    keys, item, _, _ = plb.export_lattice(ws, st, call.batch, call.n, call.pd, call.vd, reference=ref, sdims=call.sdims,
+                                          spatial_std=call.spatial_std, feature_std=call.feature_std, max_entries=0)
+    both = torch.cat([item.view(-1, 1).to(torch.int16), keys], 1)
+    assert len(torch.unique(both, dim=0)) == st.num_vertices
+    total = 0
+    for b in range(2):
+        alone, ws1, _ = plb.lattice_filter_raw(x[b:b + 1], ref[b:b + 1], True, 8.0, 0.1, 1.0, mode="deterministic",
+                                               max_entries=0, workspace_owner="alone")
+        assert torch.equal(out[b:b + 1], alone)
+        total += plb.lattice_stats(ws1).num_vertices
+    assert total == st.num_vertices
