@@ -68,7 +68,7 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
     const u32 stride = blocks * blockDim.x, dv = stride / vpr, dj = stride - dv * vpr;
     u64 e = (u64)block * blockDim.x + threadIdx.x;
     u32 v = (u32)e / vpr, j = (u32)e - v * vpr;   // item e is V j of vertex v's row (the first e fits 32 bits)
-    int2 n = (v < M) ? __ldg(nb + v) : make_int2(-1, -1);
+    int2 n = (v < M) ? load_once(nb + v) : make_int2(-1, -1);
     after_previous_kernel();
     if (hdr->status != 0) return;
     const V zero = {};
@@ -83,7 +83,7 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
                 j -= vpr;
                 v++;
             }
-            if (v < M) n = __ldg(nb + v);
+            if (v < M) n = load_once(nb + v);
             dst[e] = mix(a, b, c);
             e += stride;
         }
@@ -131,7 +131,7 @@ __device__ __forceinline__ void blur_pair_rows(const Header* hdr, const int* __r
     int2 n[3];     // theirs along a
     auto look_up = [&]() {
         int2 beside = make_int2(-1, -1);
-        if (v < M && nb) beside = __ldg(nb + v);
+        if (v < M && nb) beside = load_once(nb + v);
         u[0] = v < M ? (int)v : -1;
         u[1] = beside.x;
         u[2] = beside.y;
@@ -313,8 +313,8 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     const float* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
     for (int r = 0; r <= PD; r++) {
-        l[r] = valid ? rec_tile[r * TP + tid] : 0;
-        w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
+        l[r] = valid ? load_record<PD>(rec_tile + r * TP + tid) : 0;
+        w[r] = valid ? load_record<PD>(recw_tile + r * TP + tid) : 0.f;
     }
     if (status != 0) {
         poison_tile_output(g, output, C);
@@ -410,9 +410,9 @@ slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* 
     float w[PD + 1];
     u32 v[PD + 1];
 #pragma unroll
-    for (int r = 0; r <= PD; r++) v[r] = valid ? rec[at + r * TP] : 0;
+    for (int r = 0; r <= PD; r++) v[r] = valid ? load_record<PD>(rec + at + r * TP) : 0;
 #pragma unroll
-    for (int r = 0; r <= PD; r++) w[r] = valid ? rec_w[at + r * TP] : 0.f;
+    for (int r = 0; r <= PD; r++) w[r] = valid ? load_record<PD>(rec_w + at + r * TP) : 0.f;
     if (!Cfg<PD>::COMPACT && status != 0) return stop();
     const u32* ref = list_ref + base;
 #pragma unroll
@@ -431,9 +431,9 @@ slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* 
     }
     const float inv = (float)(1.0 / (double)(C == 1 ? acc.y : C == 2 ? acc.z : acc.w));
     float* o = output + ((size_t)item * g.n + pix) * C;
-    o[0] = PL_FMUL(acc.x, inv);
-    if constexpr (C > 1) o[1] = PL_FMUL(acc.y, inv);
-    if constexpr (C > 2) o[2] = PL_FMUL(acc.z, inv);
+    store_once(o, PL_FMUL(acc.x, inv));
+    if constexpr (C > 1) store_once(o + 1, PL_FMUL(acc.y, inv));
+    if constexpr (C > 2) store_once(o + 2, PL_FMUL(acc.z, inv));
 }
 
 template <int PD>
@@ -473,8 +473,8 @@ slice_tiles_generic(Geom g, float* __restrict__ output, const Header* hdr, const
     const float* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
     for (int r = 0; r <= PD; r++) {
-        l[r] = valid ? rec_tile[r * TP + tid] : 0;
-        w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
+        l[r] = valid ? load_record<PD>(rec_tile + r * TP + tid) : 0;
+        w[r] = valid ? load_record<PD>(recw_tile + r * TP + tid) : 0.f;
     }
     {   // row staging: vertex numbers of CH rows first, then the copies that depend on them (see slice_tiles_fast)
         constexpr int CH = 8;

@@ -212,7 +212,32 @@ __device__ __forceinline__ void store_relaxed(u32* p, u32 v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// What a launch reads or writes once, and whose next reader comes after more than the caches hold, goes first when they need room, so that
+// what is read again and again, value rows, keys and tables, stays: the point records (the construction's stores, the loads of splat and
+// slice), the neighbours of a blur pass, the entries' keys and references beyond pd 5.  us a call, without / with: 800x1200 x 3 170 / 166.5,
+// 1024x1024 grey by RGB, forward + backward, 299.5 / 294, two volumes of 111x128x120 498.5 / 489, five CRF steps on 375x500 x 21 407 / 397,
+// 4 x 321x481 x 10 with one lattice 232.5 / 228, 1 M points with 16 features 1589 / 1566.
+template <typename T>
+__device__ __forceinline__ T load_once(const T* p) { return __ldcs(p); }
+template <typename T>
+__device__ __forceinline__ void store_once(T* p, T v) { __stcs(p, v); }
+// A point's record.  Not up to pd 2: calls by position alone, whose items share one lattice's records (see one_for_all); 8 x 512x512 x
+// 21 342 / 348.  Not beyond pd 5, where the compiler takes up to 16 registers more for it.
+template <int PD, typename T>
+__device__ __forceinline__ T load_record(const T* p) {
+    if constexpr (PD > 2 && PD <= 5) return __ldcs(p);
+    else return *p;
+}
+
 // Key read straight from L2 (no L1): for data that another CTA of the SAME launch may have written.
+template <int KW>
+__device__ __forceinline__ Key<KW> load_key_once(const Key<KW>* p) {
+    Key<KW> k;
+    const unsigned long long* w = reinterpret_cast<const unsigned long long*>(p);
+#pragma unroll
+    for (int j = 0; j < KW; j++) k.w[j] = load_once(w + j);
+    return k;
+}
 template <int KW>
 __device__ __forceinline__ Key<KW> load_key_l2(const Key<KW>* p) {
     Key<KW> k;

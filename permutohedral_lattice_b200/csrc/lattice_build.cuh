@@ -282,7 +282,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
         // the weights are final: store them now so the writes overlap the de-duplication below
         R* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
-        for (int r = 0; r <= PD; r++) recw_tile[r * TP + tid] = w[r];
+        for (int r = 0; r <= PD; r++) store_once(recw_tile + r * TP + tid, w[r]);
         // COMPACT: a point's own key is formed by steps, that of a splat it is compared with from the stored ranks.
         // The two are the same once the ranks are a permutation.
         if constexpr (COMPACT) settle_ranks<PD>(s);
@@ -473,7 +473,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
 #pragma unroll
     for (int r = 0; r <= PD; r++) {
         lfin[r] = valid ? (u16)(seg[r] + lidx_s[get_rep(r)]) : (u16)0;   // the representative has the same remainder
-        rec_tile[r * TP + tid] = lfin[r];
+        store_once(rec_tile + r * TP + tid, lfin[r]);
     }
     // The tile's splats sorted by entry (what the splat stage walks): a counting sort whose first half,
     // one shared-memory atomic per splat, returns the splat's place inside its entry's run.
@@ -743,7 +743,7 @@ __device__ __forceinline__ void finish_round(Header* hdr, InsertRound& rd, const
     if (tot) {
         int2* nb = reinterpret_cast<int2*>(vi.nbr);
         for (int a = 0; a <= vi.pd; a++)
-            for (u32 i = threadIdx.x; i < tot; i += 256) nb[(u64)a * vi.max_entries + base + i] = make_int2(-1, -1);
+            for (u32 i = threadIdx.x; i < tot; i += 256) store_once(nb + (u64)a * vi.max_entries + base + i, make_int2(-1, -1));
     }
     __syncthreads();
     if (threadIdx.x == 0) rd.count = 0;
@@ -772,7 +772,7 @@ insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>
             bool winner = false;
             u64 my_slot = 0;
             if (t < T) {
-                const Key<KW> k = list_keys[t];
+                const Key<KW> k = load_key_once<KW>(list_keys + t);
                 const u64 h = hash_key<KW>(k);
                 const u64 mine = (h & 0xFFFFFFFF00000000ull) | (u64)t;
                 u32 ref = 0xFFFFFFFFu;
@@ -807,7 +807,7 @@ insert_entries(Header* hdr, u64* __restrict__ table, u32 max_log2, const Key<KW>
                     atomicOr(&hdr->status, 1u << PL_INTERNAL_ERROR);
                     ref = t;
                 }
-                list_ref[t] = ref;   // owning entry, or (VERTEX_FLAG set) the vertex itself
+                store_once(list_ref + t, ref);   // owning entry, or (VERTEX_FLAG set) the vertex itself
             }
             round_add_winner(rd, winner, t, (u32)my_slot);
         }
@@ -975,8 +975,8 @@ __device__ __forceinline__ void link_axis(const u64* __restrict__ table, u64 mas
             if ((u32)(cur >> 32) == (u32)(h >> 32)) {
                 const u32 u = (u32)cur & ~VERTEX_FLAG;
                 if (key_equal<KW>(vkeys[u], k)) {
-                    nbr_axis[2 * (u64)v] = (int)u;
-                    nbr_axis[2 * (u64)u + 1] = (int)v;
+                    store_once(nbr_axis + 2 * (u64)v, (int)u);
+                    store_once(nbr_axis + 2 * (u64)u + 1, (int)v);
                     break;
                 }
             }
@@ -1000,8 +1000,8 @@ __device__ __forceinline__ void link_axis(const KeySlot* __restrict__ table, u32
             if ((u32)cur.y == 0xFFFFFFFFu) break;
             if (cur.x == k.w[0] && (u32)(cur.y >> 32) == key_rest<PD>(k)) {
                 const u32 u = (u32)cur.y & ~VERTEX_FLAG;
-                nbr_axis[2 * (u64)v] = (int)u;
-                nbr_axis[2 * (u64)u + 1] = (int)v;
+                store_once(nbr_axis + 2 * (u64)v, (int)u);
+                store_once(nbr_axis + 2 * (u64)u + 1, (int)v);
                 break;
             }
             s = (s + 1) & mask;

@@ -336,8 +336,8 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
         const float* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
-            l[r] = valid ? rec_tile[r * TP + tid] : 0;
-            w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
+            l[r] = valid ? load_record<PD>(rec_tile + r * TP + tid) : 0;
+            w[r] = valid ? load_record<PD>(recw_tile + r * TP + tid) : 0.f;
         }
         SplatCommon<PD>::template sort_splats<PD + 1>(valid, l, w, nloc, sorted_s, cur_s, wsum_s);
     }
@@ -594,8 +594,8 @@ __device__ __forceinline__ void splat_rows(const Geom& g, const TilePos& tpos, c
         const float* recw_tile = rec_w + (size_t)tile * SPLATS;
 #pragma unroll
         for (int r = 0; r <= PD; r++) {
-            l[r] = valid ? rec_tile[r * TP + tid] : 0;
-            w[r] = valid ? recw_tile[r * TP + tid] : 0.f;
+            l[r] = valid ? load_record<PD>(rec_tile + r * TP + tid) : 0;
+            w[r] = valid ? load_record<PD>(recw_tile + r * TP + tid) : 0.f;
         }
     }
     if (!PRE)
