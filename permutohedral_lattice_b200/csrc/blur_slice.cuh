@@ -58,7 +58,7 @@ constexpr u64 MOVED_ITEMS = 5000000;
 
 template <typename V>
 __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src,
-                                          V* __restrict__ dst, u32 vpr /* V per row */, u32 block, u32 blocks, u32 lattices /* of this size */) {
+                                          V* __restrict__ dst, u32 vpr /* V per row */, u32 block, u32 blocks) {
     // Passes after the first overlap the tail of the pass before (see after_previous_kernel).  The vertex count
     // and the neighbour table are older than any blur pass: a thread's first pair of neighbours is fetched
     // before the wait, so that one of the two dependent loads of its first row is off the critical path.
@@ -89,7 +89,7 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
         }
     };
     if constexpr (std::is_same<V, float4>::value) {
-        if (items * lattices <= MOVED_ITEMS) {
+        if (items <= MOVED_ITEMS) {
             rows([](V a, V b, V c) {
                 float2 z = make_float2(0.f, 0.f);
                 look_for_finite(z, a);
@@ -102,11 +102,10 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
     }
     rows([](V a, V b, V c) { return mix_rows(a, b, c); });
 }
-// blockIdx.y: the item, where one lattice serves several (item_v: V from one's rows to the next's).
 template <typename V>
 __global__ void __launch_bounds__(256, 8)
-blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst, u32 vpr, u64 item_v) {
-    blur_rows<V>(hdr, nbr_axis, src + blockIdx.y * item_v, dst + blockIdx.y * item_v, vpr, blockIdx.x, gridDim.x, gridDim.y);
+blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst, u32 vpr) {
+    blur_rows<V>(hdr, nbr_axis, src, dst, vpr, blockIdx.x, gridDim.x);
 }
 
 // Two passes in one launch, along axes a and then b: a thread mixes the row that pass b needs of its vertex and of that one's
@@ -176,8 +175,8 @@ __device__ __forceinline__ void blur_pair_rows(const Header* hdr, const int* __r
 template <typename V>
 __global__ void __launch_bounds__(256, PAIR_CTAS)
 blur_pair(const Header* hdr, const int* __restrict__ nbr_a, const int* __restrict__ nbr_b, const V* __restrict__ src,
-          V* __restrict__ dst, u32 vpr, u64 item_v) {
-    blur_pair_rows<V>(hdr, nbr_a, nbr_b, src + blockIdx.y * item_v, dst + blockIdx.y * item_v, vpr, blockIdx.x, gridDim.x);
+          V* __restrict__ dst, u32 vpr) {
+    blur_pair_rows<V>(hdr, nbr_a, nbr_b, src, dst, vpr, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -34,7 +34,7 @@ struct Geom {
     int calm_entries;       // entries of a tile up to which its points hardly change entry in disorder (see ColumnsSample)
     int from_positions;     // 1: features are read from a positions array
     int lattice_items;      // items that one lattice serves (see one_for_all): records and vertices are those of item 0
-    u32 item_rows;          // then: value rows (and entries) from one item's to the next's
+    u32 item_entries;       // then: entries from one item's to the next's
     u32 bound;              // then: the call's max_entries (the lattice's own is a share of it)
     float scale[MAX_PD];    // host-computed scale factors (double arithmetic rounded to float)
     // T = double calls: the same three in double
@@ -300,9 +300,9 @@ __device__ __forceinline__ TilePos tile_at(const Geom& g, int x, int z) {   // C
 }
 
 // Where one lattice serves several items (see one_for_all), every item has its own value rows and its own copy of the list of
-// entries, which names them, `item_rows` apart: what an item adds to its tiles' first entries.  (Added to the rows' address
+// entries, which names them, `item_entries` apart: what an item adds to its tiles' first entries.  (Added to the rows' address
 // instead, it cost the splat of narrow rows up to 28 bytes of spills, and at pd 5 an SM's sixth CTA.)
-__device__ __forceinline__ int first_entry_of(const Geom& g, int item) { return item * (int)g.item_rows; }
+__device__ __forceinline__ int first_entry_of(const Geom& g, int item) { return item * (int)g.item_entries; }
 
 __device__ __forceinline__ TilePos this_tile(const Geom& g) { return tile_at(g, blockIdx.x, blockIdx.z); }
 

@@ -87,14 +87,14 @@ insert_direct(Header* hdr, Direct d, u32* __restrict__ table, const Key<Cfg<PD>:
 // its slot (every slot carries a vertex index by now); the same result fills that neighbour's "-" slot.
 template <int PD>
 __global__ void __launch_bounds__(256, 8)
-link_neighbours_direct(Header* hdr, Direct d, const u32* __restrict__ table, u32* __restrict__ list_ref,
+link_neighbours_direct(Header* hdr, Direct d, const u32* __restrict__ table, const u32* owners, u32* list_ref,
                        const u32* __restrict__ vid, const Key<Cfg<PD>::KW>* __restrict__ vkeys,
                        int* __restrict__ nbr, u64 max_entries, ItemRows rows, Watch watch) {
     after_previous_kernel();
     report_to(watch, hdr);
     constexpr int KW = Cfg<PD>::KW;
     if (hdr->status != 0) return;
-    resolve_entries(hdr, list_ref, vid, rows);
+    resolve_entries(hdr, owners, list_ref, vid, rows);
     const u32 M = hdr->num_vertices;
     zero_rows_of(rows, M, grid_thread(), grid_threads());
     const u64 items = (u64)M * (PD + 1);

@@ -43,19 +43,23 @@ export_points(Geom g, const Header* hdr, const int2* __restrict__ tile_info, con
     constexpr int TP = Cfg<PD>::TP, SPLATS = Cfg<PD>::SPLATS;
     if (hdr->status != 0) return;
     const TilePos tpos = this_tile(g);
-    // (of a lattice that serves several items the records are those of the first, and the vertices counted item by item)
-    const u32 shared = hdr->items > 1 ? 1u : 0u;
-    const int tid = threadIdx.x, tile = shared ? tpos.tile % g.tiles_per_item : tpos.tile;
+    // (of a lattice that serves several items the records are those of the first, list_ref names its rows, and the vertices are counted
+    // item by item)
+    const u32 items = hdr->items;
+    const int tid = threadIdx.x, tile = items > 1 ? tpos.tile % g.tiles_per_item : tpos.tile;
     int item, pix;
     if (!tile_point(g, tpos, tid, item, pix)) return;
     const int base = tile_info[tile].x;
-    const u32 first = shared * (u32)item * hdr->num_vertices;
+    const u32 first = items > 1 ? (u32)item * hdr->num_vertices : 0u;
     const u16* rec_tile = rec + (size_t)tile * SPLATS;
     const R* recw_tile = rec_w + (size_t)tile * SPLATS;
     const size_t o = ((size_t)item * g.n + pix) * (PD + 1);
 #pragma unroll
     for (int r = 0; r <= PD; r++) {
-        if (pixel_vertex) pixel_vertex[o + r] = (int32_t)(first + list_ref[base + rec_tile[r * TP + tid]]);
+        if (pixel_vertex) {
+            const u32 row = list_ref[base + rec_tile[r * TP + tid]];
+            pixel_vertex[o + r] = (int32_t)(items > 1 ? first + row / items : row);
+        }
         if (pixel_weight) pixel_weight[o + r] = recw_tile[r * TP + tid];
     }
 }

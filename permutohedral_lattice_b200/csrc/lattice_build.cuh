@@ -652,22 +652,32 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
 // ---------------------------------------------------------------------------------------------
 // insert_entries
 // ---------------------------------------------------------------------------------------------
-// The items that the lattice serves (1, or see one_for_all), and their value rows, to be zeroed.
+// The items that the lattice serves (1, or see one_for_all), and their value rows, to be zeroed.  A vertex's rows lie together, item by
+// item: to the blur, the conversion of the fixed-point sums and the zeroing they are one long row.  With an item's rows together, each
+// of these had to walk the items one after another, in threads or blocks that have next to nothing to do for one: us a call without
+// a guide, 3 channels, so / now, 64x64x64 39 / 27, 1024x8x8 136 / 24.5, 16384x8x8 1927 / 67, 65535x4x4 15180 / 181, 8x256x256 36 / 38.
 struct ItemRows {
-    u32 items, stride;   // rows, and entries, from one item's to the next's
+    u32 items, stride;   // entries from one item's to the next's
     uint4* rows;         // float rows, rows of doubles, or the 64-bit sums of the deterministic mode; null: none
-    u32 row_quads;       // 16 bytes each
+    u32 row_quads;       // 16 bytes each, of a vertex, all items
 };
 __device__ __forceinline__ void zero_rows_of(const ItemRows& z, u32 M, u64 thread, u64 threads) {
     if (!z.rows) return;
     const u64 quads = (u64)M * z.row_quads;
-    for (u32 b = 0; b < z.items; b++)
-        for (u64 i = thread; i < quads; i += threads) z.rows[(u64)b * z.stride * z.row_quads + i] = make_uint4(0u, 0u, 0u, 0u);
+    for (u64 i = thread; i < quads; i += threads) z.rows[i] = make_uint4(0u, 0u, 0u, 0u);
 }
-// The vertex of entry t, and its rows, of every item.
-__device__ __forceinline__ void store_vertex_of(const ItemRows& z, u32* __restrict__ list_ref, u32 t, u32 v) {
-    list_ref[t] = v;
-    for (u32 b = 1; b < z.items; b++) list_ref[(u64)b * z.stride + t] = b * z.stride + v;
+// Calls store(t, b) for the T entries of every item b, spread over all threads.  (Their number fits 31 bits, as the bound does.)
+template <typename Store>
+__device__ __forceinline__ void for_entries_of(const ItemRows& z, u32 T, u32 thread, u32 threads, Store store) {
+    const u32 all = T * z.items;
+    for (u32 i = thread; i < all; i += threads) {
+        const u32 b = z.items > 1 ? i / T : 0u;
+        store(i - b * T, b);
+    }
+}
+// Entry t of item b has vertex v: the row that is its, in that item's copy of the list.
+__device__ __forceinline__ void store_vertex_of(const ItemRows& z, u32* list_ref, u32 t, u32 b, u32 v) {
+    list_ref[b * z.stride + t] = v * z.items + b;
 }
 
 // What the insert launch sets up for every vertex it creates, so that no later launch has to: the
@@ -919,15 +929,15 @@ insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cf
     }
 }
 
-// entry -> vertex: after the insert launch list_ref[t] names the entry that owns t's key; the link launch
-// turns that into the owner's vertex index (first loop of link_neighbours / link_neighbours_direct).
-__device__ __forceinline__ void resolve_entries(const Header* hdr, u32* __restrict__ list_ref,
+// entry -> vertex: after the insert launch owners[t] names the entry that owns t's key; the link launch turns that into the
+// owner's vertex index, in list_ref (first loop of link_neighbours / link_neighbours_direct).  The two are the same memory
+// where the lattice serves one item.
+__device__ __forceinline__ void resolve_entries(const Header* hdr, const u32* owners, u32* list_ref,
                                                 const u32* __restrict__ vid, const ItemRows& rows) {
-    const u32 T = hdr->num_entries;
-    for (u64 t = grid_thread(); t < T; t += grid_threads()) {
-        const u32 ref = list_ref[t];
-        store_vertex_of(rows, list_ref, (u32)t, (ref & VERTEX_FLAG) ? (ref & ~VERTEX_FLAG) : vid[ref]);
-    }
+    for_entries_of(rows, hdr->num_entries, (u32)grid_thread(), (u32)grid_threads(), [&](u32 t, u32 b) {
+        const u32 ref = owners[t];
+        store_vertex_of(rows, list_ref, t, b, (ref & VERTEX_FLAG) ? (ref & ~VERTEX_FLAG) : vid[ref]);
+    });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1021,13 +1031,13 @@ struct LinkAxis {   // link_axis of the axis this block works on, chosen once pe
 
 template <int PD, bool KEY_SLOTS, int KW = Cfg<PD>::KW>
 __global__ void __launch_bounds__(256)
-link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, u32* __restrict__ list_ref,
+link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, const u32* owners, u32* list_ref,
                 const u32* __restrict__ vid, const Key<KW>* __restrict__ vkeys, int* __restrict__ nbr,
                 u64 max_entries, ItemRows rows, Watch watch) {
     after_previous_kernel();
     report_to(watch, hdr);
     if (hdr->status != 0) return;
-    resolve_entries(hdr, list_ref, vid, rows);
+    resolve_entries(hdr, owners, list_ref, vid, rows);
     const u32 M = hdr->num_vertices;
     const u64 mask = (1ull << hdr->table_log2) - 1;
     zero_rows_of(rows, M, grid_thread(), grid_threads());   // under the latency of the lookups below

@@ -341,7 +341,7 @@ static bool make_direct(Direct& d, const Geom& g, int pd, const Layout& L) {
 // The features of a spatial-only call are those of its grid, the same in every item: one lattice does for all, with its share of the
 // bound, and value rows for every item.  The lattice's own geometry and layout, of one item; false: the call builds a lattice of all
 // its items.  A share fits where the whole would have: entries are the same in every item.  us a call, forward + backward, an own
-// lattice each / one: 8 x 512x512 x 21 414 / 346, 16 x 512x512 x 1 399 / 217; forward, 3 x 1000x700 x 3 100 / 76, 4 x 300x200 x 5 44 / 37.5.
+// lattice each / one: 8 x 512x512 x 21 414 / 334, 16 x 512x512 x 1 399 / 217; forward, 1024x8x8 x 3 28.5 / 24.5, 65535x4x4 x 3 424 / 181.
 static bool one_for_all(const Geom& g, const Layout& L, int pd, Geom& one, Layout& share) {
     one = g;
     share = L;
@@ -349,7 +349,7 @@ static bool one_for_all(const Geom& g, const Layout& L, int pd, Geom& one, Layou
     share.max_entries = L.max_entries / (u64)g.batch;
     while (share.table_slots > 1024 && share.table_slots / 2 >= 2 * share.max_entries) share.table_slots /= 2;
     one.lattice_items = g.batch;
-    one.item_rows = (u32)share.max_entries;
+    one.item_entries = (u32)share.max_entries;
     one.bound = (u32)L.max_entries;
     one.batch = 1;
     one.num_tiles = one.tiles_per_item;
@@ -577,6 +577,15 @@ static bool small_blur(const Geom& g, int pd, const Layout& L, u32 vpr) {
     const int pieces = worst_case(g, pd, L) ? 2 : SMALL_PIECES;
     return L.max_entries <= pieces * one_each && vpr <= 16;
 }
+// Where one lattice serves several items, the rows of a vertex lie together, and a cluster's 16 bytes of them far apart: up to eight
+// float4 a vertex.  us a call, two passes a launch / all in one: 64x64x64 x 1 26 / 45, 16x128x128 x 1 26 / 34, 2x256x256 x 21 32 / 37.
+constexpr u32 SMALL_SHARED = 8;
+// A batch that is small as a whole, and would have its blur in one launch with a lattice of all items but not with one for them all: such a
+// call waits for its launches, as long as the construction of all takes no longer than that of one, with a tile an SM or fewer.  us a
+// call, a lattice each / one: 64x8x8 x 1 22 / 24, 4x64x64 x 21 23.8 / 25.7; with more tiles 64x32x32 x 1 28 / 24, 16x64x64 x 21 36 / 27.
+static bool better_each(const Geom& g, int pd, const Layout& whole, u32 quads) {
+    return g.num_tiles <= num_sms() && quads * (u32)g.batch > SMALL_SHARED && small_blur(g, pd, whole, quads);
+}
 // Two passes a launch (see blur_pair_rows), by what the bound says of the vertices.  us a call, a pass / two a launch: bounds
 // of 393 k x 2 items, 115 k vertices (512x512 x 3 in double, forward + backward) 185 / 179; worst cases filled by vertices: 240 k
 // 99.3 / 98.2, 470 k 142 / 144, 960 k 239 / 254.
@@ -586,27 +595,29 @@ static bool blur_in_pairs(const Geom& g, int pd, const Layout& L, u32 vpr) {
 template <int PD, int KW>
 static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
                               const VertexInit& vinit, const ItemRows& rows, Watch watch, cudaStream_t st) {
-    const u32 entries = (u32)L.max_entries;
+    const u32 entries = (u32)L.max_entries;   // (times the items: no more than the call's bound)
     const size_t smem = SmallIndex<PD>::bytes(entries);
     PL_TRY((ensure_dynamic_smem<index_small<PD, KW>>(smem)));
-    // a thread for every axis and vertex, up to 64 CTAs
-    const u32 ctas = std::max(8u, std::min(64u, (entries * (PD + 1) + SMALL_THREADS - 1) / SMALL_THREADS));
+    // a thread for every axis and vertex, up to 64 CTAs, and for the entries and rows of all items, up to one CTA an SM
+    const u64 of_items = rows.items > 1 ? ((u64)entries * rows.items + SMALL_THREADS - 1) / SMALL_THREADS : 0;
+    const u32 ctas = std::max(std::max(8u, std::min(64u, (entries * (PD + 1) + SMALL_THREADS - 1) / SMALL_THREADS)),
+                              (u32)std::min(of_items, (u64)num_sms()));
     PL_LAUNCH_AFTER(true, (index_small<PD, KW>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, rows, (u32)smem, watch);
     return PL_OK;
 }
 template <typename V, int PIECES>
-static int launch_small_blur_as(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, u32 items, u64 item_v, cudaStream_t st) {
+static int launch_small_blur_as(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
     const size_t smem = sizeof(V) * 2 * PIECES * SMALL_THREADS;
     PL_TRY((ensure_dynamic_smem<blur_small<V, PIECES>>(smem)));
-    PL_LAUNCH_AFTER(true, (blur_small<V, PIECES>), dim3(SMALL_CTAS * vpr, items), SMALL_THREADS, smem, st, hdr, nbr, L.max_entries, v, vpr, axes, reverse, item_v);
+    PL_LAUNCH_AFTER(true, (blur_small<V, PIECES>), SMALL_CTAS * vpr, SMALL_THREADS, smem, st, hdr, nbr, L.max_entries, v, vpr, axes, reverse);
     return PL_OK;
 }
 template <typename V>
-static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, u32 items, u64 item_v, cudaStream_t st) {
+static int launch_small_blur(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
     const u64 pieces = (L.max_entries + SMALL_CTAS * SMALL_THREADS - 1) / (SMALL_CTAS * SMALL_THREADS);   // a thread
-    return pieces <= 1   ? launch_small_blur_as<V, 1>(hdr, nbr, L, v, vpr, axes, reverse, items, item_v, st)
-           : pieces <= 2 ? launch_small_blur_as<V, 2>(hdr, nbr, L, v, vpr, axes, reverse, items, item_v, st)
-                         : launch_small_blur_as<V, SMALL_PIECES>(hdr, nbr, L, v, vpr, axes, reverse, items, item_v, st);
+    return pieces <= 1   ? launch_small_blur_as<V, 1>(hdr, nbr, L, v, vpr, axes, reverse, st)
+           : pieces <= 2 ? launch_small_blur_as<V, 2>(hdr, nbr, L, v, vpr, axes, reverse, st)
+                         : launch_small_blur_as<V, SMALL_PIECES>(hdr, nbr, L, v, vpr, axes, reverse, st);
 }
 
 // The header's counters and, in calls that keep one, the sketch behind it.
@@ -639,10 +650,10 @@ static int run_filter(const Geom& call, float* output, const float* input, const
     // g, L: of the whole call; the lattice is that of `one`, within `share` of the bound (see one_for_all)
     Geom g = call, one;
     Layout share;
-    const bool together = phases == (PH_BUILD | PH_APPLY) && one_for_all(call, whole, PD, one, share);
+    const bool together = phases == (PH_BUILD | PH_APPLY) && !better_each(call, PD, whole, (u32)padded_vd(vd) / 4) && one_for_all(call, whole, PD, one, share);
     if (together) {
         g.lattice_items = one.lattice_items;
-        g.item_rows = one.item_rows;
+        g.item_entries = one.item_entries;
     } else {
         one = call;
         share = whole;
@@ -718,15 +729,17 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         vinit.pd = PD;
         ItemRows rows;
         rows.items = items;
-        rows.stride = one.item_rows;
+        rows.stride = one.item_entries;
         rows.rows = (phases & PH_APPLY) ? (v64 ? reinterpret_cast<uint4*>(v64) : reinterpret_cast<uint4*>(v0)) : nullptr;
-        rows.row_quads = (u32)padded_vd(vd) / (v64 ? 2u : 4u);
+        rows.row_quads = (u32)padded_vd(vd) / (v64 ? 2u : 4u) * items;
+        // what the insert says of an entry and the link resolves: in a list that is not the items', whose entries come from it, all of them
+        u32* owners = together ? vid + share.max_entries : list_ref;
         if constexpr (PD <= MAX_SDIMS) {
             if (use_direct) {
                 u32* table32 = reinterpret_cast<u32*>(table);
                 if (!cleared) PL_LAUNCH_AFTER(true, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
-                PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
-                PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
+                PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, owners, vid, vkeys, vinit);
+                PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, owners, list_ref, vid, vkeys, nbr,
                                                                  share.max_entries, rows, watch);
             }
         }
@@ -738,10 +751,10 @@ static int run_filter(const Geom& call, float* output, const float* input, const
                 constexpr bool KEYS = decltype(keys_in_slots)::value;
                 if (!cleared) PL_LAUNCH_AFTER(true, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
                 if constexpr (KEYS)
-                    PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
+                    PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, owners, vid, vkeys, vinit, cleared);
                 else
-                    PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
-                PL_LAUNCH_AFTER(true, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, share.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr,
+                    PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, owners, vid, vkeys, vinit, cleared);
+                PL_LAUNCH_AFTER(true, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, share.max_entries), 256, 0, st, hdr, table, (u32)table_log2, owners, list_ref, vid, vkeys, nbr,
                                                           share.max_entries, rows, watch);
                 return PL_OK;
             };
@@ -763,10 +776,7 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         PL_CUDA(cudaGetLastError());
         return PL_OK;
     }
-    // the blur passes (and the conversion of the fixed-point sums): a row of blocks for every item that the lattice serves
-    const u32 qpr = (u32)padded_vd(vd) / 4;
-    const u64 item_v = (u64)one.item_rows * qpr;
-    auto rows_of_blocks = [&](int blocks) { return (unsigned)((blocks + (int)items - 1) / (int)items); };
+    const u32 qpr = (u32)padded_vd(vd) / 4 * items;   // float4 of a vertex, in the rows of all items
     int rc = PL_OK;
     if (v64) {
         if (vd > widest_vd_fixed(PD)) return PL_UNSUPPORTED_DIMS;
@@ -774,7 +784,7 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         rc = (phases & PH_BUILD) ? launch_splat_fixed<PD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st)
                                  : launch_splat_fixed<PD, true>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st);
         if (rc != PL_OK) return rc;
-        PL_LAUNCH_AFTER(true, (convert_fixed), dim3(rows_of_blocks(wide), items), 256, 0, st, hdr, v64, v0, padded_vd(vd), item_v * 4);
+        PL_LAUNCH_AFTER(true, (convert_fixed), wide, 256, 0, st, hdr, v64, v0, qpr * 4);
         PL_COUNT_LAUNCHES(1);   // convert_fixed (the splat itself is counted below)
     } else {
         rc = PL_SPLAT_FOR(PD, vd, g, input, hdr, tile_info, rec, rec_w, srec, !(phases & PH_BUILD), list_ref, v0, vd, st);
@@ -784,22 +794,22 @@ static int run_filter(const Geom& call, float* output, const float* input, const
     if (ev) PL_CUDA(cudaEventRecord(ev[3], st));
     float* src = v0;
     float* dst = v1;
-    const bool one_blur = small_blur(one, PD, share, qpr * items);
+    const bool one_blur = small_blur(one, PD, share, qpr) && (items == 1 || qpr <= SMALL_SHARED);
     if (one_blur) {
-        PL_TRY(launch_small_blur(hdr, nbr, share, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, items, item_v, st));
+        PL_TRY(launch_small_blur(hdr, nbr, share, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, st));
         PL_COUNT_LAUNCHES(1);
-    } else if (blur_in_pairs(one, PD, share, qpr * items)) {
+    } else if (blur_in_pairs(one, PD, share, qpr)) {
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * share.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * share.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<float4>), dim3(rows_of_blocks(sms * PAIR_CTAS), items), 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
+            PL_LAUNCH_AFTER(true, (blur_pair<float4>), sms * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
             std::swap(src, dst);
             PL_COUNT_LAUNCHES(1);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * share.max_entries * 2;
-        PL_LAUNCH_AFTER(true, (blur_axis<float4>), dim3(rows_of_blocks(wide), items), 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
+        PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
         float* tmp = src; src = dst; dst = tmp;
         PL_COUNT_LAUNCHES(1);
     }
@@ -864,7 +874,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         if (use_direct) {
             if (!cleared) PL_LAUNCH_AFTER(true, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
             PL_LAUNCH_AFTER(before_insert, (insert_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_keys, list_ref, vid, vkeys, vinit);
-            PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, vid, vkeys, nbr,
+            PL_LAUNCH_AFTER(true, (link_neighbours_direct<PD>), wide, 256, 0, st, hdr, direct, table32, list_ref, list_ref, vid, vkeys, nbr,
                                                              L.max_entries, rows, watch);
         }
     }
@@ -876,7 +886,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
             PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
         else
             PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
-        PL_LAUNCH_AFTER(true, (link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, vid, vkeys, nbr, L.max_entries,
+        PL_LAUNCH_AFTER(true, (link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   rows, watch);
     }
     PL_LAUNCH_AFTER(true, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
@@ -885,17 +895,17 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     double* dst = v1;
     const bool one_blur = small_blur(g, PD, L, (u32)vp / 2), pairs = blur_in_pairs(g, PD, L, (u32)vp / 2);
     if (one_blur) {
-        PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<double2*>(v0), (u32)vp / 2, PD + 1, reverse, 1, 0, st));
+        PL_TRY(launch_small_blur(hdr, nbr, L, reinterpret_cast<double2*>(v0), (u32)vp / 2, PD + 1, reverse, st));
     } else if (pairs) {
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
+            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
             std::swap(src, dst);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
+        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
         double* tmp = src; src = dst; dst = tmp;
     }
     PL_LAUNCH_AFTER(vd <= 4 || slice_overlap(g, one_blur), (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
@@ -985,11 +995,11 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     const float *va = a.v0, *vs = s.v0;
     int launches = 3;
     if (small_s) {
-        PL_TRY(launch_small_blur(s.hdr, s.nbr, LS, reinterpret_cast<float4*>(s.v0), quads, PDS + 1, 0, 1, 0, st));
+        PL_TRY(launch_small_blur(s.hdr, s.nbr, LS, reinterpret_cast<float4*>(s.v0), quads, PDS + 1, 0, st));
         launches++;
     }
     if (small_a) {
-        PL_TRY(launch_small_blur(a.hdr, a.nbr, LA, reinterpret_cast<float4*>(a.v0), quads, PDA + 1, 0, 1, 0, st));
+        PL_TRY(launch_small_blur(a.hdr, a.nbr, LA, reinterpret_cast<float4*>(a.v0), quads, PDA + 1, 0, st));
         launches++;
     }
     const bool pairs = blur_in_pairs(g, PDA, LA, quads) && blur_in_pairs(g, PDS, LS, quads);
@@ -1014,7 +1024,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     auto rest_of = [&](const LatticeRows& l, int step, int pd, const float*& v) -> int {   // from pass `step` on
         for (; step <= pd; step++) {
             const Pass p = pass_of(l, step);
-            PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads, (u64)0);
+            PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads);
             launches++;
             v = reinterpret_cast<const float*>(p.dst);
         }

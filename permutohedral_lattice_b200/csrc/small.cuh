@@ -163,10 +163,10 @@ index_small(Header* hdr, const Key<KW>* __restrict__ list_keys, u32* __restrict_
         hdr->table_log2 = lg;
         report_to(watch, hdr);
     }
-    for (u32 t = me; t < T; t += all) {
+    for_entries_of(rows, T, me, all, [&](u32 t, u32 b) {
         const u32 v = table_s[slot_s[t]] >> 16;
-        store_vertex_of(rows, list_ref, t, v);
-        if (owner_s[v] == t) {
+        store_vertex_of(rows, list_ref, t, b, v);
+        if (b == 0 && owner_s[v] == t) {
             if constexpr (SI::EXACT) {
                 Key<KW> k;
                 k.w[0] = first_s[t];
@@ -176,7 +176,7 @@ index_small(Header* hdr, const Key<KW>* __restrict__ list_keys, u32* __restrict_
                 vkeys[v] = list_keys[t];
             }
         }
-    }
+    });
     zero_rows_of(rows, M, me, all);
     int2* nb = reinterpret_cast<int2*>(vi.nbr);
     for (u32 i = me; i < M * (PD + 1); i += all) {
@@ -250,14 +250,14 @@ __device__ __forceinline__ double2 load_cluster(u32 addr, u32 cta, double2) {
 }
 template <typename V, int PIECES>
 __global__ void __cluster_dims__(SMALL_CTAS, 1, 1) __launch_bounds__(SMALL_THREADS)
-blur_small(const Header* hdr, const int* __restrict__ nbr, u64 max_entries, V* v, u32 vpr, int axes, int reverse, u64 item_v) {
+blur_small(const Header* hdr, const int* __restrict__ nbr, u64 max_entries, V* v, u32 vpr, int axes, int reverse) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* const buf = reinterpret_cast<V*>(smem_raw);
     const u32 M = hdr->num_vertices;   // (older than the splat before this)
     u32 chunk_log2 = 5;
     while ((u32)SMALL_CTAS << chunk_log2 < M) chunk_log2++;
     const u32 chunk = 1u << chunk_log2, first = (blockIdx.x % SMALL_CTAS) << chunk_log2;
-    v += blockIdx.x / SMALL_CTAS + blockIdx.y * item_v;
+    v += blockIdx.x / SMALL_CTAS;
     const int2* __restrict__ nb = reinterpret_cast<const int2*>(nbr);
     auto axis = [&](int step) { return (u64)(reverse ? axes - 1 - step : step) * max_entries; };
     int2 even[PIECES], odd[PIECES];   // neighbours of vertex first + at(p) in the next pass of either kind
