@@ -592,18 +592,26 @@ static bool better_each(const Geom& g, int pd, const Layout& whole, u32 quads) {
 static bool blur_in_pairs(const Geom& g, int pd, const Layout& L, u32 vpr) {
     return L.max_entries * vpr <= (worst_case(g, pd, L) ? PAIR_ITEMS_WORST : PAIR_ITEMS);
 }
-template <int PD, int KW>
-static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
+template <int PD, int KW, bool SHARED>
+static int launch_small_index_as(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
                               const VertexInit& vinit, const ItemRows& rows, Watch watch, cudaStream_t st) {
     const u32 entries = (u32)L.max_entries;   // (times the items: no more than the call's bound)
     const size_t smem = SmallIndex<PD>::bytes(entries);
-    PL_TRY((ensure_dynamic_smem<index_small<PD, KW>>(smem)));
+    PL_TRY((ensure_dynamic_smem<index_small<PD, KW, SHARED>>(smem)));
     // a thread for every axis and vertex, up to 64 CTAs, and for the entries and rows of all items, up to one CTA an SM
-    const u64 of_items = rows.items > 1 ? ((u64)entries * rows.items + SMALL_THREADS - 1) / SMALL_THREADS : 0;
+    const u64 of_items = SHARED ? ((u64)entries * rows.items + SMALL_THREADS - 1) / SMALL_THREADS : 0;
     const u32 ctas = std::max(std::max(8u, std::min(64u, (entries * (PD + 1) + SMALL_THREADS - 1) / SMALL_THREADS)),
                               (u32)std::min(of_items, (u64)num_sms()));
-    PL_LAUNCH_AFTER(true, (index_small<PD, KW>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, rows, (u32)smem, watch);
+    PL_LAUNCH_AFTER(true, (index_small<PD, KW, SHARED>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, rows, (u32)smem, watch);
     return PL_OK;
+}
+template <int PD, int KW>
+static int launch_small_index(Header* hdr, const Layout& L, const Key<KW>* list_keys, u32* list_ref, Key<KW>* vkeys,
+                              const VertexInit& vinit, const ItemRows& rows, Watch watch, cudaStream_t st) {
+    if constexpr (PD <= MAX_SDIMS) {
+        if (rows.items > 1) return launch_small_index_as<PD, KW, true>(hdr, L, list_keys, list_ref, vkeys, vinit, rows, watch, st);
+    }
+    return launch_small_index_as<PD, KW, false>(hdr, L, list_keys, list_ref, vkeys, vinit, rows, watch, st);
 }
 template <typename V, int PIECES>
 static int launch_small_blur_as(const Header* hdr, const int* nbr, const Layout& L, V* v, u32 vpr, int axes, int reverse, cudaStream_t st) {
