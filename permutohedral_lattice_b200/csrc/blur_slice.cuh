@@ -55,6 +55,10 @@ __device__ __forceinline__ bool all_finite(float2 z) { return PL_FADD(z.x, z.y) 
 // Beyond so many pieces of 16 bytes the rows do not stay in L2, and conversions are as fast as moves or faster: 8 x 512x512 x 21
 // of a noisy lattice (20 M pieces) 3768 / 3841 us a call.
 constexpr u64 MOVED_ITEMS = 5000000;
+// Nor do lines of neighbours that are loaded evict-first stay until the next block wants its part of them, so that beyond it the loop loads them
+// plainly: us a call, evict-first / plain, 8 x 512x512 x 21 of a noisy guide, 3.5 M vertices 2577 / 2453, 60 k points x 21 at pd 16, 1 M vertices 1056 / 1011.
+// Below, evict-first leaves L2 to the rows: 800x1200 x 3 163 / 165, five CRF steps on 375x500 x 21 371 / 378, 200 k points x 7 at pd 16 328 / 341.
+// (Two loops: chosen in the loop, it cost up to 4 %.)
 
 template <typename V>
 __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src,
@@ -72,7 +76,7 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
     after_previous_kernel();
     if (hdr->status != 0) return;
     const V zero = {};
-    auto rows = [&](auto mix) {
+    auto rows = [&](auto once, auto mix) {
         while (e < items) {
             const V b = src[e];
             const V a = (n.x >= 0) ? src[(u64)n.x * vpr + j] : zero;
@@ -83,14 +87,18 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
                 j -= vpr;
                 v++;
             }
-            if (v < M) n = load_once(nb + v);
+            if constexpr (decltype(once)::value) {
+                if (v < M) n = load_once(nb + v);
+            } else {
+                if (v < M) n = __ldg(nb + v);
+            }
             dst[e] = mix(a, b, c);
             e += stride;
         }
     };
     if constexpr (std::is_same<V, float4>::value) {
         if (items <= MOVED_ITEMS) {
-            rows([](V a, V b, V c) {
+            rows(std::true_type{}, [](V a, V b, V c) {
                 float2 z = make_float2(0.f, 0.f);
                 look_for_finite(z, a);
                 look_for_finite(z, b);
@@ -100,7 +108,7 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
             return;
         }
     }
-    rows([](V a, V b, V c) { return mix_rows(a, b, c); });
+    rows(std::is_same<V, double2>{}, [](V a, V b, V c) { return mix_rows(a, b, c); });
 }
 template <typename V>
 __global__ void __launch_bounds__(256, 8)
