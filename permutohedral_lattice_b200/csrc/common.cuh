@@ -55,7 +55,7 @@ struct Header {   // first 256 bytes of the workspace
     u32 reported;      // status bits that the call's watch has told the host of (see Watch)
     u32 calm_entries;  // of the Geom that the lattice was built with
     u32 items;         // items that the lattice serves: entries and vertices are those of one of them
-    u32 mostly_new;    // in calls with a sketch: most of the entries are vertices (see insert_keys)
+    u32 mostly_new;    // in calls with a sketch: 30 % of the entries or more are vertices, in a table that stays in L2 (see insert_keys)
     u32 pad[51];
 };
 

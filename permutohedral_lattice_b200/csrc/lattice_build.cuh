@@ -582,7 +582,7 @@ __device__ __forceinline__ u32 log2_of_slots(u64 need, u32 max_log2) {
 constexpr u64 KEY_SLOTS_WHOLE = 1ull << 21;   // 32 MB
 constexpr u64 TAG_SLOTS_WHOLE = 1ull << 23;   // 64 MB
 constexpr u64 TAG_SLOTS_MOST = 1ull << 25;    // beyond, half as many would not stay in L2 either
-constexpr float MOSTLY_NEW = 0.3f;            // see insert_keys
+constexpr float MOSTLY_NEW = 0.3f;            // vertices an entry, see insert_keys
 template <bool KEY_SLOTS>
 __global__ void __launch_bounds__(256)
 clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift) {
@@ -633,7 +633,7 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         hdr->table_log2 = lg;
         hdr->filter_log2 = filter_log2;
-        hdr->mostly_new = mostly_new ? 1u : 0u;
+        hdr->mostly_new = mostly_new && (1ull << lg) <= KEY_SLOTS_WHOLE ? 1u : 0u;
     }
     if constexpr (!KEY_SLOTS) {
         if (filter_log2) {
@@ -865,9 +865,13 @@ __device__ __forceinline__ u32 key_rest(const Key<Cfg<PD>::KW>& k) {
 // the vertex.
 // A compare-and-swap on a line that was just read takes longer than one on a line that was not: in a table of 32 MB a ns sees 175 loads of
 // random slots, 80 swaps, 50 times load, swap and store of an empty slot, 70 times swap and store.  So slots are claimed unseen where the sketch
-// says that MOSTLY_NEW of the entries are vertices and, in calls without one, by a warp as long as a third of what it claims is free,
-// which the first of the entries mostly are, whatever the lattice.  us a call, a
-// look first / not: 800x1200 x 3, 54 % vertices, 172 / 169.5, 1024x1024 grey by RGB, 33 %, 300 / 298.5; 16 x 512x512 x 21, 16 %, 1764 / 1791.
+// says that MOSTLY_NEW of the entries or more are vertices and the table stays in L2 (up to 32 MB; beyond, the load brings the line in for the
+// swap).  us a call, a look first / not, by the share of vertices, below the line 14 %, 8 x 512x512 x 3 251 / 255, 19 % 225 / 226, 24 %, 4 x 512x512 x 3
+// 148 / 147, 30 %, 1024x1024 x 3 121 / 120, but 2 x 111x128x120 of a noisy guide, 20 to 30 %, 423 / 432; above it 1024x1024 x 3, 31 % 122 / 122, 34 % 162
+// / 159, 39 % 238 / 236, 800x1200 x 3, 52 % 155 / 152, 57 % 206 / 203.  Tables of 64 MB and more: 8 x 512x512 x 3, noise 0.16, 730 / 755, 0.25
+// 1166 / 1193, 800x1200 x 3, 73 %, 714 / 720.
+// In calls without a sketch a warp does as long as a third of what it claims is free, which the first of the entries mostly are, whatever
+// the lattice: 300x400 x 3, 29 % 36 / 36, 32 % 41.4 / 40.3, 35 % 44 / 42.6, 40 % 56 / 54.5, 46 % 80.7 / 80.9, 512x512 x 3, 51 % 55.7 / 54.7, 63 % 99.6 / 100.
 template <int PD>
 __global__ void __launch_bounds__(256, 8)   // as many as it is launched with
 insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cfg<PD>::KW>* __restrict__ list_keys,
