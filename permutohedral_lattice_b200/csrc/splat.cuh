@@ -149,9 +149,11 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
 // Bound by the latency of its loads (most stalls are for them; its reductions are none, L2 is at 34 %).  Two volumes of
 // 111x128x120 points, 20 splats an entry: sorted 106 us (LSU pipe at 82 %), in columns of eight points, which left 3 of 8 warps
 // without work, 87, so 83.  us a call, eight points / so: 16 x 512x512 x 1 without a guide 208 / 186, x 3 198 / 189; 96x128x128 x
-// 1 without a guide, forward + backward, 207 / 200.  (The figures below are those of eight points.)  The records of
-// two channels at pd 4 are loaded evict-first, which leaves L1 to the points' rows: the two volumes, forward + backward, 490.5 -> 483.7; with one and
-// three channels, 4 x 512x512 guided by two, a call 84.9 -> 85.7 and 101.8 -> 103, so not there.
+// 1 without a guide, forward + backward, 207 / 200.  (The figures below are those of eight points.)  At pd 4 the records of
+// one and two channels are loaded evict-first, which leaves L1 to the points' rows.  us a call, plain / so, volumes of 0.5 to 8 M points and
+// images of 1 to 4 M: one channel 64x80x96 64.7 / 64.8, two of them 86.1 / 86.8, two of 111x128x120 262.6 / 258.8 (theta 10: 255 / 247), 200x200x200 552 / 550, images 105.3
+// / 105.4 to 308 / 308; two channels 54.6 / 54.7, 87 / 87, 263 / 260 (253 / 247), 555 / 555.5, images 94.4 / 94.6 to 315.2 / 315.5.  Not with three, 56 / 56.5, 88.6 /
+// 89.7, 268 / 269 (259 / 257), 568 / 577, images 96 / 97 to 324 / 326, nor at pd 3: 8 volumes of 64x64x64 without a guide 75 / 74, 83 / 84 and 83 / 83.
 // Where (us a splat, columns / sorted): rows of more than one float4 from 2 pd splats an entry on (8 x 512x512, pd 2,
 // 21 channels, 4.8 splats 95 / 110, 14.7 splats 76 / 98); narrow ones as NarrowColumns says.  pd 5, us a call: 8
 // splats an entry 201 / 197, 36 splats 158 / 138: up to pd 4.  Tiles of points in one dimension, which are all there are with pd 1, have no columns.
@@ -221,7 +223,7 @@ __device__ __forceinline__ void splat_columns(const Geom& g, const TilePos& tpos
                                               const float* __restrict__ recw_tile,
                                               const u32* __restrict__ list_ref, float* __restrict__ v0, bool halves) {
     constexpr int TP = Cfg<PD>::TP, C = VD - 1, VP = (VD + 3) & ~3;
-    constexpr bool ONCE = PD == 4 && VD == 3;
+    constexpr bool ONCE = PD == 4 && VD <= 3;   // (see above)
     constexpr int PIECES = TP / (16 * (PD + 1));   // of 16 points of a column, or two; a tile has TX columns of 256 / TX points
     const int tid = threadIdx.x, r = halves ? tid / 32 : tid / (16 * PIECES), c = halves ? tid % 32 : tid % (16 * PIECES);
     const int lx = c & (g.TX - 1), s = c >> g.tx_log2, k = halves ? s % 2 : s % PIECES;
