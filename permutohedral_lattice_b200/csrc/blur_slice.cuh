@@ -308,7 +308,7 @@ slice_tiles_fast(Geom g, float* __restrict__ output, const Header* hdr, const in
     const int tid = threadIdx.x, tile = tpos.tile;
     const u32 status = hdr->status;   // final by now, the same in every thread; one round trip with all that follows
     const int2 info = tile_info[tile];
-    const int base = info.x + first_entry_of(g, tpos.item), cnt = info.y;
+    const int base = info.x + first_entry_of<PD>(g, tpos.item), cnt = info.y;
     const int nrows = min(cnt, rows_cap);
     const float4* v4 = reinterpret_cast<const float4*>(vsrc);
     int item, pix;
@@ -404,7 +404,7 @@ slice_points(Geom g, float* __restrict__ output, const Header* hdr, const int2* 
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x;
     const u32 status = hdr->status;   // final by now: the same in every thread
-    const int base = tile_info[tpos.tile].x + first_entry_of(g, tpos.item);
+    const int base = tile_info[tpos.tile].x + first_entry_of<PD>(g, tpos.item);
     int item, pix;
     const bool valid = tile_point(g, tpos, tid, item, pix);
     auto stop = [&]() {
@@ -468,7 +468,7 @@ slice_tiles_generic(Geom g, float* __restrict__ output, const Header* hdr, const
     const TilePos tpos = this_tile(g);
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
-    const int base = info.x + first_entry_of(g, tpos.item), cnt = info.y;
+    const int base = info.x + first_entry_of<PD>(g, tpos.item), cnt = info.y;
     const int nrows = min(cnt, rows_cap);
     const float4* v4 = reinterpret_cast<const float4*>(vsrc);
     int item, pix;

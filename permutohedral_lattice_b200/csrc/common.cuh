@@ -301,8 +301,13 @@ __device__ __forceinline__ TilePos tile_at(const Geom& g, int x, int z) {   // C
 
 // Where one lattice serves several items (see one_for_all), every item has its own value rows and its own copy of the list of
 // entries, which names them, `item_entries` apart: what an item adds to its tiles' first entries.  (Added to the rows' address
-// instead, it cost the splat of narrow rows up to 28 bytes of spills, and at pd 5 an SM's sixth CTA.)
-__device__ __forceinline__ int first_entry_of(const Geom& g, int item) { return item * (int)g.item_entries; }
+// instead, it cost the splat of narrow rows up to 28 bytes of spills, and at pd 5 an SM's sixth CTA.)  A call by position alone has at most MAX_SDIMS
+// feature dimensions.  (Without that said, slice_tiles_fast<16, 24> spilled 40 -> 104 bytes.)
+template <int PD>
+__device__ __forceinline__ int first_entry_of(const Geom& g, int item) {
+    if constexpr (PD <= MAX_SDIMS) return item * (int)g.item_entries;
+    else return 0;
+}
 
 __device__ __forceinline__ TilePos this_tile(const Geom& g) { return tile_at(g, blockIdx.x, blockIdx.z); }
 

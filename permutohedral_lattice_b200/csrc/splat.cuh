@@ -294,7 +294,7 @@ splat_tiles_fast(Geom g, const float* __restrict__ input, Header* hdr, const int
     if constexpr (NC::EVER) halves = hdr->num_entries > NC::SHARED * hdr->num_vertices;
     if (call_failed(hdr)) return;
     if (PRE && !lattice_is_sorted(hdr)) return;
-    const int base = info.x + first_entry_of(g, tpos.item), nloc = info.y;
+    const int base = info.x + first_entry_of<PD>(g, tpos.item), nloc = info.y;
     using CS = ColumnsSample<PD>;
     if constexpr (NC::EVER) {
         if (in_columns<PD>(g, nloc, NC::LEAST) && CS::smooth(g, tpos, hdr, rec, nloc, CS::NARROW)) {
@@ -576,7 +576,7 @@ __device__ __forceinline__ void splat_rows(const Geom& g, const TilePos& tpos, c
     }
     const int tid = threadIdx.x, tile = tpos.tile, lane = tid & 31, warp = tid >> 5;
     const int2 info = tile_info[tile];
-    const int base = info.x + first_entry_of(g, tpos.item), nloc = info.y;
+    const int base = info.x + first_entry_of<PD>(g, tpos.item), nloc = info.y;
     using CS = ColumnsSample<PD>;
     constexpr bool SAMPLED = CS::TAKEN && WideColumns<PD, PRE, Sum>::EVER;
     bool columns = WideColumns<PD, PRE, Sum>::take(g, nloc, LR);   // (so far; then by the sample)
