@@ -62,7 +62,7 @@ constexpr u64 MOVED_ITEMS = 5000000;
 
 template <typename V>
 __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src,
-                                          V* __restrict__ dst, u32 vpr /* V per row */, u32 block, u32 blocks) {
+                                          V* __restrict__ dst, u32 vpr /* V per row */, u32 block, u32 blocks, u32 lattices /* of this size */) {
     // Passes after the first overlap the tail of the pass before (see after_previous_kernel).  The vertex count
     // and the neighbour table are older than any blur pass: a thread's first pair of neighbours is fetched
     // before the wait, so that one of the two dependent loads of its first row is off the critical path.
@@ -97,7 +97,7 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
         }
     };
     if constexpr (std::is_same<V, float4>::value) {
-        if (items <= MOVED_ITEMS) {
+        if (items * lattices <= MOVED_ITEMS) {
             rows(std::true_type{}, [](V a, V b, V c) {
                 float2 z = make_float2(0.f, 0.f);
                 look_for_finite(z, a);
@@ -110,10 +110,11 @@ __device__ __forceinline__ void blur_rows(const Header* hdr, const int* __restri
     }
     rows(std::is_same<V, double2>{}, [](V a, V b, V c) { return mix_rows(a, b, c); });
 }
+// blockIdx.y: the item, where one lattice serves several whose rows lie apart (item_v: V from one's rows to the next's).
 template <typename V>
 __global__ void __launch_bounds__(256, 8)
-blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst, u32 vpr) {
-    blur_rows<V>(hdr, nbr_axis, src, dst, vpr, blockIdx.x, gridDim.x);
+blur_axis(const Header* hdr, const int* __restrict__ nbr_axis, const V* __restrict__ src, V* __restrict__ dst, u32 vpr, u64 item_v) {
+    blur_rows<V>(hdr, nbr_axis, src + blockIdx.y * item_v, dst + blockIdx.y * item_v, vpr, blockIdx.x, gridDim.x, gridDim.y);
 }
 
 // Two passes in one launch, along axes a and then b: a thread mixes the row that pass b needs of its vertex and of that one's
@@ -183,8 +184,8 @@ __device__ __forceinline__ void blur_pair_rows(const Header* hdr, const int* __r
 template <typename V>
 __global__ void __launch_bounds__(256, PAIR_CTAS)
 blur_pair(const Header* hdr, const int* __restrict__ nbr_a, const int* __restrict__ nbr_b, const V* __restrict__ src,
-          V* __restrict__ dst, u32 vpr) {
-    blur_pair_rows<V>(hdr, nbr_a, nbr_b, src, dst, vpr, blockIdx.x, gridDim.x);
+          V* __restrict__ dst, u32 vpr, u64 item_v) {
+    blur_pair_rows<V>(hdr, nbr_a, nbr_b, src + blockIdx.y * item_v, dst + blockIdx.y * item_v, vpr, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -35,6 +35,7 @@ struct Geom {
     int from_positions;     // 1: features are read from a positions array
     int lattice_items;      // items that one lattice serves (see one_for_all): records and vertices are those of item 0
     u32 item_entries;       // then: entries from one item's to the next's
+    u32 row_step;           // value rows from a vertex's to the next's: the items where theirs lie together (see ItemRows), else 1
     u32 bound;              // then: the call's max_entries (the lattice's own is a share of it)
     float scale[MAX_PD];    // host-computed scale factors (double arithmetic rounded to float)
     // T = double calls: the same three in double
@@ -56,7 +57,8 @@ struct Header {   // first 256 bytes of the workspace
     u32 calm_entries;  // of the Geom that the lattice was built with
     u32 items;         // items that the lattice serves: entries and vertices are those of one of them
     u32 mostly_new;    // in calls with a sketch: 30 % of the entries or more are vertices, in a table that stays in L2 (see insert_keys)
-    u32 pad[51];
+    u32 row_step;      // of the Geom that the lattice was built with
+    u32 pad[50];
 };
 
 // Sketch of the lattice's size, behind the header (zeroed with it): a bitmap in which build_tiles sets one bit

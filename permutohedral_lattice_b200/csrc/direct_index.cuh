@@ -96,7 +96,7 @@ link_neighbours_direct(Header* hdr, Direct d, const u32* __restrict__ table, con
     if (hdr->status != 0) return;
     resolve_entries(hdr, owners, list_ref, vid, rows);
     const u32 M = hdr->num_vertices;
-    zero_rows_of(rows, M, grid_thread(), grid_threads());
+    zero_rows_of(rows, M, (u32)grid_thread(), (u32)grid_threads());
     const u64 items = (u64)M * (PD + 1);
     for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < items; e += (u64)gridDim.x * blockDim.x) {
         const u32 v = (u32)(e / (PD + 1));

@@ -58,7 +58,7 @@ export_points(Geom g, const Header* hdr, const int2* __restrict__ tile_info, con
     for (int r = 0; r <= PD; r++) {
         if (pixel_vertex) {
             const u32 row = list_ref[base + rec_tile[r * TP + tid]];
-            pixel_vertex[o + r] = (int32_t)(items > 1 ? first + row / items : row);
+            pixel_vertex[o + r] = (int32_t)(items > 1 ? first + row / hdr->row_step : row);
         }
         if (pixel_weight) pixel_weight[o + r] = recw_tile[r * TP + tid];
     }

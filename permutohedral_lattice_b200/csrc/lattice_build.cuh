@@ -454,6 +454,7 @@ build_tiles(Geom g, const R* __restrict__ positions, const R* __restrict__ refer
         hdr->sorted = SORTED ? 1u : 0u;
         hdr->calm_entries = (u32)g.calm_entries;
         hdr->items = (u32)g.lattice_items;
+        hdr->row_step = g.row_step;
     }
     if (tid == 0) {
         u32 base = atomicAdd(&hdr->num_entries, (u32)cnt);
@@ -652,32 +653,59 @@ clear_table(Header* hdr, u64* __restrict__ table, u32 max_log2, int sketch_shift
 // ---------------------------------------------------------------------------------------------
 // insert_entries
 // ---------------------------------------------------------------------------------------------
-// The items that the lattice serves (1, or see one_for_all), and their value rows, to be zeroed.  A vertex's rows lie together, item by
-// item: to the blur, the conversion of the fixed-point sums and the zeroing they are one long row.  With an item's rows together, each
-// of these had to walk the items one after another, in threads or blocks that have next to nothing to do for one: us a call without
-// a guide, 3 channels, so / now, 64x64x64 39 / 27, 1024x8x8 136 / 24.5, 16384x8x8 1927 / 67, 65535x4x4 15180 / 181, 8x256x256 36 / 38.
+// The items that the lattice serves (1, or see one_for_all), and their value rows, to be zeroed: a vertex's together, item by item, so that
+// to the blur, the conversion of the fixed-point sums and the zeroing they are one long row, or an item's together, in large lattices (see
+// rows_together).
 struct ItemRows {
-    u32 items, stride;   // entries from one item's to the next's
-    uint4* rows;         // float rows, rows of doubles, or the 64-bit sums of the deterministic mode; null: none
-    u32 row_quads;       // 16 bytes each, of a vertex, all items
+    u32 items, stride;         // entries from one item's to the next's
+    u32 row_step, item_step;   // rows from a vertex's to the next's, and from an item's to the next's
+    uint4* rows;               // float rows, rows of doubles, or the 64-bit sums of the deterministic mode; null: none
+    u32 row_quads;             // 16 bytes each
 };
-__device__ __forceinline__ void zero_rows_of(const ItemRows& z, u32 M, u64 thread, u64 threads) {
+__device__ __forceinline__ void zero_rows_of(const ItemRows& z, u32 M, u32 thread, u32 threads) {
     if (!z.rows) return;
-    const u64 quads = (u64)M * z.row_quads;
-    for (u64 i = thread; i < quads; i += threads) z.rows[i] = make_uint4(0u, 0u, 0u, 0u);
+    const u64 quads = (u64)M * z.row_step * z.row_quads;
+    if (z.item_step <= 1) {
+        for (u64 i = thread; i < quads; i += threads) z.rows[i] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
+    // quads of every item, one stretch after another
+    if (quads == 0) return;
+    const u32 fit = quads <= threads ? (u32)quads : 0u;   // (else a step stays within two items)
+    const u32 items_on = fit ? threads / fit : 0u, on = threads - items_on * fit;
+    u32 b = fit ? thread / fit : 0u;
+    u64 i = thread - b * fit;
+    while (b < z.items) {
+        z.rows[(u64)b * z.item_step * z.row_quads + i] = make_uint4(0u, 0u, 0u, 0u);
+        b += items_on;
+        i += on;
+        if (i >= quads) {
+            i -= quads;
+            b++;
+        }
+    }
 }
-// Calls store(t, b) for the T entries of every item b, spread over all threads.  (Their number fits 31 bits, as the bound does.)
-template <typename Store>
-__device__ __forceinline__ void for_entries_of(const ItemRows& z, u32 T, u32 thread, u32 threads, Store store) {
+// Calls store(t, b, vertex) for the T entries of every item b, where find(t) is an entry's vertex.  A thread goes through the items of its
+// entry, which it looks up once, while an eighth of the threads have one; fewer entries are spread over all threads (16x300x300, 200 k
+// entries of 303 k threads, 137 / 142 us a call).  (Their number in all items fits 31 bits, as the bound does.)
+template <typename Find, typename Store>
+__device__ __forceinline__ void for_entries_of(const ItemRows& z, u32 T, u32 thread, u32 threads, Find find, Store store) {
+    if (z.items == 1 || T >= threads / 8) {
+        for (u32 t = thread; t < T; t += threads) {
+            const u32 v = find(t);
+            for (u32 b = 0; b < z.items; b++) store(t, b, v);
+        }
+        return;
+    }
     const u32 all = T * z.items;
     for (u32 i = thread; i < all; i += threads) {
-        const u32 b = z.items > 1 ? i / T : 0u;
-        store(i - b * T, b);
+        const u32 b = i / T, t = i - b * T;
+        store(t, b, find(t));
     }
 }
 // Entry t of item b has vertex v: the row that is its, in that item's copy of the list.
 __device__ __forceinline__ void store_vertex_of(const ItemRows& z, u32* list_ref, u32 t, u32 b, u32 v) {
-    list_ref[b * z.stride + t] = v * z.items + b;
+    list_ref[b * z.stride + t] = v * z.row_step + b * z.item_step;
 }
 
 // What the insert launch sets up for every vertex it creates, so that no later launch has to: the
@@ -938,10 +966,13 @@ insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cf
 // where the lattice serves one item.
 __device__ __forceinline__ void resolve_entries(const Header* hdr, const u32* owners, u32* list_ref,
                                                 const u32* __restrict__ vid, const ItemRows& rows) {
-    for_entries_of(rows, hdr->num_entries, (u32)grid_thread(), (u32)grid_threads(), [&](u32 t, u32 b) {
-        const u32 ref = owners[t];
-        store_vertex_of(rows, list_ref, t, b, (ref & VERTEX_FLAG) ? (ref & ~VERTEX_FLAG) : vid[ref]);
-    });
+    for_entries_of(
+        rows, hdr->num_entries, (u32)grid_thread(), (u32)grid_threads(),
+        [&](u32 t) {
+            const u32 ref = owners[t];
+            return (ref & VERTEX_FLAG) ? (ref & ~VERTEX_FLAG) : vid[ref];
+        },
+        [&](u32 t, u32 b, u32 v) { store_vertex_of(rows, list_ref, t, b, v); });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1044,7 +1075,7 @@ link_neighbours(Header* hdr, u64* __restrict__ table, u32 max_log2, const u32* o
     resolve_entries(hdr, owners, list_ref, vid, rows);
     const u32 M = hdr->num_vertices;
     const u64 mask = (1ull << hdr->table_log2) - 1;
-    zero_rows_of(rows, M, grid_thread(), grid_threads());   // under the latency of the lookups below
+    zero_rows_of(rows, M, (u32)grid_thread(), (u32)grid_threads());   // under the latency of the lookups below
     if constexpr (KEY_SLOTS) {
         LinkAxis<PD, KW, 0>::run((int)blockIdx.y, reinterpret_cast<const KeySlot*>(table), (u32)mask, vkeys, M, nbr, max_entries);
     } else {

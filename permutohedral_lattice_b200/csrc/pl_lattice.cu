@@ -235,6 +235,7 @@ static int make_geom(Geom& g, int batch, int n, int pd, int n_sdims, const int* 
     g.n = n;
     g.from_positions = from_positions ? 1 : 0;
     g.lattice_items = 1;
+    g.row_step = 1;
     g.n_sdims = n_sdims;
     g.R = R;
     g.spatial_std = spatial_std;
@@ -338,11 +339,26 @@ static bool make_direct(Direct& d, const Geom& g, int pd, const Layout& L) {
     return direct_bounds(d, pd, g.sdims, g.spatial_std, g.scale, g.batch, L.index_words);
 }
 
+// Where one lattice serves several items: whether a vertex's rows lie together, or an item's.  With an item's, conversion and blur have a row of
+// blocks for every item, which have next to nothing to do in a small lattice, and ask for a vertex's neighbours once an item; with a
+// vertex's, rows of one float4 share their lines with other items' and not with those of the tile's other vertices, and of large lattices
+// more lines come from DRAM.  So by the bounds, of an item's entries and, for longer rows, of all rows.  us a call without a guide, an item's
+// / a vertex's together: 65535x4x4 x 3 15180 / 181, 1024x8x8 x 3 136 / 24.5, 64x64x64 x 3 39 / 27, 300x5000 x 1 81 / 46 (these with the zeroing
+// item by item too); bounds of 67 to 196 k entries an item, 8x512x512 x 1, theta 8, 65 / 58, theta 2 79 / 83, 1 128 / 139, 0.7 217 / 261, 16x300x300
+// x 3, theta 2, 65 / 67; 8x512x512 x 10, theta 2 164 / 162, 1 372 / 362, 0.7 667 / 745, x 21, theta 3, 173 / 168, 1 585 / 585, 0.7 1291 / 1415,
+// 2x1000x1000 x 21, theta 1, 606 / 620, 64x100x120 x 21, theta 1, 247 / 198, 3x100x100x100 x 10, theta 1, 940 / 803.
+constexpr u64 TOGETHER_ENTRIES = 16384;
+constexpr u64 TOGETHER_BYTES = 256u << 20;
+static bool rows_together(const Layout& whole, const Layout& share, int vd) {
+    const u64 row_bytes = sizeof(float) * (u64)padded_vd(vd);
+    return share.max_entries <= TOGETHER_ENTRIES || (row_bytes > 16 && whole.max_entries * row_bytes <= TOGETHER_BYTES);
+}
+
 // The features of a spatial-only call are those of its grid, the same in every item: one lattice does for all, with its share of the
 // bound, and value rows for every item.  The lattice's own geometry and layout, of one item; false: the call builds a lattice of all
 // its items.  A share fits where the whole would have: entries are the same in every item.  us a call, forward + backward, an own
 // lattice each / one: 8 x 512x512 x 21 414 / 334, 16 x 512x512 x 1 399 / 217; forward, 1024x8x8 x 3 28.5 / 24.5, 65535x4x4 x 3 424 / 181.
-static bool one_for_all(const Geom& g, const Layout& L, int pd, Geom& one, Layout& share) {
+static bool one_for_all(const Geom& g, const Layout& L, int pd, int vd, Geom& one, Layout& share) {
     one = g;
     share = L;
     if (g.from_positions || g.R != 0 || pd != g.n_sdims || g.batch < 2 || L.max_entries < (u64)g.batch) return false;
@@ -351,6 +367,7 @@ static bool one_for_all(const Geom& g, const Layout& L, int pd, Geom& one, Layou
     one.lattice_items = g.batch;
     one.item_entries = (u32)share.max_entries;
     one.bound = (u32)L.max_entries;
+    one.row_step = rows_together(L, share, vd) ? (u32)g.batch : 1u;
     one.batch = 1;
     one.num_tiles = one.tiles_per_item;
     one.grid3 = (one.tiles_y <= 65535 && one.outer <= 65535) ? 1 : 0;
@@ -658,7 +675,7 @@ static int run_filter(const Geom& call, float* output, const float* input, const
     // g, L: of the whole call; the lattice is that of `one`, within `share` of the bound (see one_for_all)
     Geom g = call, one;
     Layout share;
-    const bool together = phases == (PH_BUILD | PH_APPLY) && !better_each(call, PD, whole, (u32)padded_vd(vd) / 4) && one_for_all(call, whole, PD, one, share);
+    const bool together = phases == (PH_BUILD | PH_APPLY) && !better_each(call, PD, whole, (u32)padded_vd(vd) / 4) && one_for_all(call, whole, PD, vd, one, share);
     if (together) {
         g.lattice_items = one.lattice_items;
         g.item_entries = one.item_entries;
@@ -738,8 +755,10 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         ItemRows rows;
         rows.items = items;
         rows.stride = one.item_entries;
+        rows.row_step = one.row_step;
+        rows.item_step = one.row_step > 1 ? 1u : one.item_entries;
         rows.rows = (phases & PH_APPLY) ? (v64 ? reinterpret_cast<uint4*>(v64) : reinterpret_cast<uint4*>(v0)) : nullptr;
-        rows.row_quads = (u32)padded_vd(vd) / (v64 ? 2u : 4u) * items;
+        rows.row_quads = (u32)padded_vd(vd) / (v64 ? 2u : 4u);
         // what the insert says of an entry and the link resolves: in a list that is not the items', whose entries come from it, all of them
         u32* owners = together ? vid + share.max_entries : list_ref;
         if constexpr (PD <= MAX_SDIMS) {
@@ -784,7 +803,10 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         PL_CUDA(cudaGetLastError());
         return PL_OK;
     }
-    const u32 qpr = (u32)padded_vd(vd) / 4 * items;   // float4 of a vertex, in the rows of all items
+    // the blur passes (and the conversion of the fixed-point sums): on the rows of a vertex, or with a row of blocks for every item
+    const u32 quads = (u32)padded_vd(vd) / 4, qpr = quads * one.row_step, apart = one.row_step > 1 ? 1u : items;
+    const u64 item_v = (u64)one.item_entries * quads;
+    auto blocks_of = [&](int blocks) { return dim3((unsigned)((blocks + (int)apart - 1) / (int)apart), apart); };
     int rc = PL_OK;
     if (v64) {
         if (vd > widest_vd_fixed(PD)) return PL_UNSUPPORTED_DIMS;
@@ -792,7 +814,7 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         rc = (phases & PH_BUILD) ? launch_splat_fixed<PD, false>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st)
                                  : launch_splat_fixed<PD, true>(g, input, hdr, tile_info, rec, rec_w, srec, list_ref, v64, vd, st);
         if (rc != PL_OK) return rc;
-        PL_LAUNCH_AFTER(true, (convert_fixed), wide, 256, 0, st, hdr, v64, v0, qpr * 4);
+        PL_LAUNCH_AFTER(true, (convert_fixed), blocks_of(wide), 256, 0, st, hdr, v64, v0, qpr * 4, item_v * 4);
         PL_COUNT_LAUNCHES(1);   // convert_fixed (the splat itself is counted below)
     } else {
         rc = PL_SPLAT_FOR(PD, vd, g, input, hdr, tile_info, rec, rec_w, srec, !(phases & PH_BUILD), list_ref, v0, vd, st);
@@ -802,22 +824,22 @@ static int run_filter(const Geom& call, float* output, const float* input, const
     if (ev) PL_CUDA(cudaEventRecord(ev[3], st));
     float* src = v0;
     float* dst = v1;
-    const bool one_blur = small_blur(one, PD, share, qpr) && (items == 1 || qpr <= SMALL_SHARED);
+    const bool one_blur = apart == 1 && small_blur(one, PD, share, qpr) && (items == 1 || qpr <= SMALL_SHARED);
     if (one_blur) {
         PL_TRY(launch_small_blur(hdr, nbr, share, reinterpret_cast<float4*>(v0), qpr, PD + 1, reverse, st));
         PL_COUNT_LAUNCHES(1);
-    } else if (blur_in_pairs(one, PD, share, qpr)) {
+    } else if (blur_in_pairs(one, PD, share, quads * items)) {
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * share.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * share.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<float4>), sms * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
+            PL_LAUNCH_AFTER(true, (blur_pair<float4>), blocks_of(sms * PAIR_CTAS), 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
             std::swap(src, dst);
             PL_COUNT_LAUNCHES(1);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * share.max_entries * 2;
-        PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr);
+        PL_LAUNCH_AFTER(true, (blur_axis<float4>), blocks_of(wide), 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
         float* tmp = src; src = dst; dst = tmp;
         PL_COUNT_LAUNCHES(1);
     }
@@ -877,7 +899,7 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     vinit.nbr = nbr;
     vinit.max_entries = L.max_entries;
     vinit.pd = PD;
-    const ItemRows rows = {1u, 0u, reinterpret_cast<uint4*>(v0), (u32)vp / 2};   // rows of vp doubles
+    const ItemRows rows = {1u, 0u, 1u, 0u, reinterpret_cast<uint4*>(v0), (u32)vp / 2};   // rows of vp doubles
     if constexpr (PD <= MAX_SDIMS) {
         if (use_direct) {
             if (!cleared) PL_LAUNCH_AFTER(true, (clear_direct), wide, 256, 0, st, hdr, table32, direct.slots);
@@ -908,12 +930,12 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
             std::swap(src, dst);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2);
+        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
         double* tmp = src; src = dst; dst = tmp;
     }
     PL_LAUNCH_AFTER(vd <= 4 || slice_overlap(g, one_blur), (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
@@ -1032,7 +1054,7 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     auto rest_of = [&](const LatticeRows& l, int step, int pd, const float*& v) -> int {   // from pass `step` on
         for (; step <= pd; step++) {
             const Pass p = pass_of(l, step);
-            PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads);
+            PL_LAUNCH_AFTER(true, (blur_axis<float4>), wide, 256, 0, st, l.hdr, p.nbr, p.src, p.dst, quads, (u64)0);
             launches++;
             v = reinterpret_cast<const float*>(p.dst);
         }

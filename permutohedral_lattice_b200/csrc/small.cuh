@@ -180,7 +180,8 @@ index_small(Header* hdr, const Key<KW>* __restrict__ list_keys, u32* __restrict_
         }
     }
     if constexpr (SHARED) {
-        for_entries_of(rows, T, me, all, [&](u32 t, u32 b) { store_vertex_of(rows, list_ref, t, b, table_s[slot_s[t]] >> 16); });
+        for_entries_of(rows, T, me, all, [&](u32 t) { return table_s[slot_s[t]] >> 16; },
+                       [&](u32 t, u32 b, u32 v) { store_vertex_of(rows, list_ref, t, b, v); });
         zero_rows_of(rows, M, me, all);
     } else if (rows.rows) {   // (fewer than 2^32 pieces)
         for (u32 i = me; i < M * rows.row_quads; i += all) rows.rows[i] = make_uint4(0u, 0u, 0u, 0u);

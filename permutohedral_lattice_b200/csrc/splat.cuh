@@ -833,8 +833,10 @@ absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
 
 // fixed-point sums -> float rows
 __global__ void __launch_bounds__(256)
-convert_fixed(const Header* hdr, const long long* __restrict__ v64, float* __restrict__ v0, u32 vp) {
+convert_fixed(const Header* hdr, const long long* __restrict__ v64, float* __restrict__ v0, u32 vp, u64 item_cells) {
     after_previous_kernel();
+    v64 += blockIdx.y * item_cells;
+    v0 += blockIdx.y * item_cells;
     if (hdr->status != 0) return;
     const double inv = __longlong_as_double((long long)(1023 - fixed_exponent(hdr)) << 52);
     const u64 cells = (u64)hdr->num_vertices * vp;

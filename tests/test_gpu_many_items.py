@@ -1,5 +1,5 @@
-"""Batches of many small grids without a guide: one lattice serves every item, and what is done for each of them (its value
-rows, its copy of the list of entries, its share of the blur) is spread over the whole GPU, not walked item by item."""
+"""Batches without a guide, of many small grids above all: one lattice serves every item, and what is done for each of them (its
+value rows, its copy of the list of entries, its share of the blur) is spread over the whole GPU, not walked item by item."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -15,6 +15,10 @@ pytestmark = pytest.mark.gpu
     (260, (4, 5, 6), 3, 1.0, True),      # volumes
     (2, (16, 16), 7, 2.0, False),
     (40, (16, 16), 35, 2.0, False),      # rows of nine float4, 360 of them a vertex
+    (40, (90, 100), 3, 30.0, False),     # an item's rows together, by the bound: fewer entries than threads
+    (3, (420, 500), 2, 0.4, False),      # more
+    (2, (420, 500), 1, 0.4, True),
+    (4, (512, 512), 21, 0.7, False),     # beyond 256 MB of rows
 ])
 def test_every_item_as_if_alone(batch, shape, c, theta, hashed):
     import torch
