@@ -67,7 +67,6 @@ struct Header {   // first 256 bytes of the workspace
 // there are up to 40 times as many.  The shift keeps the bitmap at most about half full in the worst case.
 constexpr int SKETCH_LOG2 = 16;
 constexpr int SKETCH_WORDS = (1 << SKETCH_LOG2) / 32;
-constexpr u64 SKETCH_MIN_ENTRIES = 1ull << 18;   // below, a table sized by entries is small anyway
 
 // Filter in front of a large hash table: 2^FILTER_BITS_LOG2 bits a slot, one set for every vertex (by its key's hash).
 // Most neighbour lookups of a sparse lattice find nothing; a table that does not stay in L2 costs each of them an

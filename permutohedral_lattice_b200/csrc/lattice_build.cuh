@@ -21,7 +21,6 @@ struct ClearTable {
 };
 constexpr u32 CLEAR_QUADS = 1u << 20;         // 16 MB, at most; 8 MB where the build waits for it at its start (pd 16)
 constexpr u32 CLEAR_QUADS_ALONE = 1u << 19;
-static_assert(2 * SKETCH_MIN_ENTRIES <= CLEAR_QUADS_ALONE, "the largest table of a call that is too small for a sketch, slots of 16 bytes");
 __global__ void __launch_bounds__(256) clear_header(Header* hdr, u32 quads, ClearTable clear) {
     after_previous_kernel();
     if (blockIdx.x == 0)

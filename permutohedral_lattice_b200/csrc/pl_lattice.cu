@@ -190,9 +190,9 @@ static cudaError_t launch_kernel(bool overlap, void (*kernel)(Params...), dim3 g
 // The header and the sketch behind it.
 constexpr size_t HEADER_BYTES = sizeof(Header) + sizeof(u32) * SKETCH_WORDS;
 
-// Sampling of the sketch (see SKETCH_LOG2): so that a lattice of max_entries vertices sets about half its bits.
+// Sampling of the sketch (see SKETCH_LOG2): so that a lattice of max_entries vertices sets about half its bits.  A call keeps one when its table is
+// cleared by a launch of its own, which sizes it by the sketch (see ClearTable: bounds of more than 2^19 entries).
 static int sketch_shift_of(u64 max_entries) {
-    if (max_entries < SKETCH_MIN_ENTRIES) return -1;
     int shift = 0;
     while (shift < 20 && (max_entries >> shift) > (1ull << (SKETCH_LOG2 - 1))) shift++;
     return shift;
