@@ -215,22 +215,25 @@ __device__ __forceinline__ void store_relaxed(u32* p, u32 v) {
 
 // What a launch reads or writes once, and whose next reader comes after more than the caches hold, goes first when they need room, so that
 // what is read again and again, value rows, keys and tables, stays: the point records (the construction's stores, the loads of splat and
-// slice), the neighbours of a blur pass, the entries' keys and references beyond pd 5.  us a call, without / with: 800x1200 x 3 170 / 166.5,
-// 1024x1024 grey by RGB, forward + backward, 299.5 / 294, two volumes of 111x128x120 498.5 / 489, five CRF steps on 375x500 x 21 407 / 397,
-// 4 x 321x481 x 10 with one lattice 232.5 / 228, 1 M points with 16 features 1589 / 1566.
+// slice), the neighbours of a blur pass, the entries' keys and references beyond pd 5, new slots of the neighbour table.  us a call, plain / so:
+// the records, 800x1200 x 3 167.3 / 165.2, 1024x1024 grey by RGB, forward + backward, 292 / 286, two volumes of 111x128x120 505 / 488, 8 x 512x512 x 3
+// 242 / 237; the neighbours 167.3 / 165.2, 291 / 286, five CRF steps on 375x500 x 21 381 / 374.5, 200 k points x 7 at pd 16 341 / 328 (beyond
+// what stays in L2 see MOVED_ITEMS); the rest 164 / 165.2, 8 x 512x512 x 3 of noise 0.16 771 / 760, 1 M points with 16 features 1630 / 1613.
 template <typename T>
 __device__ __forceinline__ T load_once(const T* p) { return __ldcs(p); }
 template <typename T>
 __device__ __forceinline__ void store_once(T* p, T v) { __stcs(p, v); }
-// A point's record.  Not up to pd 2: calls by position alone, whose items share one lattice's records (see one_for_all); 8 x 512x512 x
-// 21 342 / 348.  Not beyond pd 5, where the compiler takes up to 16 registers more for it.
+// A point's record.  Not up to pd 2, most calls of which are by position alone, where the items of a batch share one lattice's records (see
+// one_for_all): 8 x 512x512 x 21 342 / 348.  Three to five dimensions may be positions alone too: 8 volumes of 64x64x64 x 21 181 / 185, but
+// x 1 to 3 and four dimensions within 0.4 % of one another, and a choice at every load costs all calls 3 to 17 %.  Not beyond pd 5, where
+// the compiler takes up to 16 registers more for it.
 template <int PD, typename T>
 __device__ __forceinline__ T load_record(const T* p) {
     if constexpr (PD > 2 && PD <= 5) return __ldcs(p);
     else return *p;
 }
 
-// Key read straight from L2 (no L1): for data that another CTA of the SAME launch may have written.
+// load_once of a key: not for keys that this launch writes.
 template <int KW>
 __device__ __forceinline__ Key<KW> load_key_once(const Key<KW>* p) {
     Key<KW> k;
@@ -239,6 +242,7 @@ __device__ __forceinline__ Key<KW> load_key_once(const Key<KW>* p) {
     for (int j = 0; j < KW; j++) k.w[j] = load_once(w + j);
     return k;
 }
+// Key read straight from L2 (no L1): for data that another CTA of the SAME launch may have written.
 template <int KW>
 __device__ __forceinline__ Key<KW> load_key_l2(const Key<KW>* p) {
     Key<KW> k;
@@ -545,12 +549,17 @@ __device__ __forceinline__ void fence_async_proxy() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// First statement of every kernel of a filter call.  A kernel launched with programmatic stream serialisation
-// may become resident while the kernel before it in the stream is still draining: the first instruction waits
-// until that kernel has finished and its writes are visible, the second lets the kernel AFTER this one become
-// resident in its turn (its CTAs are scheduled once every CTA of this grid has got here).  Every kernel waits
-// before it reads anything, so "the kernel before has finished" implies that all earlier ones have.  The release
-// comes after the wait on purpose: released first, a waiting kernel lets the one after it wait beside it, and
+// A kernel launched with programmatic stream serialisation may become resident while the kernel before it in the
+// stream is still draining: the first instruction waits until that kernel has finished and its writes are visible,
+// the second lets the kernel AFTER this one become resident in its turn (its CTAs are scheduled once every CTA of
+// this grid has got here).  First statement of most kernels; some wait later (the tile kernels, the blur passes, absmax_kernel) and until
+// then read only what is older than the kernel before them (build_tiles also writes records, which no kernel of an earlier call still reads:
+// clear_header is launched plainly), which holds since:
+//   - no thread that releases has not waited, absmax_kernel aside, so that a kernel finds all finished but the one before it;
+//   - absmax_kernel reads the call's input alone before it waits, and every CTA of it waits before it ends, so that it is finished after the
+//     kernel before it.  That one is clear_header, launched plainly, or zero_rows, the first of an apply and overlapped with whoever wrote the
+//     input: either has waited when absmax_kernel starts.
+// The release comes after the wait on purpose: released first, a waiting kernel lets the one after it wait beside it, and
 // two kernels' worth of waiting CTAs on the SMs slowed a long-running tile kernel by a quarter (pd = 16).
 // Both instructions do nothing in a plain launch.
 __device__ __forceinline__ void after_previous_kernel() {

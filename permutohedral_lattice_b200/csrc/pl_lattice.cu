@@ -177,7 +177,8 @@ static cudaError_t launch_kernel(bool overlap, void (*kernel)(Params...), dim3 g
 }
 #define PL_LAUNCH(kernel, grid, block, smem, st, ...) \
     PL_CUDA(launch_kernel(false, kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
-// A launch that may overlap the tail of the kernel before it: all but the first of a call and those whose callers say why not.
+// A launch that may overlap the tail of the kernel before it: all but clear_header, which starts a call, and those whose callers say why not (an apply
+// and a CRF step start with a kernel that overlaps whatever came before the call).
 // What each gave when it was measured by itself, all others as they are now, us a call or step, plain / overlapped: the blur passes after one
 // another, 16 and 2 items of 512x512 x 21, 2023 / 2007 and 353 / 342; the slice after the last pass and the splat after the link 2002 and 335;
 // clear_table after the build 1993 and 331; the insert after clear_table 1992 and 328.  The link after the insert and the first

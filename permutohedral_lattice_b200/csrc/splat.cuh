@@ -790,7 +790,7 @@ splat_tiles_rows(Geom g, const float* __restrict__ input, Header* hdr, const int
 // splat.  Behind the link launch, where it stood alone, 2 x 512x512 x 21, forward + backward, took 414.6 us, so 408.2.
 __global__ void __launch_bounds__(256)
 absmax_kernel(const float* __restrict__ input, u64 count, Header* hdr) {
-    let_next_kernel_start();   // (the input is older than the kernel before this)
+    let_next_kernel_start();   // (the input is older than the kernel before this, which has waited: see after_previous_kernel)
     u32 m = 0;
     auto take = [&](float x) { m = max(m, __float_as_uint(fabsf(x))); };
     const u64 lead = min(count, (u64)(((16u - ((u32)(uintptr_t)input & 15u)) & 15u) >> 2));
@@ -844,7 +844,8 @@ convert_fixed(const Header* hdr, const long long* __restrict__ v64, float* __res
         v0[i] = (float)PL_DMUL(__ll2double_rn(v64[i]), inv);
 }
 
-// Start of an apply on an already built lattice: value rows (or fixed-point sums) back to zero.
+// Start of an apply on an already built lattice: value rows (or fixed-point sums) back to zero.  It overlaps the kernel before the call, and the
+// kernels after it (absmax_kernel, the splat's staging) read the caller's input before they wait: it must not release them before it has waited.
 __global__ void __launch_bounds__(256)
 zero_rows(Header* hdr, float* __restrict__ v0, long long* __restrict__ v64, int vp) {
     after_previous_kernel();
