@@ -56,7 +56,8 @@ __device__ __forceinline__ bool all_finite(float2 z) { return PL_FADD(z.x, z.y) 
 // of a noisy lattice (20 M pieces) 3768 / 3841 us a call.
 constexpr u64 MOVED_ITEMS = 5000000;
 // Nor do lines of neighbours that are loaded evict-first stay until the next block wants its part of them, so that beyond it the loop loads them
-// plainly: us a call, evict-first / plain, 8 x 512x512 x 21 of a noisy guide, 3.5 M vertices 2577 / 2453, 60 k points x 21 at pd 16, 1 M vertices 1056 / 1011.
+// plainly: us a call, evict-first / plain, 8 x 512x512 x 21 of a noisy guide, 3.5 M vertices 2577 / 2453, 60 k points x 21 at pd 16, 1 M vertices
+// 1056 / 1011.
 // Below, evict-first leaves L2 to the rows: 800x1200 x 3 163 / 165, five CRF steps on 375x500 x 21 371 / 378, 200 k points x 7 at pd 16 328 / 341.
 // (Two loops: chosen in the loop, it cost up to 4 %.)
 

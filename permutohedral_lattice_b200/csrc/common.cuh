@@ -216,7 +216,8 @@ __device__ __forceinline__ void store_relaxed(u32* p, u32 v) {
 // What a launch reads or writes once, and whose next reader comes after more than the caches hold, goes first when they need room, so that
 // what is read again and again, value rows, keys and tables, stays: the point records (the construction's stores, the loads of splat and
 // slice), the neighbours of a blur pass, the entries' keys and references beyond pd 5, new slots of the neighbour table.  us a call, plain / so:
-// the records, 800x1200 x 3 167.3 / 165.2, 1024x1024 grey by RGB, forward + backward, 292 / 286, two volumes of 111x128x120 505 / 488, 8 x 512x512 x 3
+// the records, 800x1200 x 3 167.3 / 165.2, 1024x1024 grey by RGB, forward + backward, 292 / 286, two volumes of 111x128x120 505 / 488, 8 x 512x512
+// x 3
 // 242 / 237; the neighbours 167.3 / 165.2, 291 / 286, five CRF steps on 375x500 x 21 381 / 374.5, 200 k points x 7 at pd 16 341 / 328 (beyond
 // what stays in L2 see MOVED_ITEMS); the rest 164 / 165.2, 8 x 512x512 x 3 of noise 0.16 771 / 760, 1 M points with 16 features 1630 / 1613.
 template <typename T>

@@ -193,7 +193,8 @@ __global__ void __launch_bounds__(256, 8)
 crf_blur(const Header* hdr_a, const int* nbr_a, const float4* src_a, float4* dst_a, const Header* hdr_s, const int* nbr_s,
          const float4* src_s, float4* dst_s, u32 quads) {
     const bool second = blockIdx.y != 0;
-    blur_rows<float4>(second ? hdr_s : hdr_a, second ? nbr_s : nbr_a, second ? src_s : src_a, second ? dst_s : dst_a, quads, blockIdx.x, gridDim.x, 1);
+    blur_rows<float4>(second ? hdr_s : hdr_a, second ? nbr_s : nbr_a, second ? src_s : src_a, second ? dst_s : dst_a, quads,
+            blockIdx.x, gridDim.x, 1);
 }
 
 // Both slices and the update of a Potts model (see crf_update, whose arithmetic this is).  A thread a point: the tile's rows

@@ -893,12 +893,15 @@ __device__ __forceinline__ u32 key_rest(const Key<Cfg<PD>::KW>& k) {
 // A compare-and-swap on a line that was just read takes longer than one on a line that was not: in a table of 32 MB a ns sees 175 loads of
 // random slots, 80 swaps, 50 times load, swap and store of an empty slot, 70 times swap and store.  So slots are claimed unseen where the sketch
 // says that MOSTLY_NEW of the entries or more are vertices and the table stays in L2 (up to 32 MB; beyond, the load brings the line in for the
-// swap).  us a call, a look first / not, by the share of vertices, below the line 14 %, 8 x 512x512 x 3 251 / 255, 19 % 225 / 226, 24 %, 4 x 512x512 x 3
-// 148 / 147, 30 %, 1024x1024 x 3 121 / 120, but 2 x 111x128x120 of a noisy guide, 20 to 30 %, 423 / 432; above it 1024x1024 x 3, 31 % 122 / 122, 34 % 162
+// swap).  us a call, a look first / not, by the share of vertices, below the line 14 %, 8 x 512x512 x 3 251 / 255, 19 % 225 / 226, 24 %, 4 x
+// 512x512 x 3
+// 148 / 147, 30 %, 1024x1024 x 3 121 / 120, but 2 x 111x128x120 of a noisy guide, 20 to 30 %, 423 / 432; above it 1024x1024 x 3, 31 % 122 / 122,
+// 34 % 162
 // / 159, 39 % 238 / 236, 800x1200 x 3, 52 % 155 / 152, 57 % 206 / 203.  Tables of 64 MB and more: 8 x 512x512 x 3, noise 0.16, 730 / 755, 0.25
 // 1166 / 1193, 800x1200 x 3, 73 %, 714 / 720.
 // In calls without a sketch a warp does as long as a third of what it claims is free, which the first of the entries mostly are, whatever
-// the lattice: 300x400 x 3, 29 % 36 / 36, 32 % 41.4 / 40.3, 35 % 44 / 42.6, 40 % 56 / 54.5, 46 % 80.7 / 80.9, 512x512 x 3, 51 % 55.7 / 54.7, 63 % 99.6 / 100.
+// the lattice: 300x400 x 3, 29 % 36 / 36, 32 % 41.4 / 40.3, 35 % 44 / 42.6, 40 % 56 / 54.5, 46 % 80.7 / 80.9, 512x512 x 3, 51 % 55.7 / 54.7, 63 %
+// 99.6 / 100.
 template <int PD>
 __global__ void __launch_bounds__(256, 8)   // as many as it is launched with
 insert_keys(Header* hdr, KeySlot* __restrict__ table, u32 max_log2, const Key<Cfg<PD>::KW>* __restrict__ list_keys,

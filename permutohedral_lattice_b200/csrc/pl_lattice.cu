@@ -177,14 +177,16 @@ static cudaError_t launch_kernel(bool overlap, void (*kernel)(Params...), dim3 g
 }
 #define PL_LAUNCH(kernel, grid, block, smem, st, ...) \
     PL_CUDA(launch_kernel(false, kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
-// A launch that may overlap the tail of the kernel before it: all but clear_header, which starts a call, and those whose callers say why not (an apply
+// A launch that may overlap the tail of the kernel before it: all but clear_header, which starts a call, and those whose callers say why not (an
+// apply
 // and a CRF step start with a kernel that overlaps whatever came before the call).
 // What each gave when it was measured by itself, all others as they are now, us a call or step, plain / overlapped: the blur passes after one
 // another, 16 and 2 items of 512x512 x 21, 2023 / 2007 and 353 / 342; the slice after the last pass and the splat after the link 2002 and 335;
 // clear_table after the build 1993 and 331; the insert after clear_table 1992 and 328.  The link after the insert and the first
 // blur pass after the splat, which gain only where the insert and the splat release them at their end (see
 // wait_for_previous_kernel): 800x1200 x 3 176.6 / 172.3, 1024x1024 grey by RGB, forward + backward, 306.9 / 299.4, five CRF steps on
-// 375x500 x 21 427 / 411 (and 408 with the index stage of the two kept lattices), two volumes of 111x128x120 509 / 502, 8 x 512x512 x 21 without a guide 424 / 415, 16 x 512x512 x 21 1764 / 1764.
+// 375x500 x 21 427 / 411 (and 408 with the index stage of the two kept lattices), two volumes of 111x128x120 509 / 502, 8 x 512x512 x 21 without a
+// guide 424 / 415, 16 x 512x512 x 21 1764 / 1764.
 #define PL_LAUNCH_AFTER(overlap, kernel, grid, block, smem, st, ...) \
     PL_CUDA(launch_kernel((overlap), kernel, dim3(grid), dim3(block), smem, st, __VA_ARGS__))
 
@@ -489,7 +491,8 @@ static int launch_splat_as(const Geom& g, const float* input, Header* hdr, const
         // five CTAs per SM need nearly all of the SM's shared memory: ask for the largest carve-out
         PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, VD, PRE, FloatSum, float>>(smem, true)));
         const bool bulk = bulk_staging_ok(g, input, vd);
-        PL_LAUNCH_AFTER(true, (splat_tiles_rows<PD, VD, PRE, FloatSum, float>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+        PL_LAUNCH_AFTER(true, (splat_tiles_rows<PD, VD, PRE, FloatSum, float>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr,
+                tile_info, rec, rec_w,
                                                                               srec, list_ref, v0, vd, bulk ? 1 : 0);
     }
     return PL_OK;
@@ -503,7 +506,8 @@ static int launch_splat_fixed(const Geom& g, const float* input, Header* hdr, co
     const size_t smem = SplatRows<PD, 0, PRE>::bytes(vd);
     PL_TRY((ensure_dynamic_smem<splat_tiles_rows<PD, 0, PRE, FixedSum, long long>>(smem, true)));
     const bool bulk = bulk_staging_ok(g, input, vd);
-    PL_LAUNCH_AFTER(true, (splat_tiles_rows<PD, 0, PRE, FixedSum, long long>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr, tile_info, rec, rec_w,
+    PL_LAUNCH_AFTER(true, (splat_tiles_rows<PD, 0, PRE, FixedSum, long long>), tile_grid(g), Cfg<PD>::TP, smem, st, g, input, hdr,
+            tile_info, rec, rec_w,
                                                                           srec, list_ref, v64, vd, bulk ? 1 : 0);
     return PL_OK;
 }
@@ -620,7 +624,8 @@ static int launch_small_index_as(Header* hdr, const Layout& L, const Key<KW>* li
     const u64 of_items = SHARED ? ((u64)entries * rows.items + SMALL_THREADS - 1) / SMALL_THREADS : 0;
     const u32 ctas = std::max(std::max(8u, std::min(64u, (entries * (PD + 1) + SMALL_THREADS - 1) / SMALL_THREADS)),
                               (u32)std::min(of_items, (u64)num_sms()));
-    PL_LAUNCH_AFTER(true, (index_small<PD, KW, SHARED>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, rows, (u32)smem, watch);
+    PL_LAUNCH_AFTER(true, (index_small<PD, KW, SHARED>), ctas, SMALL_THREADS, smem, st, hdr, list_keys, list_ref, vkeys, vinit, rows,
+            (u32)smem, watch);
     return PL_OK;
 }
 template <int PD, int KW>
@@ -676,7 +681,8 @@ static int run_filter(const Geom& call, float* output, const float* input, const
     // g, L: of the whole call; the lattice is that of `one`, within `share` of the bound (see one_for_all)
     Geom g = call, one;
     Layout share;
-    const bool together = phases == (PH_BUILD | PH_APPLY) && !better_each(call, PD, whole, (u32)padded_vd(vd) / 4) && one_for_all(call, whole, PD, vd, one, share);
+    const bool together = phases == (PH_BUILD | PH_APPLY) && !better_each(call, PD, whole, (u32)padded_vd(vd) / 4) && one_for_all(call,
+            whole, PD, vd, one, share);
     if (together) {
         g.lattice_items = one.lattice_items;
         g.item_entries = one.item_entries;
@@ -739,8 +745,10 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         constexpr bool beside_clear = !Cfg<PD>::COMPACT;
         // a lattice built to be applied later (no values in this call) also gets its splats sorted
         if (phases & PH_APPLY) {
-            PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, false, KW>), tile_grid(one), TP, Cfg<PD>::build_smem(false), st, one, positions, reference, hdr,
-                                                                         tile_info, rec, rec_w, srec, list_keys, (u32)share.max_entries, sketch_shift);
+            PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, false, KW>), tile_grid(one), TP, Cfg<PD>::build_smem(false), st, one,
+                    positions, reference, hdr,
+                                                                         tile_info, rec, rec_w, srec, list_keys,
+                                                                                 (u32)share.max_entries, sketch_shift);
         } else {
             PL_TRY((ensure_dynamic_smem<build_tiles<PD, float, true, KW>>(Cfg<PD>::build_smem(true))));
             PL_LAUNCH_AFTER(beside_clear, (build_tiles<PD, float, true, KW>), tile_grid(g), TP, Cfg<PD>::build_smem(true), st, g, positions, reference, hdr,
@@ -779,10 +787,13 @@ static int run_filter(const Geom& call, float* output, const float* input, const
                 constexpr bool KEYS = decltype(keys_in_slots)::value;
                 if (!cleared) PL_LAUNCH_AFTER(true, (clear_table<KEYS>), wide, 256, 0, st, hdr, table, (u32)table_log2, sketch_shift);
                 if constexpr (KEYS)
-                    PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, owners, vid, vkeys, vinit, cleared);
+                    PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table),
+                            (u32)table_log2, list_keys, owners, vid, vkeys, vinit, cleared);
                 else
-                    PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, owners, vid, vkeys, vinit, cleared);
-                PL_LAUNCH_AFTER(true, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, share.max_entries), 256, 0, st, hdr, table, (u32)table_log2, owners, list_ref, vid, vkeys, nbr,
+                    PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys,
+                            owners, vid, vkeys, vinit, cleared);
+                PL_LAUNCH_AFTER(true, (link_neighbours<PD, KEYS, KW>), link_grid<PD>(wide, share.max_entries), 256, 0, st, hdr, table,
+                        (u32)table_log2, owners, list_ref, vid, vkeys, nbr,
                                                           share.max_entries, rows, watch);
                 return PL_OK;
             };
@@ -833,14 +844,16 @@ static int run_filter(const Geom& call, float* output, const float* input, const
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * share.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * share.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<float4>), blocks_of(sms * PAIR_CTAS), 256, 0, st, hdr, nb, then, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
+            PL_LAUNCH_AFTER(true, (blur_pair<float4>), blocks_of(sms * PAIR_CTAS), 256, 0, st, hdr, nb, then,
+                    reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
             std::swap(src, dst);
             PL_COUNT_LAUNCHES(1);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
         const int* nb = nbr + (size_t)axis * share.max_entries * 2;
-        PL_LAUNCH_AFTER(true, (blur_axis<float4>), blocks_of(wide), 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), qpr, item_v);
+        PL_LAUNCH_AFTER(true, (blur_axis<float4>), blocks_of(wide), 256, 0, st, hdr, nb, reinterpret_cast<const float4*>(src),
+                reinterpret_cast<float4*>(dst), qpr, item_v);
         float* tmp = src; src = dst; dst = tmp;
         PL_COUNT_LAUNCHES(1);
     }
@@ -894,7 +907,8 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
     const bool small_table = L.index_words <= (1ull << 24);   // (as for float)
     const bool before_insert = cleared || small_table;
 
-    PL_LAUNCH_AFTER(!Cfg<PD>::COMPACT, (build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions, reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
+    PL_LAUNCH_AFTER(!Cfg<PD>::COMPACT, (build_tiles<PD, double>), tile_grid(g), TP, Cfg<PD>::build_smem(false), st, g, positions,
+            reference, hdr, tile_info, rec, rec_w, static_cast<uint2*>(nullptr), list_keys, (u32)L.max_entries, sketch_shift);
     u32* table32 = reinterpret_cast<u32*>(table);
     VertexInit vinit;
     vinit.nbr = nbr;
@@ -917,7 +931,8 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
             PL_LAUNCH_AFTER(before_insert, (insert_keys<PD>), wide, 256, 0, st, hdr, reinterpret_cast<KeySlot*>(table), (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
         else
             PL_LAUNCH_AFTER(before_insert, (insert_entries<KW>), wide, 256, 0, st, hdr, table, (u32)table_log2, list_keys, list_ref, vid, vkeys, vinit, cleared);
-        PL_LAUNCH_AFTER(true, (link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table, (u32)table_log2, list_ref, list_ref, vid, vkeys, nbr, L.max_entries,
+        PL_LAUNCH_AFTER(true, (link_neighbours<PD, Cfg<PD>::KEY_SLOTS>), link_grid<PD>(wide, L.max_entries), 256, 0, st, hdr, table,
+                (u32)table_log2, list_ref, list_ref, vid, vkeys, nbr, L.max_entries,
                                                   rows, watch);
     }
     PL_LAUNCH_AFTER(true, (splat_tiles_f64<PD>), tile_grid(g), TP, splat_smem, st, g, input, hdr, tile_info, rec, rec_w,
@@ -931,15 +946,18 @@ static int run_filter_f64(const Geom& g, double* output, const double* input, co
         for (int step = 0; step <= PD; step += 2) {
             const int* nb = nbr + (size_t)(reverse ? PD - step : step) * L.max_entries * 2;
             const int* then = step == PD ? nullptr : nbr + (size_t)(reverse ? PD - step - 1 : step + 1) * L.max_entries * 2;
-            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
+            PL_LAUNCH_AFTER(true, (blur_pair<double2>), num_sms() * PAIR_CTAS, 256, 0, st, hdr, nb, then,
+                    reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
             std::swap(src, dst);
         }
     } else for (int step = 0; step <= PD; step++) {
         const int axis = reverse ? PD - step : step;
-        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2, reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
+        PL_LAUNCH_AFTER(true, (blur_axis<double2>), wide, 256, 0, st, hdr, nbr + (size_t)axis * L.max_entries * 2,
+                reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), (u32)vp / 2, (u64)0);
         double* tmp = src; src = dst; dst = tmp;
     }
-    PL_LAUNCH_AFTER(vd <= 4 || slice_overlap(g, one_blur), (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info, rec, rec_w, list_ref, src, vd, watch);
+    PL_LAUNCH_AFTER(vd <= 4 || slice_overlap(g, one_blur), (slice_tiles_f64<PD>), tile_grid(g), TP, 0, st, g, output, hdr, tile_info,
+            rec, rec_w, list_ref, src, vd, watch);
     PL_COUNT_LAUNCHES((small ? 2 : cleared ? 3 : 4) + 1 + (one_blur ? 1 : pairs ? PD / 2 + 1 : PD + 1) + 1);   // build and index; splat; blur; slice
     PL_CUDA(cudaGetLastError());
     return PL_OK;
@@ -1037,7 +1055,8 @@ static int run_crf_step(const Geom& g, float* q_out, const float* q, const float
     for (int pair = 0; pairs && pair <= std::max(PDA, PDS) / 2; pair++) {
         const bool pass_a = !small_a && 2 * pair <= PDA, pass_s = !small_s && 2 * pair <= PDS, both = pass_a && pass_s;
         if (!pass_a && !pass_s) continue;
-        PL_LAUNCH_AFTER(true, (crf_blur_pair<PDA, PDS>), dim3(num_sms() * PAIR_CTAS / (both ? 2 : 1), both ? 2 : 1), 256, 0, st, a, s, both ? 0 : pass_a ? 1 : 2, pair, quads);
+        PL_LAUNCH_AFTER(true, (crf_blur_pair<PDA, PDS>), dim3(num_sms() * PAIR_CTAS / (both ? 2 : 1), both ? 2 : 1), 256, 0, st, a, s,
+                both ? 0 : pass_a ? 1 : 2, pair, quads);
         launches++;
         if (pass_a) va = (pair & 1) ? a.v0 : a.v1;
         if (pass_s) vs = (pair & 1) ? s.v0 : s.v1;

@@ -151,9 +151,12 @@ __device__ __forceinline__ void flush_row(float* vrow, float* acc) {
 // without work, 87, so 83.  us a call, eight points / so: 16 x 512x512 x 1 without a guide 208 / 186, x 3 198 / 189; 96x128x128 x
 // 1 without a guide, forward + backward, 207 / 200.  (The figures below are those of eight points.)  At pd 4 the records of
 // one and two channels are loaded evict-first, which leaves L1 to the points' rows.  us a call, plain / so, volumes of 0.5 to 8 M points and
-// images of 1 to 4 M: one channel 64x80x96 64.7 / 64.8, two of them 86.1 / 86.8, two of 111x128x120 262.6 / 258.8 (theta 10: 255 / 247), 200x200x200 552 / 550, images 105.3
-// / 105.4 to 308 / 308; two channels 54.6 / 54.7, 87 / 87, 263 / 260 (253 / 247), 555 / 555.5, images 94.4 / 94.6 to 315.2 / 315.5.  Not with three, 56 / 56.5, 88.6 /
-// 89.7, 268 / 269 (259 / 257), 568 / 577, images 96 / 97 to 324 / 326, nor at pd 3: 8 volumes of 64x64x64 without a guide 75 / 74, 83 / 84 and 83 / 83.
+// images of 1 to 4 M: one channel 64x80x96 64.7 / 64.8, two of them 86.1 / 86.8, two of 111x128x120 262.6 / 258.8 (theta 10: 255 / 247),
+// 200x200x200 552 / 550, images 105.3
+// / 105.4 to 308 / 308; two channels 54.6 / 54.7, 87 / 87, 263 / 260 (253 / 247), 555 / 555.5, images 94.4 / 94.6 to 315.2 / 315.5.  Not with
+// three, 56 / 56.5, 88.6 /
+// 89.7, 268 / 269 (259 / 257), 568 / 577, images 96 / 97 to 324 / 326, nor at pd 3: 8 volumes of 64x64x64 without a guide 75 / 74, 83 / 84 and 83
+// / 83.
 // Where (us a splat, columns / sorted): rows of more than one float4 from 2 pd splats an entry on (8 x 512x512, pd 2,
 // 21 channels, 4.8 splats 95 / 110, 14.7 splats 76 / 98); narrow ones as NarrowColumns says.  pd 5, us a call: 8
 // splats an entry 201 / 197, 36 splats 158 / 138: up to pd 4.  Tiles of points in one dimension, which are all there are with pd 1, have no columns.
